@@ -233,8 +233,8 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
 int32_t wick_cuda_gemm_q8_tc(wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n,
                              float* out_dev, int32_t* block_sums_dev, void* stream);
 /* The bit-exact product on the tensor cores (the default GEMM of forward_prefill): same result as
- * wick_cuda_gemm_q8, bit for bit.  Needs k % 128 == 0.  Allocates a temporary for the masked
- * activations and synchronises `stream` (operator entry point for tests). */
+ * wick_cuda_gemm_q8, bit for bit.  Needs k % 128 == 0.  Synchronises `stream` (operator entry point for
+ * tests) and, like wick_cuda_gemm_q8_tc, makes the weight's int8 copy on its first call. */
 int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n,
                                    float* out_dev, void* stream);
 /* int32 block dot sums S[i][b] = sum over the 32 elements of block b of row i (the vdotq_s32

@@ -57,9 +57,14 @@ struct alignas(1024) TcStage {
     float sx[TC_KB_PER_STAGE][BN];            // activation scales, transposed to [block][token]
 };
 
+// Bytes of the constant operand of the exact GEMM's bias instruction: 128 rows x 32 bytes, all equal (64 x 64 x 32 = 2^17).
+constexpr int TC_BIAS_BYTES = TC_BM * QK;
+constexpr uint32_t TC_BIAS_WORD = 0x40404040u;
+
 template <int BN>
 struct TcSmem {
     TcStage<BN> stage[tc_stages<BN>()];
+    uint32_t bias[TC_BIAS_BYTES / 4];           // exact GEMM only
     unsigned long long full[tc_stages<BN>()];   // TMA bytes landed + scales written
     unsigned long long empty[tc_stages<BN>()];  // MMAs of the stage retired + epilogue done with its scales
     unsigned long long tmem_full[512 / BN];   // block sums of one k-block are in the buffer
@@ -131,12 +136,24 @@ __device__ __forceinline__ unsigned long long umma_desc_sw128(uint32_t smem_addr
     return d;
 }
 
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc) {
+// K-major operand tile of 32-byte rows without swizzle: 8 x 16-byte core matrices of 128 bytes, the two halves of a row one
+// core matrix apart, 8-row groups 256 bytes apart (only ever used on a tile whose bytes are all equal).
+__device__ __forceinline__ unsigned long long umma_desc_plain32(uint32_t smem_addr) {
+    unsigned long long d = 0;
+    d |= (unsigned long long)((smem_addr >> 4) & 0x3FFF);
+    d |= (unsigned long long)(128 >> 4) << 16;
+    d |= (unsigned long long)(256 >> 4) << 32;
+    d |= 1ull << 46;
+    return d;
+}
+
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc,
+                                        uint32_t accumulate = 0) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(0u), "r"(0u)
+        "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -241,10 +258,10 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     static_assert(TC_KB_PER_STAGE % UNIT == 0 && NBUF >= NB2, "two hand-over units that tile a stage");
     constexpr int TC_STAGES = tc_stages<BN>();
     constexpr int COLS = BN / TC_COL_GROUPS;  // columns per epilogue thread
-    // EXACT: a column is (token, NEON lane group); the activation rows arrive masked to one lane group
-    // each (tc_mask_expand), so a tile covers BN/4 tokens and the MMA yields the four lane partials
+    // EXACT: a column is (token, NEON lane group); each activation row of the operand is masked to one lane group (warp 3
+    // spreads the words), so a tile covers BN/4 tokens and the MMA yields the four lane partials.  Column order inside a
+    // pair of tokens is (lane group, token of the pair): the epilogue's packed arithmetic works on two tokens at a time.
     constexpr int TOK = EXACT ? BN / 4 : BN;  // tokens per tile
-    constexpr int XROWS = EXACT ? 4 : 1;      // rows of the activation operand per token
     static_assert(!EXACT || ((COLS == 16 || COLS == 8) && !SUMS), "exact epilogue: 4 (or 2) tokens x 4 lane groups per thread");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = k / QK;
@@ -254,7 +271,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < TC_STAGES; s++) {
-            mbar_init(smem_u32(&sm->full[s]), 1 + 32);            // producer (with tx bytes) + every lane of the scale warp
+            // producer (with tx bytes) + every lane of the scale warp + the exact GEMM's activation warp
+            mbar_init(smem_u32(&sm->full[s]), 1 + 32 + (EXACT ? 1 : 0));
             mbar_init(smem_u32(&sm->empty[s]), 1 + TC_EPI_WARPS);  // MMA commit + epilogue warps
         }
         for (int b = 0; b < NBUF; b++) {
@@ -263,6 +281,13 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         }
         sm->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if constexpr (EXACT) {
+        // the words that the lane-group masks zero are written once: every refill of a stage stores to the same other words
+        for (int s = 0; s < TC_STAGES; s++)
+            for (int i = threadIdx.x; i < BN * TC_KSTAGE / 16; i += TC_THREADS) reinterpret_cast<uint4*>(sm->stage[s].b)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = threadIdx.x; i < TC_BIAS_BYTES / 4; i += TC_THREADS) sm->bias[i] = TC_BIAS_WORD;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
@@ -289,9 +314,9 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     ok = mbar_wait<BN, 256>(sm, smem_u32(&sm->empty[s]), (u & 1) ^ 1, err, 1);
                     if (!ok) break;
                     const uint32_t bar = smem_u32(&sm->full[s]);
-                    mbar_arrive_expect_tx(bar, (TC_BM + BN) * TC_KSTAGE);
+                    mbar_arrive_expect_tx(bar, (EXACT ? TC_BM : TC_BM + BN) * TC_KSTAGE);
                     tma_load_2d(smem_u32(sm->stage[s].a), mw, bar, ks * TC_KSTAGE, tl.m0);
-                    tma_load_2d(smem_u32(sm->stage[s].b), &map_x, bar, ks * TC_KSTAGE, tl.n0 * XROWS);
+                    if constexpr (!EXACT) tma_load_2d(smem_u32(sm->stage[s].b), &map_x, bar, ks * TC_KSTAGE, tl.n0);
                 }
             }
         }
@@ -299,6 +324,10 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         // ── MMA issuer ───────────────────────────────────────────────────────
         if (lane == 0) {
             const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+            // EXACT: every block's tile starts from 2^17 (a constant x constant product of the same shape), so that the
+            // int32 results are positive: see the epilogue
+            const unsigned long long d_bias = EXACT ? umma_desc_plain32(smem_u32(sm->bias)) : 0ull;
+            (void)d_bias;
             uint32_t g = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -324,7 +353,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                             tc_fence_after();
                         }
                         // 32 bytes further along K inside the swizzle atom: +2 in the 16-byte address field
-                        umma_i8(tmem_base + buf * BN, da + (unsigned long long)(kk * 2), db + (unsigned long long)(kk * 2), idesc);
+                        if constexpr (EXACT) umma_i8(tmem_base + buf * BN, d_bias, d_bias, idesc);
+                        umma_i8(tmem_base + buf * BN, da + (unsigned long long)(kk * 2), db + (unsigned long long)(kk * 2), idesc, EXACT);
                         if (kk % UNIT == UNIT - 1) umma_commit(smem_u32(&sm->tmem_full[(j / UNIT) & 1u]));
                     }
                     if (ok) umma_commit(smem_u32(&sm->empty[s]));
@@ -369,6 +399,47 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&sm->full[s])) : "memory");
             }
         }
+    } else if (EXACT && warp == 3) {
+        // ── activation warp (exact GEMM) ─────────────────────────────────────
+        // Word l of a token's 16-byte half block belongs to lane group l (simd.rs:381-383: vdotq_s32 lane l), so it goes to
+        // row (pair of tokens, l, token of the pair) of the 128B-swizzled operand and the row's other words stay zero.  Done
+        // here the operand costs a quarter of the L2 reads of an expanded copy in memory, and no pass that writes one.
+        // A warp's 32 words of a token are 128 contiguous bytes of global memory and 32 different banks.
+        constexpr int LAG = 4;  // copies of so many stages are in flight before the oldest one is handed on
+        uint32_t g = 0, done = 0;
+        bool ok = true;
+        const int chunk = lane >> 2, l = lane & 3;
+        auto hand_on = [&]() {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sm->full[done % TC_STAGES]));
+            done++;
+        };
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
+            for (int ks = 0; ks < k_stages; ks++, g++) {
+                const int s = g % TC_STAGES;
+                ok = mbar_wait<BN, 256>(sm, smem_u32(&sm->empty[s]), ((g / TC_STAGES) & 1) ^ 1, err, 7);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const uint32_t b = smem_u32(sm->stage[s].b) + l * 4;
+                const int8_t* src = job.xq + ks * TC_KSTAGE + lane * 4;
+#pragma unroll
+                for (int j = 0; j < TOK; j++) {
+                    const int tok = min(tl.n0 + j, n - 1);  // rows past the last token repeat it; their outputs are not stored
+                    const int r7 = 2 * l + (j & 1);
+                    cp_async_4(b + (j >> 1) * 1024 + r7 * 128 + ((chunk ^ r7) << 4), src + (size_t)tok * k);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (g >= LAG) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
+                    hand_on();
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (ok)
+            while (done < g) hand_on();
     } else if (warp >= 4) {
         // ── epilogue ─────────────────────────────────────────────────────────
         const int quarter = warp & 3, cg = (warp - 4) >> 2;
@@ -446,21 +517,29 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             // The arithmetic of gemm_q*_q8_0_neon (simd.rs:696-1019) bit for bit: per output eight unfused
             // chains acc[parity of the block][lane group] += float(lane partial) * (f16(d_w) * d_x), blocks
             // in ascending order, combined at the end as ((a0+a1)+(a2+a3)) per parity, even + odd.
-            constexpr int TPT = COLS / 4;  // tokens per thread
-            // The products are formed one by one; the chain additions go out two lanes at a time (add.rn.f32x2).  A packed
-            // multiply feeding a packed add directly is turned into a fused multiply-add by the assembler, whatever the
-            // rounding modifiers say (wrong rounding for this contract); scalar products into a packed add are left alone.
-            f32x2 acc2[TPT][2][2];
+            //
+            // Bound: instruction issue and the FMA pipe.  Per (output, block) there are four lane partials p and, in the
+            // plain form, 4 int->float conversions + 4 products + 4 additions + the scale product.  Here it is 2 packed fused
+            // multiply-adds + 2 packed additions + 1/2 + 1/2 for the scales, two tokens per instruction:
+            //  - tensor memory holds v = p + 2^17 > 0 (the bias instruction).  Read as an f32, a positive integer below 2^23
+            //    is the denormal v * 2^-149, which the FMA pipe takes at full rate: no conversion.
+            //  - d = f16(d_w) * d_x is exact (two 11-bit significands), and so are D = d * 2^95 (f16 scales: |d| < 2^32) and
+            //    2^17 * D.  Hence fma(v * 2^-149, D, -2^-132 * D) rounds (v - 2^17) * d * 2^-54 once: it IS
+            //    RN(float(p) * d) * 2^-54, the reference's rounded product, and no contraction with the addition can occur.
+            //  - the chains run scaled by 2^-54.  Every f16-scaled term is a multiple of 2^-48, so nothing comes near the
+            //    denormal range (2^-102) and every rounding is the unscaled one; the final sum is multiplied back.
+            // 512 x 6144 x 2048: see launch_gemm_tc_exact.
+            constexpr int TP = COLS / 8;  // token pairs per thread
+            const f32x2 unbias = pack2(-__uint_as_float(1u << 17), -__uint_as_float(1u << 17));  // -2^-132
+            f32x2 acc2[TP][2][4];         // [pair][block parity][lane group], halves = the pair's tokens
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
                 const int m = job.m[tl.mat];
                 const int row = tl.m0 + row_in_tile;
 #pragma unroll
-                for (int i = 0; i < TPT; i++)
+                for (int i = 0; i < TP; i++)
 #pragma unroll
-                    for (int l = 0; l < 4; l++) {
-                        acc2[i][0][l >> 1] = acc2[i][1][l >> 1] = pack2(0.f, 0.f);
-                    }
+                    for (int l = 0; l < 4; l++) acc2[i][0][l] = acc2[i][1][l] = pack2(0.f, 0.f);
                 for (int ks = 0; ks < k_stages && ok; ks++, g++) {
                     const int s = g % TC_STAGES;
                     const uint32_t u = g / TC_STAGES;
@@ -477,22 +556,24 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                         // the load of block kk + 1 is in flight while the chains of block kk run
                         int32_t SA[COLS], SB[COLS];
                         auto chains = [&](const int32_t (&S)[COLS], const int kk) {
-                            const float sw = st.sw[kk][row_in_tile];
-                            float xs[TPT];
-                            if constexpr (TPT == 4) {
-                                const float4 x = *reinterpret_cast<const float4*>(&st.sx[kk][cg * TPT]);
-                                xs[0] = x.x, xs[1] = x.y, xs[2] = x.z, xs[3] = x.w;
-                            } else {
-                                const float2 x = *reinterpret_cast<const float2*>(&st.sx[kk][cg * TPT]);
+                            const float sw = st.sw[kk][row_in_tile] * 0x1p95f;
+                            const f32x2 sw2 = pack2(sw, sw);
+                            f32x2 xs[TP];
+                            if constexpr (TP == 2) {
+                                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&st.sx[kk][cg * 4]);
                                 xs[0] = x.x, xs[1] = x.y;
+                            } else {
+                                xs[0] = *reinterpret_cast<const unsigned long long*>(&st.sx[kk][cg * 2]);
                             }
 #pragma unroll
-                            for (int i = 0; i < TPT; i++) {
-                                const float d = __fmul_rn(sw, xs[i]);
+                            for (int i = 0; i < TP; i++) {
+                                const f32x2 d = mul2(sw2, xs[i]);
+                                const f32x2 c = mul2(d, unbias);
 #pragma unroll
-                                for (int l = 0; l < 4; l += 2)
-                                    acc2[i][kk & 1][l >> 1] = add2(acc2[i][kk & 1][l >> 1], pack2(__fmul_rn(__int2float_rn(S[i * 4 + l]), d),
-                                                                                                 __fmul_rn(__int2float_rn(S[i * 4 + l + 1]), d)));
+                                for (int l = 0; l < 4; l++) {
+                                    const f32x2 v = pack2(__int_as_float(S[i * 8 + 2 * l]), __int_as_float(S[i * 8 + 2 * l + 1]));
+                                    acc2[i][kk & 1][l] = add2(acc2[i][kk & 1][l], fma2(v, d, c));
+                                }
                             }
                         };
                         const uint32_t t0 = lane_base + (unit * TC_KB_PER_STAGE) * BN;
@@ -518,18 +599,14 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                 if (ok && row < m) {
                     float* out = job.out[tl.mat];
 #pragma unroll
-                    for (int i = 0; i < TPT; i++) {
-                        const int tok = tl.n0 + cg * TPT + i;
-                        float acc[1][2][4];
-                        unpack2(acc2[i][0][0], acc[0][0][0], acc[0][0][1]);
-                        unpack2(acc2[i][0][1], acc[0][0][2], acc[0][0][3]);
-                        unpack2(acc2[i][1][0], acc[0][1][0], acc[0][1][1]);
-                        unpack2(acc2[i][1][1], acc[0][1][2], acc[0][1][3]);
-#define WICK_ACC(p, l) acc[0][p][l]
-                        const float e = __fadd_rn(__fadd_rn(WICK_ACC(0, 0), WICK_ACC(0, 1)), __fadd_rn(WICK_ACC(0, 2), WICK_ACC(0, 3)));
-                        const float o = __fadd_rn(__fadd_rn(WICK_ACC(1, 0), WICK_ACC(1, 1)), __fadd_rn(WICK_ACC(1, 2), WICK_ACC(1, 3)));
-#undef WICK_ACC
-                        if (tok < n) out[(size_t)tok * m + row] = __fadd_rn(e, o);
+                    for (int i = 0; i < TP; i++) {
+                        const int tok = tl.n0 + cg * 2 * TP + 2 * i;
+                        const f32x2 e = add2(add2(acc2[i][0][0], acc2[i][0][1]), add2(acc2[i][0][2], acc2[i][0][3]));
+                        const f32x2 o = add2(add2(acc2[i][1][0], acc2[i][1][1]), add2(acc2[i][1][2], acc2[i][1][3]));
+                        float r0, r1;
+                        unpack2(add2(e, o), r0, r1);
+                        if (tok < n) out[(size_t)tok * m + row] = r0 * 0x1p54f;
+                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = r1 * 0x1p54f;
                     }
                 }
             }
@@ -649,20 +726,6 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     return cudaGetLastError();
 }
 
-// One thread per 16 input bytes (half a quantisation block): NEON lane group l owns bytes 4l..4l+3
-// of each half (simd.rs:381-383: vdotq_s32 lane l), so output row 4*j + l keeps word l and zeroes the rest.
-__global__ void k_tc_mask_expand(const uint4* __restrict__ xq, uint4* __restrict__ xm, size_t n_chunks, int chunks_per_row) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_chunks) return;
-    const uint4 v = xq[i];
-    const size_t row = i / chunks_per_row, c = i % chunks_per_row;
-    uint4* o = xm + (row * 4) * chunks_per_row + c;
-    o[0] = make_uint4(v.x, 0u, 0u, 0u);
-    o[(size_t)chunks_per_row] = make_uint4(0u, v.y, 0u, 0u);
-    o[(size_t)2 * chunks_per_row] = make_uint4(0u, 0u, v.z, 0u);
-    o[(size_t)3 * chunks_per_row] = make_uint4(0u, 0u, 0u, v.w);
-}
-
 cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, int count, int tiles_n) {
     memset(&job, 0, sizeof(job));
     job.count = count;
@@ -728,16 +791,8 @@ cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* con
                     : launch_tc<128, false>(st, job, map_x[1], x_scales, n, w[0]->k, sums, err);
 }
 
-void launch_tc_mask_expand(cudaStream_t st, const int8_t* xq, int n, int k, int8_t* xm) {
-    const size_t chunks = (size_t)n * (k / 16);
-    if (!chunks) return;
-    g_kernel_launches++;
-    k_tc_mask_expand<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(xq), reinterpret_cast<uint4*>(xm),
-                                                                         chunks, k / 16);
-}
-
-cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap& map_xm,
-                                 const float* x_scales, int n, uint32_t* err, const CUtensorMap* map_xm_narrow) {
+cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,
+                                 const float* x_scales, int n, uint32_t* err) {
     if (n <= 0 || count <= 0) return cudaSuccess;
     if (count > 3) return cudaErrorInvalidValue;
     TcJob job;
@@ -745,14 +800,13 @@ cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, floa
     // decode step): a tile's time is set by its K loop, so more, smaller tiles only pay when they run side by side
     int row_tiles = 0;
     for (int i = 0; i < count; i++) row_tiles += w[i]->m_pad / TC_BM;
-    if (map_xm_narrow && 2 * row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) <= 148) {
-        cudaError_t e = fill_job(job, w, out, count, (n + TC_EXACT_TOKENS / 2 - 1) / (TC_EXACT_TOKENS / 2));
-        if (e != cudaSuccess) return e;
-        return launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, *map_xm_narrow, x_scales, n, w[0]->k, nullptr, err);
-    }
-    cudaError_t e = fill_job(job, w, out, count, (n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS);
+    const bool narrow = 2 * row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) <= 148;
+    const int tok = narrow ? TC_EXACT_TOKENS / 2 : TC_EXACT_TOKENS;
+    cudaError_t e = fill_job(job, w, out, count, (n + tok - 1) / tok);
     if (e != cudaSuccess) return e;
-    return launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, map_xm, x_scales, n, w[0]->k, nullptr, err);
+    job.xq = xq;
+    return narrow ? launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, CUtensorMap{}, x_scales, n, w[0]->k, nullptr, err)
+                  : launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, CUtensorMap{}, x_scales, n, w[0]->k, nullptr, err);
 }
 
 }  // namespace wick

@@ -24,6 +24,7 @@ struct TcJob {
     CUtensorMap map_w[3];
     const float* scales_t[3];
     float* out[3];        // [n][m[i]] each
+    const int8_t* xq;     // exact GEMM: the quantised activations [n][k] (the other one reads them through a tensor map)
     int m[3], m_pad[3];
     int tile_start[4];    // first linear tile of each matrix; [count..3] = total
     int count;
@@ -49,15 +50,12 @@ cudaError_t tc_make_activation_map(const int8_t* xq, int rows_cap, int k, int bn
 cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap* map_x,
                            const float* x_scales, int n, int32_t* sums, uint32_t* err);
 
-// The bit-exact variant (the arithmetic of gemm_q*_q8_0_neon, simd.rs:696-1019, in its order): the
-// activation operand is the masked expansion xm [4 * n][k] of xq (row 4*j + l = token j with every
-// byte outside NEON lane group l zeroed), so that one MMA yields the four lane partials of a block
-// as four columns; the epilogue keeps the reference's eight unfused chains per output.
+// The bit-exact variant (the arithmetic of gemm_q*_q8_0_neon, simd.rs:696-1019, in its order): every token's activations
+// become four rows of the operand, one per NEON lane group with the other groups' bytes zero, so that one MMA yields the
+// four lane partials of a block as four columns; the epilogue keeps the reference's eight unfused chains per output.
+// xq: int8 [n][k], 4-byte aligned.
 constexpr int TC_EXACT_TOKENS = 16;  // tokens per tile (64 MMA columns)
-void launch_tc_mask_expand(cudaStream_t st, const int8_t* xq, int n, int k, int8_t* xm);
-// map_xm: tc_make_activation_map(xm, 4 * rows_cap, k, 64, ..); map_xm_narrow (optional): the same with 32 rows per box,
-// for the 8-token tiles small batches run with.
-cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap& map_xm,
-                                 const float* x_scales, int n, uint32_t* err, const CUtensorMap* map_xm_narrow = nullptr);
+cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,
+                                 const float* x_scales, int n, uint32_t* err);
 
 }  // namespace wick
