@@ -49,6 +49,9 @@ constexpr int TC_EPI_WARPS = 4 * TC_COL_GROUPS;
 constexpr int TC_THREADS = 32 * (4 + TC_EPI_WARPS);
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
 
+// Weight scales are stored times 2^72 (exact): what the exact epilogue needs, see there.
+constexpr float TC_SCALE_UP = 0x1p72f, TC_SCALE_DOWN = 0x1p-72f, TC_EXACT_DOWN = 0x1p77f;
+
 template <int BN>
 struct alignas(1024) TcStage {
     int8_t a[TC_BM * TC_KSTAGE];              // 16 KB, rows of 128 B, 128B-swizzled by TMA
@@ -155,6 +158,11 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, unsigned long long da, 
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(tmem_d),
         "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p;
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -273,7 +281,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         for (int s = 0; s < TC_STAGES; s++) {
             // producer (with tx bytes) + every lane of the scale warp + the exact GEMM's activation warp
             mbar_init(smem_u32(&sm->full[s]), 1 + 32 + (EXACT ? 1 : 0));
-            mbar_init(smem_u32(&sm->empty[s]), 1 + TC_EPI_WARPS);  // MMA commit + epilogue warps
+            // MMA commit + epilogue warps; exact GEMM: the MMA issuer alone, two stages later (see there)
+            mbar_init(smem_u32(&sm->empty[s]), EXACT ? 1 : 1 + TC_EPI_WARPS);
         }
         for (int b = 0; b < NBUF; b++) {
             mbar_init(smem_u32(&sm->tmem_full[b]), 1);
@@ -322,42 +331,53 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         }
     } else if (warp == 1) {
         // ── MMA issuer ───────────────────────────────────────────────────────
-        if (lane == 0) {
-            const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-            // EXACT: every block's tile starts from 2^17 (a constant x constant product of the same shape), so that the
-            // int32 results are positive: see the epilogue
-            const unsigned long long d_bias = EXACT ? umma_desc_plain32(smem_u32(sm->bias)) : 0ull;
-            (void)d_bias;
-            uint32_t g = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                for (int ks = 0; ks < k_stages && ok; ks++, g++) {
-                    const int s = g % TC_STAGES;
-                    const uint32_t u = g / TC_STAGES;
-                    ok = mbar_wait<BN, 128>(sm, smem_u32(&sm->full[s]), u & 1, err, 2);
+        // The whole warp runs the loop and one elected lane issues: descriptors and barrier addresses then stay in uniform
+        // registers.  (With a single-lane loop the eight instructions of an exact stage took about 1000 of its 1800 cycles
+        // to issue, every descriptor going through general registers first, and this warp set the pace of the kernel.)
+        const uint32_t leader = elect_one();
+        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+        // EXACT: every block's tile starts from 2^17 (a constant x constant product of the same shape), so that the
+        // int32 results are positive: see the epilogue
+        const unsigned long long d_bias = EXACT ? umma_desc_plain32(smem_u32(sm->bias)) : 0ull;
+        (void)d_bias;
+        uint32_t g = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            for (int ks = 0; ks < k_stages && ok; ks++, g++) {
+                const int s = g % TC_STAGES;
+                const uint32_t u = g / TC_STAGES;
+                ok = mbar_wait<BN, 128>(sm, smem_u32(&sm->full[s]), u & 1, err, 2);
+                if (!ok) break;
+                tc_fence_after();
+                const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
+                const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
+#pragma unroll
+                for (int h = 0; h < TC_KB_PER_STAGE / UNIT; h++) {
+                    // Buffers are handed over half of tensor memory (UNIT blocks) at a time: every hand-over
+                    // costs each epilogue warp a barrier wait and an arrival, both long dependent steps of its
+                    // loop, and that loop - not the tensor pipe - sets the pace of the kernel
+                    const uint32_t un = g * (TC_KB_PER_STAGE / UNIT) + h;
+                    ok = mbar_wait<BN, 64>(sm, smem_u32(&sm->tmem_empty[un & 1u]), ((un >> 1) & 1) ^ 1, err, 3);
                     if (!ok) break;
                     tc_fence_after();
-                    const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
-                    const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
+                    const uint32_t d0 = tmem_base + (un & 1u) * (UNIT * BN);
+                    if (leader) {
+                        // EXACT: that wait also says that the epilogue is done with the scales of the stage before the last
+                        if (EXACT && g >= 2) mbar_arrive(smem_u32(&sm->empty[(g - 2) % TC_STAGES]));
 #pragma unroll
-                    for (int kk = 0; kk < TC_KB_PER_STAGE; kk++) {
-                        const uint32_t j = g * TC_KB_PER_STAGE + kk;
-                        const uint32_t buf = j % NB2;
-                        if (kk % UNIT == 0) {
-                            // Buffers are handed over half of tensor memory (UNIT blocks) at a time: every hand-over
-                            // costs each epilogue warp a barrier wait and an arrival, both long dependent steps of its
-                            // loop, and that loop - not the tensor pipe - sets the pace of the kernel
-                            const uint32_t un = j / UNIT;
-                            ok = mbar_wait<BN, 64>(sm, smem_u32(&sm->tmem_empty[un & 1u]), ((un >> 1) & 1) ^ 1, err, 3);
-                            if (!ok) break;
-                            tc_fence_after();
+                        for (int kk = 0; kk < UNIT; kk++) {
+                            // 32 bytes further along K inside the swizzle atom: +2 in the 16-byte address field
+                            const unsigned long long off = (unsigned long long)((h * UNIT + kk) * 2);
+                            if constexpr (EXACT) umma_i8(d0 + kk * BN, d_bias, d_bias, idesc);
+                            umma_i8(d0 + kk * BN, da + off, db + off, idesc, EXACT);
                         }
-                        // 32 bytes further along K inside the swizzle atom: +2 in the 16-byte address field
-                        if constexpr (EXACT) umma_i8(tmem_base + buf * BN, d_bias, d_bias, idesc);
-                        umma_i8(tmem_base + buf * BN, da + (unsigned long long)(kk * 2), db + (unsigned long long)(kk * 2), idesc, EXACT);
-                        if (kk % UNIT == UNIT - 1) umma_commit(smem_u32(&sm->tmem_full[(j / UNIT) & 1u]));
+                        umma_commit(smem_u32(&sm->tmem_full[un & 1u]));
                     }
-                    if (ok) umma_commit(smem_u32(&sm->empty[s]));
+                    __syncwarp();
+                }
+                if constexpr (!EXACT) {
+                    if (ok && leader) umma_commit(smem_u32(&sm->empty[s]));
+                    __syncwarp();
                 }
             }
         }
@@ -405,10 +425,11 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         // row (pair of tokens, l, token of the pair) of the 128B-swizzled operand and the row's other words stay zero.  Done
         // here the operand costs a quarter of the L2 reads of an expanded copy in memory, and no pass that writes one.
         // A warp's 32 words of a token are 128 contiguous bytes of global memory and 32 different banks.
-        constexpr int LAG = 4;  // copies of so many stages are in flight before the oldest one is handed on
+        constexpr int LAG = 3;  // copies of so many stages are in flight before the oldest one is handed on
         uint32_t g = 0, done = 0;
         bool ok = true;
         const int chunk = lane >> 2, l = lane & 3;
+        const uint32_t dst0 = l * 4 + (2 * l) * 128 + ((chunk ^ (2 * l)) << 4), dst1 = l * 4 + (2 * l + 1) * 128 + ((chunk ^ (2 * l + 1)) << 4);
         auto hand_on = [&]() {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -417,18 +438,22 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         };
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
             const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
+            const int8_t* src[TOK];
+#pragma unroll
+            for (int j = 0; j < TOK; j++)  // rows past the last token repeat it; their outputs are not stored
+                src[j] = job.xq + (size_t)min(tl.n0 + j, n - 1) * k + lane * 4;
             for (int ks = 0; ks < k_stages; ks++, g++) {
                 const int s = g % TC_STAGES;
                 ok = mbar_wait<BN, 256>(sm, smem_u32(&sm->empty[s]), ((g / TC_STAGES) & 1) ^ 1, err, 7);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const uint32_t b = smem_u32(sm->stage[s].b) + l * 4;
-                const int8_t* src = job.xq + ks * TC_KSTAGE + lane * 4;
+                // row 8 * (j / 2) + 2 * l + (j & 1); its place among the eight rows of a swizzle atom is 2 * l + (j & 1)
+                const uint32_t b = smem_u32(sm->stage[s].b);
+                const uint32_t b0 = b + dst0, b1 = b + dst1;
 #pragma unroll
                 for (int j = 0; j < TOK; j++) {
-                    const int tok = min(tl.n0 + j, n - 1);  // rows past the last token repeat it; their outputs are not stored
-                    const int r7 = 2 * l + (j & 1);
-                    cp_async_4(b + (j >> 1) * 1024 + r7 * 128 + ((chunk ^ r7) << 4), src + (size_t)tok * k);
+                    cp_async_4(((j & 1) ? b1 : b0) + (j >> 1) * 1024, src[j]);
+                    src[j] += TC_KSTAGE;
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
                 if (g >= LAG) {
@@ -508,8 +533,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                         const int tok = tl.n0 + cg * COLS + c;
                         float a0, a1;
                         unpack2(acc[c / 2], a0, a1);
-                        if (tok < n) out[(size_t)tok * m + row] = a0;
-                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = a1;
+                        if (tok < n) out[(size_t)tok * m + row] = a0 * TC_SCALE_DOWN;
+                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = a1 * TC_SCALE_DOWN;
                     }
                 }
             }
@@ -523,11 +548,11 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             // multiply-adds + 2 packed additions + 1/2 + 1/2 for the scales, two tokens per instruction:
             //  - tensor memory holds v = p + 2^17 > 0 (the bias instruction).  Read as an f32, a positive integer below 2^23
             //    is the denormal v * 2^-149, which the FMA pipe takes at full rate: no conversion.
-            //  - d = f16(d_w) * d_x is exact (two 11-bit significands), and so are D = d * 2^95 (f16 scales: |d| < 2^32) and
-            //    2^17 * D.  Hence fma(v * 2^-149, D, -2^-132 * D) rounds (v - 2^17) * d * 2^-54 once: it IS
-            //    RN(float(p) * d) * 2^-54, the reference's rounded product, and no contraction with the addition can occur.
-            //  - the chains run scaled by 2^-54.  Every f16-scaled term is a multiple of 2^-48, so nothing comes near the
-            //    denormal range (2^-102) and every rounding is the unscaled one; the final sum is multiplied back.
+            //  - d = f16(d_w) * d_x rounds the same when the weight scale is stored times 2^72 (D = d * 2^72), and 2^17 * D is
+            //    exact.  Hence fma(v * 2^-149, D, -2^-132 * D) rounds (v - 2^17) * d * 2^-77 once: it IS
+            //    RN(float(p) * d) * 2^-77, the reference's rounded product, and no contraction with the addition can occur.
+            //  - the chains run scaled by 2^-77.  Scales are f16 values, so every term is a multiple of 2^-48: nothing falls
+            //    into the denormal range (2^-125) and every rounding is the unscaled one; the final sum is multiplied back.
             // 512 x 6144 x 2048: see launch_gemm_tc_exact.
             constexpr int TP = COLS / 8;  // token pairs per thread
             const f32x2 unbias = pack2(-__uint_as_float(1u << 17), -__uint_as_float(1u << 17));  // -2^-132
@@ -541,60 +566,65 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
 #pragma unroll
                     for (int l = 0; l < 4; l++) acc2[i][0][l] = acc2[i][1][l] = pack2(0.f, 0.f);
                 for (int ks = 0; ks < k_stages && ok; ks++, g++) {
-                    const int s = g % TC_STAGES;
-                    const uint32_t u = g / TC_STAGES;
-                    // (every lane of a warp runs the same wait on the same barrier and gets the same answer)
-                    ok = mbar_wait(sm, smem_u32(&sm->full[s]), u & 1, err, 5);  // the stage's scales
-                    if (!ok) break;
                     static_assert(UNIT == TC_KB_PER_STAGE, "the exact epilogue takes a whole stage per hand-over");
-                    const uint32_t unit = g & 1u;                                // the half of tensor memory with its 4 blocks
+                    const uint32_t unit = g & 1u;  // the half of tensor memory with the stage's 4 blocks
+                    // One wait and one arrival per stage.  The wait covers the stage's scales too: the MMA issuer had seen
+                    // their barrier (full[s]) before it issued what this one reports.  The arrival stands for both the tensor
+                    // memory and the scales, all of which are in registers by then.
+                    // (every lane of a warp runs the same wait on the same barrier and gets the same answer)
                     ok = mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g >> 1) & 1, err, 6);
                     if (!ok) break;
                     tc_fence_after();
-                    const TcStage<BN>& st = sm->stage[s];
-                    {
-                        // the load of block kk + 1 is in flight while the chains of block kk run
-                        int32_t SA[COLS], SB[COLS];
-                        auto chains = [&](const int32_t (&S)[COLS], const int kk) {
-                            const float sw = st.sw[kk][row_in_tile] * 0x1p95f;
-                            const f32x2 sw2 = pack2(sw, sw);
-                            f32x2 xs[TP];
-                            if constexpr (TP == 2) {
-                                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&st.sx[kk][cg * 4]);
-                                xs[0] = x.x, xs[1] = x.y;
-                            } else {
-                                xs[0] = *reinterpret_cast<const unsigned long long*>(&st.sx[kk][cg * 2]);
-                            }
+                    const TcStage<BN>& st = sm->stage[g % TC_STAGES];
+                    // the load of block kk + 1 is in flight while the chains of block kk run
+                    int32_t SA[COLS], SB[COLS];
+                    struct Scales {
+                        float w;
+                        f32x2 x[TP];
+                    };
+                    auto scales = [&](const int kk) {
+                        Scales c;
+                        c.w = st.sw[kk][row_in_tile];
+                        if constexpr (TP == 2) {
+                            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&st.sx[kk][cg * 4]);
+                            c.x[0] = x.x, c.x[1] = x.y;
+                        } else {
+                            c.x[0] = *reinterpret_cast<const unsigned long long*>(&st.sx[kk][cg * 2]);
+                        }
+                        return c;
+                    };
+                    auto chains = [&](const int32_t (&S)[COLS], const int p, const Scales& sc) {
+                        const f32x2 sw2 = pack2(sc.w, sc.w);
 #pragma unroll
-                            for (int i = 0; i < TP; i++) {
-                                const f32x2 d = mul2(sw2, xs[i]);
-                                const f32x2 c = mul2(d, unbias);
+                        for (int i = 0; i < TP; i++) {
+                            const f32x2 d = mul2(sw2, sc.x[i]);
+                            const f32x2 c = mul2(d, unbias);
 #pragma unroll
-                                for (int l = 0; l < 4; l++) {
-                                    const f32x2 v = pack2(__int_as_float(S[i * 8 + 2 * l]), __int_as_float(S[i * 8 + 2 * l + 1]));
-                                    acc2[i][kk & 1][l] = add2(acc2[i][kk & 1][l], fma2(v, d, c));
-                                }
+                            for (int l = 0; l < 4; l++) {
+                                const f32x2 v = pack2(__int_as_float(S[i * 8 + 2 * l]), __int_as_float(S[i * 8 + 2 * l + 1]));
+                                acc2[i][p][l] = add2(acc2[i][p][l], fma2(v, d, c));
                             }
-                        };
-                        const uint32_t t0 = lane_base + (unit * TC_KB_PER_STAGE) * BN;
-                        tmem_ld<COLS>(t0, SA);
-                        tmem_ld_wait();
-                        tmem_ld<COLS>(t0 + BN, SB);
-                        chains(SA, 0);
-                        tmem_ld_wait();
-                        tmem_ld<COLS>(t0 + 2 * BN, SA);
-                        chains(SB, 1);
-                        tmem_ld_wait();
-                        tmem_ld<COLS>(t0 + 3 * BN, SB);
-                        chains(SA, 2);
-                        tmem_ld_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&sm->tmem_empty[unit]));
-                        chains(SB, 3);
-                    }
+                        }
+                    };
+                    const uint32_t t0 = lane_base + unit * (TC_KB_PER_STAGE * BN);
+                    tmem_ld<COLS>(t0, SA);
+                    const Scales c0 = scales(0), c1 = scales(1);
+                    tmem_ld_wait();
+                    tmem_ld<COLS>(t0 + BN, SB);
+                    chains(SA, 0, c0);
+                    const Scales c2 = scales(2);
+                    tmem_ld_wait();
+                    tmem_ld<COLS>(t0 + 2 * BN, SA);
+                    chains(SB, 1, c1);
+                    const Scales c3 = scales(3);
+                    tmem_ld_wait();
+                    tmem_ld<COLS>(t0 + 3 * BN, SB);
+                    chains(SA, 0, c2);
+                    tmem_ld_wait();
+                    tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&sm->empty[s]));
+                    if (lane == 0) mbar_arrive(smem_u32(&sm->tmem_empty[unit]));
+                    chains(SB, 1, c3);
                 }
                 if (ok && row < m) {
                     float* out = job.out[tl.mat];
@@ -605,8 +635,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                         const f32x2 o = add2(add2(acc2[i][1][0], acc2[i][1][1]), add2(acc2[i][1][2], acc2[i][1][3]));
                         float r0, r1;
                         unpack2(add2(e, o), r0, r1);
-                        if (tok < n) out[(size_t)tok * m + row] = r0 * 0x1p54f;
-                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = r1 * 0x1p54f;
+                        if (tok < n) out[(size_t)tok * m + row] = r0 * TC_EXACT_DOWN;
+                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = r1 * TC_EXACT_DOWN;
                     }
                 }
             }
@@ -639,7 +669,7 @@ __global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restri
     const int g = row >> 2, r = row & 3;
     const __half* dg = w.d + (size_t)g * nb * 4;
     const uint32_t* qg = reinterpret_cast<const uint32_t*>(w.q + (size_t)g * w.q_group_bytes());
-    scales_t[(size_t)b * m_pad + row] = __half2float(dg[b * 4 + r]);
+    scales_t[(size_t)b * m_pad + row] = __half2float(dg[b * 4 + r]) * TC_SCALE_UP;
     uint32_t o[8];
     if (w.dtype == DT_Q4_0) {
 #pragma unroll

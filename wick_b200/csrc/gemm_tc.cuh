@@ -11,7 +11,7 @@ namespace wick {
 // layout, plus its scales as f32, block-major so that one k-block's 128 row scales are contiguous.
 struct TcWeight {
     int8_t* q = nullptr;      // [m_pad][k]
-    float* scales_t = nullptr;  // [k/32][m_pad]
+    float* scales_t = nullptr;  // [k/32][m_pad], times 2^72
     int m = 0, k = 0, m_pad = 0;
     CUtensorMap map;          // rows of this matrix, box 128 bytes x 128 rows, 128B swizzle
     size_t q_bytes() const { return (size_t)m_pad * k; }
