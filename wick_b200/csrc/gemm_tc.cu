@@ -44,9 +44,9 @@ constexpr int TC_KB_PER_STAGE = TC_KSTAGE / QK;  // 4 quantisation blocks per st
 // the MMA issuer needs it; with four stages that left about one microsecond, less than a loaded L2 round trip.
 template <int BN>
 __host__ __device__ constexpr int tc_stages() { return BN <= 64 ? 8 : 6; }
-constexpr int TC_COL_GROUPS = 4;    // epilogue warps per TMEM lane quarter; each takes BN/4 columns
-constexpr int TC_EPI_WARPS = 4 * TC_COL_GROUPS;
-constexpr int TC_THREADS = 32 * (4 + TC_EPI_WARPS);
+// Epilogue warps per TMEM lane quarter; each takes 1 / groups of a tile's columns
+__host__ __device__ constexpr int tc_col_groups(bool exact) { return exact ? 2 : 4; }
+__host__ __device__ constexpr int tc_threads(bool exact) { return 32 * (4 + 4 * tc_col_groups(exact)); }
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
 
 // Weight scales are stored times 2^72 (exact): what the exact epilogue needs, see there.
@@ -253,7 +253,7 @@ __device__ __forceinline__ TcTile tc_decode_tile(const TcJob& job, int t, int ti
 }
 
 template <int BN, bool SUMS, bool EXACT>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(tc_threads(EXACT), 1)
 k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap map_x,
           const float* __restrict__ x_scales,  // [n][k/32]
           int32_t* __restrict__ sums,          // optional [n][m][k/32] (single-matrix jobs only)
@@ -265,12 +265,13 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     constexpr int NB2 = 2 * UNIT;  // buffers in use (32-column tiles leave half of tensor memory unused)
     static_assert(TC_KB_PER_STAGE % UNIT == 0 && NBUF >= NB2, "two hand-over units that tile a stage");
     constexpr int TC_STAGES = tc_stages<BN>();
+    constexpr int TC_COL_GROUPS = tc_col_groups(EXACT), TC_EPI_WARPS = 4 * TC_COL_GROUPS, TC_THREADS = tc_threads(EXACT);
     constexpr int COLS = BN / TC_COL_GROUPS;  // columns per epilogue thread
     // EXACT: a column is (token, NEON lane group); each activation row of the operand is masked to one lane group (warp 3
     // spreads the words), so a tile covers BN/4 tokens and the MMA yields the four lane partials.  Column order inside a
     // pair of tokens is (lane group, token of the pair): the epilogue's packed arithmetic works on two tokens at a time.
     constexpr int TOK = EXACT ? BN / 4 : BN;  // tokens per tile
-    static_assert(!EXACT || ((COLS == 16 || COLS == 8) && !SUMS), "exact epilogue: 4 (or 2) tokens x 4 lane groups per thread");
+    static_assert(!EXACT || ((COLS == 32 || COLS == 16 || COLS == 8) && !SUMS), "exact epilogue: 8, 4 or 2 tokens x 4 lane groups per thread");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = k / QK;
     const int k_stages = k / TC_KSTAGE;
@@ -585,9 +586,12 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     auto scales = [&](const int kk) {
                         Scales c;
                         c.w = st.sw[kk][row_in_tile];
-                        if constexpr (TP == 2) {
-                            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&st.sx[kk][cg * 4]);
-                            c.x[0] = x.x, c.x[1] = x.y;
+                        if constexpr (TP >= 2) {
+#pragma unroll
+                            for (int i = 0; i < TP; i += 2) {
+                                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&st.sx[kk][(cg * TP + i) * 2]);
+                                c.x[i] = x.x, c.x[i + 1] = x.y;
+                            }
                         } else {
                             c.x[0] = *reinterpret_cast<const unsigned long long*>(&st.sx[kk][cg * 2]);
                         }
@@ -748,11 +752,11 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     g_kernel_launches++;
     if constexpr (!EXACT) {
         if (sums) {
-            k_gemm_tc<BN, true, false><<<grid, TC_THREADS, smem, st>>>(job, map_x, x_scales, sums, n, k, err);
+            k_gemm_tc<BN, true, false><<<grid, tc_threads(false), smem, st>>>(job, map_x, x_scales, sums, n, k, err);
             return cudaGetLastError();
         }
     }
-    k_gemm_tc<BN, false, EXACT><<<grid, TC_THREADS, smem, st>>>(job, map_x, x_scales, nullptr, n, k, err);
+    k_gemm_tc<BN, false, EXACT><<<grid, tc_threads(EXACT), smem, st>>>(job, map_x, x_scales, nullptr, n, k, err);
     return cudaGetLastError();
 }
 
