@@ -8,8 +8,8 @@
 // S_b is the same integer the NEON kernels produce per block (simd.rs:696-1019, the four lane
 // partials added up); what differs from them is the f32 accumulation: one fused chain per output in
 // block order instead of 2 x 4 unfused lane chains, so outputs agree to f32 rounding (~1e-6 relative),
-// not bit for bit.  The bit-exact order lives in k_gemm (kernels_gemv.cu); this kernel is the
-// throughput path of forward_prefill.
+// not bit for bit.  The EXACT instantiation (the default of forward_prefill) keeps the four lane partials apart as columns
+// and their eight chains in the epilogue, bit for bit; this one is the throughput option.
 //
 // One MMA instruction covers exactly one quantisation block (K = 32 int8), writes a fresh 128 x BN
 // int32 tile into one of 512/BN tensor-memory buffers and never accumulates across blocks, because
@@ -17,12 +17,12 @@
 // and apply the scales on the CUDA cores: 3 instructions per (output, block), which is what bounds the
 // kernel (the tensor pipe needs about 1/6 of that time).
 //
-// Roles in a CTA of 20 warps (one CTA per SM, persistent over output tiles):
-//   warp 0  lane 0: TMA producer, one K=128 stage (4 blocks) of W rows and activation rows per step
-//   warp 1  lane 0: issues tcgen05.mma / tcgen05.commit; the whole warp owns the TMEM allocation
+// Roles in a CTA (one CTA per SM, persistent over output tiles; 12 warps for EXACT, else 20):
+//   warp 0  lane 0: TMA producer, one K=128 stage (4 blocks) of W rows (and, not for EXACT, activation rows) per step
+//   warp 1        : issues tcgen05.mma / tcgen05.commit from one elected lane and owns the TMEM allocation
 //   warp 2        : copies the stage's weight scales and (transposed) activation scales into smem (cp.async)
-//   warps 4..19   : epilogue; warp w reads TMEM lanes 32*(w%4).. and columns (w-4)/4 * BN/4 ..; four
-//                   warps per scheduler hide the tensor-memory load and barrier latencies
+//   warp 3        : EXACT: spreads the activation words over the lane-group rows of the operand (cp.async)
+//   warps 4..     : epilogue; warp w reads TMEM lanes 32*(w%4).. and its group's share of the columns
 // Every wait is bounded: on expiry the kernel records an error code, all roles leave their loops and
 // the CTA frees its tensor memory and exits.
 #include <cuda.h>
@@ -99,6 +99,18 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
     return ok;
 }
 
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {  // asks once, never suspends
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait.  Returns false once the limit is hit or another role has already given up.
 // SLEEP_NS > 0 is for the producer, MMA and scale-loader roles: they run stages ahead of the epilogue, and a
 // tight poll loop in those warps would take issue slots from the epilogue warps that bound the kernel.
@@ -150,14 +162,28 @@ __device__ __forceinline__ unsigned long long umma_desc_plain32(uint32_t smem_ad
     return d;
 }
 
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc,
-                                        uint32_t accumulate = 0) {
+template <bool ACC>
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(da), "l"(db), "r"(idesc), "n"(ACC ? 1 : 0)
         : "memory");
+}
+// The constant product: several in a row read the same A operand, which stays in the collector (N = 32: 20 cycles instead
+// of 40, the A operand being read at 64 bytes a cycle).  WHICH: 0 first, 1 between, 2 last.
+template <int WHICH>
+__device__ __forceinline__ void umma_i8_same_a(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc) {
+#define WICK_UMMA_COLLECT(how)                                                                                      \
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"                                                   \
+                 "tcgen05.mma.cta_group::1.kind::i8.collector::a::" how " [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), \
+                 "l"(da), "l"(db), "r"(idesc)                                                                       \
+                 : "memory")
+    if constexpr (WHICH == 0) WICK_UMMA_COLLECT("fill");
+    else if constexpr (WHICH == 1) WICK_UMMA_COLLECT("use");
+    else WICK_UMMA_COLLECT("lastuse");
+#undef WICK_UMMA_COLLECT
 }
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t p;
@@ -230,6 +256,20 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
+}
+// Shared-memory loads by 32-bit address (a pointer derived from the aligned raw buffer is a generic one to the compiler)
+__device__ __forceinline__ float lds_f32(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ f32x2 lds_64(uint32_t a) {
+    f32x2 v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void lds_2x64(uint32_t a, f32x2& v0, f32x2& v1) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v0), "=l"(v1) : "r"(a));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -341,42 +381,69 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         // int32 results are positive: see the epilogue
         const unsigned long long d_bias = EXACT ? umma_desc_plain32(smem_u32(sm->bias)) : 0ull;
         (void)d_bias;
-        uint32_t g = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-            for (int ks = 0; ks < k_stages && ok; ks++, g++) {
-                const int s = g % TC_STAGES;
-                const uint32_t u = g / TC_STAGES;
-                ok = mbar_wait<BN, 128>(sm, smem_u32(&sm->full[s]), u & 1, err, 2);
-                if (!ok) break;
+        if constexpr (EXACT) {
+            // Asking a barrier costs 66 cycles even when it completed long ago: a stage's two questions go out together, and
+            // only a "not yet" is followed by a wait.
+            static_assert(UNIT == TC_KB_PER_STAGE, "one hand-over per stage");
+            const uint32_t g_total = (uint32_t)((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * (uint32_t)k_stages;
+            for (uint32_t g = 0; g < g_total; g++) {
+                const uint32_t s = g % TC_STAGES, unit = g & 1u, par = ((g >> 1) & 1) ^ 1;
+                const uint32_t fbar = smem_u32(&sm->full[s]), fpar = (g / TC_STAGES) & 1;
+                const uint32_t ebar = smem_u32(&sm->tmem_empty[unit]);
+                const bool pf = mbar_test(fbar, fpar), pe = mbar_test(ebar, par);
+                if (!__all_sync(0xffffffffu, pf) && !__all_sync(0xffffffffu, mbar_wait<BN, 128>(sm, fbar, fpar, err, 2))) break;
+                if (!__all_sync(0xffffffffu, pe) && !__all_sync(0xffffffffu, mbar_wait<BN, 64>(sm, ebar, par, err, 3))) break;
                 tc_fence_after();
                 const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
                 const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
+                const uint32_t d = tmem_base + unit * (UNIT * BN);
+                if (leader) {
+                    // that wait also says that the epilogue is done with the scales of the stage before the last
+                    if (g >= 2) mbar_arrive(smem_u32(&sm->empty[(g - 2) % TC_STAGES]));
+                    umma_i8_same_a<0>(d, d_bias, d_bias, idesc);
+                    umma_i8_same_a<1>(d + BN, d_bias, d_bias, idesc);
+                    umma_i8_same_a<1>(d + 2 * BN, d_bias, d_bias, idesc);
+                    umma_i8_same_a<2>(d + 3 * BN, d_bias, d_bias, idesc);
 #pragma unroll
-                for (int h = 0; h < TC_KB_PER_STAGE / UNIT; h++) {
-                    // Buffers are handed over half of tensor memory (UNIT blocks) at a time: every hand-over
-                    // costs each epilogue warp a barrier wait and an arrival, both long dependent steps of its
-                    // loop, and that loop - not the tensor pipe - sets the pace of the kernel
-                    const uint32_t un = g * (TC_KB_PER_STAGE / UNIT) + h;
-                    ok = mbar_wait<BN, 64>(sm, smem_u32(&sm->tmem_empty[un & 1u]), ((un >> 1) & 1) ^ 1, err, 3);
+                    for (int kk = 0; kk < UNIT; kk++)  // 32 bytes further along K inside the swizzle atom: +2 in the address field
+                        umma_i8<true>(d + kk * BN, da + kk * 2, db + kk * 2, idesc);
+                    umma_commit(smem_u32(&sm->tmem_full[unit]));
+                }
+                __syncwarp();
+            }
+        } else {
+            uint32_t g = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+                for (int ks = 0; ks < k_stages && ok; ks++, g++) {
+                    const int s = g % TC_STAGES;
+                    const uint32_t u = g / TC_STAGES;
+                    ok = mbar_wait<BN, 128>(sm, smem_u32(&sm->full[s]), u & 1, err, 2);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t d0 = tmem_base + (un & 1u) * (UNIT * BN);
-                    if (leader) {
-                        // EXACT: that wait also says that the epilogue is done with the scales of the stage before the last
-                        if (EXACT && g >= 2) mbar_arrive(smem_u32(&sm->empty[(g - 2) % TC_STAGES]));
+                    const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
+                    const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
 #pragma unroll
-                        for (int kk = 0; kk < UNIT; kk++) {
-                            // 32 bytes further along K inside the swizzle atom: +2 in the 16-byte address field
-                            const unsigned long long off = (unsigned long long)((h * UNIT + kk) * 2);
-                            if constexpr (EXACT) umma_i8(d0 + kk * BN, d_bias, d_bias, idesc);
-                            umma_i8(d0 + kk * BN, da + off, db + off, idesc, EXACT);
+                    for (int h = 0; h < TC_KB_PER_STAGE / UNIT; h++) {
+                        // Buffers are handed over half of tensor memory (UNIT blocks) at a time: every hand-over
+                        // costs each epilogue warp a barrier wait and an arrival, both long dependent steps of its
+                        // loop, and that loop - not the tensor pipe - sets the pace of the kernel
+                        const uint32_t un = g * (TC_KB_PER_STAGE / UNIT) + h;
+                        ok = mbar_wait<BN, 64>(sm, smem_u32(&sm->tmem_empty[un & 1u]), ((un >> 1) & 1) ^ 1, err, 3);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t d0 = tmem_base + (un & 1u) * (UNIT * BN);
+                        if (leader) {
+#pragma unroll
+                            for (int kk = 0; kk < UNIT; kk++) {
+                                // 32 bytes further along K inside the swizzle atom: +2 in the 16-byte address field
+                                const unsigned long long off = (unsigned long long)((h * UNIT + kk) * 2);
+                                umma_i8<false>(d0 + kk * BN, da + off, db + off, idesc);
+                            }
+                            umma_commit(smem_u32(&sm->tmem_full[un & 1u]));
                         }
-                        umma_commit(smem_u32(&sm->tmem_full[un & 1u]));
+                        __syncwarp();
                     }
-                    __syncwarp();
-                }
-                if constexpr (!EXACT) {
                     if (ok && leader) umma_commit(smem_u32(&sm->empty[s]));
                     __syncwarp();
                 }
@@ -554,9 +621,14 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             //    RN(float(p) * d) * 2^-77, the reference's rounded product, and no contraction with the addition can occur.
             //  - the chains run scaled by 2^-77.  Scales are f16 values, so every term is a multiple of 2^-48: nothing falls
             //    into the denormal range (2^-125) and every rounding is the unscaled one; the final sum is multiplied back.
-            // 512 x 6144 x 2048: see launch_gemm_tc_exact.
+            // 6144 x 2048 at 512 tokens: 157 -> 117 us (110 TFLOP/s); FMA pipe two thirds busy, the rest is the hand-over: both
+            // warps of a scheduler wait at the same time.  Tried: columns split between the groups with barriers and MMAs of
+            // their own (123), the groups kept half a stage apart (144), sixteen warps of 4 tokens (131), the next stage's
+            // first block loaded before the last chains (145 to 179).
             constexpr int TP = COLS / 8;  // token pairs per thread
             const f32x2 unbias = pack2(-__uint_as_float(1u << 17), -__uint_as_float(1u << 17));  // -2^-132
+            const uint32_t sw0 = smem_u32(&sm->stage[0].sw[0][row_in_tile]), sx0 = smem_u32(&sm->stage[0].sx[0][cg * 2 * TP]);
+            bool ready = false;  // the answer of a question asked during the stage before
             f32x2 acc2[TP][2][4];         // [pair][block parity][lane group], halves = the pair's tokens
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
@@ -573,10 +645,12 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     // their barrier (full[s]) before it issued what this one reports.  The arrival stands for both the tensor
                     // memory and the scales, all of which are in registers by then.
                     // (every lane of a warp runs the same wait on the same barrier and gets the same answer)
-                    ok = mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g >> 1) & 1, err, 6);
-                    if (!ok) break;
+                    if (!ready) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g >> 1) & 1, err, 6));
+                        if (!ok) break;
+                    }
                     tc_fence_after();
-                    const TcStage<BN>& st = sm->stage[g % TC_STAGES];
+                    const uint32_t st_off = (g % TC_STAGES) * (uint32_t)sizeof(TcStage<BN>), st_sw = sw0 + st_off, st_sx = sx0 + st_off;
                     // the load of block kk + 1 is in flight while the chains of block kk run
                     int32_t SA[COLS], SB[COLS];
                     struct Scales {
@@ -585,15 +659,12 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     };
                     auto scales = [&](const int kk) {
                         Scales c;
-                        c.w = st.sw[kk][row_in_tile];
+                        c.w = lds_f32(st_sw + kk * (TC_BM * 4));
                         if constexpr (TP >= 2) {
 #pragma unroll
-                            for (int i = 0; i < TP; i += 2) {
-                                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&st.sx[kk][(cg * TP + i) * 2]);
-                                c.x[i] = x.x, c.x[i + 1] = x.y;
-                            }
+                            for (int i = 0; i < TP; i += 2) lds_2x64(st_sx + kk * (BN * 4) + i * 8, c.x[i], c.x[i + 1]);
                         } else {
-                            c.x[0] = *reinterpret_cast<const unsigned long long*>(&st.sx[kk][cg * 2]);
+                            c.x[0] = lds_64(st_sx + kk * (BN * 4));
                         }
                         return c;
                     };
@@ -623,10 +694,11 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     const Scales c3 = scales(3);
                     tmem_ld_wait();
                     tmem_ld<COLS>(t0 + 3 * BN, SB);
+                    const bool q = mbar_test(smem_u32(&sm->tmem_full[unit ^ 1u]), ((g + 1) >> 1) & 1);
                     chains(SA, 0, c2);
                     tmem_ld_wait();
                     tc_fence_before();
-                    __syncwarp();
+                    ready = __all_sync(0xffffffffu, q);
                     if (lane == 0) mbar_arrive(smem_u32(&sm->tmem_empty[unit]));
                     chains(SB, 1, c3);
                 }
