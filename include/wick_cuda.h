@@ -220,7 +220,8 @@ int32_t wick_cuda_quantize_q8_0(const float* x_dev, uint32_t n, uint32_t k, floa
 int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const int8_t* xq_dev,
                           float* y_dev, void* stream);
 /* gemm_q4_0_q8_0_neon / gemm_q8_0_q8_0_neon (simd.rs:696-925, :937-1019) over n pre-quantised
- * columns; the result is token-major out[j*m + i] (the reference writes out[i*n + j]). */
+ * columns; the result is token-major out[j*m + i] (the reference writes out[i*n + j]).  With more than 8 columns
+ * and k % 128 == 0 it runs on the tensor cores (same bits; the weight's int8 copy is made by the first such call). */
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev,
                           uint32_t n, float* out_dev, void* stream);
 /* The same product on the tensor cores (tcgen05 int8 MMA, one instruction per 32-element block, int32

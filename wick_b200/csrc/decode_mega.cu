@@ -439,7 +439,7 @@ __device__ void prologue_norm(Ctx& c, const MegaPhase& ph, uint32_t token, const
             v[j] = 0.0f;
             if (b < nb) {
                 if (ph.embed) {
-                    v[j] = P.embd_q6k ? q6k_elem(P.embd6, token, e) : embed_elem(P.embd, token, e);
+                    v[j] = P.embedding ? __ldcg(P.embedding + e) : P.embd_q6k ? q6k_elem(P.embd6, token, e) : embed_elem(P.embd, token, e);
                     if (e >= e0 && e < e1) P.hidden[e] = v[j];
                 } else {
                     v[j] = __ldcg(P.hidden + e);

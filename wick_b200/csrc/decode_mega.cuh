@@ -77,6 +77,7 @@ struct MegaParams {
     // (skip_logits): output norm, logits, argmax and the control-block update run as separate kernels
     int embd_q6k, skip_logits;
     DevQ6K embd6;
+    const float* embedding;  // the first phase's row instead of the token's embedding, or NULL
     float *hidden, *proj, *qbuf, *kbuf, *vbuf, *attn_out, *gate, *up, *logits;
     const float *rope_cos, *rope_sin;
     DecodeCtl* ctl;
