@@ -32,6 +32,7 @@ constexpr int NCT = NC * 32;
 constexpr int TEAM_WARPS = MEGA_TEAM_WARPS;  // consumer warps work on ring slots in teams
 constexpr int NTEAMS = MEGA_TEAMS;
 constexpr int TEAM_THREADS = TEAM_WARPS * 32;
+constexpr int SPLIT_PAIR_STEPS = 48;  // two groups in a slot are split over the team's warps above this many steps
 constexpr unsigned SPIN_LIMIT = 1u << 22;  // x ~0.25-2 us per iteration
 constexpr unsigned WAIT_NS = 2000;         // hardware suspend limit of one mbarrier test
 
@@ -194,7 +195,7 @@ __device__ __forceinline__ Plan plan_phase(const MegaPhase& ph, int cta, int nct
     p.lo = share(cta, gt, ncta);
     p.hi = share(cta + 1, gt, ncta);
     int cap = slot_bytes / gb;
-    cap = cap < 1 ? 1 : (cap > 4 ? 4 : cap);
+    cap = cap < 1 ? 1 : cap >= 2 * TEAM_WARPS ? 2 * TEAM_WARPS : cap >= TEAM_WARPS ? TEAM_WARPS : cap;  // whole rounds of a team's warps
     int rg = (p.hi - p.lo + NTEAMS - 1) / NTEAMS;  // spread a small phase over all teams
     rg = rg < 1 ? 1 : rg;
     p.rg = rg > cap ? cap : rg;
@@ -933,92 +934,82 @@ __device__ __forceinline__ float reduce_row8(float a) {
     return a;
 }
 
-// The mat-vec over one ring slot is done by a TEAM of three consumer warps in two steps.
-//  1. products: every (row, block, lane-word) term  float(p) * (f16(d_w) * d_x)  is independent of
-//     every other one, so the team's 96 threads compute them all in parallel and write each one
-//     over the weight word it came from (same size: 4 bytes; for Q8_0 over the low word of the pair);
-//  2. chains: one warp per 4-row group, lane = p*16 + r*4 + l, adds its chain's products in block
-//     order (the only part of the reference's arithmetic that is serial), then the three shuffle-adds.
-// Both steps touch shared memory as 32 consecutive words per warp access (no bank conflicts).
 __device__ __forceinline__ void team_sync(int team) {
     asm volatile("bar.sync %0, %1;" ::"r"(2 + team), "n"(TEAM_THREADS) : "memory");
 }
 
-// One thread takes one (block, row) of the group per step: its four lane-words are 16 contiguous
-// bytes (as are the matching input words), so weights, inputs and products move as 128-bit
-// shared-memory accesses and the scale product is formed once per four terms.
-template <int DT, int U = (DT == DT_Q4_0 ? 3 : 2)>
-__device__ __forceinline__ void stage_products(uint32_t* __restrict__ qs, const __half* __restrict__ ds, int nb, int tt,
-                                               const int* __restrict__ xq32, const float* __restrict__ xsc) {
-    const int ni = nb * 4;  // (block, row) items of the group
-    for (int i0 = tt; i0 < ni; i0 += TEAM_THREADS * U) {
-        uint4 wa[U], wb[U];
-        int4 xl[U], xh[U];
-        float d[U];
-        int at[U];
+// The mat-vec over the 4-row groups of a ring slot.  Lane = p*16 + r*4 + l of a warp IS the chain (parity p, row r, lane group
+// l) of the reference's arithmetic: it walks the group's blocks p, p + 2, ... in order, forms the term
+// float(lane partial) * (f16(d_w) * d_x) and adds it.  Weight words of a step are 32 consecutive words, the input words 16 bytes
+// per parity (broadcast over the rows): five shared-memory wavefronts per step of 2 blocks x 4 rows, three of them shared
+// when a warp walks two groups at once (gate and up of the same rows).
+// (Before, all threads of a team first turned the words into terms in place and one warp then added them up: 18 wavefronts per
+// 8 blocks x 4 rows plus the terms' second trip, and shared memory was what bounded it - 430 ns per group of a 2048-long row
+// and team, and twice as many barriers.  Gate + up of the 1.6B model took 5.2 us per layer for 2.4 us of weight traffic.)
+//
+// Terms of steps [s, s + U) of G groups; use(u, g, term) takes them in step order per group.
+template <int DT, int G, int U, class F>
+__device__ __forceinline__ void chain_batch(const uint32_t* const (&q)[G], const __half* const (&d)[G], const int* x, const float* xs, int s, F&& use) {
+    uint32_t w[U][G], w2[U][G];
+    int xl[U], xh[U];
+    float dw[U][G], dx[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) {  // every load of the U independent items first
-            const int i = i0 + u * TEAM_THREADS, is = i < ni ? i : i0;
-            const int b = is >> 2, r = is & 3;
-            at[u] = DT == DT_Q4_0 ? q4_word(b, r, 0) : q8_word(b, 0, r, 0);
-            wa[u] = *reinterpret_cast<const uint4*>(qs + at[u]);
-            if (DT == DT_Q8_0) wb[u] = *reinterpret_cast<const uint4*>(qs + at[u] + 32);
-            xl[u] = *reinterpret_cast<const int4*>(xq32 + b * 8);
-            xh[u] = *reinterpret_cast<const int4*>(xq32 + b * 8 + 4);
-            d[u] = __fmul_rn(__half2float(ds[is]), xsc[b]);  // scale plane index b*4 + r == item index
-        }
+    for (int u = 0; u < U; u++) {  // every load of the batch first
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            int s0, s1, s2, s3;
-            if (DT == DT_Q4_0) {  // 16 * lane sum; xsc already carries the 1/16
-#define WICK_Q4_TERM(w, lo_x, hi_x) \
-    __dp4a((int)(((w)&0xF0F0F0F0u) ^ 0x80808080u), hi_x, __dp4a((int)((((w) << 4) & 0xF0F0F0F0u) ^ 0x80808080u), lo_x, 0))
-                s0 = WICK_Q4_TERM(wa[u].x, xl[u].x, xh[u].x);
-                s1 = WICK_Q4_TERM(wa[u].y, xl[u].y, xh[u].y);
-                s2 = WICK_Q4_TERM(wa[u].z, xl[u].z, xh[u].z);
-                s3 = WICK_Q4_TERM(wa[u].w, xl[u].w, xh[u].w);
-#undef WICK_Q4_TERM
-            } else {
-                s0 = __dp4a((int)wb[u].x, xh[u].x, __dp4a((int)wa[u].x, xl[u].x, 0));
-                s1 = __dp4a((int)wb[u].y, xh[u].y, __dp4a((int)wa[u].y, xl[u].y, 0));
-                s2 = __dp4a((int)wb[u].z, xh[u].z, __dp4a((int)wa[u].z, xl[u].z, 0));
-                s3 = __dp4a((int)wb[u].w, xh[u].w, __dp4a((int)wa[u].w, xl[u].w, 0));
-            }
-            if (i0 + u * TEAM_THREADS < ni) {
-                uint4 o;
-                o.x = __float_as_uint(__fmul_rn((float)s0, d[u]));
-                o.y = __float_as_uint(__fmul_rn((float)s1, d[u]));
-                o.z = __float_as_uint(__fmul_rn((float)s2, d[u]));
-                o.w = __float_as_uint(__fmul_rn((float)s3, d[u]));
-                *reinterpret_cast<uint4*>(qs + at[u]) = o;
-            }
+        for (int g = 0; g < G; g++) {
+            w[u][g] = q[g][(s + u) * (DT == DT_Q4_0 ? 32 : 64)];
+            if (DT == DT_Q8_0) w2[u][g] = q[g][(s + u) * 64 + 32];
+            dw[u][g] = __half2float(d[g][(s + u) * 8]);
         }
+        xl[u] = x[(s + u) * 16];
+        xh[u] = x[(s + u) * 16 + 4];
+        dx[u] = xs[(s + u) * 2];
     }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            int p;
+            if (DT == DT_Q4_0)  // 16 * lane partial; xs carries the 1/16
+                p = __dp4a((int)((w[u][g] & 0xF0F0F0F0u) ^ 0x80808080u), xh[u], __dp4a((int)(((w[u][g] << 4) & 0xF0F0F0F0u) ^ 0x80808080u), xl[u], 0));
+            else
+                p = __dp4a((int)w2[u][g], xh[u], __dp4a((int)w[u][g], xl[u], 0));
+            use(u, g, __fmul_rn((float)p, __fmul_rn(dw[u][g], dx[u])));
+        }
 }
 
-template <int DT, int U>
-__device__ __forceinline__ void chain_batches(const uint32_t* __restrict__ pp, int nb, int& b, float& acc) {
-    for (; b + 2 * (U - 1) < nb; b += 2 * U) {
-        float t[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) t[u] = __uint_as_float(DT == DT_Q4_0 ? pp[(b + 2 * u) * 16] : pp[((b + 2 * u) >> 1) * 64]);
-#pragma unroll
-        for (int u = 0; u < U; u++) acc = __fadd_rn(acc, t[u]);
-    }
+// Adds steps [s, s1) of G groups to their chains.
+template <int DT, int G>
+__device__ __forceinline__ void chain_steps(const uint32_t* const (&q)[G], const __half* const (&d)[G], const int* x, const float* xs, int s, int s1,
+                                            float (&acc)[G]) {
+    auto add = [&](int, int g, float t) { acc[g] = __fadd_rn(acc[g], t); };
+    for (; s + 8 <= s1; s += 8) chain_batch<DT, G, 8>(q, d, x, xs, s, add);
+    for (; s + 4 <= s1; s += 4) chain_batch<DT, G, 4>(q, d, x, xs, s, add);
+    for (; s < s1; s++) chain_batch<DT, G, 1>(q, d, x, xs, s, add);
 }
 
-// The chain of one (row, parity, lane group): its products in block order.  The additions are serial by contract; the
-// operand loads are not, so they are issued 32 at a time (then 8 at a time for what is left) ahead of the additions:
-// with 8 at a time the 32 terms of a 2048-long row took ~620 cycles, most of it shared-memory latency between batches.
+// Writes the terms of steps [s, s1) of one group over the weight words they come from.
 template <int DT>
-__device__ __forceinline__ float group_chain_sum(const uint32_t* __restrict__ qs, int nb, int lane) {
-    const int p = lane >> 4;
-    const uint32_t* pp = DT == DT_Q4_0 ? qs + (lane & 15) : qs + lane;
-    float acc = 0.0f;
-    int b = p;
-    chain_batches<DT, 32>(pp, nb, b, acc);
-    chain_batches<DT, 8>(pp, nb, b, acc);
-    for (; b < nb; b += 2) acc = __fadd_rn(acc, __uint_as_float(DT == DT_Q4_0 ? pp[b * 16] : pp[(b >> 1) * 64]));
+__device__ __forceinline__ void chain_terms(uint32_t* q, const __half* d, const int* x, const float* xs, int s, int s1) {
+    const uint32_t* const qa[1] = {q};
+    const __half* const da[1] = {d};
+    auto put = [&](int s0) { return [=](int u, int, float t) { q[(s0 + u) * (DT == DT_Q4_0 ? 32 : 64)] = __float_as_uint(t); }; };
+    for (; s + 4 <= s1; s += 4) chain_batch<DT, 1, 4>(qa, da, x, xs, s, put(s));
+    for (; s < s1; s++) chain_batch<DT, 1, 1>(qa, da, x, xs, s, put(s));
+}
+
+// Adds the stored terms of steps [s, s1) to a chain: the operand loads are issued 8 at a time ahead of the serial additions.
+template <int DT>
+__device__ __forceinline__ float chain_stored(const uint32_t* q, int s, int s1, float acc) {
+    constexpr int W = DT == DT_Q4_0 ? 32 : 64;
+    for (; s + 8 <= s1; s += 8) {
+        float t[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) t[u] = __uint_as_float(q[(s + u) * W]);
+#pragma unroll
+        for (int u = 0; u < 8; u++) acc = __fadd_rn(acc, t[u]);
+    }
+    for (; s < s1; s++) acc = __fadd_rn(acc, __uint_as_float(q[s * W]));
     return acc;
 }
 
@@ -1039,7 +1030,9 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
     const uint32_t pos0 = __ldcg(&P.ctl->pos), step0 = __ldcg(&P.ctl->step);
     uint32_t token = __ldcg(&P.ctl->token);
     unsigned owed = 0;  // arrivals of flag_out phases not yet added to the barrier counter
-    const int* xq32 = reinterpret_cast<const int*>(S.xq);
+    // this lane's input words and scales: parity cp, lane group lane & 3
+    const int cp = c.lane >> 4;
+    const int* const xw = reinterpret_cast<const int*>(S.xq) + cp * 8 + (c.lane & 3);
     for (int t = 0; t < P.n_tokens; t++) {
         const int pos = (int)pos0 + t;
         unsigned long long best = 0;
@@ -1079,7 +1072,6 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                 // slots until it has the two sums of each row and can apply SwiGLU (n_slots is a multiple of
                 // 2 * NTEAMS, so within the phase a slot always returns to the same team)
                 const DevWeight& wg = ph.mat[0].w;
-                const DevWeight& wu = ph.mat[1].w;
                 const int nb = wg.k / QK;
                 const uint32_t qgb = (uint32_t)wg.q_group_bytes();
                 float* act = ph.mat[0].y;
@@ -1095,7 +1087,9 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                     par ^= (slot == 0);
                     if (pj % NTEAMS != team) continue;
                     const int ng = pl.rg < pl.hi - g0 ? pl.rg : pl.hi - g0;
-                    uint8_t* bases[2] = {S.ring + (size_t)slot_a * P.slot_bytes, S.ring + (size_t)slot_b * P.slot_bytes};
+                    const uint8_t* base_a = S.ring + (size_t)slot_a * P.slot_bytes;
+                    const uint8_t* base_b = S.ring + (size_t)slot_b * P.slot_bytes;
+#pragma unroll 1
                     for (int half = 0; half < 2; half++) {
                         unsigned spins = 0;
                         while (!mbar_try_wait_for(&S.full[half ? slot_b : slot_a], half ? par_b : par_a, WAIT_NS) && !*S.abort) {
@@ -1105,26 +1099,19 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                                 break;
                             }
                         }
-                        const DevWeight& w = half ? wu : wg;
-                        const __half* dbase = reinterpret_cast<const __half*>(bases[half] + (size_t)ng * qgb);
-                        for (int gi = 0; gi < ng; gi++) {
-                            uint32_t* qs = reinterpret_cast<uint32_t*>(bases[half] + (size_t)gi * qgb);
-                            if (is_q4<DTK>(w.dtype)) stage_products<DT_Q4_0>(qs, dbase + (size_t)gi * nb * 4, nb, tt, xq32, S.xs16);
-                            else stage_products<DT_Q8_0>(qs, dbase + (size_t)gi * nb * 4, nb, tt, xq32, S.xs);
-                        }
                     }
-                    team_sync(team);
                     for (int gi = tw; gi < ng; gi += TEAM_WARPS) {
-                        const uint32_t* qa = reinterpret_cast<const uint32_t*>(bases[0] + (size_t)gi * qgb);
-                        const uint32_t* qb = reinterpret_cast<const uint32_t*>(bases[1] + (size_t)gi * qgb);
-                        float ga = is_q4<DTK>(wg.dtype) ? group_chain_sum<DT_Q4_0>(qa, nb, c.lane) : group_chain_sum<DT_Q8_0>(qa, nb, c.lane);
-                        float ua = is_q4<DTK>(wu.dtype) ? group_chain_sum<DT_Q4_0>(qb, nb, c.lane) : group_chain_sum<DT_Q8_0>(qb, nb, c.lane);
-                        ga = reduce_row8(ga);
-                        ua = reduce_row8(ua);
+                        const uint32_t* const q[2] = {reinterpret_cast<const uint32_t*>(base_a + (size_t)gi * qgb) + c.lane,
+                                                      reinterpret_cast<const uint32_t*>(base_b + (size_t)gi * qgb) + c.lane};
+                        const size_t d_off = (size_t)ng * qgb + (size_t)gi * nb * 8 + (c.lane >> 2) * 2;
+                        const __half* const d[2] = {reinterpret_cast<const __half*>(base_a + d_off), reinterpret_cast<const __half*>(base_b + d_off)};
+                        float acc[2] = {0.0f, 0.0f};
+                        if (is_q4<DTK>(wg.dtype)) chain_steps<DT_Q4_0, 2>(q, d, xw, S.xs16 + cp, 0, nb >> 1, acc);
+                        else chain_steps<DT_Q8_0, 2>(q, d, xw, S.xs + cp, 0, nb >> 1, acc);
+                        const float ga = reduce_row8(acc[0]), ua = reduce_row8(acc[1]);
                         const int row = (g0 + gi) * 4 + ((c.lane >> 2) & 3);
                         if ((c.lane & 19) == 0 && row < wg.m) act[row] = silu_mul_elem(ga, ua);  // cpu.rs:668-673
                     }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     team_sync(team);
                     if (tt == 0) {
                         mbar_arrive(&S.empty[slot_a]);
@@ -1157,12 +1144,11 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                         }
                         if (c.stamp && nst < 4) c.stamp[nst * 4 + 1] = globaltimer_ns();
                         uint8_t* base = S.ring + (size_t)slot * P.slot_bytes;
-                        const __half* dbase = reinterpret_cast<const __half*>(base + (size_t)ng * qgb);
-                        for (int gi = 0; gi < ng; gi++) {
-                            uint32_t* qs = reinterpret_cast<uint32_t*>(base + (size_t)gi * qgb);
-                            if (is_q4<DTK>(w.dtype)) stage_products<DT_Q4_0>(qs, dbase + (size_t)gi * nb * 4, nb, tt, xq32, S.xs16);
-                            else stage_products<DT_Q8_0>(qs, dbase + (size_t)gi * nb * 4, nb, tt, xq32, S.xs);
-                        }
+                        const int n = nb >> 1;
+                        // One group (or two long ones) per team: the steps of each are shared out to the team's warps, the
+                        // owner takes the first part and adds the others' terms after the sync
+                        const bool split = ng == 1 || (ng == 2 && n > SPLIT_PAIR_STEPS);
+                        const int part = ((n + TEAM_WARPS - 1) / TEAM_WARPS + 3) & ~3;  // whole batches
                         // residual-add epilogue: the old value of the row is fetched now, so that its latency runs
                         // under the chain step instead of after it (a warp owns at most two groups of a slot)
                         float resid[2] = {0.0f, 0.0f};
@@ -1173,11 +1159,42 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                                 if (gi < ng && row < wm) resid[q] = __ldcg(y + row);
                             }
                         }
-                        team_sync(team);
+                        float first = 0.0f;  // split: the owner's part of its group
+                        if (split) {
+                            for (int gi = 0; gi < ng; gi++) {
+                                uint32_t* q = reinterpret_cast<uint32_t*>(base + (size_t)gi * qgb) + c.lane;
+                                const __half* d = reinterpret_cast<const __half*>(base + (size_t)ng * qgb + (size_t)gi * nb * 8 + (c.lane >> 2) * 2);
+                                const int role = tw >= gi ? tw - gi : tw - gi + TEAM_WARPS;
+                                const int s0 = role * part < n ? role * part : n, s1 = s0 + part < n ? s0 + part : n;
+                                if (role == 0) {
+                                    const uint32_t* const qa[1] = {q};
+                                    const __half* const da[1] = {d};
+                                    float a[1] = {0.0f};
+                                    if (is_q4<DTK>(w.dtype)) chain_steps<DT_Q4_0, 1>(qa, da, xw, S.xs16 + cp, s0, s1, a);
+                                    else chain_steps<DT_Q8_0, 1>(qa, da, xw, S.xs + cp, s0, s1, a);
+                                    first = a[0];
+                                } else if (is_q4<DTK>(w.dtype)) {
+                                    chain_terms<DT_Q4_0>(q, d, xw, S.xs16 + cp, s0, s1);
+                                } else {
+                                    chain_terms<DT_Q8_0>(q, d, xw, S.xs + cp, s0, s1);
+                                }
+                            }
+                            team_sync(team);
+                        }
                         if (c.stamp && nst < 4) c.stamp[nst * 4 + 2] = globaltimer_ns();
                         for (int gi = tw; gi < ng; gi += TEAM_WARPS) {
-                            const uint32_t* qs = reinterpret_cast<const uint32_t*>(base + (size_t)gi * qgb);
-                            float acc = is_q4<DTK>(w.dtype) ? group_chain_sum<DT_Q4_0>(qs, nb, c.lane) : group_chain_sum<DT_Q8_0>(qs, nb, c.lane);
+                            const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (size_t)gi * qgb) + c.lane;
+                            float acc = first;
+                            if (split) {
+                                acc = is_q4<DTK>(w.dtype) ? chain_stored<DT_Q4_0>(q, part, n, acc) : chain_stored<DT_Q8_0>(q, part, n, acc);
+                            } else {
+                                const uint32_t* const qa[1] = {q};
+                                const __half* const da[1] = {reinterpret_cast<const __half*>(base + (size_t)ng * qgb + (size_t)gi * nb * 8 + (c.lane >> 2) * 2)};
+                                float a[1] = {0.0f};
+                                if (is_q4<DTK>(w.dtype)) chain_steps<DT_Q4_0, 1>(qa, da, xw, S.xs16 + cp, 0, n, a);
+                                else chain_steps<DT_Q8_0, 1>(qa, da, xw, S.xs + cp, 0, n, a);
+                                acc = a[0];
+                            }
                             acc = reduce_row8(acc);
                             const int row = (g0 + gi) * 4 + ((c.lane >> 2) & 3);
                             if ((c.lane & 19) == 0 && row < wm) {
@@ -1194,8 +1211,8 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                                 }
                             }
                         }
-                        // the slot was written through the generic proxy (products); order that before the
-                        // bulk copy (async proxy) that will refill it
+                        // a split slot was written through the generic proxy (terms); order that before the bulk copy
+                        // (async proxy) that will refill it
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         team_sync(team);
                         if (c.stamp && nst < 4) c.stamp[nst * 4 + 3] = globaltimer_ns();
