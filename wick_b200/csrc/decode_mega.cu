@@ -119,12 +119,15 @@ struct Plan {
     int lo, hi, rg, pad;
 };
 
+// Offset of the odd blocks' scales in xs / xs16 (even, so that two steps' scales load as one 64-bit word).
+__host__ __device__ __forceinline__ int xs_half(const MegaParams& P) { return (P.kmax / QK / 2 + 3) & ~3; }
+
 struct Smem {
     Plan* plan;    // [n_phases]
     uint8_t* ring;
     float* xf;     // attention phase: normalised scores, then gathered V rows
-    int8_t* xq;    // quantised phase input
-    float* xs;     // its block scales
+    int8_t* xq;    // quantised phase input; in a block the words of lane group l (elements 4l.., 16 + 4l..) lie side by side
+    float* xs;     // its block scales, those of the even blocks first, then (from xs_half) those of the odd ones
     float* xs16;   // scales / 16 (Q4_0 lane sums are kept multiplied by 16)
     double* red;   // [NC]
     float* redf;   // [NC]
@@ -146,9 +149,9 @@ __device__ __forceinline__ Smem carve(uint8_t* base, const MegaParams& P) {
     s.xf = (float*)(base + o);
     o += (size_t)nf * 4;
     s.xs = (float*)(base + o);
-    o += (size_t)(P.kmax / QK) * 4;
+    o += (size_t)xs_half(P) * 8;
     s.xs16 = (float*)(base + o);
-    o += (size_t)(P.kmax / QK) * 4;
+    o += (size_t)xs_half(P) * 8;
     o = (o + 15) & ~(size_t)15;
     s.xq = (int8_t*)(base + o);
     o += (size_t)P.kmax;
@@ -328,15 +331,16 @@ __device__ __forceinline__ void quantize_blocks(Ctx& c, const float (&v)[J], int
         const int b = c.cw + (j0 + jm) * NC;
         if ((c.lane & ((1 << SH) - 1)) == 0 && jm < J && b < nb) {
             const float sc = __half2float(__float2half_rn(d));
-            c.S.xs[b] = sc;
-            c.S.xs16[b] = __fmul_rn(sc, 0.0625f);
+            const int at = (b & 1) * xs_half(c.P) + (b >> 1);
+            c.S.xs[at] = sc;
+            c.S.xs16[at] = __fmul_rn(sc, 0.0625f);
         }
     }
 #pragma unroll
     for (int j = 0; j < J; j++) {
         const float idj = __shfl_sync(0xffffffffu, id, j << SH);
         const int b = c.cw + (j0 + j) * NC;
-        if (b < nb) c.S.xq[b * QK + c.lane] = (int8_t)__float2int_rn(__fmul_rn(v[j], idj));
+        if (b < nb) c.S.xq[b * QK + ((c.lane & 12) << 1) + ((c.lane & 16) >> 2) + (c.lane & 3)] = (int8_t)__float2int_rn(__fmul_rn(v[j], idj));
     }
 }
 
@@ -928,8 +932,8 @@ __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
 }
 
 __device__ __forceinline__ float reduce_row8(float a) {
-    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 1));
-    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 2));
+    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 4));
+    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 8));
     a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 16));
     return a;
 }
@@ -938,18 +942,19 @@ __device__ __forceinline__ void team_sync(int team) {
     asm volatile("bar.sync %0, %1;" ::"r"(2 + team), "n"(TEAM_THREADS) : "memory");
 }
 
-// The mat-vec over the 4-row groups of a ring slot.  Lane = p*16 + r*4 + l of a warp IS the chain (parity p, row r, lane group
-// l) of the reference's arithmetic: it walks the group's blocks p, p + 2, ... in order, forms the term
-// float(lane partial) * (f16(d_w) * d_x) and adds it.  Weight words of a step are 32 consecutive words, the input words 16 bytes
-// per parity (broadcast over the rows): five shared-memory wavefronts per step of 2 blocks x 4 rows, three of them shared
-// when a warp walks two groups at once (gate and up of the same rows).
+// The mat-vec over the 4-row groups of a ring slot.  Lane = p*16 + l*4 + r of a warp IS the chain (parity p, lane group l, row r)
+// of the reference's arithmetic: it walks the group's blocks p, p + 2, ... in order, forms the term
+// float(lane partial) * (f16(d_w) * d_x) and adds it.  Bound: shared-memory wavefronts (12 to 15 warps at one per cycle).  A step
+// of 2 blocks x 4 rows takes 1 for the weight words, 1 for both input words (a 64-bit load is one wavefront when four
+// neighbouring lanes share it, two otherwise: hence the rows in the low lane bits), 1 for d_w and 1/2 for d_x; the last
+// two kinds are shared when a warp walks two groups at once (gate and up of the same rows).
 // (Before, all threads of a team first turned the words into terms in place and one warp then added them up: 18 wavefronts per
 // 8 blocks x 4 rows plus the terms' second trip, and shared memory was what bounded it - 430 ns per group of a 2048-long row
 // and team, and twice as many barriers.  Gate + up of the 1.6B model took 5.2 us per layer for 2.4 us of weight traffic.)
 //
 // Terms of steps [s, s + U) of G groups; use(u, g, term) takes them in step order per group.
 template <int DT, int G, int U, class F>
-__device__ __forceinline__ void chain_batch(const uint32_t* const (&q)[G], const __half* const (&d)[G], const int* x, const float* xs, int s, F&& use) {
+__device__ __forceinline__ void chain_batch(const uint32_t* const (&q)[G], const __half* const (&d)[G], const int2* x, const float* xs, int s, F&& use) {
     uint32_t w[U][G], w2[U][G];
     int xl[U], xh[U];
     float dw[U][G], dx[U];
@@ -961,9 +966,14 @@ __device__ __forceinline__ void chain_batch(const uint32_t* const (&q)[G], const
             if (DT == DT_Q8_0) w2[u][g] = q[g][(s + u) * 64 + 32];
             dw[u][g] = __half2float(d[g][(s + u) * 8]);
         }
-        xl[u] = x[(s + u) * 16];
-        xh[u] = x[(s + u) * 16 + 4];
-        dx[u] = xs[(s + u) * 2];
+        const int2 xx = x[(s + u) * 8];
+        xl[u] = xx.x, xh[u] = xx.y;
+        if constexpr (U == 1) {
+            dx[u] = xs[s + u];
+        } else if ((u & 1) == 0) {  // batches start at even steps
+            const float2 dd = *reinterpret_cast<const float2*>(xs + s + u);
+            dx[u] = dd.x, dx[u + 1] = dd.y;
+        }
     }
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -980,7 +990,7 @@ __device__ __forceinline__ void chain_batch(const uint32_t* const (&q)[G], const
 
 // Adds steps [s, s1) of G groups to their chains.
 template <int DT, int G>
-__device__ __forceinline__ void chain_steps(const uint32_t* const (&q)[G], const __half* const (&d)[G], const int* x, const float* xs, int s, int s1,
+__device__ __forceinline__ void chain_steps(const uint32_t* const (&q)[G], const __half* const (&d)[G], const int2* x, const float* xs, int s, int s1,
                                             float (&acc)[G]) {
     auto add = [&](int, int g, float t) { acc[g] = __fadd_rn(acc[g], t); };
     for (; s + 8 <= s1; s += 8) chain_batch<DT, G, 8>(q, d, x, xs, s, add);
@@ -990,7 +1000,7 @@ __device__ __forceinline__ void chain_steps(const uint32_t* const (&q)[G], const
 
 // Writes the terms of steps [s, s1) of one group over the weight words they come from.
 template <int DT>
-__device__ __forceinline__ void chain_terms(uint32_t* q, const __half* d, const int* x, const float* xs, int s, int s1) {
+__device__ __forceinline__ void chain_terms(uint32_t* q, const __half* d, const int2* x, const float* xs, int s, int s1) {
     const uint32_t* const qa[1] = {q};
     const __half* const da[1] = {d};
     auto put = [&](int s0) { return [=](int u, int, float t) { q[(s0 + u) * (DT == DT_Q4_0 ? 32 : 64)] = __float_as_uint(t); }; };
@@ -1030,9 +1040,11 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
     const uint32_t pos0 = __ldcg(&P.ctl->pos), step0 = __ldcg(&P.ctl->step);
     uint32_t token = __ldcg(&P.ctl->token);
     unsigned owed = 0;  // arrivals of flag_out phases not yet added to the barrier counter
-    // this lane's input words and scales: parity cp, lane group lane & 3
-    const int cp = c.lane >> 4;
-    const int* const xw = reinterpret_cast<const int*>(S.xq) + cp * 8 + (c.lane & 3);
+    // this lane's chain: parity, lane group, row; its place among a step's weight words and scales, input words and scales
+    const int cp = c.lane >> 4, cl = (c.lane >> 2) & 3, cr = c.lane & 3;
+    const int w_at = cp * 16 + cr * 4 + cl, d_at = (cp * 4 + cr) * 2;
+    const int2* const xw = reinterpret_cast<const int2*>(S.xq) + cp * 4 + cl;
+    const float *const x16 = S.xs16 + cp * xs_half(P), *const x1 = S.xs + cp * xs_half(P);
     for (int t = 0; t < P.n_tokens; t++) {
         const int pos = (int)pos0 + t;
         unsigned long long best = 0;
@@ -1101,16 +1113,16 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                         }
                     }
                     for (int gi = tw; gi < ng; gi += TEAM_WARPS) {
-                        const uint32_t* const q[2] = {reinterpret_cast<const uint32_t*>(base_a + (size_t)gi * qgb) + c.lane,
-                                                      reinterpret_cast<const uint32_t*>(base_b + (size_t)gi * qgb) + c.lane};
-                        const size_t d_off = (size_t)ng * qgb + (size_t)gi * nb * 8 + (c.lane >> 2) * 2;
+                        const uint32_t* const q[2] = {reinterpret_cast<const uint32_t*>(base_a + (size_t)gi * qgb) + w_at,
+                                                      reinterpret_cast<const uint32_t*>(base_b + (size_t)gi * qgb) + w_at};
+                        const size_t d_off = (size_t)ng * qgb + (size_t)gi * nb * 8 + d_at;
                         const __half* const d[2] = {reinterpret_cast<const __half*>(base_a + d_off), reinterpret_cast<const __half*>(base_b + d_off)};
                         float acc[2] = {0.0f, 0.0f};
-                        if (is_q4<DTK>(wg.dtype)) chain_steps<DT_Q4_0, 2>(q, d, xw, S.xs16 + cp, 0, nb >> 1, acc);
-                        else chain_steps<DT_Q8_0, 2>(q, d, xw, S.xs + cp, 0, nb >> 1, acc);
+                        if (is_q4<DTK>(wg.dtype)) chain_steps<DT_Q4_0, 2>(q, d, xw, x16, 0, nb >> 1, acc);
+                        else chain_steps<DT_Q8_0, 2>(q, d, xw, x1, 0, nb >> 1, acc);
                         const float ga = reduce_row8(acc[0]), ua = reduce_row8(acc[1]);
-                        const int row = (g0 + gi) * 4 + ((c.lane >> 2) & 3);
-                        if ((c.lane & 19) == 0 && row < wg.m) act[row] = silu_mul_elem(ga, ua);  // cpu.rs:668-673
+                        const int row = (g0 + gi) * 4 + c.lane;
+                        if (c.lane < 4 && row < wg.m) act[row] = silu_mul_elem(ga, ua);  // cpu.rs:668-673
                     }
                     team_sync(team);
                     if (tt == 0) {
@@ -1152,52 +1164,52 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                         // residual-add epilogue: the old value of the row is fetched now, so that its latency runs
                         // under the chain step instead of after it (a warp owns at most two groups of a slot)
                         float resid[2] = {0.0f, 0.0f};
-                        if (epi == MEP_ADD && (c.lane & 19) == 0) {
+                        if (epi == MEP_ADD && c.lane < 4) {
 #pragma unroll
                             for (int q = 0; q < 2; q++) {
-                                const int gi = tw + q * TEAM_WARPS, row = (g0 + gi) * 4 + ((c.lane >> 2) & 3);
+                                const int gi = tw + q * TEAM_WARPS, row = (g0 + gi) * 4 + c.lane;
                                 if (gi < ng && row < wm) resid[q] = __ldcg(y + row);
                             }
                         }
                         float first = 0.0f;  // split: the owner's part of its group
                         if (split) {
                             for (int gi = 0; gi < ng; gi++) {
-                                uint32_t* q = reinterpret_cast<uint32_t*>(base + (size_t)gi * qgb) + c.lane;
-                                const __half* d = reinterpret_cast<const __half*>(base + (size_t)ng * qgb + (size_t)gi * nb * 8 + (c.lane >> 2) * 2);
+                                uint32_t* q = reinterpret_cast<uint32_t*>(base + (size_t)gi * qgb) + w_at;
+                                const __half* d = reinterpret_cast<const __half*>(base + (size_t)ng * qgb + (size_t)gi * nb * 8 + d_at);
                                 const int role = tw >= gi ? tw - gi : tw - gi + TEAM_WARPS;
                                 const int s0 = role * part < n ? role * part : n, s1 = s0 + part < n ? s0 + part : n;
                                 if (role == 0) {
                                     const uint32_t* const qa[1] = {q};
                                     const __half* const da[1] = {d};
                                     float a[1] = {0.0f};
-                                    if (is_q4<DTK>(w.dtype)) chain_steps<DT_Q4_0, 1>(qa, da, xw, S.xs16 + cp, s0, s1, a);
-                                    else chain_steps<DT_Q8_0, 1>(qa, da, xw, S.xs + cp, s0, s1, a);
+                                    if (is_q4<DTK>(w.dtype)) chain_steps<DT_Q4_0, 1>(qa, da, xw, x16, s0, s1, a);
+                                    else chain_steps<DT_Q8_0, 1>(qa, da, xw, x1, s0, s1, a);
                                     first = a[0];
                                 } else if (is_q4<DTK>(w.dtype)) {
-                                    chain_terms<DT_Q4_0>(q, d, xw, S.xs16 + cp, s0, s1);
+                                    chain_terms<DT_Q4_0>(q, d, xw, x16, s0, s1);
                                 } else {
-                                    chain_terms<DT_Q8_0>(q, d, xw, S.xs + cp, s0, s1);
+                                    chain_terms<DT_Q8_0>(q, d, xw, x1, s0, s1);
                                 }
                             }
                             team_sync(team);
                         }
                         if (c.stamp && nst < 4) c.stamp[nst * 4 + 2] = globaltimer_ns();
                         for (int gi = tw; gi < ng; gi += TEAM_WARPS) {
-                            const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (size_t)gi * qgb) + c.lane;
+                            const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (size_t)gi * qgb) + w_at;
                             float acc = first;
                             if (split) {
                                 acc = is_q4<DTK>(w.dtype) ? chain_stored<DT_Q4_0>(q, part, n, acc) : chain_stored<DT_Q8_0>(q, part, n, acc);
                             } else {
                                 const uint32_t* const qa[1] = {q};
-                                const __half* const da[1] = {reinterpret_cast<const __half*>(base + (size_t)ng * qgb + (size_t)gi * nb * 8 + (c.lane >> 2) * 2)};
+                                const __half* const da[1] = {reinterpret_cast<const __half*>(base + (size_t)ng * qgb + (size_t)gi * nb * 8 + d_at)};
                                 float a[1] = {0.0f};
-                                if (is_q4<DTK>(w.dtype)) chain_steps<DT_Q4_0, 1>(qa, da, xw, S.xs16 + cp, 0, n, a);
-                                else chain_steps<DT_Q8_0, 1>(qa, da, xw, S.xs + cp, 0, n, a);
+                                if (is_q4<DTK>(w.dtype)) chain_steps<DT_Q4_0, 1>(qa, da, xw, x16, 0, n, a);
+                                else chain_steps<DT_Q8_0, 1>(qa, da, xw, x1, 0, n, a);
                                 acc = a[0];
                             }
                             acc = reduce_row8(acc);
-                            const int row = (g0 + gi) * 4 + ((c.lane >> 2) & 3);
-                            if ((c.lane & 19) == 0 && row < wm) {
+                            const int row = (g0 + gi) * 4 + c.lane;
+                            if (c.lane < 4 && row < wm) {
                                 if (epi == MEP_ADD) {
                                     const float hv = __fadd_rn(gi == tw ? resid[0] : resid[1], acc);
                                     y[row] = hv;
@@ -1316,7 +1328,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_decode_mega(const MegaParam
 
 size_t mega_smem_bytes(const MegaParams& P) {
     int nf = xf_floats(P);
-    size_t o = (size_t)P.n_slots * P.slot_bytes + (size_t)nf * 4 + (size_t)(P.kmax / QK) * 8;
+    size_t o = (size_t)P.n_slots * P.slot_bytes + (size_t)nf * 4 + (size_t)xs_half(P) * 16;
     o = (o + 15) & ~(size_t)15;
     o += P.kmax;
     o = (o + 15) & ~(size_t)15;
