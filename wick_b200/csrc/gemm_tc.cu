@@ -43,7 +43,7 @@ constexpr int TC_KB_PER_STAGE = TC_KSTAGE / QK;  // 4 quantisation blocks per st
 // only refilled after the epilogue has finished with its scales, and the refill has to be back from L2 before
 // the MMA issuer needs it; with four stages that left about one microsecond, less than a loaded L2 round trip.
 template <int BN>
-__host__ __device__ constexpr int tc_stages() { return BN <= 64 ? 8 : 6; }
+__host__ __device__ constexpr int tc_stages() { return BN <= 32 ? 9 : BN <= 64 ? 8 : 6; }
 // Epilogue warps per TMEM lane quarter; each takes 1 / groups of a tile's columns
 __host__ __device__ constexpr int tc_col_groups(bool exact) { return exact ? 2 : 4; }
 __host__ __device__ constexpr int tc_threads(bool exact) { return 32 * (4 + 4 * tc_col_groups(exact)); }
@@ -302,8 +302,11 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     TcSmem<BN>* sm = reinterpret_cast<TcSmem<BN>*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int NBUF = 512 / BN;
     constexpr int UNIT = NBUF / 2 < TC_KB_PER_STAGE ? NBUF / 2 : TC_KB_PER_STAGE;  // blocks per hand-over: two units in flight
-    constexpr int NB2 = 2 * UNIT;  // buffers in use (32-column tiles leave half of tensor memory unused)
-    static_assert(TC_KB_PER_STAGE % UNIT == 0 && NBUF >= NB2, "two hand-over units that tile a stage");
+    // Hand-over units in flight.  The narrow exact tiles fill tensor memory with four: with two, a stage could not take less than
+    // half the way round (release, MMA issue, MMAs, wait, loads), ~860 cycles for the work of ~400.
+    constexpr int NU = EXACT ? NBUF / UNIT : 2;
+    constexpr int NB2 = NU * UNIT;
+    static_assert(TC_KB_PER_STAGE % UNIT == 0 && NBUF >= NB2 && (NU & (NU - 1)) == 0, "hand-over units that tile a stage");
     constexpr int TC_STAGES = tc_stages<BN>();
     constexpr int TC_COL_GROUPS = tc_col_groups(EXACT), TC_EPI_WARPS = 4 * TC_COL_GROUPS, TC_THREADS = tc_threads(EXACT);
     constexpr int COLS = BN / TC_COL_GROUPS;  // columns per epilogue thread
@@ -387,7 +390,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             static_assert(UNIT == TC_KB_PER_STAGE, "one hand-over per stage");
             const uint32_t g_total = (uint32_t)((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * (uint32_t)k_stages;
             for (uint32_t g = 0; g < g_total; g++) {
-                const uint32_t s = g % TC_STAGES, unit = g & 1u, par = ((g >> 1) & 1) ^ 1;
+                const uint32_t s = g % TC_STAGES, unit = g % NU, par = ((g / NU) & 1) ^ 1;
                 const uint32_t fbar = smem_u32(&sm->full[s]), fpar = (g / TC_STAGES) & 1;
                 const uint32_t ebar = smem_u32(&sm->tmem_empty[unit]);
                 const bool pf = mbar_test(fbar, fpar), pe = mbar_test(ebar, par);
@@ -398,8 +401,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                 const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
                 const uint32_t d = tmem_base + unit * (UNIT * BN);
                 if (leader) {
-                    // that wait also says that the epilogue is done with the scales of the stage before the last
-                    if (g >= 2) mbar_arrive(smem_u32(&sm->empty[(g - 2) % TC_STAGES]));
+                    // that wait also says that the epilogue is done with the scales of the stage NU before this one
+                    if (g >= NU) mbar_arrive(smem_u32(&sm->empty[(g - NU) % TC_STAGES]));
                     umma_i8_same_a<0>(d, d_bias, d_bias, idesc);
                     umma_i8_same_a<1>(d + BN, d_bias, d_bias, idesc);
                     umma_i8_same_a<1>(d + 2 * BN, d_bias, d_bias, idesc);
@@ -640,13 +643,13 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     for (int l = 0; l < 4; l++) acc2[i][0][l] = acc2[i][1][l] = pack2(0.f, 0.f);
                 for (int ks = 0; ks < k_stages && ok; ks++, g++) {
                     static_assert(UNIT == TC_KB_PER_STAGE, "the exact epilogue takes a whole stage per hand-over");
-                    const uint32_t unit = g & 1u;  // the half of tensor memory with the stage's 4 blocks
+                    const uint32_t unit = g % NU;  // the part of tensor memory with the stage's 4 blocks
                     // One wait and one arrival per stage.  The wait covers the stage's scales too: the MMA issuer had seen
                     // their barrier (full[s]) before it issued what this one reports.  The arrival stands for both the tensor
                     // memory and the scales, all of which are in registers by then.
                     // (every lane of a warp runs the same wait on the same barrier and gets the same answer)
                     if (!ready) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g >> 1) & 1, err, 6));
+                        ok = __all_sync(0xffffffffu, mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g / NU) & 1, err, 6));
                         if (!ok) break;
                     }
                     tc_fence_after();
@@ -694,7 +697,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     const Scales c3 = scales(3);
                     tmem_ld_wait();
                     tmem_ld<COLS>(t0 + 3 * BN, SB);
-                    const bool q = mbar_test(smem_u32(&sm->tmem_full[unit ^ 1u]), ((g + 1) >> 1) & 1);
+                    const bool q = mbar_test(smem_u32(&sm->tmem_full[(g + 1) % NU]), ((g + 1) / NU) & 1);
                     chains(SA, 0, c2);
                     tmem_ld_wait();
                     tc_fence_before();
