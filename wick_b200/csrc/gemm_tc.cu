@@ -298,6 +298,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
           const float* __restrict__ x_scales,  // [n][k/32]
           int32_t* __restrict__ sums,          // optional [n][m][k/32] (single-matrix jobs only)
           int n, int k, uint32_t* err) {
+    pdl_trigger();
     extern __shared__ uint8_t tc_smem_raw[];
     TcSmem<BN>* sm = reinterpret_cast<TcSmem<BN>*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int NBUF = 512 / BN;
@@ -352,6 +353,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = sm->tmem_base;
+    // Everything up to here, and the weight tiles of the exact GEMM (constant data), needs nothing of the kernel before
+    if (!(EXACT && warp == 0) && warp != 1) pdl_wait();
 
     if (warp == 0) {
         // ── TMA producer ─────────────────────────────────────────────────────
@@ -827,12 +830,10 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     g_kernel_launches++;
     if constexpr (!EXACT) {
         if (sums) {
-            k_gemm_tc<BN, true, false><<<grid, tc_threads(false), smem, st>>>(job, map_x, x_scales, sums, n, k, err);
-            return cudaGetLastError();
+            return launch_pdl(st, k_gemm_tc<BN, true, false>, dim3(grid), dim3(tc_threads(false)), smem, job, map_x, x_scales, sums, n, k, err);
         }
     }
-    k_gemm_tc<BN, false, EXACT><<<grid, tc_threads(EXACT), smem, st>>>(job, map_x, x_scales, nullptr, n, k, err);
-    return cudaGetLastError();
+    return launch_pdl(st, k_gemm_tc<BN, false, EXACT>, dim3(grid), dim3(tc_threads(EXACT)), smem, job, map_x, x_scales, nullptr, n, k, err);
 }
 
 cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, int count, int tiles_n) {

@@ -9,6 +9,31 @@ namespace wick {
 // recorded into a stream capture).
 extern thread_local unsigned long long g_kernel_launches;
 
+// Programmatic dependent launch.  Kernels launched with launch_pdl may start while their predecessor in the stream is still
+// running; pdl_enter() lets the successor do the same and then waits until the predecessor has finished and its writes are
+// visible, so it stands before the first access to memory that any other kernel writes or reads.  A prompt or a batched
+// step is a chain of ~150 kernels of 2 to 20 us: the launch and the ramp of one now lie under the tail of the one before.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+    pdl_trigger();
+    pdl_wait();
+}
+template <class... P, class... A>
+inline cudaError_t launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Device-resident control block of the decode step: lets one captured CUDA graph
 // serve every position (kernels read the token and position from here).
 struct DecodeCtl {

@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(NAIVE_THREADS) k_attention_naive(const float* 
                                                                     float* __restrict__ out, int start_pos,
                                                                     const DecodeCtl* __restrict__ ctl, int n_heads,
                                                                     int n_kv_heads, int hd, int max_seq) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     __shared__ double red[32];
     __shared__ float redf[32];
@@ -149,7 +150,7 @@ void launch_attention_naive(cudaStream_t st, const float* q, const float* k_cach
     size_t smem = naive_attention_smem_bytes(head_dim, max_seq);
     raise_naive_attention_smem(smem);  // no-op once granted; a failure surfaces as the launch error
     g_kernel_launches++;
-    k_attention_naive<<<grid, NAIVE_THREADS, smem, st>>>(q, k_cache, v_cache, out, start_pos, ctl, n_heads, n_kv_heads,
+    launch_pdl(st, k_attention_naive, dim3(grid), dim3(NAIVE_THREADS), smem, q, k_cache, v_cache, out, start_pos, ctl, n_heads, n_kv_heads,
                                                         head_dim, max_seq);
 }
 
@@ -214,6 +215,7 @@ template <int HD, int BQ, int MAXW>  // MAXW: the most consumer warps a launch o
 __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_FA_MIN_CTAS : 2) : 1) k_attention_flash(const float* __restrict__ q, const float* __restrict__ k_cache,
                                                           const float* __restrict__ v_cache, float* __restrict__ out, int n, int start_pos,
                                                           int n_heads, int n_kv_heads, int qb, int wave_size, uint32_t* __restrict__ err) {
+    pdl_enter();
     constexpr int ROW = HD + 4;          // padded row, floats
     constexpr int DPL = HD / 4;          // output dims per lane
     extern __shared__ __align__(128) uint8_t fa_smem[];
@@ -512,8 +514,8 @@ static cudaError_t launch_flash_hd(cudaStream_t st, const float* q, const float*
     const unsigned grid = (unsigned)(n_kv_heads * ((n + qb - 1) / qb));
     const int threads = (n_cw + 1) * 32;
     g_kernel_launches++;
-    if (n_cw <= 4) k_attention_flash<HD, BQ, 4><<<grid, threads, smem, st>>>(q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, qb, wave, err);
-    else k_attention_flash<HD, BQ, 8><<<grid, threads, smem, st>>>(q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, qb, wave, err);
+    if (n_cw <= 4) launch_pdl(st, k_attention_flash<HD, BQ, 4>, dim3(grid), dim3(threads), smem, q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, qb, wave, err);
+    else launch_pdl(st, k_attention_flash<HD, BQ, 8>, dim3(grid), dim3(threads), smem, q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, qb, wave, err);
     return cudaSuccess;
 }
 

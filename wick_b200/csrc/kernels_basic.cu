@@ -40,6 +40,7 @@ void launch_repack(cudaStream_t st, const DevWeight& w, const uint8_t* raw, uint
 // ── embedding ──────────────────────────────────────────────────────────────
 __global__ void k_embed(DevWeight w, const uint32_t* __restrict__ tokens, const DecodeCtl* __restrict__ ctl,
                         float* __restrict__ out) {
+    pdl_enter();
     int j = blockIdx.x;
     uint32_t tok = tokens ? tokens[j] : ctl->token;
     if (tok >= (uint32_t)w.m) tok = 0;  // host validates ids; never index outside the table
@@ -63,7 +64,7 @@ __global__ void k_embed(DevWeight w, const uint32_t* __restrict__ tokens, const 
 
 void launch_embed(cudaStream_t st, const DevWeight& w, const uint32_t* tokens, const DecodeCtl* ctl, float* out, int n) {
     g_kernel_launches++;
-    k_embed<<<n, 256, 0, st>>>(w, tokens, ctl, out);
+    launch_pdl(st, k_embed, dim3(n), dim3(256), 0, w, tokens, ctl, out);
 }
 
 // ── residual add + RMSNorm + Q8_0 quantise ─────────────────────────────────
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_quant(float* __restrict__ h
                                                           const float* __restrict__ weight, float eps, int dim,
                                                           float* __restrict__ q8s, int8_t* __restrict__ q8q,
                                                           float* __restrict__ normed_out) {
+    pdl_enter();
     extern __shared__ float xs[];
     __shared__ double red[32];
     const int row = blockIdx.x;
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_quant(float* __restrict__ h
 void launch_add_rmsnorm_quant(cudaStream_t st, float* hidden, const float* add, const float* weight, float eps, int n,
                               int dim, float* q8s, int8_t* q8q, float* normed_out) {
     g_kernel_launches++;
-    k_add_rmsnorm_quant<<<n, 256, dim * sizeof(float), st>>>(hidden, add, weight, eps, dim, q8s, q8q, normed_out);
+    launch_pdl(st, k_add_rmsnorm_quant, dim3(n), dim3(256), dim * sizeof(float), hidden, add, weight, eps, dim, q8s, q8q, normed_out);
 }
 
 __global__ void __launch_bounds__(256) k_rmsnorm_generic(float* __restrict__ x, const float* __restrict__ weight, int dim,
@@ -137,6 +139,7 @@ void launch_rmsnorm(cudaStream_t st, float* x, const float* weight, int n, int d
 // ── plain Q8_0 quantisation of rows ────────────────────────────────────────
 __global__ void k_quant_rows(const float* __restrict__ x, size_t total_blocks, float* __restrict__ q8s,
                              int8_t* __restrict__ q8q) {
+    pdl_enter();
     // 8 lanes per block, 4 consecutive elements per lane; lanes past the end still take part in the shuffles
     const size_t gt = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t b = gt >> 3;
@@ -156,12 +159,13 @@ void launch_quant_rows(cudaStream_t st, const float* x, int n, int k, float* q8s
     if (!total) return;
     unsigned grid = (unsigned)((total * 8 + 255) / 256);
     g_kernel_launches++;
-    k_quant_rows<<<grid, 256, 0, st>>>(x, total, q8s, q8q);
+    launch_pdl(st, k_quant_rows, dim3(grid), dim3(256), 0, x, total, q8s, q8q);
 }
 
 // ── SwiGLU + quantise ──────────────────────────────────────────────────────
 __global__ void k_silu_mul_quant(const float* __restrict__ gate, const float* __restrict__ up, size_t total_blocks,
                                  float* __restrict__ q8s, int8_t* __restrict__ q8q, float* __restrict__ act_out) {
+    pdl_enter();
     const size_t gt = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t b = gt >> 3;
     const bool in = b < total_blocks;
@@ -186,7 +190,7 @@ void launch_silu_mul_quant(cudaStream_t st, const float* gate, const float* up, 
     if (!total) return;
     unsigned grid = (unsigned)((total * 8 + 255) / 256);
     g_kernel_launches++;
-    k_silu_mul_quant<<<grid, 256, 0, st>>>(gate, up, total, q8s, q8q, act_out);
+    launch_pdl(st, k_silu_mul_quant, dim3(grid), dim3(256), 0, gate, up, total, q8s, q8q, act_out);
 }
 
 __global__ void k_silu_mul(float* __restrict__ gate, const float* __restrict__ up, size_t count) {
@@ -218,6 +222,7 @@ void launch_expf(cudaStream_t st, const float* x, float* y, size_t count) {
 __global__ void k_shortconv(const float* __restrict__ proj, const float* __restrict__ conv_w,
                             const float* __restrict__ state, int n, int hs, int ks, float* __restrict__ out,
                             float* __restrict__ q8s, int8_t* __restrict__ q8q) {
+    pdl_enter();
     const int dc = ks - 1;
     size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
@@ -253,6 +258,7 @@ __global__ void k_shortconv(const float* __restrict__ proj, const float* __restr
 // inside the old buffer (n < d_conv).  One thread per channel, ascending k, so the in-place
 // shift never reads a slot it already overwrote.
 __global__ void k_shortconv_state(const float* __restrict__ proj, float* __restrict__ state, int n, int hs, int ks) {
+    pdl_enter();
     const int dc = ks - 1;
     int ch = blockIdx.x * blockDim.x + threadIdx.x;
     if (ch >= hs) return;
@@ -274,8 +280,8 @@ void launch_shortconv(cudaStream_t st, const float* proj, const float* conv_w, f
     size_t warps = (size_t)n * (hs / QK);
     if (!warps) return;
     g_kernel_launches++;
-    k_shortconv<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(proj, conv_w, state, n, hs, ks, out, q8s, q8q);
-    if (ks > 1) g_kernel_launches++, k_shortconv_state<<<(hs + 255) / 256, 256, 0, st>>>(proj, state, n, hs, ks);
+    launch_pdl(st, k_shortconv, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, state, n, hs, ks, out, q8s, q8q);
+    if (ks > 1) g_kernel_launches++, launch_pdl(st, k_shortconv_state, dim3((hs + 255) / 256), dim3(256), 0, proj, state, n, hs, ks);
 }
 
 // ── per-head QK RMSNorm + RoPE + KV append ─────────────────────────────────
@@ -291,6 +297,7 @@ __global__ void __launch_bounds__(32) k_qknorm_rope_kv(float* __restrict__ q, co
                                                       float* __restrict__ v_cache, int start_pos,
                                                       const DecodeCtl* __restrict__ ctl, int n_heads, int n_kv_heads,
                                                       int hd) {
+    pdl_enter();
     __shared__ float xs[256];
     const int j = blockIdx.x, head = blockIdx.y, lane = threadIdx.x;
     const int hs = n_heads * hd, kv_dim = n_kv_heads * hd, half = hd / 2;
@@ -328,7 +335,7 @@ void launch_qknorm_rope_kv(cudaStream_t st, float* q, const float* k, const floa
                            int head_dim) {
     dim3 grid(n, n_heads + n_kv_heads);
     g_kernel_launches++;
-    k_qknorm_rope_kv<<<grid, 32, 0, st>>>(q, k, v, q_norm, k_norm, eps, rope_cos, rope_sin, k_cache, v_cache, start_pos,
+    launch_pdl(st, k_qknorm_rope_kv, dim3(grid), dim3(32), 0, q, k, v, q_norm, k_norm, eps, rope_cos, rope_sin, k_cache, v_cache, start_pos,
                                           ctl, n_heads, n_kv_heads, head_dim);
 }
 
@@ -350,6 +357,7 @@ void launch_rope(cudaStream_t st, float* q, float* k, const float* cos_row, cons
 
 // ── argmax ─────────────────────────────────────────────────────────────────
 __global__ void k_argmax_partial(const float* __restrict__ x, int count, unsigned long long* __restrict__ acc) {
+    pdl_enter();
     unsigned long long best = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         unsigned long long p = argmax_pack(x[i], (uint32_t)i);
@@ -363,6 +371,7 @@ __global__ void k_argmax_partial(const float* __restrict__ x, int count, unsigne
     if ((threadIdx.x & 31) == 0) atomicMax(acc, best);
 }
 __global__ void k_argmax_finish(unsigned long long* __restrict__ acc, uint32_t* __restrict__ out) {
+    pdl_enter();
     *out = (uint32_t)(*acc & 0xffffffffull);
     *acc = 0;
 }
@@ -371,13 +380,14 @@ void launch_argmax(cudaStream_t st, const float* logits, int count, unsigned lon
     if (grid > 148) grid = 148;
     if (grid < 1) grid = 1;
     g_kernel_launches++;
-    k_argmax_partial<<<grid, 256, 0, st>>>(logits, count, scratch);
+    launch_pdl(st, k_argmax_partial, dim3(grid), dim3(256), 0, logits, count, scratch);
     g_kernel_launches++;
-    k_argmax_finish<<<1, 1, 0, st>>>(scratch, out);
+    launch_pdl(st, k_argmax_finish, dim3(1), dim3(1), 0, scratch, out);
 }
 
 __global__ void k_decode_advance(DecodeCtl* __restrict__ ctl, const uint32_t* __restrict__ argmax_tok,
                                  uint32_t* __restrict__ ring, int ring_len) {
+    pdl_enter();
     uint32_t t = *argmax_tok;
     ctl->token = t;
     ctl->pos += 1;
@@ -386,7 +396,7 @@ __global__ void k_decode_advance(DecodeCtl* __restrict__ ctl, const uint32_t* __
 }
 void launch_decode_advance(cudaStream_t st, DecodeCtl* ctl, const uint32_t* argmax_tok, uint32_t* ring, int ring_len) {
     g_kernel_launches++;
-    k_decode_advance<<<1, 1, 0, st>>>(ctl, argmax_tok, ring, ring_len);
+    launch_pdl(st, k_decode_advance, dim3(1), dim3(1), 0, ctl, argmax_tok, ring, ring_len);
 }
 
 // ── n_keep context shift ────────────────────────────────────────────────────

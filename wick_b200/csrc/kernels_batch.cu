@@ -14,6 +14,7 @@ namespace wick {
 // buffer [d_conv][hs] is read, used and advanced by the thread that owns the channel.
 __global__ void k_shortconv_rows(const float* __restrict__ proj, const float* __restrict__ conv_w, float* const* __restrict__ states,
                                  int n, int hs, int ks, float* __restrict__ q8s, int8_t* __restrict__ q8q) {
+    pdl_enter();
     const int dc = ks - 1;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -47,7 +48,7 @@ void launch_shortconv_rows(cudaStream_t st, const float* proj, const float* conv
     const size_t warps = (size_t)n * (hs / QK);
     if (!warps) return;
     g_kernel_launches++;
-    k_shortconv_rows<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(proj, conv_w, states, n, hs, ks, q8s, q8q);
+    launch_pdl(st, k_shortconv_rows, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, states, n, hs, ks, q8s, q8q);
 }
 
 // ── per-head QK RMSNorm + RoPE + KV append, per-row position and caches (lfm2.rs:783-855) ──
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(32) k_qknorm_rope_kv_rows(float* __restrict__ 
                                                            const float* __restrict__ rope_cos, const float* __restrict__ rope_sin,
                                                            float* const* __restrict__ k_caches, float* const* __restrict__ v_caches,
                                                            const uint32_t* __restrict__ positions, int n_heads, int n_kv_heads, int hd) {
+    pdl_enter();
     __shared__ float xs[256];
     const int j = blockIdx.x, head = blockIdx.y, lane = threadIdx.x;
     const int hs = n_heads * hd, kv_dim = n_kv_heads * hd, half = hd / 2;
@@ -93,7 +95,7 @@ void launch_qknorm_rope_kv_rows(cudaStream_t st, float* q, const float* k, const
                                 const uint32_t* positions, int n, int n_heads, int n_kv_heads, int head_dim) {
     dim3 grid(n, n_heads + n_kv_heads);
     g_kernel_launches++;
-    k_qknorm_rope_kv_rows<<<grid, 32, 0, st>>>(q, k, v, q_norm, k_norm, eps, rope_cos, rope_sin, k_caches, v_caches, positions, n_heads,
+    launch_pdl(st, k_qknorm_rope_kv_rows, dim3(grid), dim3(32), 0, q, k, v, q_norm, k_norm, eps, rope_cos, rope_sin, k_caches, v_caches, positions, n_heads,
                                                n_kv_heads, head_dim);
 }
 
@@ -124,6 +126,7 @@ __device__ __forceinline__ float qk_dot_rows(const float* __restrict__ q, const 
 __global__ void __launch_bounds__(ROWS_ATTN_THREADS) k_attention_rows(const float* __restrict__ q, float* const* __restrict__ k_caches,
                                                                       float* const* __restrict__ v_caches, const uint32_t* __restrict__ positions,
                                                                       float* __restrict__ out, int n_heads, int n_kv_heads, int hd, int max_seq) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     __shared__ double red[32];
     __shared__ float redf[32];
@@ -196,7 +199,7 @@ cudaError_t launch_attention_rows(cudaStream_t st, const float* q, float* const*
     }
     dim3 grid(n_heads, n);
     g_kernel_launches++;
-    k_attention_rows<<<grid, ROWS_ATTN_THREADS, smem, st>>>(q, k_caches, v_caches, positions, out, n_heads, n_kv_heads, head_dim, max_seq);
+    launch_pdl(st, k_attention_rows, dim3(grid), dim3(ROWS_ATTN_THREADS), smem, q, k_caches, v_caches, positions, out, n_heads, n_kv_heads, head_dim, max_seq);
     return cudaSuccess;
 }
 
@@ -309,6 +312,7 @@ void launch_attention_splitk(cudaStream_t st, const float* q, float* const* k_ca
 
 // ── cpu_argmax (sampler.rs:8-19) of every row of logits [n][count]; one CTA per row ──
 __global__ void __launch_bounds__(1024) k_argmax_rows(const float* __restrict__ x, int count, uint32_t* __restrict__ out) {
+    pdl_enter();
     __shared__ unsigned long long sh[32];
     const float* row = x + (size_t)blockIdx.x * count;
     unsigned long long best = 0;
@@ -332,13 +336,14 @@ __global__ void __launch_bounds__(1024) k_argmax_rows(const float* __restrict__ 
 void launch_argmax_rows(cudaStream_t st, const float* logits, int n, int count, uint32_t* out) {
     if (!n) return;
     g_kernel_launches++;
-    k_argmax_rows<<<n, 1024, 0, st>>>(logits, count, out);
+    launch_pdl(st, k_argmax_rows, dim3(n), dim3(1024), 0, logits, count, out);
 }
 
 // End of a batched step kept on the device: the chosen tokens become the next step's inputs, every position
 // advances by one, and the tokens are recorded in row `step` of the output table [steps][n].
 __global__ void k_rows_advance(uint32_t* __restrict__ tokens, const uint32_t* __restrict__ next, uint32_t* __restrict__ positions,
                                uint32_t* __restrict__ out_table, int n, int step) {
+    pdl_enter();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const uint32_t t = next[j];
@@ -350,7 +355,7 @@ __global__ void k_rows_advance(uint32_t* __restrict__ tokens, const uint32_t* __
 void launch_rows_advance(cudaStream_t st, uint32_t* tokens, const uint32_t* next, uint32_t* positions, uint32_t* out_table, int n, int step) {
     if (!n) return;
     g_kernel_launches++;
-    k_rows_advance<<<(n + 127) / 128, 128, 0, st>>>(tokens, next, positions, out_table, n, step);
+    launch_pdl(st, k_rows_advance, dim3((n + 127) / 128), dim3(128), 0, tokens, next, positions, out_table, n, step);
 }
 
 }  // namespace wick

@@ -72,6 +72,7 @@ __device__ __forceinline__ float gemv_chain(const DevWeight& w, int g, int lane,
 
 __global__ void __launch_bounds__(256) k_gemv(GemvJob job, const float* __restrict__ xs_g,
                                               const int8_t* __restrict__ xq_g) {
+    pdl_enter();
     extern __shared__ int smem_i[];
     const int k = job.w[0].k, nb = k / QK;
     int* xq32 = smem_i;                                   // k/4 words
@@ -103,7 +104,7 @@ void launch_gemv(cudaStream_t st, const GemvJob& job, const float* xs, const int
     const int k = job.w[0].k;
     size_t smem = (size_t)k + (size_t)(k / QK) * 4;
     g_kernel_launches++;
-    k_gemv<<<(groups + GEMV_GROUPS - 1) / GEMV_GROUPS, 256, smem, st>>>(job, xs, xq);
+    launch_pdl(st, k_gemv, dim3((groups + GEMV_GROUPS - 1) / GEMV_GROUPS), dim3(256), smem, job, xs, xq);
 }
 
 // ── block sums (parity tap) ────────────────────────────────────────────────
@@ -143,6 +144,7 @@ constexpr int KC = 32;       // blocks per K chunk
 template <int DT>
 __global__ void __launch_bounds__(256) k_gemm(DevWeight w, const float* __restrict__ bs, const int8_t* __restrict__ bq,
                                               int n, float* __restrict__ out) {
+    pdl_enter();
     __shared__ __align__(16) int xt[KC * 8 * TJP];
     __shared__ __align__(16) float st[KC * TJP];
     const int k = w.k, nb = k / QK, m = w.m;
@@ -219,8 +221,8 @@ __global__ void __launch_bounds__(256) k_gemm(DevWeight w, const float* __restri
 void launch_gemm(cudaStream_t st, const DevWeight& w, const float* bs, const int8_t* bq, int n, float* out) {
     if (!n || !w.m) return;
     dim3 grid((w.m + GEMM_ROWS - 1) / GEMM_ROWS, (n + TJ - 1) / TJ);
-    if (w.dtype == DT_Q4_0) g_kernel_launches++, k_gemm<DT_Q4_0><<<grid, 256, 0, st>>>(w, bs, bq, n, out);
-    else g_kernel_launches++, k_gemm<DT_Q8_0><<<grid, 256, 0, st>>>(w, bs, bq, n, out);
+    if (w.dtype == DT_Q4_0) g_kernel_launches++, launch_pdl(st, k_gemm<DT_Q4_0>, dim3(grid), dim3(256), 0, w, bs, bq, n, out);
+    else g_kernel_launches++, launch_pdl(st, k_gemm<DT_Q8_0>, dim3(grid), dim3(256), 0, w, bs, bq, n, out);
 }
 
 }  // namespace wick

@@ -19,6 +19,7 @@ __global__ void k_repack_q6k(const uint16_t* __restrict__ raw, uint16_t* ql, uin
 }
 
 __global__ void k_embed_q6k(DevQ6K w, const uint32_t* __restrict__ tokens, const DecodeCtl* __restrict__ ctl, float* __restrict__ out) {
+    pdl_enter();
     const int j = blockIdx.x;
     uint32_t tok = tokens ? tokens[j] : ctl->token;
     if (tok >= (uint32_t)w.m) tok = 0;  // host validates ids; never index outside the table
@@ -35,6 +36,7 @@ constexpr int Q6K_WARPS = 4;     // warps per CTA
 
 __global__ void __launch_bounds__(32 * Q6K_WARPS)
 k_gemv_q6k(DevQ6K w, const float* __restrict__ xs, const int8_t* __restrict__ xq, float* __restrict__ y) {
+    pdl_enter();
     extern __shared__ float q6k_terms[];  // [warp][ROWS][k/16]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = w.k, units = k / 64, nsub = k / 16;
@@ -97,7 +99,7 @@ void launch_repack_q6k(cudaStream_t st, const uint8_t* raw, const DevQ6K& w) {
 
 void launch_embed_q6k(cudaStream_t st, const DevQ6K& w, const uint32_t* tokens, const DecodeCtl* ctl, float* out, int n) {
     g_kernel_launches++;
-    k_embed_q6k<<<n, 256, 0, st>>>(w, tokens, ctl, out);
+    launch_pdl(st, k_embed_q6k, dim3(n), dim3(256), 0, w, tokens, ctl, out);
 }
 
 size_t gemv_q6k_smem(int k) { return (size_t)Q6K_WARPS * Q6K_ROWS * (k / 16) * sizeof(float); }
@@ -105,7 +107,7 @@ size_t gemv_q6k_smem(int k) { return (size_t)Q6K_WARPS * Q6K_ROWS * (k / 16) * s
 void launch_gemv_q6k(cudaStream_t st, const DevQ6K& w, const float* xs, const int8_t* xq, float* y) {
     const int rows_per_cta = Q6K_WARPS * Q6K_ROWS;
     g_kernel_launches++;
-    k_gemv_q6k<<<(w.m + rows_per_cta - 1) / rows_per_cta, 32 * Q6K_WARPS, gemv_q6k_smem(w.k), st>>>(w, xs, xq, y);
+    launch_pdl(st, k_gemv_q6k, dim3((w.m + rows_per_cta - 1) / rows_per_cta), dim3(32 * Q6K_WARPS), gemv_q6k_smem(w.k), w, xs, xq, y);
 }
 
 }  // namespace wick
