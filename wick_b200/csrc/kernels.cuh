@@ -15,9 +15,13 @@ extern thread_local unsigned long long g_kernel_launches;
 // step is a chain of ~150 kernels of 2 to 20 us: the launch and the ramp of one now lie under the tail of the one before.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_enter() {
+// `p`: the kernel's pointers.  A load through a const __restrict__ parameter may be moved anywhere by the compiler, above the
+// wait too; passing the pointers through here makes every access depend on a value that only exists behind it.
+template <class... T>
+__device__ __forceinline__ void pdl_enter(T&... p) {
     pdl_trigger();
     pdl_wait();
+    ([](auto& q) { asm volatile("" : "+l"(q) : : "memory"); }(p), ...);
 }
 template <class... P, class... A>
 inline cudaError_t launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(NAIVE_THREADS) k_attention_naive(const float* 
                                                                     float* __restrict__ out, int start_pos,
                                                                     const DecodeCtl* __restrict__ ctl, int n_heads,
                                                                     int n_kv_heads, int hd, int max_seq) {
-    pdl_enter();
+    pdl_enter(q, k_cache, v_cache, out, ctl);
     extern __shared__ __align__(16) float sm[];
     __shared__ double red[32];
     __shared__ float redf[32];
@@ -215,7 +215,7 @@ template <int HD, int BQ, int MAXW>  // MAXW: the most consumer warps a launch o
 __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_FA_MIN_CTAS : 2) : 1) k_attention_flash(const float* __restrict__ q, const float* __restrict__ k_cache,
                                                           const float* __restrict__ v_cache, float* __restrict__ out, int n, int start_pos,
                                                           int n_heads, int n_kv_heads, int qb, int wave_size, uint32_t* __restrict__ err) {
-    pdl_enter();
+    pdl_enter(q, k_cache, v_cache, out, err);
     constexpr int ROW = HD + 4;          // padded row, floats
     constexpr int DPL = HD / 4;          // output dims per lane
     extern __shared__ __align__(128) uint8_t fa_smem[];

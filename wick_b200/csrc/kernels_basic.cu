@@ -40,7 +40,7 @@ void launch_repack(cudaStream_t st, const DevWeight& w, const uint8_t* raw, uint
 // ── embedding ──────────────────────────────────────────────────────────────
 __global__ void k_embed(DevWeight w, const uint32_t* __restrict__ tokens, const DecodeCtl* __restrict__ ctl,
                         float* __restrict__ out) {
-    pdl_enter();
+    pdl_enter(tokens, ctl, out);
     int j = blockIdx.x;
     uint32_t tok = tokens ? tokens[j] : ctl->token;
     if (tok >= (uint32_t)w.m) tok = 0;  // host validates ids; never index outside the table
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_quant(float* __restrict__ h
                                                           const float* __restrict__ weight, float eps, int dim,
                                                           float* __restrict__ q8s, int8_t* __restrict__ q8q,
                                                           float* __restrict__ normed_out) {
-    pdl_enter();
+    pdl_enter(hidden, add, weight, q8s, q8q, normed_out);
     extern __shared__ float xs[];
     __shared__ double red[32];
     const int row = blockIdx.x;
@@ -139,7 +139,7 @@ void launch_rmsnorm(cudaStream_t st, float* x, const float* weight, int n, int d
 // ── plain Q8_0 quantisation of rows ────────────────────────────────────────
 __global__ void k_quant_rows(const float* __restrict__ x, size_t total_blocks, float* __restrict__ q8s,
                              int8_t* __restrict__ q8q) {
-    pdl_enter();
+    pdl_enter(x, q8s, q8q);
     // 8 lanes per block, 4 consecutive elements per lane; lanes past the end still take part in the shuffles
     const size_t gt = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t b = gt >> 3;
@@ -165,7 +165,7 @@ void launch_quant_rows(cudaStream_t st, const float* x, int n, int k, float* q8s
 // ── SwiGLU + quantise ──────────────────────────────────────────────────────
 __global__ void k_silu_mul_quant(const float* __restrict__ gate, const float* __restrict__ up, size_t total_blocks,
                                  float* __restrict__ q8s, int8_t* __restrict__ q8q, float* __restrict__ act_out) {
-    pdl_enter();
+    pdl_enter(gate, up, q8s, q8q, act_out);
     const size_t gt = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t b = gt >> 3;
     const bool in = b < total_blocks;
@@ -222,7 +222,7 @@ void launch_expf(cudaStream_t st, const float* x, float* y, size_t count) {
 __global__ void k_shortconv(const float* __restrict__ proj, const float* __restrict__ conv_w,
                             const float* __restrict__ state, int n, int hs, int ks, float* __restrict__ out,
                             float* __restrict__ q8s, int8_t* __restrict__ q8q) {
-    pdl_enter();
+    pdl_enter(proj, conv_w, state, out, q8s, q8q);
     const int dc = ks - 1;
     size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
@@ -258,7 +258,7 @@ __global__ void k_shortconv(const float* __restrict__ proj, const float* __restr
 // inside the old buffer (n < d_conv).  One thread per channel, ascending k, so the in-place
 // shift never reads a slot it already overwrote.
 __global__ void k_shortconv_state(const float* __restrict__ proj, float* __restrict__ state, int n, int hs, int ks) {
-    pdl_enter();
+    pdl_enter(proj, state);
     const int dc = ks - 1;
     int ch = blockIdx.x * blockDim.x + threadIdx.x;
     if (ch >= hs) return;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(32) k_qknorm_rope_kv(float* __restrict__ q, co
                                                       float* __restrict__ v_cache, int start_pos,
                                                       const DecodeCtl* __restrict__ ctl, int n_heads, int n_kv_heads,
                                                       int hd) {
-    pdl_enter();
+    pdl_enter(q, k, v, q_norm, k_norm, rope_cos, rope_sin, k_cache, v_cache, ctl);
     __shared__ float xs[256];
     const int j = blockIdx.x, head = blockIdx.y, lane = threadIdx.x;
     const int hs = n_heads * hd, kv_dim = n_kv_heads * hd, half = hd / 2;
@@ -357,7 +357,7 @@ void launch_rope(cudaStream_t st, float* q, float* k, const float* cos_row, cons
 
 // ── argmax ─────────────────────────────────────────────────────────────────
 __global__ void k_argmax_partial(const float* __restrict__ x, int count, unsigned long long* __restrict__ acc) {
-    pdl_enter();
+    pdl_enter(x, acc);
     unsigned long long best = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         unsigned long long p = argmax_pack(x[i], (uint32_t)i);
@@ -371,7 +371,7 @@ __global__ void k_argmax_partial(const float* __restrict__ x, int count, unsigne
     if ((threadIdx.x & 31) == 0) atomicMax(acc, best);
 }
 __global__ void k_argmax_finish(unsigned long long* __restrict__ acc, uint32_t* __restrict__ out) {
-    pdl_enter();
+    pdl_enter(acc, out);
     *out = (uint32_t)(*acc & 0xffffffffull);
     *acc = 0;
 }
@@ -387,7 +387,7 @@ void launch_argmax(cudaStream_t st, const float* logits, int count, unsigned lon
 
 __global__ void k_decode_advance(DecodeCtl* __restrict__ ctl, const uint32_t* __restrict__ argmax_tok,
                                  uint32_t* __restrict__ ring, int ring_len) {
-    pdl_enter();
+    pdl_enter(ctl, argmax_tok, ring);
     uint32_t t = *argmax_tok;
     ctl->token = t;
     ctl->pos += 1;

@@ -14,7 +14,7 @@ namespace wick {
 // buffer [d_conv][hs] is read, used and advanced by the thread that owns the channel.
 __global__ void k_shortconv_rows(const float* __restrict__ proj, const float* __restrict__ conv_w, float* const* __restrict__ states,
                                  int n, int hs, int ks, float* __restrict__ q8s, int8_t* __restrict__ q8q) {
-    pdl_enter();
+    pdl_enter(proj, conv_w, states, q8s, q8q);
     const int dc = ks - 1;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(32) k_qknorm_rope_kv_rows(float* __restrict__ 
                                                            const float* __restrict__ rope_cos, const float* __restrict__ rope_sin,
                                                            float* const* __restrict__ k_caches, float* const* __restrict__ v_caches,
                                                            const uint32_t* __restrict__ positions, int n_heads, int n_kv_heads, int hd) {
-    pdl_enter();
+    pdl_enter(q, k, v, q_norm, k_norm, rope_cos, rope_sin, k_caches, v_caches, positions);
     __shared__ float xs[256];
     const int j = blockIdx.x, head = blockIdx.y, lane = threadIdx.x;
     const int hs = n_heads * hd, kv_dim = n_kv_heads * hd, half = hd / 2;
@@ -126,7 +126,7 @@ __device__ __forceinline__ float qk_dot_rows(const float* __restrict__ q, const 
 __global__ void __launch_bounds__(ROWS_ATTN_THREADS) k_attention_rows(const float* __restrict__ q, float* const* __restrict__ k_caches,
                                                                       float* const* __restrict__ v_caches, const uint32_t* __restrict__ positions,
                                                                       float* __restrict__ out, int n_heads, int n_kv_heads, int hd, int max_seq) {
-    pdl_enter();
+    pdl_enter(q, k_caches, v_caches, positions, out);
     extern __shared__ __align__(16) float sm[];
     __shared__ double red[32];
     __shared__ float redf[32];
@@ -312,7 +312,7 @@ void launch_attention_splitk(cudaStream_t st, const float* q, float* const* k_ca
 
 // ── cpu_argmax (sampler.rs:8-19) of every row of logits [n][count]; one CTA per row ──
 __global__ void __launch_bounds__(1024) k_argmax_rows(const float* __restrict__ x, int count, uint32_t* __restrict__ out) {
-    pdl_enter();
+    pdl_enter(x, out);
     __shared__ unsigned long long sh[32];
     const float* row = x + (size_t)blockIdx.x * count;
     unsigned long long best = 0;
@@ -343,7 +343,7 @@ void launch_argmax_rows(cudaStream_t st, const float* logits, int n, int count, 
 // advances by one, and the tokens are recorded in row `step` of the output table [steps][n].
 __global__ void k_rows_advance(uint32_t* __restrict__ tokens, const uint32_t* __restrict__ next, uint32_t* __restrict__ positions,
                                uint32_t* __restrict__ out_table, int n, int step) {
-    pdl_enter();
+    pdl_enter(tokens, next, positions, out_table);
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const uint32_t t = next[j];

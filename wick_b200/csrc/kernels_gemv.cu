@@ -72,7 +72,7 @@ __device__ __forceinline__ float gemv_chain(const DevWeight& w, int g, int lane,
 
 __global__ void __launch_bounds__(256) k_gemv(GemvJob job, const float* __restrict__ xs_g,
                                               const int8_t* __restrict__ xq_g) {
-    pdl_enter();
+    pdl_enter(xs_g, xq_g);
     extern __shared__ int smem_i[];
     const int k = job.w[0].k, nb = k / QK;
     int* xq32 = smem_i;                                   // k/4 words
@@ -144,7 +144,7 @@ constexpr int KC = 32;       // blocks per K chunk
 template <int DT>
 __global__ void __launch_bounds__(256) k_gemm(DevWeight w, const float* __restrict__ bs, const int8_t* __restrict__ bq,
                                               int n, float* __restrict__ out) {
-    pdl_enter();
+    pdl_enter(bs, bq, out);
     __shared__ __align__(16) int xt[KC * 8 * TJP];
     __shared__ __align__(16) float st[KC * TJP];
     const int k = w.k, nb = k / QK, m = w.m;

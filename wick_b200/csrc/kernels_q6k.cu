@@ -19,7 +19,7 @@ __global__ void k_repack_q6k(const uint16_t* __restrict__ raw, uint16_t* ql, uin
 }
 
 __global__ void k_embed_q6k(DevQ6K w, const uint32_t* __restrict__ tokens, const DecodeCtl* __restrict__ ctl, float* __restrict__ out) {
-    pdl_enter();
+    pdl_enter(tokens, ctl, out);
     const int j = blockIdx.x;
     uint32_t tok = tokens ? tokens[j] : ctl->token;
     if (tok >= (uint32_t)w.m) tok = 0;  // host validates ids; never index outside the table
@@ -36,7 +36,7 @@ constexpr int Q6K_WARPS = 4;     // warps per CTA
 
 __global__ void __launch_bounds__(32 * Q6K_WARPS)
 k_gemv_q6k(DevQ6K w, const float* __restrict__ xs, const int8_t* __restrict__ xq, float* __restrict__ y) {
-    pdl_enter();
+    pdl_enter(xs, xq, y);
     extern __shared__ float q6k_terms[];  // [warp][ROWS][k/16]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = w.k, units = k / 64, nsub = k / 16;
