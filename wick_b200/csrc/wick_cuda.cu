@@ -1110,8 +1110,8 @@ int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) 
 
 // One decode step for n rows: tokens in m->rows_tok, positions in m->rows_pos, per-row state pointers in m->rows_ptrs
 // (run_layers, lfm2.rs:1020-1124, for every row; the mat-vecs as batched GEMMs, bit-identical to the mat-vec per row,
-// simd.rs:1440-1623).  Leaves the logits of every row in m->logits_rows.
-int32_t enqueue_decode_rows(wick_cuda_model* m, int n) {
+// simd.rs:1440-1623).  Leaves the logits of every row in m->logits_rows.  seq_bound: no row attends more keys than this.
+int32_t enqueue_decode_rows(wick_cuda_model* m, int n, int seq_bound) {
     cudaStream_t st = m->stream;
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size, hd = m->head_dim, cap = m->batch_cap;
     const float eps = m->cfg.rms_norm_eps;
@@ -1135,7 +1135,7 @@ int32_t enqueue_decode_rows(wick_cuda_model* m, int n) {
                 launch_attention_splitk(st, m->qbuf, p0, p1, nullptr, nullptr, m->rows_pos, m->attn_out, m->splitk_scratch, n, m->cfg.n_heads, L.n_kv,
                                         hd, m->cfg.max_seq_len);
             else
-                CU_TRY(launch_attention_rows(st, m->qbuf, p0, p1, m->rows_pos, m->attn_out, n, m->cfg.n_heads, L.n_kv, hd, m->cfg.max_seq_len));
+                CU_TRY(launch_attention_rows(st, m->qbuf, p0, p1, m->rows_pos, m->attn_out, n, m->cfg.n_heads, L.n_kv, hd, seq_bound));
             launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q);
             gemms({{&L.o, &L.tc_o, m->block_out}});
         }
@@ -1166,10 +1166,12 @@ int32_t decode_rows(wick_cuda_model* m, const uint32_t* tokens_host, const uint3
     if (!tokens_host || !seq_ids_host || (!out_tokens_host && !logits_host)) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
     if (bs > MAX_BATCH_ROWS) return fail(WICK_CUDA_ERR_BAD_ARG, "batch of " + std::to_string(bs) + " rows exceeds " + std::to_string(MAX_BATCH_ROWS));
     std::vector<uint8_t> seen(m->seqs.size(), 0);
+    uint32_t longest = 0;  // cached rows of the longest sequence
     for (uint32_t j = 0; j < bs; j++) {
         W_TRY(check_seq(m, seq_ids_host[j]));
         if (seen[seq_ids_host[j]]) return fail(WICK_CUDA_ERR_BAD_ARG, "sequence " + std::to_string(seq_ids_host[j]) + " appears twice in one batch");
         seen[seq_ids_host[j]] = 1;
+        longest = std::max(longest, m->seqs[seq_ids_host[j]].seq_len);
         if (tokens_host[j] >= m->cfg.vocab_size)
             return fail(WICK_CUDA_ERR_BAD_ARG, "token_id " + std::to_string(tokens_host[j]) + " out of range (vocab_size=" + std::to_string(m->cfg.vocab_size) + ")");
         if ((uint64_t)m->seqs[seq_ids_host[j]].seq_len + n_steps > m->cfg.max_seq_len)
@@ -1202,7 +1204,7 @@ int32_t decode_rows(wick_cuda_model* m, const uint32_t* tokens_host, const uint3
     CU_TRY(cudaMemcpyAsync(m->rows_ptrs, h_ptr, nl * 2 * cap * sizeof(float*), cudaMemcpyHostToDevice, m->stream));
     const unsigned long long before = g_kernel_launches;
     for (uint32_t s_i = 0; s_i < n_steps; s_i++) {
-        W_TRY(enqueue_decode_rows(m, (int)bs));
+        W_TRY(enqueue_decode_rows(m, (int)bs, (int)(longest + n_steps)));
         if (!logits_host) {
             launch_argmax_rows(m->stream, m->logits_rows, (int)bs, (int)m->cfg.vocab_size, m->rows_next);
             launch_rows_advance(m->stream, m->rows_tok, m->rows_next, m->rows_pos, m->rows_out, (int)bs, (int)s_i);
