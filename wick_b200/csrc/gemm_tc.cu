@@ -39,14 +39,14 @@ namespace {
 constexpr int TC_BM = 128;          // weight rows per tile == TMEM lanes
 constexpr int TC_KSTAGE = 128;      // int8 elements (bytes) per row per stage == one 128B swizzle atom
 constexpr int TC_KB_PER_STAGE = TC_KSTAGE / QK;  // 4 quantisation blocks per stage
-// Shared-memory stages: as many as fit (27.6 KB each for 64-column tiles, 36.9 KB for 128).  A stage is
+// Shared-memory stages: as many as fit (27.6 KB each for 64-column tiles, 23.5 KB for 32).  A stage is
 // only refilled after the epilogue has finished with its scales, and the refill has to be back from L2 before
 // the MMA issuer needs it; with four stages that left about one microsecond, less than a loaded L2 round trip.
 template <int BN>
-__host__ __device__ constexpr int tc_stages() { return BN <= 32 ? 9 : BN <= 64 ? 8 : 6; }
-// Epilogue warps per TMEM lane quarter; each takes 1 / groups of a tile's columns
-__host__ __device__ constexpr int tc_col_groups(bool exact) { return exact ? 2 : 4; }
-__host__ __device__ constexpr int tc_threads(bool exact) { return 32 * (4 + 4 * tc_col_groups(exact)); }
+__host__ __device__ constexpr int tc_stages() { return BN <= 32 ? 9 : 8; }
+constexpr int TC_COL_GROUPS = 2;    // epilogue warps per TMEM lane quarter; each takes half of a tile's columns
+constexpr int TC_EPI_WARPS = 4 * TC_COL_GROUPS;
+constexpr int TC_THREADS = 32 * (4 + TC_EPI_WARPS);
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
 
 // Weight scales are stored times 2^72 (exact): what the exact epilogue needs, see there.
@@ -293,7 +293,7 @@ __device__ __forceinline__ TcTile tc_decode_tile(const TcJob& job, int t, int ti
 }
 
 template <int BN, bool SUMS, bool EXACT>
-__global__ void __launch_bounds__(tc_threads(EXACT), 1)
+__global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap map_x,
           const float* __restrict__ x_scales,  // [n][k/32]
           int32_t* __restrict__ sums,          // optional [n][m][k/32] (single-matrix jobs only)
@@ -302,14 +302,12 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     extern __shared__ uint8_t tc_smem_raw[];
     TcSmem<BN>* sm = reinterpret_cast<TcSmem<BN>*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int NBUF = 512 / BN;
-    constexpr int UNIT = NBUF / 2 < TC_KB_PER_STAGE ? NBUF / 2 : TC_KB_PER_STAGE;  // blocks per hand-over: two units in flight
-    // Hand-over units in flight.  The narrow exact tiles fill tensor memory with four: with two, a stage could not take less than
+    constexpr int UNIT = TC_KB_PER_STAGE;  // blocks per hand-over of tensor memory: a stage
+    // Hand-over units in flight.  32-column tiles fill tensor memory with four: with two, a stage could not take less than
     // half the way round (release, MMA issue, MMAs, wait, loads), ~860 cycles for the work of ~400.
-    constexpr int NU = EXACT ? NBUF / UNIT : 2;
-    constexpr int NB2 = NU * UNIT;
-    static_assert(TC_KB_PER_STAGE % UNIT == 0 && NBUF >= NB2 && (NU & (NU - 1)) == 0, "hand-over units that tile a stage");
+    constexpr int NU = NBUF / UNIT;
+    static_assert(NU >= 2 && (NU & (NU - 1)) == 0, "hand-over units that tile tensor memory");
     constexpr int TC_STAGES = tc_stages<BN>();
-    constexpr int TC_COL_GROUPS = tc_col_groups(EXACT), TC_EPI_WARPS = 4 * TC_COL_GROUPS, TC_THREADS = tc_threads(EXACT);
     constexpr int COLS = BN / TC_COL_GROUPS;  // columns per epilogue thread
     // EXACT: a column is (token, NEON lane group); each activation row of the operand is masked to one lane group (warp 3
     // spreads the words), so a tile covers BN/4 tokens and the MMA yields the four lane partials.  Column order inside a
@@ -326,8 +324,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         for (int s = 0; s < TC_STAGES; s++) {
             // producer (with tx bytes) + every lane of the scale warp + the exact GEMM's activation warp
             mbar_init(smem_u32(&sm->full[s]), 1 + 32 + (EXACT ? 1 : 0));
-            // MMA commit + epilogue warps; exact GEMM: the MMA issuer alone, two stages later (see there)
-            mbar_init(smem_u32(&sm->empty[s]), EXACT ? 1 : 1 + TC_EPI_WARPS);
+            mbar_init(smem_u32(&sm->empty[s]), 1);  // the MMA issuer alone, NU stages later (see there)
         }
         for (int b = 0; b < NBUF; b++) {
             mbar_init(smem_u32(&sm->tmem_full[b]), 1);
@@ -390,73 +387,36 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         // int32 results are positive: see the epilogue
         const unsigned long long d_bias = EXACT ? umma_desc_plain32(smem_u32(sm->bias)) : 0ull;
         (void)d_bias;
-        if constexpr (EXACT) {
-            // Asking a barrier costs 66 cycles even when it completed long ago: a stage's two questions go out together, and
-            // only a "not yet" is followed by a wait.
-            static_assert(UNIT == TC_KB_PER_STAGE, "one hand-over per stage");
-            const uint32_t g_total = (uint32_t)((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * (uint32_t)k_stages;
-            for (uint32_t g = 0; g < g_total; g++) {
-                const uint32_t s = g % TC_STAGES, unit = g % NU, par = ((g / NU) & 1) ^ 1;
-                const uint32_t fbar = smem_u32(&sm->full[s]), fpar = (g / TC_STAGES) & 1;
-                const uint32_t ebar = smem_u32(&sm->tmem_empty[unit]);
-                const bool pf = mbar_test(fbar, fpar), pe = mbar_test(ebar, par);
-                if (!__all_sync(0xffffffffu, pf) && !__all_sync(0xffffffffu, mbar_wait<BN, 128>(sm, fbar, fpar, err, 2))) break;
-                if (!__all_sync(0xffffffffu, pe) && !__all_sync(0xffffffffu, mbar_wait<BN, 64>(sm, ebar, par, err, 3))) break;
-                tc_fence_after();
-                const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
-                const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
-                const uint32_t d = tmem_base + unit * (UNIT * BN);
-                if (leader) {
-                    // that wait also says that the epilogue is done with the scales of the stage NU before this one
-                    if (g >= NU) mbar_arrive(smem_u32(&sm->empty[(g - NU) % TC_STAGES]));
+        // Asking a barrier costs 66 cycles even when it completed long ago: a stage's two questions go out together, and
+        // only a "not yet" is followed by a wait.
+        static_assert(UNIT == TC_KB_PER_STAGE, "one hand-over per stage");
+        const uint32_t g_total = (uint32_t)((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * (uint32_t)k_stages;
+        for (uint32_t g = 0; g < g_total; g++) {
+            const uint32_t s = g % TC_STAGES, unit = g % NU, par = ((g / NU) & 1) ^ 1;
+            const uint32_t fbar = smem_u32(&sm->full[s]), fpar = (g / TC_STAGES) & 1;
+            const uint32_t ebar = smem_u32(&sm->tmem_empty[unit]);
+            const bool pf = mbar_test(fbar, fpar), pe = mbar_test(ebar, par);
+            if (!__all_sync(0xffffffffu, pf) && !__all_sync(0xffffffffu, mbar_wait<BN, 128>(sm, fbar, fpar, err, 2))) break;
+            if (!__all_sync(0xffffffffu, pe) && !__all_sync(0xffffffffu, mbar_wait<BN, 64>(sm, ebar, par, err, 3))) break;
+            tc_fence_after();
+            const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
+            const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
+            const uint32_t d = tmem_base + unit * (UNIT * BN);
+            if (leader) {
+                // that wait also says that the epilogue is done with the scales of the stage NU before this one
+                if (g >= NU) mbar_arrive(smem_u32(&sm->empty[(g - NU) % TC_STAGES]));
+                if constexpr (EXACT) {
                     umma_i8_same_a<0>(d, d_bias, d_bias, idesc);
                     umma_i8_same_a<1>(d + BN, d_bias, d_bias, idesc);
                     umma_i8_same_a<1>(d + 2 * BN, d_bias, d_bias, idesc);
                     umma_i8_same_a<2>(d + 3 * BN, d_bias, d_bias, idesc);
-#pragma unroll
-                    for (int kk = 0; kk < UNIT; kk++)  // 32 bytes further along K inside the swizzle atom: +2 in the address field
-                        umma_i8<true>(d + kk * BN, da + kk * 2, db + kk * 2, idesc);
-                    umma_commit(smem_u32(&sm->tmem_full[unit]));
                 }
-                __syncwarp();
-            }
-        } else {
-            uint32_t g = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                for (int ks = 0; ks < k_stages && ok; ks++, g++) {
-                    const int s = g % TC_STAGES;
-                    const uint32_t u = g / TC_STAGES;
-                    ok = mbar_wait<BN, 128>(sm, smem_u32(&sm->full[s]), u & 1, err, 2);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const unsigned long long da = umma_desc_sw128(smem_u32(sm->stage[s].a));
-                    const unsigned long long db = umma_desc_sw128(smem_u32(sm->stage[s].b));
 #pragma unroll
-                    for (int h = 0; h < TC_KB_PER_STAGE / UNIT; h++) {
-                        // Buffers are handed over half of tensor memory (UNIT blocks) at a time: every hand-over
-                        // costs each epilogue warp a barrier wait and an arrival, both long dependent steps of its
-                        // loop, and that loop - not the tensor pipe - sets the pace of the kernel
-                        const uint32_t un = g * (TC_KB_PER_STAGE / UNIT) + h;
-                        ok = mbar_wait<BN, 64>(sm, smem_u32(&sm->tmem_empty[un & 1u]), ((un >> 1) & 1) ^ 1, err, 3);
-                        if (!ok) break;
-                        tc_fence_after();
-                        const uint32_t d0 = tmem_base + (un & 1u) * (UNIT * BN);
-                        if (leader) {
-#pragma unroll
-                            for (int kk = 0; kk < UNIT; kk++) {
-                                // 32 bytes further along K inside the swizzle atom: +2 in the 16-byte address field
-                                const unsigned long long off = (unsigned long long)((h * UNIT + kk) * 2);
-                                umma_i8<false>(d0 + kk * BN, da + off, db + off, idesc);
-                            }
-                            umma_commit(smem_u32(&sm->tmem_full[un & 1u]));
-                        }
-                        __syncwarp();
-                    }
-                    if (ok && leader) umma_commit(smem_u32(&sm->empty[s]));
-                    __syncwarp();
-                }
+                for (int kk = 0; kk < UNIT; kk++)  // 32 bytes further along K inside the swizzle atom: +2 in the address field
+                    umma_i8<EXACT>(d + kk * BN, da + kk * 2, db + kk * 2, idesc);
+                umma_commit(smem_u32(&sm->tmem_full[unit]));
             }
+            __syncwarp();
         }
     } else if (warp == 2) {
         // ── scale loader ─────────────────────────────────────────────────────
@@ -553,7 +513,12 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         uint32_t g = 0;
         bool ok = true;
         if constexpr (!EXACT) {
+            // One fused chain per output: per block a conversion per output and one packed product and one packed multiply-add
+            // per two.  Same hand-over as below (6144 x 2048 at 512 tokens: see launch_gemm_tc).
+            static_assert(COLS == 32, "64 tokens per tile");
             f32x2 acc[COLS / 2];
+            bool ready = false;
+            const uint32_t sw0 = smem_u32(&sm->stage[0].sw[0][row_in_tile]), sx0 = smem_u32(&sm->stage[0].sx[0][cg * COLS]);
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
                 const int m = job.m[tl.mat];
@@ -561,37 +526,24 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
 #pragma unroll
                 for (int c = 0; c < COLS / 2; c++) acc[c] = pack2(0.f, 0.f);
                 for (int ks = 0; ks < k_stages && ok; ks++, g++) {
-                    const int s = g % TC_STAGES;
-                    const uint32_t u = g / TC_STAGES;
-                    // (every lane of a warp runs the same wait on the same barrier and gets the same answer)
-                    ok = mbar_wait(sm, smem_u32(&sm->full[s]), u & 1, err, 5);
-                    if (!ok) break;
-                    const TcStage<BN>& st = sm->stage[s];
-#pragma unroll(BN == 64 && !SUMS ? TC_KB_PER_STAGE : 1)
-                    for (int kk = 0; kk < TC_KB_PER_STAGE; kk++) {
-                        const uint32_t j = g * TC_KB_PER_STAGE + kk;
-                        const uint32_t buf = j % NB2, un = j / UNIT;
-                        if (kk % UNIT == 0) {
-                            ok = mbar_wait(sm, smem_u32(&sm->tmem_full[un & 1u]), (un >> 1) & 1, err, 6);
-                            if (!ok) break;
-                            tc_fence_after();
-                        }
-                        int32_t S[COLS];
-                        tmem_ld<COLS>(lane_base + buf * BN, S);
-                        tmem_ld_wait();
-                        if (kk % UNIT == UNIT - 1) {  // the unit's blocks are all in registers or consumed
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(smem_u32(&sm->tmem_empty[un & 1u]));
-                        }
-                        const float sw = st.sw[kk][row_in_tile];
+                    const uint32_t unit = g % NU;
+                    if (!ready) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g / NU) & 1, err, 6));
+                        if (!ok) break;
+                    }
+                    tc_fence_after();
+                    const uint32_t st_off = (g % TC_STAGES) * (uint32_t)sizeof(TcStage<BN>), st_sw = sw0 + st_off, st_sx = sx0 + st_off;
+                    const uint32_t t0 = lane_base + unit * (UNIT * BN);
+                    int32_t SA[COLS], SB[COLS];
+                    auto chain = [&](const int32_t (&S)[COLS], const int kk) {
+                        const float sw = lds_f32(st_sw + kk * (TC_BM * 4));
                         const f32x2 sw2 = pack2(sw, sw);
-                        const float4* sx4 = reinterpret_cast<const float4*>(&st.sx[kk][cg * COLS]);
 #pragma unroll
                         for (int c = 0; c < COLS; c += 4) {
-                            const float4 x = sx4[c >> 2];
-                            acc[c / 2 + 0] = fma2(pack2(__int2float_rn(S[c + 0]), __int2float_rn(S[c + 1])), mul2(sw2, pack2(x.x, x.y)), acc[c / 2 + 0]);
-                            acc[c / 2 + 1] = fma2(pack2(__int2float_rn(S[c + 2]), __int2float_rn(S[c + 3])), mul2(sw2, pack2(x.z, x.w)), acc[c / 2 + 1]);
+                            f32x2 x0, x1;
+                            lds_2x64(st_sx + kk * (BN * 4) + c * 4, x0, x1);
+                            acc[c / 2 + 0] = fma2(pack2(__int2float_rn(S[c + 0]), __int2float_rn(S[c + 1])), mul2(sw2, x0), acc[c / 2 + 0]);
+                            acc[c / 2 + 1] = fma2(pack2(__int2float_rn(S[c + 2]), __int2float_rn(S[c + 3])), mul2(sw2, x1), acc[c / 2 + 1]);
                         }
                         if (SUMS && row < m) {
                             const int b = ks * TC_KB_PER_STAGE + kk;
@@ -601,10 +553,23 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                                 if (tok < n) sums[((size_t)tok * m + row) * nb + b] = S[c];
                             }
                         }
-                    }
-                    if (!ok) break;
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&sm->empty[s]));
+                    };
+                    tmem_ld<COLS>(t0, SA);
+                    tmem_ld_wait();
+                    tmem_ld<COLS>(t0 + BN, SB);
+                    chain(SA, 0);
+                    tmem_ld_wait();
+                    tmem_ld<COLS>(t0 + 2 * BN, SA);
+                    chain(SB, 1);
+                    tmem_ld_wait();
+                    tmem_ld<COLS>(t0 + 3 * BN, SB);
+                    const bool q = mbar_test(smem_u32(&sm->tmem_full[(g + 1) % NU]), ((g + 1) / NU) & 1);
+                    chain(SA, 2);
+                    tmem_ld_wait();
+                    chain(SB, 3);  // (the scales are read in here: the stage is handed back behind it)
+                    tc_fence_before();
+                    ready = __all_sync(0xffffffffu, q);
+                    if (lane == 0) mbar_arrive(smem_u32(&sm->tmem_empty[unit]));
                 }
                 if (ok && row < m) {
                     float* out = job.out[tl.mat];
@@ -836,10 +801,10 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     g_kernel_launches++;
     if constexpr (!EXACT) {
         if (sums) {
-            return launch_pdl(st, k_gemm_tc<BN, true, false>, dim3(grid), dim3(tc_threads(false)), smem, job, map_x, x_scales, sums, n, k, err);
+            return launch_pdl(st, k_gemm_tc<BN, true, false>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, sums, n, k, err);
         }
     }
-    return launch_pdl(st, k_gemm_tc<BN, false, EXACT>, dim3(grid), dim3(tc_threads(EXACT)), smem, job, map_x, x_scales, nullptr, n, k, err);
+    return launch_pdl(st, k_gemm_tc<BN, false, EXACT>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, nullptr, n, k, err);
 }
 
 cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, int count, int tiles_n) {
@@ -866,13 +831,6 @@ cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, in
 
 bool tc_gemm_supported(int m, int k) { return m > 0 && k > 0 && k % TC_KSTAGE == 0; }
 
-int tc_gemm_bn(int n, int row_tiles) {
-    // 128-token tiles halve the weight-tile traffic; 64-token tiles are used while the wider ones
-    // would leave the grid at less than two tiles per SM
-    if (n <= 64) return 64;
-    return row_tiles * ((n + 127) / 128) < 2 * 148 ? 64 : 128;
-}
-
 cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out) {
     out->m = w.m;
     out->k = w.k;
@@ -893,18 +851,14 @@ cudaError_t tc_make_activation_map(const int8_t* xq, int rows_cap, int k, int bn
     return encode_rows_map(xq, rows_cap, k, bn, out);
 }
 
-cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap* map_x,
+cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap& map_x,
                            const float* x_scales, int n, int32_t* sums, uint32_t* err) {
     if (n <= 0 || count <= 0) return cudaSuccess;
     if (count > 3 || (sums && count != 1)) return cudaErrorInvalidValue;
-    int rows = 0;
-    for (int i = 0; i < count; i++) rows += w[i]->m_pad / TC_BM;
-    const int bn = tc_gemm_bn(n, rows);
     TcJob job;
-    cudaError_t e = fill_job(job, w, out, count, (n + bn - 1) / bn);
+    cudaError_t e = fill_job(job, w, out, count, (n + TC_TENSOR_TOKENS - 1) / TC_TENSOR_TOKENS);
     if (e != cudaSuccess) return e;
-    return bn == 64 ? launch_tc<64, false>(st, job, map_x[0], x_scales, n, w[0]->k, sums, err)
-                    : launch_tc<128, false>(st, job, map_x[1], x_scales, n, w[0]->k, sums, err);
+    return launch_tc<TC_TENSOR_TOKENS, false>(st, job, map_x, x_scales, n, w[0]->k, sums, err);
 }
 
 cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,

@@ -32,8 +32,6 @@ struct TcJob {
 
 // True when the shapes meet the kernel's requirements (k a multiple of 128).
 bool tc_gemm_supported(int m, int k);
-// Tokens per tile (64 or 128) the launcher chooses for n tokens and `row_tiles` 128-row tiles.
-int tc_gemm_bn(int n, int row_tiles);
 
 // Fills `out` (q / scales_t must already point at q_bytes() / s_bytes() of device memory, zeroed by
 // this call) from the grouped layout of `w`, and encodes its tensor map.  Returns cudaSuccess or the
@@ -44,10 +42,11 @@ cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out);
 cudaError_t tc_make_activation_map(const int8_t* xq, int rows_cap, int k, int bn, CUtensorMap* out);
 
 // out[i][j][r] for matrix i < count (<= 3, equal k), token j < n, row r < m_i (token-major, like
-// launch_gemm).  map_x[0] / map_x[1]: activation maps with 64 / 128 rows per box.  sums: optional
+// launch_gemm).  map_x: activation map with TC_TENSOR_TOKENS rows per box.  sums: optional
 // [n][m][k/32] int32 block sums (count == 1 only).  err: device word that receives a non-zero code
 // if a bounded wait expired.
-cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap* map_x,
+constexpr int TC_TENSOR_TOKENS = 64;  // tokens per tile
+cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap& map_x,
                            const float* x_scales, int n, int32_t* sums, uint32_t* err);
 
 // The bit-exact variant (the arithmetic of gemm_q*_q8_0_neon, simd.rs:696-1019, in its order): every token's activations

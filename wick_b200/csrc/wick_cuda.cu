@@ -85,7 +85,7 @@ struct wick_cuda_model {
     bool tc_ok = false;     // the model's shapes allow the tensor-core GEMM
     bool tc_built = false;  // its int8 weight copies and buffers exist (made by the first call that needs them)
     int prefill_mode = WICK_CUDA_PREFILL_EXACT;
-    CUtensorMap map_x_hs[2], map_x_is[2];  // activations [max_chunk][hs | is], box of 64 / 128 rows
+    CUtensorMap map_x_hs, map_x_is;  // activations [max_chunk][hs | is] for the fused-chain GEMM
     float* normed_last = nullptr;  // output-normed hidden row of the last prefilled token
     float* rope_delta = nullptr;   // [head_dim]: cos then sin of the n_keep shift rotation
     uint32_t* tc_err = nullptr;
@@ -816,10 +816,8 @@ int32_t ensure_tc(wick_cuda_model* m) {
         W_TRY(fill(L.up, &L.tc_up));
         W_TRY(fill(L.down, &L.tc_down));
     }
-    for (int i = 0; i < 2; i++) {
-        CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, hs, i ? 128 : 64, &m->map_x_hs[i]));
-        CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, is, i ? 128 : 64, &m->map_x_is[i]));
-    }
+    CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, hs, TC_TENSOR_TOKENS, &m->map_x_hs));
+    CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, is, TC_TENSOR_TOKENS, &m->map_x_is));
     CU_TRY(cudaStreamSynchronize(m->stream));
     m->tc_built = true;
     return WICK_CUDA_OK;
@@ -2034,9 +2032,8 @@ int32_t wick_cuda_gemm_q8_tc(wick_cuda_weight* w, const float* bs_dev, const int
     if (n == 0) return WICK_CUDA_OK;
     cudaStream_t st = (cudaStream_t)stream;
     W_TRY(ensure_tc_weight(w, st));
-    CUtensorMap map_x[2];
-    CU_TRY(tc_make_activation_map(bq_dev, (int)n, w->w.k, 64, &map_x[0]));
-    CU_TRY(tc_make_activation_map(bq_dev, (int)n, w->w.k, 128, &map_x[1]));
+    CUtensorMap map_x;
+    CU_TRY(tc_make_activation_map(bq_dev, (int)n, w->w.k, TC_TENSOR_TOKENS, &map_x));
     const TcWeight* tw[1] = {&w->tc};
     float* outs[1] = {out_dev};
     CU_TRY(launch_gemm_tc(st, tw, outs, 1, map_x, bs_dev, (int)n, block_sums_dev, w->tc_err));
