@@ -232,31 +232,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, int32_t* r) {
     else if constexpr (COLS == 16) tmem_ld16(taddr, r);
     else tmem_ld32(taddr, r);
 }
-// Two f32 lanes per instruction (sm_100 packed f32x2 arithmetic), used by the fused-chain epilogue,
-// which is bound by instruction issue: each half of a packed multiply or fused multiply-add is rounded
-// like the scalar instruction.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 // Shared-memory loads by 32-bit address (a pointer derived from the aligned raw buffer is a generic one to the compiler)
 __device__ __forceinline__ float lds_f32(uint32_t a) {
     float v;

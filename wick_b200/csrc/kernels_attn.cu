@@ -208,16 +208,20 @@ __device__ __forceinline__ bool fa_wait(uint64_t* bar, uint32_t parity, volatile
     return !*abort;
 }
 
-#ifndef WICK_FA_MIN_CTAS
-#define WICK_FA_MIN_CTAS 4
-#endif
-#ifndef WICK_FA_BQ
-#define WICK_FA_BQ 1
-#endif
-template <int HD, int BQ, int MAXW>  // MAXW: the most consumer warps a launch of this instance has (4 or 8)
-__global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_FA_MIN_CTAS : 2) : 1) k_attention_flash(const float* __restrict__ q, const float* __restrict__ k_cache,
+__device__ __forceinline__ f32x2 shfl_xor2(f32x2 v, int mask) {
+    float a, b;
+    unpack2(v, a, b);
+    return pack2(__shfl_xor_sync(0xffffffffu, a, mask), __shfl_xor_sync(0xffffffffu, b, mask));
+}
+
+// Up to FLASH_MAX_CW consumer warps and one producer: 8 warps, two CTAs of them to an SM, leave 128 registers a thread, which is
+// what the blocks below need (at 4 consumer warps + 1 and four CTAs it was 96, with spills: 20.5 ms of attention in a
+// 4096-token prompt of the 1.6B model, 14.9 in one of the 350M model).
+constexpr int FLASH_MAX_CW = 7;
+template <int HD, int BQ>
+__global__ void __launch_bounds__((FLASH_MAX_CW + 1) * 32, HD <= 64 ? 2 : 1) k_attention_flash(const float* __restrict__ q, const float* __restrict__ k_cache,
                                                           const float* __restrict__ v_cache, float* __restrict__ out, int n, int start_pos,
-                                                          int n_heads, int n_kv_heads, int qb, int wave_size, uint32_t* __restrict__ err) {
+                                                          int n_heads, int n_kv_heads, int n_cw_max, int wave_size, uint32_t* __restrict__ err) {
     pdl_enter(q, k_cache, v_cache, out, err);
     constexpr int ROW = HD + 4;          // padded row, floats
     constexpr int DPL = HD / 4;          // output dims per lane
@@ -230,13 +234,15 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
     float* Qs = Vs + 2 * FLASH_TILE * ROW;                            // [consumer warps][8 * BQ][ROW]
 
     const int group = n_heads / n_kv_heads;
-    const int n_cw = group * (qb / (8 * BQ));  // consumer warps (<= MAXW)
-    // Which (KV head, query block) this CTA takes.  All CTAs of a launch are resident together, 3 or 4 to an SM, and a
-    // CTA's work grows with its query block (causal), so the launch ends when the SM with the heaviest set ends.  The
-    // items are ranked by descending work and dealt to the block indices in waves of one block per SM, forwards in
-    // even waves and backwards in odd ones: with the usual placement (blocks b, b + #SMs, b + 2 #SMs, ... on one SM)
-    // every SM then holds about the same work.  Any placement is correct; only the balance depends on it.
-    const int n_qblocks = (n + qb - 1) / qb;
+    // The work of a KV head is a list of (run of 8 * BQ queries, query head of its group) items, one per warp, n_cw_max of them to
+    // a CTA.  Which (KV head, part of the list) this CTA takes: a CTA's work grows with its place in the list (causal) and
+    // several CTAs share an SM, so the launch ends when the SM with the heaviest set ends.  The parts are ranked by
+    // descending work and dealt to the block indices in waves of one block per SM, forwards in even waves and backwards in
+    // odd ones: with the usual placement (blocks b, b + #SMs, b + 2 #SMs, ... on one SM) every SM then holds about the same
+    // work.  Any placement is correct; only the balance depends on it.
+    constexpr int QPW = 8 * BQ;
+    const int n_items = (n + QPW - 1) / QPW * group;
+    const int n_qblocks = (n_items + n_cw_max - 1) / n_cw_max;
     int kvh, qblock;
     {
         const int b = blockIdx.x, total = gridDim.x;
@@ -248,8 +254,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hs = n_heads * HD, kv_dim = n_kv_heads * HD;
-    const int j_first = qblock * qb;
-    const int j_last = min(n, j_first + qb) - 1;
+    const int item0 = qblock * n_cw_max, n_cw = min(n_cw_max, n_items - item0);
+    const int j_last = min(n, ((item0 + n_cw - 1) / group + 1) * QPW) - 1;
     const int cta_max = start_pos + j_last + 1;  // keys this CTA needs
     const int n_tiles = (cta_max + FLASH_TILE - 1) / FLASH_TILE;
 
@@ -264,7 +270,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
     }
     __syncthreads();
 
-    if (warp == n_cw) {
+    if (warp == n_cw_max) {
         // producer: tile `it` goes to buffer it & 1 once its previous user has been released by every consumer warp
         for (int it = 0; it < n_tiles; it++) {
             const int buf = it & 1;
@@ -295,7 +301,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
         }
         return;
     }
-    if (warp > n_cw) return;
+    if (warp >= n_cw) return;
 
     // A consumer warp owns QPW = 8 * BQ consecutive queries of one head.  lane = (part g = lane / 8, chain c = lane % 8).
     //   q.k: part g owns keys t = 8 (u / 2) + 2 g + (u % 2), u = 0..7, of the tile (rows two apart for neighbouring
@@ -307,11 +313,10 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
     //   query c of the pass (a + b == b + a bit for bit, so both partners hold the same sums).
     //   softmax and weighted V: lane (g, c) is "slot c, part g": it owns the scores of queries c, c + 8, ... for its part's
     //   keys and, of those queries' outputs, the 4-float pieces g, g + 4, g + 8, ... of the head.
-    constexpr int QPW = 8 * BQ;
-    const int g = warp % group, run = warp / group;
+    const int g = (item0 + warp) % group;
     const int part = lane >> 3, c = lane & 7;
     const int h = kvh * group + g;
-    const int j0 = j_first + run * QPW;
+    const int j0 = (item0 + warp) / group * QPW;
     const float scale = __fdiv_rn(1.0f, sqrtf((float)HD));
     int my_max[BQ];
 #pragma unroll
@@ -330,13 +335,13 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
         reinterpret_cast<float4*>(qw + r * ROW)[cc] = v;
     }
     __syncwarp();
-    float acc[BQ][DPL];
+    f32x2 acc[BQ][DPL / 2];  // pairs of output dims
     float running_max[BQ];
     double running_sum[BQ];
 #pragma unroll
     for (int u = 0; u < BQ; u++) {
 #pragma unroll
-        for (int d = 0; d < DPL; d++) acc[u][d] = 0.0f;
+        for (int d = 0; d < DPL / 2; d++) acc[u][d] = pack2(0.0f, 0.0f);
         running_max[u] = __int_as_float(0xFF800000);
         running_sum[u] = 0.0;
     }
@@ -360,11 +365,11 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
 #pragma unroll
             for (int pass = 0; pass < BQ; pass++) {
                 // chain c of the 8 x 8 dots of this pass
-                float d8[8][8];
+                f32x2 d8[8][4];  // [query][pair of keys]
 #pragma unroll
                 for (int j = 0; j < 8; j++)
 #pragma unroll
-                    for (int u = 0; u < 8; u++) d8[j][u] = 0.0f;
+                    for (int u = 0; u < 4; u++) d8[j][u] = pack2(0.0f, 0.0f);
                 const float* qp = qw + (pass * 8) * ROW + c;
                 const float* kp = Kt + (2 * part) * ROW + c;
 #pragma unroll 2
@@ -375,43 +380,51 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
 #pragma unroll
                     for (int u = 0; u < 8; u++) kv[u] = kp[(8 * (u >> 1) + (u & 1)) * ROW + i];
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
+                    for (int j = 0; j < 8; j++) {
+                        const f32x2 qq = pack2(qv[j], qv[j]);
 #pragma unroll
-                        for (int u = 0; u < 8; u++) d8[j][u] = __fmaf_rn(qv[j], kv[u], d8[j][u]);
+                        for (int u = 0; u < 4; u++) d8[j][u] = fma2(qq, pack2(kv[2 * u], kv[2 * u + 1]), d8[j][u]);
+                    }
                 }
                 // sum0[l] + sum1[l]: exchange with lane c ^ 4, keeping the queries whose bit 2 equals this lane's
-                float r1[4][8];
+                f32x2 r1[4][4];
                 const bool hi4 = (c & 4) != 0;
 #pragma unroll
                 for (int jj = 0; jj < 4; jj++)
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        const float mine = hi4 ? d8[jj + 4][u] : d8[jj][u];
-                        const float other = hi4 ? d8[jj][u] : d8[jj + 4][u];
-                        r1[jj][u] = __fadd_rn(mine, __shfl_xor_sync(0xffffffffu, other, 4));
+                    for (int u = 0; u < 4; u++) {
+                        const f32x2 mine = hi4 ? d8[jj + 4][u] : d8[jj][u];
+                        const f32x2 other = hi4 ? d8[jj][u] : d8[jj + 4][u];
+                        r1[jj][u] = add2(mine, shfl_xor2(other, 4));
                     }
                 // (v0 + v1), (v2 + v3): exchange with lane c ^ 1, keeping the queries whose bit 0 equals this lane's
-                float r2[2][8];
+                f32x2 r2[2][4];
                 const bool hi1 = (c & 1) != 0;
 #pragma unroll
                 for (int m = 0; m < 2; m++)
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        const float mine = hi1 ? r1[2 * m + 1][u] : r1[2 * m][u];
-                        const float other = hi1 ? r1[2 * m][u] : r1[2 * m + 1][u];
-                        r2[m][u] = __fadd_rn(mine, __shfl_xor_sync(0xffffffffu, other, 1));
+                    for (int u = 0; u < 4; u++) {
+                        const f32x2 mine = hi1 ? r1[2 * m + 1][u] : r1[2 * m][u];
+                        const f32x2 other = hi1 ? r1[2 * m][u] : r1[2 * m + 1][u];
+                        r2[m][u] = add2(mine, shfl_xor2(other, 1));
                     }
                 // (v0 + v1) + (v2 + v3): exchange with lane c ^ 2: query c of the pass remains
                 const bool hi2 = (c & 2) != 0;
                 float mx = __int_as_float(0xFF800000);
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    const float mine = hi2 ? r2[1][u] : r2[0][u];
-                    const float other = hi2 ? r2[0][u] : r2[1][u];
-                    const float sc = __fmul_rn(__fadd_rn(mine, __shfl_xor_sync(0xffffffffu, other, 2)), scale);
-                    const bool in = part_key(u) < len[pass];
-                    e[pass][u] = in ? sc : __int_as_float(0xFF800000);
-                    if (in && sc > mx) mx = sc;
+                for (int u2 = 0; u2 < 4; u2++) {
+                    const f32x2 mine = hi2 ? r2[1][u2] : r2[0][u2];
+                    const f32x2 other = hi2 ? r2[0][u2] : r2[1][u2];
+                    float s2[2];
+                    unpack2(add2(mine, shfl_xor2(other, 2)), s2[0], s2[1]);
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const int u = 2 * u2 + k;
+                        const float sc = __fmul_rn(s2[k], scale);
+                        const bool in = part_key(u) < len[pass];
+                        e[pass][u] = in ? sc : __int_as_float(0xFF800000);
+                        if (in && sc > mx) mx = sc;
+                    }
                 }
                 tmax[pass] = mx;
             }
@@ -425,7 +438,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
 #pragma unroll
                 for (int i = 0; i < 8; i++) e[u][i] = (part_key(i) < len[u]) ? ggml_expf(__fsub_rn(e[u][i], new_max[u])) : 0.0f;
 #pragma unroll
-                for (int d = 0; d < DPL; d++) acc[u][d] = __fmul_rn(acc[u][d], rescale);
+                for (int d = 0; d < DPL / 2; d++) acc[u][d] = mul2(acc[u][d], pack2(rescale, rescale));
                 if (len[u] > 0) running_sum[u] = running_sum[u] * (double)rescale;  // (+ the tile sum, below)
             }
             double tsum[BQ];
@@ -438,20 +451,19 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
 #pragma unroll
                 for (int u = 0; u < BQ; u++) p[u] = __shfl_sync(0xffffffffu, e[u][2 * (t >> 3) + (t & 1)], (((t & 7) >> 1) << 3) | c);
                 if (t < len_max) {
-                    float4 vv[DPL / 4];
-                    const float4* vp = reinterpret_cast<const float4*>(Vt + t * ROW) + part;
+                    ulonglong2 vv[DPL / 4];  // four floats as two packed pairs
+                    const ulonglong2* vp = reinterpret_cast<const ulonglong2*>(Vt + t * ROW) + part;
 #pragma unroll
                     for (int cc = 0; cc < DPL / 4; cc++) vv[cc] = vp[4 * cc];  // the four parts read 64 consecutive bytes
 #pragma unroll
                     for (int u = 0; u < BQ; u++)
                         if (t < len[u]) {
                             tsum[u] += (double)p[u];
+                            const f32x2 pp = pack2(p[u], p[u]);
 #pragma unroll
                             for (int cc = 0; cc < DPL / 4; cc++) {
-                                acc[u][4 * cc + 0] = __fmaf_rn(p[u], vv[cc].x, acc[u][4 * cc + 0]);
-                                acc[u][4 * cc + 1] = __fmaf_rn(p[u], vv[cc].y, acc[u][4 * cc + 1]);
-                                acc[u][4 * cc + 2] = __fmaf_rn(p[u], vv[cc].z, acc[u][4 * cc + 2]);
-                                acc[u][4 * cc + 3] = __fmaf_rn(p[u], vv[cc].w, acc[u][4 * cc + 3]);
+                                acc[u][2 * cc + 0] = fma2(pp, vv[cc].x, acc[u][2 * cc + 0]);
+                                acc[u][2 * cc + 1] = fma2(pp, vv[cc].y, acc[u][2 * cc + 1]);
                             }
                         }
                 }
@@ -473,9 +485,12 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MAXW == 4 ? (HD <= 64 ? WICK_
             const float inv = (float)(1.0 / running_sum[u]);
             float4* op = reinterpret_cast<float4*>(out + (size_t)j * hs + h * HD) + part;
 #pragma unroll
-            for (int cc = 0; cc < DPL / 4; cc++)
-                op[4 * cc] = make_float4(__fmul_rn(acc[u][4 * cc + 0], inv), __fmul_rn(acc[u][4 * cc + 1], inv), __fmul_rn(acc[u][4 * cc + 2], inv),
-                                     __fmul_rn(acc[u][4 * cc + 3], inv));
+            for (int cc = 0; cc < DPL / 4; cc++) {
+                float4 o;
+                unpack2(mul2(acc[u][2 * cc + 0], pack2(inv, inv)), o.x, o.y);
+                unpack2(mul2(acc[u][2 * cc + 1], pack2(inv, inv)), o.z, o.w);
+                op[4 * cc] = o;
+            }
         }
     }
 }
@@ -488,37 +503,38 @@ bool attention_flash_supported(int n_heads, int n_kv_heads, int head_dim) {
 template <int HD>
 static cudaError_t launch_flash_hd(cudaStream_t st, const float* q, const float* k_cache, const float* v_cache, float* out, int n,
                                    int start_pos, int n_heads, int n_kv_heads, uint32_t* err) {
-    constexpr int BQ = WICK_FA_BQ;
+    constexpr int BQ = 1;
     const int group = n_heads / n_kv_heads;
-    const int runs = group >= 4 ? 1 : 4 / group;  // runs of 8 * BQ queries per head and CTA: 4 consumer warps (8 when group is 5..8)
-    const int qb = runs * 8 * BQ;                 // queries per CTA
-    const int n_cw = group * runs;
-    const size_t smem = 64 + (size_t)(4 * FLASH_TILE + n_cw * 8 * BQ) * (HD + 4) * sizeof(float);
-    static size_t configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    static int sm_count[64] = {};
+    if (dev >= 0 && dev < 64 && sm_count[dev] == 0) cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+    const int wave = (dev >= 0 && dev < 64 && sm_count[dev] > 0) ? sm_count[dev] : 148;
+    // Consumer warps per CTA: the number that leaves the fewest on the fullest SM, and of equals the largest (fewer CTAs fetch
+    // the same keys).  512 queries of 32 heads: 7, 296 CTAs, 14 warps on every SM; of 16 heads: 4, at most 8 warps.
+    const int n_items = (n + 8 * BQ - 1) / (8 * BQ) * group;
+    int n_cw = FLASH_MAX_CW, grid = 0;
+    for (int w = FLASH_MAX_CW, best = 0; w >= 3; w--) {
+        const int ctas = n_kv_heads * ((n_items + w - 1) / w);
+        const int fullest = (ctas + wave - 1) / wave * w;
+        if (best == 0 || fullest < best) best = fullest, n_cw = w, grid = ctas;
+    }
+    const size_t smem = 64 + (size_t)(4 * FLASH_TILE + n_cw * 8 * BQ) * (HD + 4) * sizeof(float);
+    static size_t configured[64] = {};
     if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || configured[dev] < smem)) {
-        e = cudaFuncSetAttribute(k_attention_flash<HD, BQ, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(k_attention_flash<HD, BQ, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k_attention_flash<HD, BQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = smem;
     }
     static bool carved[64] = {};
     if (dev >= 0 && dev < 64 && !carved[dev]) {  // several CTAs per SM only fit when the SM's L1/shared split favours shared memory
-        cudaFuncSetAttribute(k_attention_flash<HD, BQ, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(k_attention_flash<HD, BQ, 8>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(k_attention_flash<HD, BQ>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         carved[dev] = true;
     }
-    static int sm_count[64] = {};
-    if (dev >= 0 && dev < 64 && sm_count[dev] == 0) cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-    const int wave = (dev >= 0 && dev < 64 && sm_count[dev] > 0) ? sm_count[dev] : 148;
-    const unsigned grid = (unsigned)(n_kv_heads * ((n + qb - 1) / qb));
     const int threads = (n_cw + 1) * 32;
     g_kernel_launches++;
-    if (n_cw <= 4) launch_pdl(st, k_attention_flash<HD, BQ, 4>, dim3(grid), dim3(threads), smem, q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, qb, wave, err);
-    else launch_pdl(st, k_attention_flash<HD, BQ, 8>, dim3(grid), dim3(threads), smem, q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, qb, wave, err);
+    launch_pdl(st, k_attention_flash<HD, BQ>, dim3((unsigned)grid), dim3(threads), smem, q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, n_cw, wave, err);
     return cudaSuccess;
 }
 
