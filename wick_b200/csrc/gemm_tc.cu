@@ -841,11 +841,15 @@ cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, floa
     if (n <= 0 || count <= 0) return cudaSuccess;
     if (count > 3) return cudaErrorInvalidValue;
     TcJob job;
-    // 8-token tiles while twice the 16-token tiles still fit one wave (few rows and a narrow matrix: the multi-sequence
-    // decode step): a tile's time is set by its K loop, so more, smaller tiles only pay when they run side by side
+    // 16-token or 8-token tiles: whichever needs less time in waves of one tile per SM.  A stage of the small tile takes 810
+    // cycles against 1430 (0.57; 64 rows x 2048 x 6912 and 512 x 6144 x 2048), so it wins where it fills a last wave that
+    // the large one would leave mostly empty: one wave instead of half of one, 3 instead of 2 (64 rows x 6144), and so on.
     int row_tiles = 0;
     for (int i = 0; i < count; i++) row_tiles += w[i]->m_pad / TC_BM;
-    const bool narrow = 2 * row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) <= 148;
+    constexpr int SMS = 148;
+    const int wide_waves = (row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) + SMS - 1) / SMS;
+    const int narrow_waves = (row_tiles * ((n + TC_EXACT_TOKENS / 2 - 1) / (TC_EXACT_TOKENS / 2)) + SMS - 1) / SMS;
+    const bool narrow = narrow_waves * 62 < wide_waves * 100;  // (close calls go to the large tile: fewer weight reads)
     const int tok = narrow ? TC_EXACT_TOKENS / 2 : TC_EXACT_TOKENS;
     cudaError_t e = fill_job(job, w, out, count, (n + tok - 1) / tok);
     if (e != cudaSuccess) return e;
