@@ -197,7 +197,7 @@ __device__ __forceinline__ Plan plan_phase(const MegaPhase& ph, int cta, int nct
     Plan p;
     p.lo = share(cta, gt, ncta);
     p.hi = share(cta + 1, gt, ncta);
-    int cap = slot_bytes / gb;
+    int cap = slot_bytes / (ph.pair == 2 ? 2 * gb : gb);
     cap = cap < 1 ? 1 : cap >= 2 * TEAM_WARPS ? 2 * TEAM_WARPS : cap >= TEAM_WARPS ? TEAM_WARPS : cap;  // whole rounds of a team's warps
     int rg = (p.hi - p.lo + NTEAMS - 1) / NTEAMS;  // spread a small phase over all teams
     rg = rg < 1 ? 1 : rg;
@@ -218,16 +218,16 @@ __device__ unsigned long long producer(const MegaParams& P, const Smem& S, int c
             const MegaPhase& ph = S.ph[pi];
             if (ph.kind == MPH_ATTN || ph.kind == MPH_SCORES) continue;
             const Plan pl = S.plan[pi];
-            // stage list: per matrix its chunks in order; a paired phase alternates the two matrices chunk by chunk
-            const int n_seq = ph.pair ? 1 : ph.n_mat, n_alt = ph.pair ? 2 : 1;
+            // stage list: per matrix its chunks in order; a paired phase alternates the two matrices chunk by chunk (pair 1) or
+            // has both matrices' chunks in one stage, one behind the other (pair 2)
+            const int n_seq = ph.pair ? 1 : ph.n_mat, n_alt = ph.pair == 1 ? 2 : 1, n_in = ph.pair == 2 ? 2 : 1;
             int off = 0;
             for (int mi = 0; mi < n_seq; mi++) {
                 const int gm = ph.mat[mi].w.groups();
                 int a = (pl.lo > off ? pl.lo : off) - off, b = (pl.hi < off + gm ? pl.hi : off + gm) - off;
                 for (int g0 = a; g0 < b; g0 += pl.rg) {
                     for (int alt = 0; alt < n_alt; alt++, cnt++, slot = slot + 1 == P.n_slots ? 0 : slot + 1, par ^= (slot == 0)) {
-                        const DevWeight& w = ph.mat[mi + alt].w;
-                        const uint32_t qgb = (uint32_t)w.q_group_bytes(), dgb = (uint32_t)w.d_group_bytes();
+                        const uint32_t qgb = (uint32_t)ph.mat[mi + alt].w.q_group_bytes(), dgb = (uint32_t)ph.mat[mi + alt].w.d_group_bytes();
                         int ng = pl.rg < b - g0 ? pl.rg : b - g0;
                         unsigned spins = 0;
                         while (!mbar_try_wait_for(&S.empty[slot], par ^ 1, WAIT_NS)) {
@@ -239,9 +239,12 @@ __device__ unsigned long long producer(const MegaParams& P, const Smem& S, int c
                             }
                         }
                         uint8_t* dst = S.ring + (size_t)slot * P.slot_bytes;
-                        mbar_expect_tx(&S.full[slot], ng * (qgb + dgb));
-                        bulk_g2s(dst, w.q + (size_t)g0 * qgb, ng * qgb, &S.full[slot], pol);
-                        bulk_g2s(dst + (size_t)ng * qgb, (const uint8_t*)w.d + (size_t)g0 * dgb, ng * dgb, &S.full[slot], pol);
+                        mbar_expect_tx(&S.full[slot], n_in * ng * (qgb + dgb));
+                        for (int k = 0; k < n_in; k++, dst += (size_t)ng * (qgb + dgb)) {
+                            const DevWeight& w = ph.mat[mi + alt + k].w;
+                            bulk_g2s(dst, w.q + (size_t)g0 * qgb, ng * qgb, &S.full[slot], pol);
+                            bulk_g2s(dst + (size_t)ng * qgb, (const uint8_t*)w.d + (size_t)g0 * dgb, ng * dgb, &S.full[slot], pol);
+                        }
                     }
                 }
                 off += gm;
@@ -1080,9 +1083,10 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
             }
             if (prof) P.prof[pi * 4 + 1] = globaltimer_ns();
             if (kind != MPH_ATTN && kind != MPH_SCORES && pair) {
-                // gate / up as alternating stages: stage pair j goes to team j % NTEAMS, which keeps both
-                // slots until it has the two sums of each row and can apply SwiGLU (n_slots is a multiple of
-                // 2 * NTEAMS, so within the phase a slot always returns to the same team)
+                // gate / up of the same rows.  pair 1: alternating stages; stage pair j goes to team j % NTEAMS, which keeps both
+                // slots until it has the two sums of each row and can apply SwiGLU (n_slots is a multiple of 2 * NTEAMS, so
+                // within the phase a slot always returns to the same team).  pair 2, where the ring has too few slots for
+                // that: both in one slot, dealt to the teams like any other stage.
                 const DevWeight& wg = ph.mat[0].w;
                 const int nb = wg.k / QK;
                 const uint32_t qgb = (uint32_t)wg.q_group_bytes();
@@ -1093,16 +1097,19 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                     const uint32_t par_a = par;
                     slot = slot + 1 == P.n_slots ? 0 : slot + 1;
                     par ^= (slot == 0);
-                    const int slot_b = slot;
+                    int slot_b = slot_a;
                     const uint32_t par_b = par;
-                    slot = slot + 1 == P.n_slots ? 0 : slot + 1;
-                    par ^= (slot == 0);
-                    if (pj % NTEAMS != team) continue;
+                    if (pair == 1) {
+                        slot_b = slot;
+                        slot = slot + 1 == P.n_slots ? 0 : slot + 1;
+                        par ^= (slot == 0);
+                    }
+                    if ((pair == 1 ? pj : slot_a) % NTEAMS != team) continue;
                     const int ng = pl.rg < pl.hi - g0 ? pl.rg : pl.hi - g0;
                     const uint8_t* base_a = S.ring + (size_t)slot_a * P.slot_bytes;
-                    const uint8_t* base_b = S.ring + (size_t)slot_b * P.slot_bytes;
+                    const uint8_t* base_b = pair == 1 ? S.ring + (size_t)slot_b * P.slot_bytes : base_a + (size_t)ng * (qgb + nb * 8);
 #pragma unroll 1
-                    for (int half = 0; half < 2; half++) {
+                    for (int half = 0; half < (pair == 1 ? 2 : 1); half++) {
                         unsigned spins = 0;
                         while (!mbar_try_wait_for(&S.full[half ? slot_b : slot_a], half ? par_b : par_a, WAIT_NS) && !*S.abort) {
                             if (++spins > SPIN_LIMIT) {
@@ -1127,7 +1134,7 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                     team_sync(team);
                     if (tt == 0) {
                         mbar_arrive(&S.empty[slot_a]);
-                        mbar_arrive(&S.empty[slot_b]);
+                        if (pair == 1) mbar_arrive(&S.empty[slot_b]);
                     }
                 }
             } else if (kind != MPH_ATTN && kind != MPH_SCORES) {

@@ -44,8 +44,8 @@ struct MegaPhase {
     int layer;          // conv / attention layer this phase belongs to (or -1)
     int embed;          // MPH_NORM: 1 = first phase of a token
     int conv_commit;    // MPH_NORM: layer whose conv state is advanced in this prologue, or -1
-    int pair;           // 1: mat[0] / mat[1] are gate / up of equal shape, streamed as alternating stages and
-                        //    combined row by row in the epilogue (MEP_SWIGLU)
+    int pair;           // mat[0] / mat[1] are gate / up of equal shape, combined row by row in the epilogue (MEP_SWIGLU);
+                        //    1: streamed as alternating stages, 2: both in one stage
     int flag_in;        // MPH_NORM: the hidden row is taken from the flagged copy the previous phase wrote, element by
                         //    element as it arrives; no grid barrier in front of this phase
     int flag_out;       // MEP_ADD phase in front of a flag_in phase: rows are also written as (phase id, value) words

@@ -404,8 +404,13 @@ int32_t build_mega(wick_cuda_model* m) {
     P.n_slots = (int)(((size_t)max_smem - fixed - 64 * 4) / ((size_t)P.slot_bytes + 16));
     if (P.n_slots > 30) P.n_slots = 30;
     P.n_slots -= P.n_slots % MEGA_TEAMS;  // each slot is always served by the same consumer team
-    if (P.n_slots % (2 * MEGA_TEAMS))       // paired (gate/up) phases need whole pairs per ring lap
-        for (auto& q : ph) if (q.pair) { q.pair = 0; q.mat[0].epi = q.mat[1].epi = MEP_STORE; }
+    if (P.n_slots % (2 * MEGA_TEAMS))  // paired (gate/up) phases need whole pairs per ring lap, or both halves in one slot
+        for (auto& q : ph)
+            if (q.pair) {
+                const bool one_slot = 2 * (q.mat[0].w.q_group_bytes() + q.mat[0].w.d_group_bytes()) <= (size_t)P.slot_bytes;
+                q.pair = one_slot ? 2 : 0;
+                if (!one_slot) q.mat[0].epi = q.mat[1].epi = MEP_STORE;
+            }
     for (size_t i = 0; i + 1 < ph.size(); i++)
         if (ph[i].kind == MPH_NORM && ph[i].n_mat == 2 && !ph[i].pair && ph[i + 1].kind == MPH_QUANT && ph[i + 1].src == m->gate) ph[i + 1].kind = MPH_SILU;
     // A residual-add phase followed by an RMSNorm phase hands the hidden row over through flagged words instead of
