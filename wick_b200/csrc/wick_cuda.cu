@@ -64,7 +64,7 @@ struct wick_cuda_weight {
     // int8 copy for the tensor-core GEMMs, made by the first call that uses them; the lock is for that call only
     mutable std::mutex tc_lock;
     mutable TcWeight tc;
-    mutable uint32_t* tc_err = nullptr;  // pinned host word the kernels write on an expired wait, so that reading it needs no copy
+    mutable uint32_t* tc_err = nullptr;  // host word (TcErrorWords) the kernels write on an expired wait: reading it needs no copy
 };
 
 struct wick_cuda_model {
@@ -1938,13 +1938,13 @@ int32_t wick_cuda_weight_create(int32_t dtype, const uint8_t* raw_host, uint32_t
     return WICK_CUDA_OK;
 }
 
+static void release_tc_error_word(uint32_t* word);
 void wick_cuda_weight_destroy(wick_cuda_weight* w) {
     if (!w) return;
     cudaFree((void*)w->w.q);
     cudaFree((void*)w->w.d);
     cudaFree(w->tc.q);
-    cudaFree(w->tc.scales_t);
-    if (w->tc_err) cudaFreeHost(w->tc_err);
+    release_tc_error_word(w->tc_err);  // (cudaFree has waited for the weight's kernels)
     delete w;
 }
 
@@ -1971,6 +1971,44 @@ int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const 
     OP_END();
 }
 
+// Host words that kernels of operator-API weights report expired waits in: one pinned page for the process, handed out word by
+// word (pinning memory takes about 2 ms, which every weight paid for on its first product).  Weights beyond the page share its
+// first word: a report then names the wait but not the weight.
+class TcErrorWords {
+    static constexpr uint32_t N = 1024;
+    std::mutex lock;
+    uint32_t* page = nullptr;
+    std::vector<uint32_t*> unused;
+
+public:
+    cudaError_t take(uint32_t** out) {
+        std::lock_guard<std::mutex> hold(lock);
+        if (!page) {
+            cudaError_t e = cudaHostAlloc((void**)&page, N * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable);
+            if (e != cudaSuccess) return e;
+            memset(page, 0, N * sizeof(uint32_t));
+            for (uint32_t i = N - 1; i > 0; i--) unused.push_back(page + i);
+        }
+        *out = page;
+        if (!unused.empty()) {
+            *out = unused.back();
+            unused.pop_back();
+        }
+        return cudaSuccess;
+    }
+    void give_back(uint32_t* w) {
+        std::lock_guard<std::mutex> hold(lock);
+        if (w && w != page) *w = 0, unused.push_back(w);
+    }
+};
+static TcErrorWords g_tc_error_words;
+static void release_tc_error_word(uint32_t* word) { g_tc_error_words.give_back(word); }
+
+static bool has_tc_weight(const wick_cuda_weight* w) {
+    std::lock_guard<std::mutex> hold(w->tc_lock);
+    return w->tc_err != nullptr;
+}
+
 // The int8 copy of an operator-API weight, made on first use (and finished before the call goes on: later calls may come
 // on other streams).
 static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
@@ -1981,18 +2019,15 @@ static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
     t.k = w->w.k;
     t.m_pad = (w->w.m + 127) / 128 * 128;
     uint32_t* err = nullptr;
-    cudaError_t e = cudaMalloc((void**)&t.q, t.q_bytes());
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t.scales_t, t.s_bytes());
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&err, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable);
+    cudaError_t e = cudaMalloc((void**)&t.q, t.q_bytes() + t.s_bytes());  // (q_bytes is a multiple of 128 * 128)
     if (e == cudaSuccess) {
-        *err = 0;
+        t.scales_t = reinterpret_cast<float*>(t.q + t.q_bytes());
         e = tc_weight_fill(st, w->w, &t);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = g_tc_error_words.take(&err);
     if (e != cudaSuccess) {
         cudaFree(t.q);
-        cudaFree(t.scales_t);
-        if (err) cudaFreeHost(err);
         CU_TRY(e);
     }
     w->tc = t;
@@ -2017,7 +2052,7 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
         cudaStream_t st = (cudaStream_t)stream;
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CU_TRY(cudaStreamIsCapturing(st, &capturing));
-        if (w->tc_err || capturing == cudaStreamCaptureStatusNone) {  // (making the copy allocates and synchronises)
+        if (capturing == cudaStreamCaptureStatusNone || has_tc_weight(w)) {  // (making the copy allocates and synchronises)
             W_TRY(ensure_tc_weight(w, st));
             W_TRY(take_tc_error(w));
             const TcWeight* tw[1] = {&w->tc};
