@@ -750,6 +750,63 @@ __device__ void phase_scores(Ctx& c, const MegaPhase& ph, int pos) {
 // item recomputes its head's scores and softmax (cheap), then the slice's weighted V sum: the
 // needed V columns are first gathered into shared memory by all threads (one memory latency per
 // chunk), and 16 threads run the fused chains in ascending t, the reference's order.
+//
+// Long contexts: the chain (16 or 8 dependent-FMA lanes over thousands of keys) is what takes the time, so the V columns come
+// in two halves of the staging area, the 14 other warps refilling one while warp 0 works on the other, and the chain's
+// operands are loaded a batch ahead.  Where 16-wide slices leave half of the CTAs without an item, slices are 8 wide: half
+// the bytes to gather per item.  (350M, 4200 keys: 40 us per layer with gather and chain in turn.)
+__device__ __forceinline__ void chain_load8(const float* scp, const float* vp, int sl, float (&s)[8], float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(scp), b = *reinterpret_cast<const float4*>(scp + 4);
+    s[0] = a.x, s[1] = a.y, s[2] = a.z, s[3] = a.w, s[4] = b.x, s[5] = b.y, s[6] = b.z, s[7] = b.w;
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = vp[i * sl];
+}
+__device__ __forceinline__ void long_values_fetch(const Ctx& c, const float* v_cache, const float* v_new, int kv_dim, int pos, int t0, int rows, int sl,
+                                                  float* dst, int first_thread) {
+    const int sh = sl == 16 ? 2 : 1, pc = sl >> 2;  // 16-byte pieces per row
+    for (int i = c.ct - first_thread; i < rows * pc; i += NCT - first_thread) {
+        const int t = t0 + (i >> sh), q = (i & (pc - 1)) * 4;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + i * 4)), "l"(t < pos ? v_cache + (size_t)t * kv_dim + q : v_new + q)
+                     : "memory");
+    }
+}
+// The weighted sum over seq rows for the item's sl output dims; the first two chunks are on their way (one commit group each).
+__device__ __forceinline__ float long_values(Ctx& c, const float* sc, float* Vs, int half_rows, const float* v_cache, const float* v_new, int kv_dim, int pos,
+                                             int sl) {
+    const int seq = pos + 1, n_chunks = (seq + half_rows - 1) / half_rows;
+    float acc = 0.0f;
+    for (int k = 0; k < n_chunks; k++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // this thread's copies of chunk k
+        consumer_sync();
+        const int t0 = k * half_rows, rows = half_rows < seq - t0 ? half_rows : seq - t0;
+        float* V = Vs + (k & 1) * half_rows * sl;
+        if (c.ct < sl) {
+            const float* scp = sc + t0;
+            const float* vp = V + c.ct;
+            int t = 0;
+            if (rows >= 16) {
+                float s0[8], v0[8], s1[8], v1[8];
+                chain_load8(scp, vp, sl, s0, v0);
+                for (; t + 16 <= rows; t += 16) {
+                    chain_load8(scp + t + 8, vp + (t + 8) * sl, sl, s1, v1);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) acc = __fmaf_rn(s0[i], v0[i], acc);
+                    const int nx = t + 24 <= rows ? t + 16 : t;  // (not used otherwise)
+                    chain_load8(scp + nx, vp + nx * sl, sl, s0, v0);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) acc = __fmaf_rn(s1[i], v1[i], acc);
+                }
+            }
+            for (; t < rows; t++) acc = __fmaf_rn(scp[t], vp[t * sl], acc);
+        }
+        consumer_sync();  // chunk consumed
+        const int t2 = (k + 2) * half_rows;
+        if (t2 < seq && c.cw > 0) long_values_fetch(c, v_cache, v_new, kv_dim, pos, t2, half_rows < seq - t2 ? half_rows : seq - t2, sl, V, 32);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    return acc;
+}
+
 template <bool LONG>
 __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
     const MegaParams& P = c.P;
@@ -761,7 +818,8 @@ __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
     float* sc = c.S.xf;
     float *qs = c.S.head, *ks = c.S.head + 256;
     const int seq = pos + 1;
-    const int nq = hd / 16, items = n_heads * nq;
+    const int sl = LONG && 2 * n_heads * (hd / 16) <= c.ncta ? 8 : 16;  // output dims per item
+    const int nq = hd / sl, items = n_heads * nq;
     const int nf = xf_floats(P);
     const int sc_pad = (seq + 3) & ~3;
     float* Vs = sc + sc_pad;                 // [rows][16]
@@ -771,11 +829,20 @@ __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
     const int it0 = (int)(((unsigned)c.cta * items + c.ncta - 1) / c.ncta);
     const int it1 = (int)(((unsigned)(c.cta + 1) * items + c.ncta - 1) / c.ncta);
     for (int it = it0; it < it1 && it < items; it++) {
-        const int h = it / nq, d0 = (it % nq) * 16;
+        const int h = it / nq, d0 = (it % nq) * sl;
         const int kvh = h / group, off = kvh * hd;
         STAMP(c, 0);
         consumer_sync();
-        {   // The V columns of the first chunk do not depend on the scores: they are fetched now with asynchronous
+        const int half_rows = ((nf - sc_pad) / (2 * sl)) & ~3;
+        if (LONG) {
+            for (int k = 0; k < 2; k++) {
+                const int t0 = k * half_rows;
+                if (t0 < seq)
+                    long_values_fetch(c, L.v_cache + off + d0, P.vbuf + off + d0, kv_dim, pos, t0, half_rows < seq - t0 ? half_rows : seq - t0, sl,
+                                      Vs + k * half_rows * sl, 0);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+        } else {   // The V columns of the first chunk do not depend on the scores: they are fetched now with asynchronous
             // global -> shared copies (no registers held) and land while the scores and the softmax are computed.
             const int rows = chunk < seq ? chunk : seq;
             for (int i = c.ct; i < rows * 4; i += NCT) {
@@ -883,7 +950,8 @@ __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
         STAMP(c, 5);
         // attn_values (cpu.rs:1463-1509): one fused chain per output dim, ascending t
         float acc = 0.0f;
-        for (int t0 = 0; t0 < seq; t0 += chunk) {
+        if (LONG) acc = long_values(c, sc, Vs, half_rows, L.v_cache + off + d0, P.vbuf + off + d0, kv_dim, pos, sl);
+        for (int t0 = 0; t0 < seq && !LONG; t0 += chunk) {
             const int rows = chunk < seq - t0 ? chunk : seq - t0;
             consumer_sync();  // scores normalised / previous chunk consumed
             if (t0 == 0) STAMP(c, 8);
@@ -929,7 +997,7 @@ __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
             if (t0 == 0) STAMP(c, 10);
         }
         STAMP(c, 6);
-        if (c.ct < 16) P.attn_out[h * hd + d0 + c.ct] = acc;
+        if (c.ct < sl) P.attn_out[h * hd + d0 + c.ct] = acc;
     }
     STAMP(c, 7);
 }
