@@ -511,7 +511,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     const uint32_t t0 = lane_base + unit * (UNIT * BN);
                     int32_t SA[COLS], SB[COLS];
                     auto chain = [&](const int32_t (&S)[COLS], const int kk) {
-                        const float sw = lds_f32(st_sw + kk * (TC_BM * 4));
+                        const float sw = lds_f32(st_sw + kk * (TC_BM * 4)) * TC_SCALE_DOWN;
                         const f32x2 sw2 = pack2(sw, sw);
 #pragma unroll
                         for (int c = 0; c < COLS; c += 4) {
@@ -553,8 +553,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                         const int tok = tl.n0 + cg * COLS + c;
                         float a0, a1;
                         unpack2(acc[c / 2], a0, a1);
-                        if (tok < n) out[(size_t)tok * m + row] = a0 * TC_SCALE_DOWN;
-                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = a1 * TC_SCALE_DOWN;
+                        if (tok < n) out[(size_t)tok * m + row] = a0;
+                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = a1;
                     }
                 }
             }
