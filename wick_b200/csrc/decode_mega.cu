@@ -361,11 +361,6 @@ __device__ __forceinline__ float embed_elem(const DevWeight& w, uint32_t tok, in
     return __fmul_rn((float)v, d);
 }
 
-// b * x of channel ch from the in_proj output (lfm2.rs:691-695)
-__device__ __forceinline__ float conv_bx(const float* proj, int hs, int ch) {
-    return __fmul_rn(__ldcg(proj + ch), __ldcg(proj + 2 * hs + ch));
-}
-
 // Norm weights of the thread's elements; static data, fetched BEFORE the dependency wait.
 __device__ __forceinline__ void load_norm_w(const Ctx& c, const MegaPhase& ph, float (&w)[MAXJ]) {
     const int nb = ph.k / QK;
@@ -403,19 +398,6 @@ __device__ __forceinline__ float ldcg_if(bool in, const float* p) { return in ? 
 __device__ void prologue_norm(Ctx& c, const MegaPhase& ph, uint32_t token, const float (&w)[MAXJ], uint32_t id_in) {
     const MegaParams& P = c.P;
     const int k = ph.k, nb = k / QK;
-    // Conv state of the layer whose gating ran one phase ago (lfm2.rs:691-695).  The values are fetched now; the
-    // rolling buffer is overwritten further down, once every CTA is known to have finished reading the old one.
-    const MegaLayer* CL = ph.conv_commit >= 0 ? &c.S.layers[ph.conv_commit] : nullptr;
-    const int dc = P.conv_ks - 1, hs = P.hs;
-    const int cc0 = CL ? share(c.cta, hs, c.ncta) : 0, cc1 = CL ? share(c.cta + 1, hs, c.ncta) : 0;
-    float cst[3] = {0.0f, 0.0f, 0.0f};  // conv_ks <= 4
-    if (cc0 + c.ct < cc1) {
-        const int ch = cc0 + c.ct;
-#pragma unroll
-        for (int kk = 0; kk < 2; kk++)
-            if (kk + 1 < dc) cst[kk] = __ldcg(CL->conv_state + (size_t)(kk + 1) * hs + ch);
-        cst[2] = conv_bx(P.proj, hs, ch);
-    }
     STAMP(c, 0);
     float v[MAXJ];
     const int e0 = ph.embed ? share(c.cta, k, c.ncta) : 0, e1 = ph.embed ? share(c.cta + 1, k, c.ncta) : 0;
@@ -482,22 +464,6 @@ __device__ void prologue_norm(Ctx& c, const MegaPhase& ph, uint32_t token, const
     if (c.lane == 0) c.S.red[c.cw] = s;
     consumer_sync();
     STAMP(c, 2);
-    if (CL) {
-        // every CTA has passed the gating prologue that read the old buffer: either a grid barrier lies in between,
-        // or (flag_in) all rows of the mat-vec that followed that prologue have been seen by this CTA
-        for (int ch = cc0 + c.ct; ch < cc1; ch += NCT) {
-            if (ch != cc0 + c.ct) {  // rows beyond the first of this thread (hidden sizes above 480 x CTAs)
-#pragma unroll
-                for (int kk = 0; kk < 2; kk++)
-                    if (kk + 1 < dc) cst[kk] = __ldcg(CL->conv_state + (size_t)(kk + 1) * hs + ch);
-                cst[2] = conv_bx(P.proj, hs, ch);
-            }
-#pragma unroll
-            for (int kk = 0; kk < 2; kk++)
-                if (kk + 1 < dc) CL->conv_state[(size_t)kk * hs + ch] = cst[kk];
-            if (dc > 0) CL->conv_state[(size_t)(dc - 1) * hs + ch] = cst[2];
-        }
-    }
     const double tot = sum_warp_partials(c.S.red);
     // (for a power-of-two length the division is an exact scaling, as is the multiplication by its reciprocal)
     const double mean = (k & (k - 1)) == 0 ? tot * (1.0 / (double)k) : tot / (double)k;
@@ -518,10 +484,15 @@ __device__ void prologue_norm(Ctx& c, const MegaPhase& ph, uint32_t token, const
     STAMP(c, 5);
 }
 
-__device__ void prologue_conv(Ctx& c, const MegaPhase& ph) {
+// Every CTA reads the whole rolling buffer here and the owner of a channel writes its next state (lfm2.rs:691-695) to the OTHER of
+// the layer's two buffers, which the next token reads: the values are in registers, and nobody waits for anybody.  (With one
+// buffer the update had to wait for the next phase, whose prologue it held up for a microsecond, 10 times per token.)
+__device__ void prologue_conv(Ctx& c, const MegaPhase& ph, int odd) {
     const MegaParams& P = c.P;
     const MegaLayer& L = c.S.layers[ph.layer];
     const int hs = P.hs, ks = P.conv_ks, dc = ks - 1, nb = hs / QK;
+    const float* const cur = odd ? L.conv_alt : L.conv_state;
+    float* const nxt = odd ? L.conv_state : L.conv_alt;
     constexpr int MAXKS = 4;  // kernel sizes up to 4 (LFM2 uses 3); larger ones take the per-kernel path
     // five blocks per warp and pass: hidden sizes up to 2400 are done in one pass (one memory round trip)
     constexpr int CJ = FASTJ;
@@ -536,11 +507,12 @@ __device__ void prologue_conv(Ctx& c, const MegaPhase& ph) {
             pc[j] = ldcg_if(in, P.proj + hs + chs);
             px[j] = ldcg_if(in, P.proj + 2 * hs + chs);
 #pragma unroll
-            for (int kk = 0; kk < MAXKS - 1; kk++) st[j][kk] = ldcg_if(in && kk < dc, L.conv_state + (size_t)kk * hs + chs);
+            for (int kk = 0; kk < MAXKS - 1; kk++) st[j][kk] = ldcg_if(in && kk < dc, cur + (size_t)kk * hs + chs);
 #pragma unroll
             for (int kk = 0; kk < MAXKS; kk++) cw[j][kk] = in && kk < ks ? __ldg(L.conv_w + chs * ks + kk) : 0.0f;
         }
         float o[CJ];
+        const int ch0 = share(c.cta, hs, c.ncta), ch1 = share(c.cta + 1, hs, c.ncta);  // channels this CTA keeps
 #pragma unroll
         for (int j = 0; j < CJ; j++) {
             float sum = 0.0f;
@@ -553,6 +525,12 @@ __device__ void prologue_conv(Ctx& c, const MegaPhase& ph) {
             for (int kk = 1; kk < MAXKS; kk++) wl = kk == dc ? cw[j][kk] : wl;
             sum = __fadd_rn(sum, __fmul_rn(bx, wl));
             o[j] = __fmul_rn(pc[j], sum);
+            const int ch = (c.cw + (j0 + j) * NC) * QK + c.lane;
+            if (ch >= ch0 && ch < ch1) {
+#pragma unroll
+                for (int kk = 0; kk < MAXKS - 1; kk++)
+                    if (kk < dc) nxt[(size_t)kk * hs + ch] = kk + 1 < dc ? st[j][kk + 1 < MAXKS - 1 ? kk + 1 : kk] : bx;
+            }
         }
         quantize_blocks<CJ>(c, o, j0, nb);
     }
@@ -1141,7 +1119,7 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
             if (pi == 1 && cta == 0 && c.ct == 0) P.argmax_acc[(t + 1) & 1] = 0;  // free for the next step
             switch (kind) {
                 case MPH_NORM: prologue_norm(c, ph, token, nw, phase_id(P, t, pi - 1)); break;
-                case MPH_CONV: prologue_conv(c, ph); break;
+                case MPH_CONV: prologue_conv(c, ph, t & 1); break;
                 case MPH_SILU: prologue_silu(c, ph); break;
                 case MPH_QUANT: prologue_quant(c, ph); break;
                 case MPH_SCORES:
@@ -1332,6 +1310,16 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                 owed = 0;
             }
             if (prof) P.prof[pi * 4 + 3] = globaltimer_ns();
+        }
+    }
+    // after an odd number of steps the conv buffers' current state is in the second set: this CTA's share goes back (every CTA
+    // read it some phases ago, and only this one wrote it)
+    if (P.n_tokens & 1) {
+        const int dc = P.conv_ks - 1, ch0 = share(cta, P.hs, ncta), nch = share(cta + 1, P.hs, ncta) - ch0, per_layer = dc * nch;
+#pragma unroll 1
+        for (int i = c.ct; i < P.n_layers * per_layer; i += NCT) {
+            const int l = i / per_layer, r = i - l * per_layer, at = r / nch * P.hs + ch0 + r % nch;
+            if (S.layers[l].conv_state) S.layers[l].conv_state[at] = __ldcg(S.layers[l].conv_alt + at);
         }
     }
     // last step's result and the control block

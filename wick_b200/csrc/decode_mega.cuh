@@ -43,7 +43,6 @@ struct MegaPhase {
     int k;              // input length
     int layer;          // conv / attention layer this phase belongs to (or -1)
     int embed;          // MPH_NORM: 1 = first phase of a token
-    int conv_commit;    // MPH_NORM: layer whose conv state is advanced in this prologue, or -1
     int pair;           // mat[0] / mat[1] are gate / up of equal shape, combined row by row in the epilogue (MEP_SWIGLU);
                         //    1: streamed as alternating stages, 2: both in one stage
     int flag_in;        // MPH_NORM: the hidden row is taken from the flagged copy the previous phase wrote, element by
@@ -57,7 +56,8 @@ struct MegaPhase {
 
 struct MegaLayer {
     const float* conv_w;
-    float* conv_state;
+    float* conv_state;  // current state before the launch's first step; every step reads one of the two and writes the other
+    float* conv_alt;
     const float* q_norm;
     const float* k_norm;
     float* k_cache;

@@ -292,6 +292,8 @@ void fill_rope_table(int n_pos, int hd, float base, std::vector<float>& c, std::
     }
 }
 
+size_t conv_state_floats(const wick_cuda_model* m);
+
 // Phase list of one decode step for the persistent kernel (see decode_mega.cu).
 int32_t build_mega(wick_cuda_model* m) {
     const char* env = getenv("WICK_CUDA_DECODE");
@@ -303,6 +305,8 @@ int32_t build_mega(wick_cuda_model* m) {
     const int hs = c.hidden_size, is = c.intermediate_size;
     std::vector<MegaPhase> ph;
     std::vector<MegaLayer> ml(c.n_layers);
+    float* conv_alt = nullptr;
+    W_TRY(dev_alloc(m, &conv_alt, conv_state_floats(m)));
     size_t max_group = 0;
     bool ok = true;
     auto mat = [&](const DevWeight& w, float* y, int epi) {
@@ -314,22 +318,22 @@ int32_t build_mega(wick_cuda_model* m) {
         max_group = std::max(max_group, w.q_group_bytes() + w.d_group_bytes());
         return mm;
     };
-    int pending_commit = -1;
     for (uint32_t i = 0; i < c.n_layers; i++) {
         Layer& L = m->layers[i];
         MegaLayer& M = ml[i];
-        M.conv_w = L.conv_w; M.conv_state = L.conv_state; M.q_norm = L.q_norm; M.k_norm = L.k_norm;
+        M.conv_w = L.conv_w; M.conv_state = L.conv_state; M.conv_alt = nullptr; M.q_norm = L.q_norm; M.k_norm = L.k_norm;
         M.k_cache = L.k_cache; M.v_cache = L.v_cache; M.n_kv = L.n_kv;
         MegaPhase a{};
-        a.kind = MPH_NORM; a.k = hs; a.layer = (int)i; a.embed = i == 0; a.conv_commit = -1; a.norm_w = L.attn_norm;
+        a.kind = MPH_NORM; a.k = hs; a.layer = (int)i; a.embed = i == 0; a.norm_w = L.attn_norm;
         if (!L.is_attn) {
             a.n_mat = 1; a.mat[0] = mat(L.in_proj, m->proj, MEP_STORE);
             ph.push_back(a);
             MegaPhase b{};
-            b.kind = MPH_CONV; b.k = hs; b.layer = (int)i; b.conv_commit = -1; b.n_mat = 1;
+            b.kind = MPH_CONV; b.k = hs; b.layer = (int)i; b.n_mat = 1;
             b.mat[0] = mat(L.out_proj, m->hidden, MEP_ADD);
             ph.push_back(b);
-            pending_commit = (int)i;
+            M.conv_alt = conv_alt;
+            conv_alt += (size_t)std::max((int)c.conv_kernel_size - 1, 1) * hs;
         } else {
             a.n_mat = 3;
             a.mat[0] = mat(L.q, m->qbuf, MEP_STORE);
@@ -337,16 +341,15 @@ int32_t build_mega(wick_cuda_model* m) {
             a.mat[2] = mat(L.v, m->vbuf, MEP_STORE);
             ph.push_back(a);
             MegaPhase at{};
-            at.kind = MPH_ATTN; at.layer = (int)i; at.conv_commit = -1; at.k = hs;
+            at.kind = MPH_ATTN; at.layer = (int)i; at.k = hs;
             ph.push_back(at);
             MegaPhase o{};
-            o.kind = MPH_QUANT; o.src = m->attn_out; o.k = hs; o.layer = (int)i; o.conv_commit = -1; o.n_mat = 1;
+            o.kind = MPH_QUANT; o.src = m->attn_out; o.k = hs; o.layer = (int)i; o.n_mat = 1;
             o.mat[0] = mat(L.o, m->hidden, MEP_ADD);
             ph.push_back(o);
         }
         MegaPhase f{};
-        f.kind = MPH_NORM; f.k = hs; f.layer = (int)i; f.conv_commit = pending_commit; f.norm_w = L.ffn_norm; f.n_mat = 2;
-        pending_commit = -1;
+        f.kind = MPH_NORM; f.k = hs; f.layer = (int)i; f.norm_w = L.ffn_norm; f.n_mat = 2;
         // gate and up of equal shape and type are streamed as alternating stages and SwiGLU is applied
         // by the thread that holds both sums of a row; `gate` then holds silu(gate) * up
         const bool fuse = L.gate.m == L.up.m && L.gate.k == L.up.k && L.gate.dtype == L.up.dtype;
@@ -355,13 +358,13 @@ int32_t build_mega(wick_cuda_model* m) {
         f.mat[1] = mat(L.up, m->up, fuse ? MEP_SWIGLU : MEP_STORE);
         ph.push_back(f);
         MegaPhase d{};
-        d.kind = fuse ? MPH_QUANT : MPH_SILU; d.src = m->gate; d.k = is; d.layer = (int)i; d.conv_commit = -1; d.n_mat = 1;
+        d.kind = fuse ? MPH_QUANT : MPH_SILU; d.src = m->gate; d.k = is; d.layer = (int)i; d.n_mat = 1;
         d.mat[0] = mat(L.down, m->hidden, MEP_ADD);
         ph.push_back(d);
     }
     if (!m->embd_q6k) {
         MegaPhase v{};
-        v.kind = MPH_NORM; v.k = hs; v.layer = -1; v.conv_commit = -1; v.norm_w = m->output_norm; v.n_mat = 1;
+        v.kind = MPH_NORM; v.k = hs; v.layer = -1; v.norm_w = m->output_norm; v.n_mat = 1;
         v.mat[0] = mat(m->embd, m->logits, MEP_LOGITS);
         ph.push_back(v);
     }  // a Q6_K vocabulary matrix is not streamed by the persistent kernel: see run_mega
