@@ -1087,7 +1087,7 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
     uint32_t par = 0;
     const int team = c.cw / TEAM_WARPS, tw = c.cw % TEAM_WARPS, tt = tw * 32 + c.lane;
     const uint32_t pos0 = __ldcg(&P.ctl->pos), step0 = __ldcg(&P.ctl->step);
-    uint32_t token = P.first_token == MEGA_TOKEN_FROM_CTL ? __ldcg(&P.ctl->token) : P.first_token;
+    uint32_t token = __ldcg(&P.ctl->token);
     unsigned owed = 0;  // arrivals of flag_out phases not yet added to the barrier counter
     // this lane's chain: parity, lane group, row; its place among a step's weight words and scales, input words and scales
     const int cp = c.lane >> 4, cl = (c.lane >> 2) & 3, cr = c.lane & 3;

@@ -12,8 +12,6 @@ constexpr int MEGA_TEAMS = MEGA_CONSUMER_WARPS / MEGA_TEAM_WARPS;  // the ring h
 static_assert(MEGA_CONSUMER_WARPS % MEGA_TEAM_WARPS == 0, "consumer warps must split into whole teams");
 constexpr int MEGA_THREADS = 32 * (MEGA_CONSUMER_WARPS + 1);  // warp 0 issues the bulk copies
 
-constexpr uint32_t MEGA_TOKEN_FROM_CTL = 0xFFFFFFFFu;
-
 enum MegaPhaseKind : int {
     MPH_NORM = 0,   // input = RMSNorm(hidden) (first phase of a token: hidden = embedding row)
     MPH_CONV = 1,   // input = c * shortconv(b * x) from proj
@@ -71,7 +69,6 @@ struct MegaParams {
     int n_phases;
     int n_layers;
     int n_tokens;
-    uint32_t first_token;  // the first step's token, or MEGA_TOKEN_FROM_CTL
     int greedy;      // 1: feed the argmax back; 0: single step, logits only
     int hs, is, n_heads, head_dim, vocab, conv_ks, max_seq;
     float eps;

@@ -480,11 +480,10 @@ void logits_matvec(wick_cuda_model* m);
 static const uint32_t MEGA_LONG_CTX = 768;
 
 // `embedding`: device row [hidden] that takes the place of the token's embedding (one step only).
-int32_t run_mega(wick_cuda_model* m, uint32_t token, int n_tokens, bool greedy, const float* embedding = nullptr) {
+int32_t run_mega(wick_cuda_model* m, int n_tokens, bool greedy, const float* embedding = nullptr) {
     MegaParams P = m->mega;
     P.greedy = greedy ? 1 : 0;
     P.embedding = embedding;
-    P.first_token = token;  // (a launch argument: no copy to the device in front of every step)
     m->last_launch_long = m->long_ok && m->seq_len >= MEGA_LONG_CTX && getenv("WICK_CUDA_NO_SPLIT_SCORES") == nullptr;
     if (m->last_launch_long) {
         P.phases = m->d_phases_long;
@@ -507,7 +506,6 @@ int32_t run_mega(wick_cuda_model* m, uint32_t token, int n_tokens, bool greedy, 
             P.bar_base = m->bar_base;
             CU_TRY(launch_decode_mega(m->stream, P, m->mega_ctas));
             m->bar_base += (unsigned long long)P.n_phases;
-            P.first_token = MEGA_TOKEN_FROM_CTL;  // later steps: what the kernels below left there
             launch_add_rmsnorm_quant(m->stream, m->hidden, nullptr, m->output_norm, m->cfg.rms_norm_eps, 1, m->cfg.hidden_size, m->q8s,
                                      m->q8q, nullptr);
             logits_matvec(m);
@@ -1328,12 +1326,12 @@ int32_t wick_cuda_gpu_memory_bytes(const wick_cuda_model* m, uint64_t* out) {
 int32_t wick_cuda_forward(wick_cuda_model* m, uint32_t token, uint32_t pos, float* logits_host) {
     W_TRY(pre_step(m, token, pos));
     if (!logits_host) return fail(WICK_CUDA_ERR_BAD_ARG, "logits_host is NULL");
+    m->h_u32[0] = token;
     CU_TRY(cudaEventRecord(m->ev0, m->stream));
+    CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
     if (m->mega_ok) {
-        W_TRY(run_mega(m, token, 1, false));
+        W_TRY(run_mega(m, 1, false));
     } else {
-        m->h_u32[0] = token;
-        CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
         CU_TRY(cudaGraphLaunch(m->g_logits, m->stream));
         m->launches += m->nodes_logits;
     }
@@ -1349,13 +1347,11 @@ int32_t wick_cuda_forward(wick_cuda_model* m, uint32_t token, uint32_t pos, floa
 int32_t wick_cuda_forward_greedy(wick_cuda_model* m, uint32_t token, uint32_t pos, uint32_t* next_token) {
     W_TRY(pre_step(m, token, pos));
     if (!next_token) return fail(WICK_CUDA_ERR_BAD_ARG, "next_token is NULL");
+    m->h_u32[0] = token;
     CU_TRY(cudaEventRecord(m->ev0, m->stream));
-    if (!m->mega_ok) {
-        m->h_u32[0] = token;
-        CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
-    }
+    CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
     if (m->mega_ok) {
-        W_TRY(run_mega(m, token, 1, true));  // copies the control block (with the chosen token) back
+        W_TRY(run_mega(m, 1, true));  // copies the control block (with the chosen token) back
     } else {
         CU_TRY(cudaGraphLaunch(m->g_greedy, m->stream));
         m->launches += m->nodes_greedy;
@@ -1386,12 +1382,12 @@ int32_t wick_cuda_forward_sample(wick_cuda_model* m, uint32_t token, uint32_t po
         W_TRY(dev_alloc(m, &m->sample_status, 1));
         CU_TRY(cudaMemset(m->sample_status, 0, 4));
     }
+    m->h_u32[0] = token;
     CU_TRY(cudaEventRecord(m->ev0, m->stream));
+    CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
     if (m->mega_ok) {
-        W_TRY(run_mega(m, token, 1, false));
+        W_TRY(run_mega(m, 1, false));
     } else {
-        m->h_u32[0] = token;
-        CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
         CU_TRY(cudaGraphLaunch(m->g_logits, m->stream));
         m->launches += m->nodes_logits;
     }
@@ -1426,7 +1422,7 @@ int32_t wick_cuda_generate_greedy(wick_cuda_model* m, uint32_t first_token, uint
     CU_TRY(cudaEventRecord(m->ev0, m->stream));
     CU_TRY(cudaMemcpyAsync(m->ctl, m->h_u32, sizeof(init), cudaMemcpyHostToDevice, m->stream));
     if (m->mega_ok) {
-        W_TRY(run_mega(m, first_token, (int)n_steps, true));
+        W_TRY(run_mega(m, (int)n_steps, true));
     } else {
         for (uint32_t i = 0; i < n_steps; i++) CU_TRY(cudaGraphLaunch(m->g_greedy, m->stream));
         m->launches += m->nodes_greedy * n_steps;
@@ -1465,10 +1461,13 @@ static int32_t prefill_core(wick_cuda_model* m, const uint32_t* tokens_host, con
     // instead of ~160 (350M Q8_0, one frame: 3.1 -> 0.5 ms).  Slots and the category timers stay on the pipeline.
     const bool one_step = n == 1 && m->mega_ok && !m->slot_bound && !m->prof_on;
     if (one_step) {
-        if (!tokens_host) {
+        if (tokens_host) {
+            m->h_u32[0] = tokens_host[0];
+            CU_TRY(cudaMemcpyAsync(&m->ctl->token, m->h_u32, 4, cudaMemcpyHostToDevice, m->stream));
+        } else {
             CU_TRY(cudaMemcpyAsync(m->block_out, emb_host, (size_t)hs * 4, cudaMemcpyHostToDevice, m->stream));
         }
-        W_TRY(run_mega(m, tokens_host ? tokens_host[0] : 0, 1, false, tokens_host ? nullptr : m->block_out));
+        W_TRY(run_mega(m, 1, false, tokens_host ? nullptr : m->block_out));
         if (hidden_host) {
             launch_add_rmsnorm_quant(m->stream, m->hidden, nullptr, m->output_norm, m->cfg.rms_norm_eps, 1, hs, m->q8s, m->q8q, m->normed_last);
             m->launches++;
