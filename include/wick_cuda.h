@@ -132,8 +132,9 @@ int32_t wick_cuda_forward_embedding(wick_cuda_model* m, uint32_t token, uint32_t
  * WICK_CUDA_ERR_BAD_ARG. */
 int32_t wick_cuda_shift_kv(wick_cuda_model* m, uint32_t n_keep, uint32_t shift);
 
-/* Which GEMM forward_prefill uses for chunks of >= 16 tokens (shorter chunks always take the
- * CUDA-core kernel).  Decode is not affected.
+/* Which GEMM forward_prefill uses for chunks of several tokens (the first chunk of more than 8 makes the
+ * tensor-core copies of the weights; until then, and in TENSOR mode below 16 tokens, the CUDA-core kernel
+ * runs; a single token or frame is a decode step, with the same bits).  Decode is not affected.
  * EXACT (default): the arithmetic of gemm_q*_q8_0_neon (simd.rs:696-1019) bit for bit, so logits and
  *   greedy tokens equal wick's CPU path.  When hidden and feed-forward sizes are multiples of 128 it
  *   runs on the tensor cores: tcgen05 int8 MMAs against lane-group-masked activations produce the

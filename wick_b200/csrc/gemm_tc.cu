@@ -489,7 +489,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         bool ok = true;
         if constexpr (!EXACT) {
             // One fused chain per output: per block a conversion per output and one packed product and one packed multiply-add
-            // per two.  Same hand-over as below (6144 x 2048 at 512 tokens: see launch_gemm_tc).
+            // per two.  Same hand-over as below (2048-token prompt of the 1.6B model: 23.4 -> 18.4 ms).
             static_assert(COLS == 32, "64 tokens per tile");
             f32x2 acc[COLS / 2];
             bool ready = false;
