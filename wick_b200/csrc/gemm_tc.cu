@@ -31,6 +31,7 @@
 #include <mutex>
 
 #include "gemm_tc.cuh"
+#include "per_device.hpp"
 
 namespace wick {
 
@@ -754,23 +755,20 @@ cudaError_t encode_rows_map(const void* base, int rows, int k, int box_rows, CUt
 template <int BN, bool EXACT>
 cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_x, const float* x_scales, int n, int k,
                       int32_t* sums, uint32_t* err) {
-    static int sm_count = 0;
-    static bool configured = false;
+    // per device, like every attribute of a kernel: the first device of a process must not stand for the others
     const size_t smem = sizeof(TcSmem<BN>) + 1024;
-    if (!configured) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return e;
-        e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(k_gemm_tc<BN, false, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        if constexpr (!EXACT) {
-            e = cudaFuncSetAttribute(k_gemm_tc<BN, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
-        configured = true;
-    }
+    int dev = 0, sm_count = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    static RaisedPerDevice configured;
+    e = (cudaError_t)configured.raise(dev, smem, [](size_t bytes) {
+        cudaError_t r = cudaFuncSetAttribute(k_gemm_tc<BN, false, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if constexpr (!EXACT)
+            if (r == cudaSuccess) r = cudaFuncSetAttribute(k_gemm_tc<BN, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        return (int)r;
+    });
+    if (e != cudaSuccess) return e;
     const int tiles = job.tile_start[job.count];
     const int grid = tiles < sm_count ? tiles : sm_count;
     g_kernel_launches++;
