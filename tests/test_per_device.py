@@ -49,11 +49,18 @@ def test_launch_state_is_kept_per_device(tmp_path):
     assert out.returncode == 0, out.stdout
 
 
-@pytest.mark.parametrize("name", ["gemm_tc.cu"])
+@pytest.mark.parametrize("name", ["gemm_tc.cu", "kernels_attn.cu", "kernels_batch.cu"])
 def test_launchers_keep_no_state_of_their_own(name):
     """No plain function-level static in a launcher: it would be one value for all devices, unsynchronised between threads."""
     code = open(os.path.join(CSRC, name)).read()
     assert not re.findall(r"^\s+static (?:bool|int|size_t) \w+(?:\[\w+\])? = .*$", code, flags=re.M)
+
+
+@pytest.mark.parametrize("name", ["gemm_tc.cu", "kernels_attn.cu", "kernels_batch.cu", "decode_mega.cu"])
+def test_shared_memory_is_only_ever_raised(name):
+    """A bare set of a kernel's shared-memory limit lowers it under another thread that is about to launch with more."""
+    code = open(os.path.join(CSRC, name)).read()
+    assert "cudaFuncAttributeMaxDynamicSharedMemorySize" not in code and "raise_dynamic_smem" in code
 
 
 @pytest.mark.gpu

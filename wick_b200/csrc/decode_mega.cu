@@ -1405,6 +1405,8 @@ size_t mega_smem_bytes(const MegaParams& P) {
 }
 
 namespace {
+// The instantiation a launch takes, and its opt-in shared memory: per kernel and device, not per model (models of different
+// size share a kernel, and may be used from different threads), so it is only ever raised.
 const void* mega_kernel(const MegaParams& P) {
     if (P.long_ctx) {
         switch (P.uniform_dtype) {
@@ -1419,6 +1421,11 @@ const void* mega_kernel(const MegaParams& P) {
         default: return (const void*)k_decode_mega<0, false>;
     }
 }
+cudaError_t raise_mega_smem(const MegaParams& P, size_t smem) {
+    static RaisedPerDevice limit[6];
+    const int i = (P.long_ctx ? 3 : 0) + (P.uniform_dtype == DT_Q4_0 ? 0 : P.uniform_dtype == DT_Q8_0 ? 1 : 2);
+    return raise_dynamic_smem(limit[i], mega_kernel(P), smem);
+}
 }  // namespace
 
 int mega_max_ctas(const MegaParams& P) {
@@ -1426,7 +1433,7 @@ int mega_max_ctas(const MegaParams& P) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     size_t smem = mega_smem_bytes(P);
-    if (cudaFuncSetAttribute(mega_kernel(P), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (raise_mega_smem(P, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -1439,8 +1446,7 @@ int mega_max_ctas(const MegaParams& P) {
 
 cudaError_t launch_decode_mega(cudaStream_t st, const MegaParams& P, int n_ctas) {
     size_t smem = mega_smem_bytes(P);
-    // the attribute is per function, not per model: models of different size share the kernel
-    cudaError_t e = cudaFuncSetAttribute(mega_kernel(P), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = raise_mega_smem(P, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&P};
     g_kernel_launches++;

@@ -31,7 +31,6 @@
 #include <mutex>
 
 #include "gemm_tc.cuh"
-#include "per_device.hpp"
 
 namespace wick {
 
@@ -761,13 +760,10 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    static RaisedPerDevice configured;
-    e = (cudaError_t)configured.raise(dev, smem, [](size_t bytes) {
-        cudaError_t r = cudaFuncSetAttribute(k_gemm_tc<BN, false, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if constexpr (!EXACT)
-            if (r == cudaSuccess) r = cudaFuncSetAttribute(k_gemm_tc<BN, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        return (int)r;
-    });
+    static RaisedPerDevice limit, limit_sums;
+    e = raise_dynamic_smem(limit, (const void*)k_gemm_tc<BN, false, EXACT>, smem);
+    if constexpr (!EXACT)
+        if (e == cudaSuccess) e = raise_dynamic_smem(limit_sums, (const void*)k_gemm_tc<BN, true, false>, smem);
     if (e != cudaSuccess) return e;
     const int tiles = job.tile_start[job.count];
     const int grid = tiles < sm_count ? tiles : sm_count;

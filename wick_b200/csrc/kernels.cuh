@@ -2,6 +2,7 @@
 // asynchronous on `st`.  Activations are token-major: [n tokens][dim].
 #pragma once
 #include "common.cuh"
+#include "per_device.hpp"
 
 namespace wick {
 
@@ -36,6 +37,14 @@ inline cudaError_t launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, 
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Raises a kernel's opt-in shared memory on the current device; `state`: the kernel's own static object.
+inline cudaError_t raise_dynamic_smem(RaisedPerDevice& state, const void* kernel, size_t bytes) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)state.raise(dev, bytes, [kernel](size_t b) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b); });
 }
 
 // Device-resident control block of the decode step: lets one captured CUDA graph

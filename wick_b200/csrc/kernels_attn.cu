@@ -123,17 +123,9 @@ __global__ void __launch_bounds__(NAIVE_THREADS) k_attention_naive(const float* 
 // ever raised (a second model with a shorter context, or an operator call with a shorter sequence, must not
 // lower the limit under a model that still launches with its own, larger size).
 static cudaError_t raise_naive_attention_smem(size_t bytes) {
-    constexpr int MAX_DEV = 64;
-    static size_t granted[MAX_DEV] = {};  // written under the callers' own serialisation (one handle = one thread at a time);
-                                          // a lost update only repeats an idempotent cudaFuncSetAttribute
+    static RaisedPerDevice limit;
     if (bytes <= 48 * 1024) return cudaSuccess;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < MAX_DEV && granted[dev] >= bytes) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_attention_naive, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess && dev >= 0 && dev < MAX_DEV) granted[dev] = bytes;
-    return e;
+    return raise_dynamic_smem(limit, (const void*)k_attention_naive, bytes);
 }
 
 void configure_naive_attention_smem(size_t bytes) { raise_naive_attention_smem(bytes); }
@@ -508,9 +500,8 @@ static cudaError_t launch_flash_hd(cudaStream_t st, const float* q, const float*
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    static int sm_count[64] = {};
-    if (dev >= 0 && dev < 64 && sm_count[dev] == 0) cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-    const int wave = (dev >= 0 && dev < 64 && sm_count[dev] > 0) ? sm_count[dev] : 148;
+    int wave = 0;
+    if (cudaDeviceGetAttribute(&wave, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || wave <= 0) wave = 148;
     // Consumer warps per CTA: the number that leaves the fewest on the fullest SM, and of equals the largest (fewer CTAs fetch
     // the same keys).  512 queries of 32 heads: 7, 296 CTAs, 14 warps on every SM; of 16 heads: 4, at most 8 warps.
     const int n_items = (n + 8 * BQ - 1) / (8 * BQ) * group;
@@ -521,17 +512,15 @@ static cudaError_t launch_flash_hd(cudaStream_t st, const float* q, const float*
         if (best == 0 || fullest < best) best = fullest, n_cw = w, grid = ctas;
     }
     const size_t smem = 64 + (size_t)(4 * FLASH_TILE + n_cw * 8 * BQ) * (HD + 4) * sizeof(float);
-    static size_t configured[64] = {};
-    if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || configured[dev] < smem)) {
-        e = cudaFuncSetAttribute(k_attention_flash<HD, BQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static RaisedPerDevice limit, carveout;
+    if (smem > 48 * 1024) {
+        e = raise_dynamic_smem(limit, (const void*)k_attention_flash<HD, BQ>, smem);
         if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = smem;
     }
-    static bool carved[64] = {};
-    if (dev >= 0 && dev < 64 && !carved[dev]) {  // several CTAs per SM only fit when the SM's L1/shared split favours shared memory
-        cudaFuncSetAttribute(k_attention_flash<HD, BQ>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        carved[dev] = true;
-    }
+    // several CTAs per SM only fit when the SM's L1/shared split favours shared memory (a preference: a refusal is no error)
+    carveout.raise(dev, (size_t)cudaSharedmemCarveoutMaxShared, [](size_t percent) {
+        return (int)cudaFuncSetAttribute(k_attention_flash<HD, BQ>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)percent);
+    });
     const int threads = (n_cw + 1) * 32;
     g_kernel_launches++;
     launch_pdl(st, k_attention_flash<HD, BQ>, dim3((unsigned)grid), dim3(threads), smem, q, k_cache, v_cache, out, n, start_pos, n_heads, n_kv_heads, n_cw, wave, err);

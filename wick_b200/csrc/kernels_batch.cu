@@ -185,17 +185,11 @@ __global__ void __launch_bounds__(ROWS_ATTN_THREADS) k_attention_rows(const floa
 
 cudaError_t launch_attention_rows(cudaStream_t st, const float* q, float* const* k_caches, float* const* v_caches, const uint32_t* positions,
                                   float* out, int n, int n_heads, int n_kv_heads, int head_dim, int max_seq) {
-    static size_t granted[64] = {};  // opt-in shared-memory limit of this kernel per device: only ever raised
+    static RaisedPerDevice limit;
     const size_t smem = naive_attention_smem_bytes(head_dim, max_seq);
     if (smem > 48 * 1024) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
+        const cudaError_t e = raise_dynamic_smem(limit, (const void*)k_attention_rows, smem);
         if (e != cudaSuccess) return e;
-        if (dev < 0 || dev >= 64 || granted[dev] < smem) {
-            e = cudaFuncSetAttribute(k_attention_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            if (dev >= 0 && dev < 64) granted[dev] = smem;
-        }
     }
     dim3 grid(n_heads, n);
     g_kernel_launches++;
