@@ -225,6 +225,15 @@ int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const 
  * and k % 128 == 0 it runs on the tensor cores (same bits; the weight's int8 copy is made by the first such call). */
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev,
                           uint32_t n, float* out_dev, void* stream);
+/* Whether every product of this weight that has finished by now came to its end.  On the tensor cores a kernel's device-side
+ * waits are bounded (about a second each); wick_cuda_gemm_q8 does not wait for its kernel, so a wait that expired is
+ * reported here, or by the weight's next product.  Synchronises `stream` (the one the products ran on, or on which a captured
+ * graph with products was replayed), then returns WICK_CUDA_OK, or WICK_CUDA_ERR_TIMEOUT once: the outputs of the products since
+ * the last report are then undefined, the context stays usable. */
+int32_t wick_cuda_weight_status(const wick_cuda_weight* w, void* stream);
+/* Test hook: leaves `code` where a kernel of this weight reports an expired wait (BAD_ARG before the weight's first product
+ * on the tensor cores). */
+int32_t wick_cuda_debug_weight_error(const wick_cuda_weight* w, uint32_t code);
 /* The same product on the tensor cores (tcgen05 int8 MMA, one instruction per 32-element block, int32
  * block sums in tensor memory, f32 scaling in the epilogue): the throughput path of forward_prefill.
  * Block sums are the exact integers of simd.rs:806-842; the f32 accumulation is one fused chain per

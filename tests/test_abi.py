@@ -55,6 +55,8 @@ def test_bad_arguments_do_not_touch_cuda(cuda_lib):
     raw = np.zeros(18, np.uint8)
     assert cuda_lib.wick_cuda_weight_create(3, raw.ctypes.data, 1, 32, C.byref(w)) == _lib.ERR_UNSUPPORTED_DTYPE
     assert cuda_lib.wick_cuda_weight_create(2, raw.ctypes.data, 1, 33, C.byref(w)) == _lib.ERR_BAD_ARG
+    assert cuda_lib.wick_cuda_weight_status(None, None) == _lib.ERR_BAD_ARG
+    assert cuda_lib.wick_cuda_debug_weight_error(None, 1) == _lib.ERR_BAD_ARG
 
 
 def test_gguf_version_and_truncation_are_rejected(cuda_lib, model_dir):

@@ -1,0 +1,58 @@
+"""Operator-API weights around the tensor-core product: reports of expired waits."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+F32 = np.float32
+
+
+@pytest.fixture(scope="module")
+def ops(cuda_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import ops
+    return ops
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def make(ops, orc, m=128, k=128, n=9, seed=0):
+    """A weight, its raw blocks, and n quantised columns."""
+    from wick_b200 import gguf_synth as gs
+    rng = np.random.default_rng(seed)
+    raw = gs.quantize_q4_0((rng.standard_normal((m, k)) * 0.02).astype(F32))
+    bs, bq = orc.quantize_q8_0(rng.standard_normal((n, k), dtype=F32))
+    return ops.QuantWeight(ops.DT_Q4_0, raw, m, k), raw, bs, bq
+
+
+def check_product(ops, orc, w, raw, bs, bq):
+    out = ops.gemm_q8(w, dev(bs), dev(bq)).cpu().numpy()
+    for j in (0, len(bq) - 1):
+        assert np.array_equal(out[j].view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], w.m, w.k).view(np.uint32))
+
+
+def plant(w, code=6):
+    """What a kernel does whose wait has expired, done by the host."""
+    return w._lib.wick_cuda_debug_weight_error(w._h, code)
+
+
+def test_expired_wait_of_the_last_product_is_reported(ops, orc):
+    from wick_b200 import _lib
+    w, *args = make(ops, orc)
+    w.check_products()                                   # nothing has run
+    assert plant(w) == _lib.ERR_BAD_ARG                  # no word yet
+    check_product(ops, orc, w, *args)
+    w.check_products()
+    assert plant(w) == _lib.OK
+    with pytest.raises(_lib.WickCudaError) as e:
+        w.check_products()
+    assert e.value.code == _lib.ERR_TIMEOUT and "code 6" in e.value.message
+    w.check_products()                                   # reported once
+    assert plant(w) == _lib.OK
+    with pytest.raises(_lib.WickCudaError) as e:         # or by the next product
+        ops.gemm_q8(w, dev(args[1]), dev(args[2]))
+    assert e.value.code == _lib.ERR_TIMEOUT
+    check_product(ops, orc, w, *args)

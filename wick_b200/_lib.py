@@ -92,6 +92,8 @@ SIGNATURES = {
     "wick_cuda_quantize_q8_0": [_vp, _u32, _u32, _vp, _vp, _vp],
     "wick_cuda_gemv_q8": [_vp, _vp, _vp, _vp, _vp],
     "wick_cuda_gemm_q8": [_vp, _vp, _vp, _u32, _vp, _vp],
+    "wick_cuda_weight_status": [_vp, _vp],
+    "wick_cuda_debug_weight_error": [_vp, _u32],
     "wick_cuda_gemm_q8_tc": [_vp, _vp, _vp, _u32, _vp, _vp, _vp],
     "wick_cuda_gemm_q8_tc_exact": [_vp, _vp, _vp, _u32, _vp, _vp],
     "wick_cuda_block_sums": [_vp, _vp, _vp, _vp],

@@ -2037,12 +2037,24 @@ static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
     return WICK_CUDA_OK;
 }
 
-// Reports and clears what a kernel of this weight left behind on an expired wait.
+// Reports and clears what a kernel of this weight left behind on an expired wait (one exchange: of two threads one gets it).
 static int32_t take_tc_error(const wick_cuda_weight* w) {
-    const uint32_t code = *(volatile uint32_t*)w->tc_err;
+    const uint32_t code = __atomic_exchange_n(w->tc_err, 0u, __ATOMIC_ACQ_REL);
     if (code == 0) return WICK_CUDA_OK;
-    *(volatile uint32_t*)w->tc_err = 0;
     return fail(WICK_CUDA_ERR_TIMEOUT, "tensor-core GEMM: a bounded wait expired (role code " + std::to_string(code) + ")");
+}
+
+int32_t wick_cuda_weight_status(const wick_cuda_weight* w, void* stream) {
+    if (!w) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
+    CU_TRY(cudaStreamSynchronize((cudaStream_t)stream));
+    return has_tc_weight(w) ? take_tc_error(w) : WICK_CUDA_OK;
+}
+
+int32_t wick_cuda_debug_weight_error(const wick_cuda_weight* w, uint32_t code) {
+    if (!w) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
+    if (!has_tc_weight(w)) return fail(WICK_CUDA_ERR_BAD_ARG, "no product of this weight has used the tensor cores yet");
+    __atomic_store_n(w->tc_err, code, __ATOMIC_RELEASE);
+    return WICK_CUDA_OK;
 }
 
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n, float* out_dev,
@@ -2050,7 +2062,7 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
     if (!w || !bs_dev || !bq_dev || !out_dev) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
     if (n > (uint32_t)TC_BUILD_ABOVE && tc_gemm_supported(w->w.m, w->w.k)) {
         // same bits on the tensor cores (6912 x 2048 at 2002 rows: 1.71 ms on the CUDA cores); asynchronous like the other
-        // operators, so a wait that expired in an earlier call is reported by the next one
+        // operators, so a wait that expired in an earlier call is reported by wick_cuda_weight_status or by the next call
         cudaStream_t st = (cudaStream_t)stream;
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CU_TRY(cudaStreamIsCapturing(st, &capturing));

@@ -41,6 +41,10 @@ class QuantWeight:
         torch.cuda.init()
         check(self._lib.wick_cuda_weight_create(dtype, raw.ctypes.data, m, k, C.byref(self._h)))
 
+    def check_products(self):
+        """Waits for the current stream; raises TIMEOUT if a product of this weight gave up on a device-side wait."""
+        check(self._lib.wick_cuda_weight_status(self._h, _stream()))
+
     def close(self):
         if self._h.value:
             self._lib.wick_cuda_weight_destroy(self._h)
