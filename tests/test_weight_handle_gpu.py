@@ -56,3 +56,21 @@ def test_expired_wait_of_the_last_product_is_reported(ops, orc):
         ops.gemm_q8(w, dev(args[1]), dev(args[2]))
     assert e.value.code == _lib.ERR_TIMEOUT
     check_product(ops, orc, w, *args)
+
+
+def test_a_report_names_its_own_weight(ops, orc):
+    """More weights than a page of error words: none takes another's report."""
+    from wick_b200 import _lib
+    ws, args = [], None
+    for _ in range(1030):
+        w, *args = make(ops, orc, m=4)
+        ops.gemm_q8(w, dev(args[1]), dev(args[2]))
+        ws.append(w)
+    assert plant(ws[-1]) == _lib.OK
+    for w in ws[:-1]:
+        w.check_products()
+    with pytest.raises(_lib.WickCudaError):
+        ws[-1].check_products()
+    for w in ws[5:]:
+        w.close()
+    check_product(ops, orc, ws[0], *args)

@@ -20,6 +20,7 @@
 #include "decode_mega.cuh"
 #include "gemm_tc.cuh"
 #include "kernels.cuh"
+#include "word_pool.hpp"
 
 using namespace wick;
 
@@ -1973,37 +1974,18 @@ int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const 
     OP_END();
 }
 
-// Host words that kernels of operator-API weights report expired waits in: one pinned page for the process, handed out word by
-// word (pinning memory takes about 2 ms, which every weight paid for on its first product).  Weights beyond the page share its
-// first word: a report then names the wait but not the weight.
-class TcErrorWords {
-    static constexpr uint32_t N = 1024;
-    std::mutex lock;
-    uint32_t* page = nullptr;
-    std::vector<uint32_t*> unused;
-
-public:
-    cudaError_t take(uint32_t** out) {
-        std::lock_guard<std::mutex> hold(lock);
-        if (!page) {
-            cudaError_t e = cudaHostAlloc((void**)&page, N * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable);
-            if (e != cudaSuccess) return e;
-            memset(page, 0, N * sizeof(uint32_t));
-            for (uint32_t i = N - 1; i > 0; i--) unused.push_back(page + i);
-        }
-        *out = page;
-        if (!unused.empty()) {
-            *out = unused.back();
-            unused.pop_back();
-        }
-        return cudaSuccess;
+// Host words that kernels of operator-API weights report expired waits in, one for each weight that has used the tensor cores, out
+// of pinned pages for the whole process (a page of its own cost every weight about 2 ms on its first product).
+struct PinnedPage {
+    uint32_t* operator()(uint32_t words) const {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, words * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        memset(p, 0, words * sizeof(uint32_t));
+        return (uint32_t*)p;
     }
-    void give_back(uint32_t* w) {
-        std::lock_guard<std::mutex> hold(lock);
-        if (w && w != page) *w = 0, unused.push_back(w);
-    }
+    void operator()(uint32_t* page) const { cudaFreeHost(page); }
 };
-static TcErrorWords g_tc_error_words;
+static WordPool<PinnedPage, PinnedPage> g_tc_error_words{PinnedPage(), PinnedPage()};
 static void release_tc_error_word(uint32_t* word) { g_tc_error_words.give_back(word); }
 
 static bool has_tc_weight(const wick_cuda_weight* w) {
@@ -2027,7 +2009,7 @@ static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
         e = tc_weight_fill(st, w->w, &t);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = g_tc_error_words.take(&err);
+    if (e == cudaSuccess && !(err = g_tc_error_words.take())) e = cudaErrorMemoryAllocation;
     if (e != cudaSuccess) {
         cudaFree(t.q);
         CU_TRY(e);
