@@ -43,6 +43,35 @@ def test_exact_gemm_keeps_every_f16_scale(ops, orc, dtype, scales):
     assert_bits(ops.gemm_q8_tc_exact(w, dev(bs), dev(bq)), want, f"{dtype} {scales}")
 
 
+@pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("where", ["weights", "activations", "both"])
+@pytest.mark.parametrize("m,k,n", [(130, 384, 19), (6144, 128, 64)])  # 8- and 16-token tiles
+def test_exact_gemm_with_infinite_scales(ops, orc, dtype, where, m, k, n):
+    """Scales beyond f16 (a block of activations above 8.3 million; an infinity or NaN in a file): the reference's infinities and
+    NaNs, not NaN throughout.  Only the sign and payload of a NaN are free."""
+    rng = np.random.default_rng(5)
+    raw = rng.integers(0, 256, size=(m, k // 32, 18 if dtype == "q4_0" else 34), dtype=np.uint8)
+    d = rng.uniform(0.01, 0.02, size=(m, k // 32)).astype(np.float16)
+    bs = rng.uniform(0.01, 0.02, size=(n, k // 32)).astype(np.float16)
+    if where != "activations":
+        d[1, 0], d[2, 1], d[m - 1, 2], d[7, 0] = np.inf, -np.inf, np.inf, np.nan
+    if where != "weights":
+        bs[0, 0], bs[3, 1], bs[n - 1, 2], bs[5, 1:3] = np.inf, np.inf, np.inf, np.inf
+        bs[6, 0] = 0.0
+    raw[:, :, :2] = d.view(np.uint8).reshape(m, k // 32, 2)
+    bs = bs.astype(F32)
+    bq = rng.integers(1, 128, size=(n, k), dtype=np.int8) * rng.choice(np.array([-1, 1], np.int8), size=(n, 1))
+    if dtype == "q8_0":
+        raw[:, :, 2:] = rng.integers(1, 128, size=raw[:, :, 2:].shape)  # lane partials without a zero: infinities survive
+    bq[n // 2, :32] = 0                                                   # and a block with nothing but zeros
+    w = ops.QuantWeight(ops.QTYPE_ID[dtype], raw.reshape(-1), m, k)
+    got = ops.gemm_q8_tc_exact(w, dev(bs), dev(bq)).cpu().numpy()
+    want = np.stack([orc.gemv(orc.QTYPE_ID[dtype], raw.reshape(m, -1), bs[j], bq[j], m, k) for j in range(n)])
+    assert np.isinf(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert_bits(np.where(np.isnan(got), F32(0), got), np.where(np.isnan(want), F32(0), want), f"{dtype} {where}")
+
+
 @pytest.mark.parametrize("m,k,n", [(128, 128, 2), (128, 128, 7), (256, 256, 8), (256, 256, 9), (384, 128, 15), (2048, 128, 73), (6144, 128, 64),
                                    (2048, 128, 600), (100, 160, 40)])
 def test_operator_gemm_on_either_path(ops, orc, m, k, n):

@@ -22,6 +22,7 @@ struct TcWeight {
 // Q + K + V): their tiles are scheduled as one grid so that narrow matrices do not leave SMs idle.
 struct TcJob {
     CUtensorMap map_w[3];
+    const int8_t* wq[3];  // what map_w describes
     const float* scales_t[3];
     float* out[3];        // [n][m[i]] each
     const int8_t* xq;     // exact GEMM: the quantised activations [n][k] (the other one reads them through a tensor map)
