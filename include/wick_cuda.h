@@ -139,7 +139,9 @@ int32_t wick_cuda_shift_kv(wick_cuda_model* m, uint32_t n_keep, uint32_t shift);
  *   greedy tokens equal wick's CPU path.  When hidden and feed-forward sizes are multiples of 128 it
  *   runs on the tensor cores: tcgen05 int8 MMAs against lane-group-masked activations produce the
  *   four int32 lane partials of every block, and the epilogue keeps the reference's eight unfused f32
- *   chains per output; otherwise on the CUDA-core kernel.
+ *   chains per output; otherwise, and for weights with an infinite scale, on the CUDA-core kernel.  One limit: a
+ *   block of activations above 65504 x 127 (8.3 million) has an infinite scale; its token's outputs are then NaN
+ *   on the tensor cores, where the CPU path gives infinities and NaN (the operators below do as the CPU path does).
  * EXACT_CUDA_CORES (env WICK_CUDA_PREFILL=exact-cuda-cores): always the CUDA-core kernel (same bits).
  * TENSOR (env WICK_CUDA_PREFILL=tensor; needs the multiples of 128): the kernel described at
  *   wick_cuda_gemm_q8_tc.  Each product agrees with EXACT to f32 rounding, but the first last-bit

@@ -72,6 +72,31 @@ def test_exact_gemm_with_infinite_scales(ops, orc, dtype, where, m, k, n):
     assert_bits(np.where(np.isnan(got), F32(0), got), np.where(np.isnan(want), F32(0), want), f"{dtype} {where}")
 
 
+def test_model_with_infinite_weight_scales(cuda_lib, orc, model_dir, tmp_path):
+    """Infinite scales in rows of the vocabulary matrix: a batched step's logits are the CPU path's infinities and NaNs."""
+    import wick_b200.model as wick
+    from wick_b200 import gguf_synth as gs
+    clean = gs.cached_model("tiny-wide", "q4_0", 0, cache_dir=model_dir, norm_jitter=0.2, weight_std=0.05)
+    (k, vocab), _, off = orc.GgufFile(clean).tensors["token_embd.weight"]
+    data = bytearray(open(clean, "rb").read())
+    for r in range(vocab - 100, vocab):
+        at = off + (r * (k // 32) + r % (k // 32)) * 18
+        data[at:at + 2] = np.array([np.inf if r % 2 else -np.inf], np.float16).tobytes()
+    path = tmp_path / "inf.gguf"
+    path.write_bytes(bytes(data))
+    cm, rows = wick.CudaLfm2Model(str(path), 256), 10
+    ids, oms = [cm.seq_create() for _ in range(rows)], [orc.OracleModel(str(path), 256) for _ in range(rows)]
+    for i in range(rows):
+        toks = gs.random_prompt(9 + i, vocab - 100, seed=i)
+        cm.seq_prefill(ids[i], toks, 0), oms[i].forward_prefill(toks, 0)
+    for step in range(2):
+        got = cm.decode_batch_logits([3 * i + step for i in range(rows)], ids)
+        want = np.stack([oms[i].forward(3 * i + step) for i in range(rows)])
+        assert np.isinf(want).any() and np.isnan(want).any() and np.isfinite(want[:, :vocab - 100]).all()
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        assert_bits(np.where(np.isnan(got), F32(0), got), np.where(np.isnan(want), F32(0), want), f"step {step}")
+
+
 @pytest.mark.parametrize("m,k,n", [(128, 128, 2), (128, 128, 7), (256, 256, 8), (256, 256, 9), (384, 128, 15), (2048, 128, 73), (6144, 128, 64),
                                    (2048, 128, 600), (100, 160, 40)])
 def test_operator_gemm_on_either_path(ops, orc, m, k, n):

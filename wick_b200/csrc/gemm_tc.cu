@@ -267,26 +267,6 @@ __device__ __forceinline__ TcTile tc_decode_tile(const TcJob& job, int t, int ti
     return r;
 }
 
-// One output of the exact GEMM in the reference's plain form, for the rare ones that the scaled chains cannot give (see the
-// epilogue).  wq, xq: the rows' int8 values; ws: the row's scales, m_pad apart, times 2^72; xs: the token's scales.
-__device__ __noinline__ float tc_exact_plain(const int8_t* wq, const float* ws, int m_pad, const int8_t* xq, const float* xs, int nb) {
-    float acc[2][4] = {};
-#pragma unroll 1
-    for (int b = 0; b < nb; b++) {
-        const float d = __fmul_rn(ws[(size_t)b * m_pad] * TC_SCALE_DOWN, xs[b]);
-        const int *w = reinterpret_cast<const int*>(wq + b * QK), *x = reinterpret_cast<const int*>(xq + b * QK);
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const float t = __fmul_rn((float)dp4a_ss(w[4 + l], x[4 + l], dp4a_ss(w[l], x[l], 0)), d);
-            if (b & 1) acc[1][l] = __fadd_rn(acc[1][l], t);
-            else acc[0][l] = __fadd_rn(acc[0][l], t);
-        }
-    }
-    const float e = __fadd_rn(__fadd_rn(acc[0][0], acc[0][1]), __fadd_rn(acc[0][2], acc[0][3]));
-    const float o = __fadd_rn(__fadd_rn(acc[1][0], acc[1][1]), __fadd_rn(acc[1][2], acc[1][3]));
-    return __fadd_rn(e, o);
-}
-
 template <int BN, bool SUMS, bool EXACT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap map_x,
@@ -593,8 +573,9 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             //    RN(float(p) * d) * 2^-77, the reference's rounded product, and no contraction with the addition can occur.
             //  - the chains run scaled by 2^-77.  Scales are f16 values, so every term is a multiple of 2^-48: nothing falls
             //    into the denormal range (2^-125) and every rounding is the unscaled one; the final sum is multiplied back.
-            //  - an infinite scale makes every term Inf - Inf, so the output is NaN here, where the reference's may be an
-            //    infinity: an output that comes out NaN is computed again in the plain form (tc_exact_plain).
+            //  - scales outside launch_gemm_tc_exact's range are kept away from here: an infinite one would make every term
+            //    Inf - Inf.  (Looked for in this kernel - NaN outputs in the epilogue, scales in the loading warps - they cost
+            //    1 to 7 % of every product.)
             // 6144 x 2048 at 512 tokens: 157 -> 117 us (110 TFLOP/s); FMA pipe two thirds busy, the rest is the hand-over: both
             // warps of a scheduler wait at the same time.  Tried: columns split between the groups with barriers and MMAs of
             // their own (123), the groups kept half a stage apart (144), sixteen warps of 4 tokens (131), the next stage's
@@ -683,20 +664,12 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                         const int tok = tl.n0 + cg * 2 * TP + 2 * i;
                         const f32x2 e = add2(add2(acc2[i][0][0], acc2[i][0][1]), add2(acc2[i][0][2], acc2[i][0][3]));
                         const f32x2 o = add2(add2(acc2[i][1][0], acc2[i][1][1]), add2(acc2[i][1][2], acc2[i][1][3]));
-                        float r[2];
-                        unpack2(add2(e, o), r[0], r[1]);
-#pragma unroll
-                        for (int j = 0; j < 2; j++) {
-                            if (tok + j >= n) continue;
-                            float v = r[j] * TC_EXACT_DOWN;
-                            if (v != v)
-                                v = tc_exact_plain(job.wq[tl.mat] + (size_t)row * k, job.scales_t[tl.mat] + row, job.m_pad[tl.mat],
-                                                   job.xq + (size_t)(tok + j) * k, x_scales + (size_t)(tok + j) * nb, nb);
-                            out[(size_t)(tok + j) * m + row] = v;
-                        }
+                        float r0, r1;
+                        unpack2(add2(e, o), r0, r1);
+                        if (tok < n) out[(size_t)tok * m + row] = r0 * TC_EXACT_DOWN;
+                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = r1 * TC_EXACT_DOWN;
                     }
                 }
-                __syncwarp();  // (the loads from tensor memory need the whole warp together)
             }
         }
     }
@@ -719,7 +692,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
 namespace {
 
 // One thread per (row, block): widen the block's quants to int8 and store its scale.
-__global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restrict__ scales_t, int m_pad) {
+// *infinite = 1 if a scale is infinite.
+__global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restrict__ scales_t, int m_pad, uint32_t* __restrict__ infinite) {
     const int nb = w.k / QK;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)w.m * nb) return;
@@ -727,7 +701,9 @@ __global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restri
     const int g = row >> 2, r = row & 3;
     const __half* dg = w.d + (size_t)g * nb * 4;
     const uint32_t* qg = reinterpret_cast<const uint32_t*>(w.q + (size_t)g * w.q_group_bytes());
-    scales_t[(size_t)b * m_pad + row] = __half2float(dg[b * 4 + r]) * TC_SCALE_UP;
+    const float d = __half2float(dg[b * 4 + r]);
+    scales_t[(size_t)b * m_pad + row] = d * TC_SCALE_UP;
+    if (isinf(d)) *infinite = 1;
     uint32_t o[8];
     if (w.dtype == DT_Q4_0) {
 #pragma unroll
@@ -815,7 +791,6 @@ cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, in
         if (i >= count) continue;
         if (w[i]->k != w[0]->k) return cudaErrorInvalidValue;
         job.map_w[i] = w[i]->map;
-        job.wq[i] = w[i]->q;
         job.scales_t[i] = w[i]->scales_t;
         job.out[i] = out[i];
         job.m[i] = w[i]->m;
@@ -831,7 +806,7 @@ cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, in
 
 bool tc_gemm_supported(int m, int k) { return m > 0 && k > 0 && k % TC_KSTAGE == 0; }
 
-cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out) {
+cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out, uint32_t* infinite) {
     out->m = w.m;
     out->k = w.k;
     out->m_pad = (w.m + TC_BM - 1) / TC_BM * TC_BM;
@@ -841,7 +816,7 @@ cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out) {
     if (e != cudaSuccess) return e;
     const size_t n_blocks = (size_t)w.m * (w.k / QK);
     g_kernel_launches++;
-    k_tc_unpack<<<(unsigned)((n_blocks + 255) / 256), 256, 0, st>>>(w, out->q, out->scales_t, out->m_pad);
+    k_tc_unpack<<<(unsigned)((n_blocks + 255) / 256), 256, 0, st>>>(w, out->q, out->scales_t, out->m_pad, infinite);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return encode_rows_map(out->q, out->m_pad, out->k, TC_BM, &out->map);

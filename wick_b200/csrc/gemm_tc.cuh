@@ -22,7 +22,6 @@ struct TcWeight {
 // Q + K + V): their tiles are scheduled as one grid so that narrow matrices do not leave SMs idle.
 struct TcJob {
     CUtensorMap map_w[3];
-    const int8_t* wq[3];  // what map_w describes
     const float* scales_t[3];
     float* out[3];        // [n][m[i]] each
     const int8_t* xq;     // exact GEMM: the quantised activations [n][k] (the other one reads them through a tensor map)
@@ -36,8 +35,9 @@ bool tc_gemm_supported(int m, int k);
 
 // Fills `out` (q / scales_t must already point at q_bytes() / s_bytes() of device memory, zeroed by
 // this call) from the grouped layout of `w`, and encodes its tensor map.  Returns cudaSuccess or the
-// failing CUDA error; a tensor-map failure is reported as cudaErrorInvalidValue.
-cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out);
+// failing CUDA error; a tensor-map failure is reported as cudaErrorInvalidValue.  *infinite (device or mapped host memory)
+// becomes 1 if a scale is infinite: the exact GEMM does not take such a matrix.
+cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out, uint32_t* infinite);
 
 // Tensor map over quantised activations xq [rows_cap][k] int8 with a box of bn rows.
 cudaError_t tc_make_activation_map(const int8_t* xq, int rows_cap, int k, int bn, CUtensorMap* out);
@@ -53,7 +53,8 @@ cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* con
 // The bit-exact variant (the arithmetic of gemm_q*_q8_0_neon, simd.rs:696-1019, in its order): every token's activations
 // become four rows of the operand, one per NEON lane group with the other groups' bytes zero, so that one MMA yields the
 // four lane partials of a block as four columns; the epilogue keeps the reference's eight unfused chains per output.
-// xq: int8 [n][k], 4-byte aligned.
+// xq: int8 [n][k], 4-byte aligned.  It needs finite f16 weight scales, and activation scales that are 0 or in [2^-25, 2^40) by
+// magnitude (f16 values are): its chains run scaled by powers of two, see there.
 constexpr int TC_EXACT_TOKENS = 16;  // tokens per tile (64 MMA columns)
 cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,
                                  const float* x_scales, int n, uint32_t* err);

@@ -65,6 +65,7 @@ struct wick_cuda_weight {
     // int8 copy for the tensor-core GEMMs, made by the first call that uses them; the lock is for that call only
     mutable std::mutex tc_lock;
     mutable TcWeight tc;
+    mutable bool tc_exact = false;       // the copy can serve the exact product (no infinite scale)
     mutable uint32_t* tc_err = nullptr;  // host word (TcErrorWords) the kernels write on an expired wait: reading it needs no copy
 };
 
@@ -85,6 +86,7 @@ struct wick_cuda_model {
     // picks the bit-exact one (default), the fused-chain one, or the bit-exact CUDA-core kernel
     bool tc_ok = false;     // the model's shapes allow the tensor-core GEMM
     bool tc_built = false;  // its int8 weight copies and buffers exist (made by the first call that needs them)
+    bool tc_infinite = false;  // a copied matrix has an infinite scale: the exact GEMM stays on the CUDA cores
     int prefill_mode = WICK_CUDA_PREFILL_EXACT;
     CUtensorMap map_x_hs, map_x_is;  // activations [max_chunk][hs | is] for the fused-chain GEMM
     float* normed_last = nullptr;  // output-normed hidden row of the last prefilled token
@@ -696,7 +698,7 @@ struct GemmTarget {
 void run_gemms(wick_cuda_model* m, int n, std::initializer_list<GemmTarget> list) {
     cudaStream_t st = m->stream;
     const int hs = m->cfg.hidden_size;
-    const bool tc_exact = m->tc_built && n >= 2 && m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
+    const bool tc_exact = m->tc_built && !m->tc_infinite && n >= 2 && m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
     const bool tc = tc_exact || (m->tc_built && n >= TC_FUSED_MIN_TOKENS && m->prefill_mode == WICK_CUDA_PREFILL_TENSOR);
     if (tc) {
         const TcWeight* tw[3] = {};
@@ -797,6 +799,16 @@ int32_t build_tc(wick_cuda_model* m) {
     return WICK_CUDA_OK;
 }
 
+// After tc_weight_fill calls that report to the model's (otherwise idle) error word; synchronises.
+int32_t note_infinite_scales(wick_cuda_model* m) {
+    uint32_t found = 0;
+    CU_TRY(cudaMemcpyAsync(&found, m->tc_err, 4, cudaMemcpyDeviceToHost, m->stream));
+    CU_TRY(cudaMemsetAsync(m->tc_err, 0, 4, m->stream));
+    CU_TRY(cudaStreamSynchronize(m->stream));
+    m->tc_infinite = m->tc_infinite || found != 0;
+    return WICK_CUDA_OK;
+}
+
 int32_t ensure_tc(wick_cuda_model* m) {
     if (!m->tc_ok || m->tc_built || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size;
@@ -806,7 +818,7 @@ int32_t ensure_tc(wick_cuda_model* m) {
         t->k = w.k;
         W_TRY(dev_alloc(m, &t->q, t->q_bytes()));
         W_TRY(dev_alloc(m, &t->scales_t, t->s_bytes() / sizeof(float)));
-        CU_TRY(tc_weight_fill(m->stream, w, t));
+        CU_TRY(tc_weight_fill(m->stream, w, t, m->tc_err));
         return WICK_CUDA_OK;
     };
     for (Layer& L : m->layers) {
@@ -825,7 +837,7 @@ int32_t ensure_tc(wick_cuda_model* m) {
     }
     CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, hs, TC_TENSOR_TOKENS, &m->map_x_hs));
     CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, is, TC_TENSOR_TOKENS, &m->map_x_is));
-    CU_TRY(cudaStreamSynchronize(m->stream));
+    W_TRY(note_infinite_scales(m));
     m->tc_built = true;
     return WICK_CUDA_OK;
 }
@@ -1094,8 +1106,8 @@ int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) 
         t->k = m->embd.k;
         W_TRY(dev_alloc(m, &t->q, t->q_bytes()));
         W_TRY(dev_alloc(m, &t->scales_t, t->s_bytes() / sizeof(float)));
-        CU_TRY(tc_weight_fill(m->stream, m->embd, t));
-        CU_TRY(cudaStreamSynchronize(m->stream));
+        CU_TRY(tc_weight_fill(m->stream, m->embd, t, m->tc_err));
+        W_TRY(note_infinite_scales(m));
     }
     const size_t out_need = (size_t)steps * rows;
     if (out_need > m->rows_out_cap) {
@@ -1621,7 +1633,7 @@ int32_t wick_cuda_prefill_mode(const wick_cuda_model* m, int32_t* mode) {
 int32_t wick_cuda_prefill_uses_tensor_cores(const wick_cuda_model* m, int32_t* yes) {
     W_TRY(check_model(m));
     if (!yes) return fail(WICK_CUDA_ERR_BAD_ARG, "yes is NULL");
-    *yes = m->tc_ok && m->prefill_mode != WICK_CUDA_PREFILL_EXACT_CUDA_CORES;
+    *yes = m->tc_ok && m->prefill_mode != WICK_CUDA_PREFILL_EXACT_CUDA_CORES && !(m->tc_infinite && m->prefill_mode == WICK_CUDA_PREFILL_EXACT);
     return WICK_CUDA_OK;
 }
 
@@ -2002,18 +2014,19 @@ static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
     t.m = w->w.m;
     t.k = w->w.k;
     t.m_pad = (w->w.m + 127) / 128 * 128;
-    uint32_t* err = nullptr;
-    cudaError_t e = cudaMalloc((void**)&t.q, t.q_bytes() + t.s_bytes());  // (q_bytes is a multiple of 128 * 128)
+    uint32_t* err = g_tc_error_words.take();
+    cudaError_t e = err ? cudaMalloc((void**)&t.q, t.q_bytes() + t.s_bytes()) : cudaErrorMemoryAllocation;  // (q_bytes is a multiple of 128 * 128)
     if (e == cudaSuccess) {
         t.scales_t = reinterpret_cast<float*>(t.q + t.q_bytes());
-        e = tc_weight_fill(st, w->w, &t);
+        e = tc_weight_fill(st, w->w, &t, err);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess && !(err = g_tc_error_words.take())) e = cudaErrorMemoryAllocation;
     if (e != cudaSuccess) {
         cudaFree(t.q);
+        g_tc_error_words.give_back(err);
         CU_TRY(e);
     }
+    w->tc_exact = __atomic_exchange_n(err, 0u, __ATOMIC_ACQ_REL) == 0;
     w->tc = t;
     w->tc_err = err;
     return WICK_CUDA_OK;
@@ -2051,10 +2064,13 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
         if (capturing == cudaStreamCaptureStatusNone || has_tc_weight(w)) {  // (making the copy allocates and synchronises)
             W_TRY(ensure_tc_weight(w, st));
             W_TRY(take_tc_error(w));
-            const TcWeight* tw[1] = {&w->tc};
-            float* outs[1] = {out_dev};
-            CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
-            OP_END();
+            if (w->tc_exact) {
+                const TcWeight* tw[1] = {&w->tc};
+                float* outs[1] = {out_dev};
+                CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
+                launch_gemm_odd_scales(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
+                OP_END();
+            }
         }
     }
     launch_gemm((cudaStream_t)stream, w->w, bs_dev, bq_dev, (int)n, out_dev);
@@ -2086,7 +2102,13 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     W_TRY(ensure_tc_weight(w, st));
     const TcWeight* tw[1] = {&w->tc};
     float* outs[1] = {out_dev};
-    CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
+    if (w->tc_exact) {
+        CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
+        launch_gemm_odd_scales(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
+    } else {
+        launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
+    }
+    CU_TRY(cudaGetLastError());
     CU_TRY(cudaStreamSynchronize(st));
     return take_tc_error(w);
 }
