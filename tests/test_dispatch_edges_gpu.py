@@ -97,6 +97,24 @@ def test_model_with_infinite_weight_scales(cuda_lib, orc, model_dir, tmp_path):
         assert_bits(np.where(np.isnan(got), F32(0), got), np.where(np.isnan(want), F32(0), want), f"step {step}")
 
 
+@pytest.mark.parametrize("m,k,n", [(130, 384, 19), (6144, 128, 64)])  # 8- and 16-token tiles
+def test_operator_gemm_with_scales_that_are_not_f16(ops, orc, m, k, n):
+    """A caller's own quantiser need not round its scales to f16: tiny, subnormal and huge ones, alone and beside ordinary ones."""
+    from wick_b200 import gguf_synth as gs
+    rng = np.random.default_rng(9)
+    raw = gs.quantize_q4_0((rng.standard_normal((m, k)) * 0.02).astype(F32))
+    bs = (10.0 ** rng.uniform(-4, 0, size=(n, k // 32))).astype(F32)
+    bs[2] = 10.0 ** rng.uniform(-44, -8, size=k // 32)
+    bs[4, 1], bs[5, 2], bs[6, 3], bs[n - 1, 0] = 1e-12, 3e-39, 1e13, 1e30
+    bs[7], bs[8, 1:] = 2.0 ** -25, np.nextafter(F32(2.0 ** -25), F32(0))   # the last inside and the first outside
+    bs[9], bs[10, 0] = np.nextafter(F32(2.0 ** 40), F32(0)), 2.0 ** 40
+    bq = rng.integers(-127, 128, size=(n, k), dtype=np.int8)
+    w = ops.QuantWeight(ops.DT_Q4_0, raw, m, k)
+    want = np.stack([orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], m, k) for j in range(n)])
+    assert np.isfinite(want).all()
+    assert_bits(ops.gemm_q8(w, dev(bs), dev(bq)), want, f"{m} x {k}")
+
+
 @pytest.mark.parametrize("m,k,n", [(128, 128, 2), (128, 128, 7), (256, 256, 8), (256, 256, 9), (384, 128, 15), (2048, 128, 73), (6144, 128, 64),
                                    (2048, 128, 600), (100, 160, 40)])
 def test_operator_gemm_on_either_path(ops, orc, m, k, n):

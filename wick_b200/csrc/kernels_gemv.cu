@@ -226,7 +226,8 @@ void launch_gemm(cudaStream_t st, const DevWeight& w, const float* bs, const int
 }
 
 // ── behind the exact tensor-core GEMM: tokens whose scales it cannot take ───
-// It needs finite activation scales; a block of activations above 8.3 million has an infinite one.  A warp looks at one token's scales; the CTA computes the
+// It needs activation scales that are 0 or in [2^-25, 2^40) by magnitude.  The library's quantiser gives f16 values (an overflow to
+// infinity apart), but a caller of the operators may bring any f32.  A warp looks at one token's scales; the CTA computes the
 // outputs of the tokens that have others (not expected: no attempt at speed) as k_gemv does.  Bound: one launch and one trip to
 // L2, about 2 us where no token does.
 constexpr int ODD_TOKENS = 8;
@@ -235,11 +236,13 @@ __global__ void __launch_bounds__(ODD_TOKENS * 32) k_gemm_odd_scales(DevWeight w
                                                                       float* __restrict__ out) {
     pdl_enter(bs, bq, out);
     __shared__ uint32_t odd[ODD_TOKENS];
+    constexpr uint32_t LOW = 0x33000000u, END = 0x53800000u;  // 2^-25, 2^40
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = w.k, nb = k / QK;
     const int j0 = blockIdx.x * ODD_TOKENS;
     bool mine = false;
     for (int b = lane; b < nb && j0 + warp < n; b += 32) {
-        mine |= !isfinite(bs[(size_t)(j0 + warp) * nb + b]);
+        const uint32_t u = __float_as_uint(bs[(size_t)(j0 + warp) * nb + b]) & 0x7fffffffu;
+        mine |= u != 0u && u - LOW >= END - LOW;
     }
     mine = __any_sync(0xffffffffu, mine);
     if (lane == 0) odd[warp] = mine;
