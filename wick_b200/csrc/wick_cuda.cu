@@ -2022,6 +2022,7 @@ static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
+        cudaGetLastError();  // (not for the next launch to find)
         cudaFree(t.q);
         g_tc_error_words.give_back(err);
         CU_TRY(e);
@@ -2061,8 +2062,10 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
         cudaStream_t st = (cudaStream_t)stream;
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CU_TRY(cudaStreamIsCapturing(st, &capturing));
-        if (capturing == cudaStreamCaptureStatusNone || has_tc_weight(w)) {  // (making the copy allocates and synchronises)
-            W_TRY(ensure_tc_weight(w, st));
+        int32_t made = WICK_CUDA_ERR_OOM;  // (making the copy allocates and synchronises: not while the stream is captured)
+        if (capturing == cudaStreamCaptureStatusNone || has_tc_weight(w)) made = ensure_tc_weight(w, st);
+        if (made != WICK_CUDA_OK && made != WICK_CUDA_ERR_OOM) return made;
+        if (made == WICK_CUDA_OK) {
             W_TRY(take_tc_error(w));
             if (w->tc_exact) {
                 const TcWeight* tw[1] = {&w->tc};
@@ -2073,6 +2076,7 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
             }
         }
     }
+    // also where there is no memory for the copy: the product itself needs none
     launch_gemm((cudaStream_t)stream, w->w, bs_dev, bq_dev, (int)n, out_dev);
     OP_END();
 }
