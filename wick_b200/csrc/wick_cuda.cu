@@ -187,6 +187,14 @@ int32_t dev_alloc(wick_cuda_model* m, T** out, size_t count) {
     return WICK_CUDA_OK;
 }
 
+// Frees what dev_alloc has handed out since the model held `n` allocations.
+void undo_allocs(wick_cuda_model* m, size_t n, uint64_t bytes) {
+    cudaStreamSynchronize(m->stream);  // kernels that fill them may be running
+    for (; m->allocs.size() > n; m->allocs.pop_back()) cudaFree(m->allocs.back());
+    m->bytes = bytes;
+    cudaGetLastError();  // the failed allocation's error is not for the next launch to find
+}
+
 int32_t upload_f32(wick_cuda_model* m, const GgufImage& g, const std::string& name, size_t expect, float** out) {
     const GgufTensor* t = g.tensor(name);
     if (!t) return fail(WICK_CUDA_ERR_BAD_GGUF, "tensor not found: " + name);
@@ -686,7 +694,8 @@ void prof_collect(wick_cuda_model* m) {  // after the stream has been synchronis
 // the bit-exact GEMM uses them from two tokens on: its 8-token tile costs the same for 2 tokens as for 8, and the CUDA-core
 // kernel needs several times as long at any of these counts (350M, 9-token prompt: 3.7 -> 1.2 ms).  The fused-chain GEMM
 // keeps its lower limit, because below it the other kernels' results are the ones a caller has always had.
-constexpr int TC_BUILD_ABOVE = 8, TC_FUSED_MIN_TOKENS = 16;
+// From TC_REQUIRED_FROM rows on a call without memory for the copies is an error; below, the CUDA cores serve it.
+constexpr int TC_BUILD_ABOVE = 8, TC_FUSED_MIN_TOKENS = 16, TC_REQUIRED_FROM = 16;
 
 // Integer GEMMs of n quantised rows (m->q8q / m->q8s) with up to three matrices that read the same input, as one
 // launch on the tensor cores when the chunk is wide enough to fill an MMA tile, else the exact CUDA-core kernel.
@@ -809,8 +818,7 @@ int32_t note_infinite_scales(wick_cuda_model* m) {
     return WICK_CUDA_OK;
 }
 
-int32_t ensure_tc(wick_cuda_model* m) {
-    if (!m->tc_ok || m->tc_built || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
+int32_t make_tc(wick_cuda_model* m) {
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size;
     auto fill = [&](const DevWeight& w, TcWeight* t) -> int32_t {
         t->m_pad = (w.m + 127) / 128 * 128;
@@ -840,6 +848,16 @@ int32_t ensure_tc(wick_cuda_model* m) {
     W_TRY(note_infinite_scales(m));
     m->tc_built = true;
     return WICK_CUDA_OK;
+}
+
+// The copies for a call of `rows` rows.
+int32_t ensure_tc(wick_cuda_model* m, uint32_t rows) {
+    if (rows <= (uint32_t)TC_BUILD_ABOVE || !m->tc_ok || m->tc_built || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
+    const size_t n = m->allocs.size();
+    const uint64_t bytes = m->bytes;
+    const int32_t r = make_tc(m);
+    if (r != WICK_CUDA_OK) undo_allocs(m, n, bytes);
+    return r == WICK_CUDA_ERR_OOM && rows < (uint32_t)TC_REQUIRED_FROM ? WICK_CUDA_OK : r;
 }
 
 // Floats of all conv buffers of one sequence, one after another in layer order.
@@ -1085,6 +1103,17 @@ int32_t with_slot(wick_cuda_model* m, uint32_t id, F&& fn) {
 
 constexpr uint32_t MAX_BATCH_ROWS = 1024;
 
+int32_t make_tc_embd(wick_cuda_model* m) {
+    TcWeight* t = &m->tc_embd;
+    t->m_pad = (m->embd.m + 127) / 128 * 128;
+    t->m = m->embd.m;
+    t->k = m->embd.k;
+    W_TRY(dev_alloc(m, &t->q, t->q_bytes()));
+    W_TRY(dev_alloc(m, &t->scales_t, t->s_bytes() / sizeof(float)));
+    CU_TRY(tc_weight_fill(m->stream, m->embd, t, m->tc_err));
+    return note_infinite_scales(m);
+}
+
 int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) {
     const size_t nl = m->layers.size();
     if ((int)rows > m->batch_cap) {
@@ -1100,14 +1129,14 @@ int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) 
     }
     if (m->tc_built && !m->embd_q6k && !m->tc_embd.q && rows >= 2) {
         // the vocabulary head of a batched step is a GEMM over all rows: worth a tensor-core copy of the matrix
-        TcWeight* t = &m->tc_embd;
-        t->m_pad = (m->embd.m + 127) / 128 * 128;
-        t->m = m->embd.m;
-        t->k = m->embd.k;
-        W_TRY(dev_alloc(m, &t->q, t->q_bytes()));
-        W_TRY(dev_alloc(m, &t->scales_t, t->s_bytes() / sizeof(float)));
-        CU_TRY(tc_weight_fill(m->stream, m->embd, t, m->tc_err));
-        W_TRY(note_infinite_scales(m));
+        const size_t n_allocs = m->allocs.size();
+        const uint64_t bytes = m->bytes;
+        const int32_t r = make_tc_embd(m);
+        if (r != WICK_CUDA_OK) {
+            undo_allocs(m, n_allocs, bytes);
+            m->tc_embd = TcWeight();  // (its first plane may have been allocated, which is what the calls look at)
+            if (r != WICK_CUDA_ERR_OOM || rows >= (uint32_t)TC_REQUIRED_FROM) return r;
+        }
     }
     const size_t out_need = (size_t)steps * rows;
     if (out_need > m->rows_out_cap) {
@@ -1196,7 +1225,7 @@ int32_t decode_rows(wick_cuda_model* m, const uint32_t* tokens_host, const uint3
                                                         std::to_string(m->cfg.max_seq_len));
     }
     CU_TRY(cudaSetDevice(m->device));
-    if (bs > (uint32_t)TC_BUILD_ABOVE) W_TRY(ensure_tc(m));
+    W_TRY(ensure_tc(m, bs));
     if (m->attn_splitk) W_TRY(ensure_splitk_scratch(m, (int)bs));
     W_TRY(ensure_batch_buffers(m, bs, n_steps));
     const size_t nl = m->layers.size();
@@ -1466,7 +1495,7 @@ static int32_t prefill_core(wick_cuda_model* m, const uint32_t* tokens_host, con
         return fail(WICK_CUDA_ERR_CONTEXT_FULL, "start_pos + n = " + std::to_string((uint64_t)start_pos + n) +
                                                     " exceeds max_seq_len " + std::to_string(m->cfg.max_seq_len));
     CU_TRY(cudaSetDevice(m->device));
-    if (n > (uint32_t)TC_BUILD_ABOVE) W_TRY(ensure_tc(m));
+    W_TRY(ensure_tc(m, n));
     if (start_pos == 0) W_TRY(reset_sequence(m));  // new sequence, metal_lfm2.rs:2361-2397
     const bool flash = n >= 256;  // FLASH_ATTN_THRESHOLD, lfm2.rs:1646-1647
     CU_TRY(cudaEventRecord(m->ev0, m->stream));
