@@ -1,4 +1,4 @@
-"""Operator-API weights around the tensor-core product: reports of expired waits."""
+"""Operator-API weights around the tensor-core product: reports of expired waits, captures of other streams."""
 import numpy as np
 import pytest
 
@@ -74,3 +74,41 @@ def test_a_report_names_its_own_weight(ops, orc):
     for w in ws[5:]:
         w.close()
     check_product(ops, orc, ws[0], *args)
+
+
+def test_first_product_beside_a_capture(ops, orc):
+    """A weight's first product on one stream while another stream is captured (in torch's default, global mode) disturbs neither."""
+    w, raw, bs, bq = make(ops, orc)
+    x, dbs, dbq = torch.zeros(4, device="cuda"), dev(bs), dev(bq)
+    out, side = torch.empty((len(bq), w.m), device="cuda"), torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        x += 1
+        with torch.cuda.stream(side):
+            ops.gemm_q8(w, dbs, dbq, out)
+    side.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 4
+    assert np.array_equal(out[8].cpu().numpy().view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[8], bq[8], w.m, w.k).view(np.uint32))
+
+
+def test_captured_products(ops, orc):
+    """Captured before and after the weight has its copy; replayed on new columns."""
+    for warm in (False, True):
+        w, raw, bs, bq = make(ops, orc, n=20)
+        xs, xq, out = dev(bs), dev(bq), torch.empty((20, w.m), device="cuda")
+        if warm:
+            ops.gemm_q8(w, xs, xq, out)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            ops.gemm_q8(w, xs, xq, out)
+        _, _, bs, bq = make(ops, orc, n=20, seed=1)
+        xs.copy_(dev(bs)), xq.copy_(dev(bq))
+        g.replay()
+        torch.cuda.synchronize()
+        w.check_products()
+        for j in (0, 19):
+            assert np.array_equal(out[j].cpu().numpy().view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], w.m, w.k).view(np.uint32))

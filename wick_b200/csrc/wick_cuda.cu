@@ -187,6 +187,14 @@ int32_t dev_alloc(wick_cuda_model* m, T** out, size_t count) {
     return WICK_CUDA_OK;
 }
 
+// Another thread may be capturing a graph in the global mode, in which an allocation by this thread is an error that also ends
+// that capture.  The allocations here have nothing to do with it, so they are made in the relaxed mode.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Frees what dev_alloc has handed out since the model held `n` allocations.
 void undo_allocs(wick_cuda_model* m, size_t n, uint64_t bytes) {
     cudaStreamSynchronize(m->stream);  // kernels that fill them may be running
@@ -853,6 +861,7 @@ int32_t make_tc(wick_cuda_model* m) {
 // The copies for a call of `rows` rows.
 int32_t ensure_tc(wick_cuda_model* m, uint32_t rows) {
     if (rows <= (uint32_t)TC_BUILD_ABOVE || !m->tc_ok || m->tc_built || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
+    RelaxedCapture relaxed;
     const size_t n = m->allocs.size();
     const uint64_t bytes = m->bytes;
     const int32_t r = make_tc(m);
@@ -1129,6 +1138,7 @@ int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) 
     }
     if (m->tc_built && !m->embd_q6k && !m->tc_embd.q && rows >= 2) {
         // the vocabulary head of a batched step is a GEMM over all rows: worth a tensor-core copy of the matrix
+        RelaxedCapture relaxed;
         const size_t n_allocs = m->allocs.size();
         const uint64_t bytes = m->bytes;
         const int32_t r = make_tc_embd(m);
@@ -2039,6 +2049,7 @@ static bool has_tc_weight(const wick_cuda_weight* w) {
 static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
     std::lock_guard<std::mutex> hold(w->tc_lock);
     if (w->tc_err) return WICK_CUDA_OK;
+    RelaxedCapture relaxed;
     TcWeight t;
     t.m = w->w.m;
     t.k = w->w.k;
