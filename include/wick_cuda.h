@@ -223,8 +223,12 @@ int32_t wick_cuda_quantize_q8_0(const float* x_dev, uint32_t n, uint32_t k, floa
 int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const int8_t* xq_dev,
                           float* y_dev, void* stream);
 /* gemm_q4_0_q8_0_neon / gemm_q8_0_q8_0_neon (simd.rs:696-925, :937-1019) over n pre-quantised
- * columns; the result is token-major out[j*m + i] (the reference writes out[i*n + j]).  With more than 8 columns
- * and k % 128 == 0 it runs on the tensor cores (same bits; the weight's int8 copy is made by the first such call). */
+ * columns; the result is token-major out[j*m + i] (the reference writes out[i*n + j]).  bq must be 4-byte aligned; bs may hold
+ * any f32.  With more than 8 columns and k % 128 == 0 it runs on the tensor cores, with the same bits: the weight's first such
+ * call makes an int8 copy of it (1.125 bytes per parameter, kept until the weight is destroyed) and waits for that; repeated
+ * products are then 3.7 times as fast as on the CUDA cores, the first one 1.8 times.  Without memory for the copy, while `stream`
+ * is captured before the copy exists, and for weights with an infinite scale it runs on the CUDA cores.  A weight created
+ * with WICK_CUDA_PREFILL=exact-cuda-cores in the environment always does, and never makes the copy. */
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev,
                           uint32_t n, float* out_dev, void* stream);
 /* Whether every product of this weight that has finished by now came to its end.  On the tensor cores a kernel's device-side

@@ -1,4 +1,5 @@
-"""Operator-API weights around the tensor-core product: reports of expired waits, captures of other streams."""
+"""Operator-API weights around the tensor-core product: reports of expired waits, captures of
+other streams, and weights that are to stay at their packed size."""
 import numpy as np
 import pytest
 
@@ -112,3 +113,23 @@ def test_captured_products(ops, orc):
         w.check_products()
         for j in (0, 19):
             assert np.array_equal(out[j].cpu().numpy().view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], w.m, w.k).view(np.uint32))
+
+
+def test_weight_that_stays_on_the_cuda_cores(ops, orc, monkeypatch):
+    """The environment switch of the models, for operator weights: no copy, the same bits."""
+    from wick_b200 import _lib
+    monkeypatch.setenv("WICK_CUDA_PREFILL", "exact-cuda-cores")
+    w, *args = make(ops, orc, m=16384, k=1024, n=40)
+    monkeypatch.delenv("WICK_CUDA_PREFILL")
+    x = dev(args[1]), dev(args[2])
+    out = torch.empty((40, w.m), device="cuda")
+    ops.gemm_q8(make(ops, orc)[0], *(dev(a) for a in make(ops, orc)[2:]))   # (loads the kernels)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ops.gemm_q8(w, *x, out)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] > free - (8 << 20)                  # the copy would take 18.9 MB
+    assert plant(w) == _lib.ERR_BAD_ARG
+    check_product(ops, orc, w, *args)
+    same, *_ = make(ops, orc, m=16384, k=1024, n=40)
+    assert torch.equal(out.view(torch.int32), ops.gemm_q8(same, *x).view(torch.int32))

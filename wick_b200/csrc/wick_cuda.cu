@@ -65,6 +65,7 @@ struct wick_cuda_weight {
     // int8 copy for the tensor-core GEMMs, made by the first call that uses them; the lock is for that call only
     mutable std::mutex tc_lock;
     mutable TcWeight tc;
+    bool cuda_cores = false;             // products stay on the CUDA cores (WICK_CUDA_PREFILL=exact-cuda-cores at creation): no copy is made
     mutable bool tc_exact = false;       // the copy can serve the exact product (no infinite scale)
     mutable uint32_t* tc_err = nullptr;  // host word (TcErrorWords) the kernels write on an expired wait: reading it needs no copy
 };
@@ -1968,6 +1969,8 @@ int32_t wick_cuda_weight_create(int32_t dtype, const uint8_t* raw_host, uint32_t
     if (k == 0 || k % QK || mrows == 0) return fail(WICK_CUDA_ERR_BAD_ARG, "k must be a positive multiple of 32 and m > 0");
     std::unique_ptr<wick_cuda_weight> w(new wick_cuda_weight());
     CU_TRY(cudaGetDevice(&w->device));
+    const char* mode = getenv("WICK_CUDA_PREFILL");
+    w->cuda_cores = mode && strcmp(mode, "exact-cuda-cores") == 0;
     w->w.m = (int)mrows;
     w->w.k = (int)k;
     w->w.dtype = dtype;
@@ -2096,7 +2099,7 @@ int32_t wick_cuda_debug_weight_error(const wick_cuda_weight* w, uint32_t code) {
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n, float* out_dev,
                           void* stream) {
     if (!w || !bs_dev || !bq_dev || !out_dev) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
-    if (n > (uint32_t)TC_BUILD_ABOVE && tc_gemm_supported(w->w.m, w->w.k)) {
+    if (n > (uint32_t)TC_BUILD_ABOVE && !w->cuda_cores && tc_gemm_supported(w->w.m, w->w.k)) {
         // same bits on the tensor cores (6912 x 2048 at 2002 rows: 1.71 ms on the CUDA cores); asynchronous like the other
         // operators, so a wait that expired in an earlier call is reported by wick_cuda_weight_status or by the next call
         cudaStream_t st = (cudaStream_t)stream;
