@@ -34,3 +34,15 @@ def cuda_lib():
     from wick_b200 import _lib, build
     build.build()
     return _lib.load()
+
+
+@pytest.fixture
+def cuda_core_weight(cuda_lib, monkeypatch):
+    """Makes operator weights whose products stay on the CUDA cores, to compare the tensor-core kernels with (a plain weight's
+    product of more than 8 columns is one of them itself)."""
+    def make(dtype, raw, m, k):
+        from wick_b200 import ops
+        with monkeypatch.context() as mp:
+            mp.setenv("WICK_CUDA_PREFILL", "exact-cuda-cores")
+            return ops.QuantWeight(dtype, raw, m, k)
+    return make

@@ -31,8 +31,8 @@ def _path(model_dir, spec, qtype, **kw):
 
 @pytest.mark.parametrize("spec,qtype,n_seq", [("tiny", "q4_0", 5), ("tiny-wide", "q8_0", 3), ("tiny-wide", "q4_0", 20)])
 def test_batched_decode_matches_oracle_per_sequence(wick, orc, model_dir, spec, qtype, n_seq):
-    """Ragged prompts (1 .. 300 tokens, so both prefill attention paths and both GEMM paths, n < 16 and n >= 16 rows,
-    are used), then interleaved batched steps: logits and tokens of every row equal the oracle's."""
+    """Ragged prompts (1 .. 300 tokens, so both prefill attention paths are used; the first of more than 8 tokens moves the
+    GEMMs of 2 rows and more to the tensor cores), then interleaved batched steps: logits and tokens of every row equal the oracle's."""
     from wick_b200 import gguf_synth as gs
     path = _path(model_dir, spec, qtype, norm_jitter=0.2, weight_std=0.05)
     cm = wick.CudaLfm2Model(path, 512)

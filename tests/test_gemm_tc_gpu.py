@@ -34,7 +34,7 @@ def rand_weights(rng, dtype, m, k, std=0.02):
     return gs.quantize_q4_0(w) if dtype == "q4_0" else gs.quantize_q8_0(w)
 
 
-def check_against_oracle(ops, orc, dtype, m, k, n, seed, oracle_tokens):
+def check_against_oracle(ops, orc, cuda_core_weight, dtype, m, k, n, seed, oracle_tokens):
     rng = np.random.default_rng(seed)
     raw = rand_weights(rng, dtype, m, k)
     x = rng.standard_normal((n, k), dtype=F32)
@@ -44,7 +44,7 @@ def check_against_oracle(ops, orc, dtype, m, k, n, seed, oracle_tokens):
     dbs, dbq = dev(bs), dev(bq)
     out, sums = ops.gemm_q8_tc(w, dbs, dbq, want_sums=True)
     out, sums = host(out), host(sums)
-    exact = host(ops.gemm_q8(w, dbs, dbq))                      # bit-exact path, itself checked against the oracle
+    exact = host(ops.gemm_q8(cuda_core_weight(dt, raw, m, k), dbs, dbq))  # bit-exact, itself checked against the oracle
     scale = np.abs(exact).max()
     assert np.abs(out - exact).max() <= 1e-5 * scale, f"{dtype} {m}x{k}x{n}: {np.abs(out - exact).max()} vs scale {scale}"
     for j in oracle_tokens:
@@ -68,15 +68,15 @@ def check_against_oracle(ops, orc, dtype, m, k, n, seed, oracle_tokens):
     (130, 384, 129),     # one token into the second token tile
     (64, 128, 1),        # single token, fewer rows than a tile
 ])
-def test_gemm_tc_shapes(ops, orc, dtype, m, k, n):
-    check_against_oracle(ops, orc, dtype, m, k, n, seed=m + k + n, oracle_tokens=sorted({0, n // 2, n - 1}))
+def test_gemm_tc_shapes(ops, orc, cuda_core_weight, dtype, m, k, n):
+    check_against_oracle(ops, orc, cuda_core_weight, dtype, m, k, n, seed=m + k + n, oracle_tokens=sorted({0, n // 2, n - 1}))
 
 
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("n", [8, 128, 2002])
-def test_gemm_tc_matmul_sweep(ops, orc, dtype, n):
+def test_gemm_tc_matmul_sweep(ops, orc, cuda_core_weight, dtype, n):
     """The isolated matmul sweep shape (m=6912, k=2048): more tiles than SMs, so CTAs loop over tiles."""
-    check_against_oracle(ops, orc, dtype, 6912, 2048, n, seed=3, oracle_tokens=sorted({0, n - 1}))
+    check_against_oracle(ops, orc, cuda_core_weight, dtype, 6912, 2048, n, seed=3, oracle_tokens=sorted({0, n - 1}))
 
 
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
@@ -84,7 +84,7 @@ def test_gemm_tc_matmul_sweep(ops, orc, dtype, n):
     (128, 128, 16), (128, 512, 64), (256, 1152, 17), (384, 2048, 128), (200, 256, 37), (130, 384, 129), (64, 128, 1),
     (6912, 2048, 8), (6912, 2048, 128), (6912, 2048, 2002), (2048, 6912, 130),
 ])
-def test_gemm_tc_exact_is_bit_exact(ops, orc, dtype, m, k, n):
+def test_gemm_tc_exact_is_bit_exact(ops, orc, cuda_core_weight, dtype, m, k, n):
     """The default prefill GEMM: tensor-core lane partials + the reference's eight chains.  Bit-equal to
     the CUDA-core kernel for every output, and to the oracle for sampled tokens."""
     rng = np.random.default_rng(m * 7 + k + n)
@@ -95,7 +95,7 @@ def test_gemm_tc_exact_is_bit_exact(ops, orc, dtype, m, k, n):
     w = ops.QuantWeight(dt, raw, m, k)
     dbs, dbq = dev(bs), dev(bq)
     out = host(ops.gemm_q8_tc_exact(w, dbs, dbq))
-    exact = host(ops.gemm_q8(w, dbs, dbq))
+    exact = host(ops.gemm_q8(cuda_core_weight(dt, raw, m, k), dbs, dbq))
     assert np.array_equal(out.view(np.uint32), exact.view(np.uint32)), \
         f"{dtype} {m}x{k}x{n}: {int((out.view(np.uint32) != exact.view(np.uint32)).sum())} outputs differ"
     for j in sorted({0, n // 2, n - 1}):
@@ -103,7 +103,7 @@ def test_gemm_tc_exact_is_bit_exact(ops, orc, dtype, m, k, n):
         assert np.array_equal(out[j].view(np.uint32), ref.view(np.uint32))
 
 
-def test_gemm_tc_exact_full_size_properties(ops, orc):
+def test_gemm_tc_exact_full_size_properties(ops, orc, cuda_core_weight):
     """n = 4096 (256 token tiles per row tile, CTAs loop over tiles): equals the CUDA-core kernel bit for
     bit, and sampled tokens equal the oracle."""
     m, k, n = 1024, 2048, 4096
@@ -113,13 +113,13 @@ def test_gemm_tc_exact_full_size_properties(ops, orc):
     w = ops.QuantWeight(orc.DT_Q4_0, raw, m, k)
     bs, bq = ops.quantize_f32_to_q8_0(dev(x))
     out = ops.gemm_q8_tc_exact(w, bs, bq)
-    assert torch.equal(out, ops.gemm_q8(w, bs, bq))
+    assert torch.equal(out, ops.gemm_q8(cuda_core_weight(orc.DT_Q4_0, raw, m, k), bs, bq))
     for j in (0, 1777, 4095):
         ref = orc.gemv(orc.DT_Q4_0, raw, host(bs[j]), host(bq[j]), m, k)
         assert np.array_equal(host(out[j]).view(np.uint32), ref.view(np.uint32))
 
 
-def test_gemm_tc_extreme_values(ops, orc):
+def test_gemm_tc_extreme_values(ops, orc, cuda_core_weight):
     """Largest possible block sums: all weights at -8 (Q4_0) against activations at +/-127."""
     m, k, n = 128, 256, 32
     from wick_b200 import gguf_synth as gs
@@ -133,11 +133,11 @@ def test_gemm_tc_extreme_values(ops, orc):
     S1 = orc.block_sums(orc.DT_Q4_0, raw, bq[1], m, k)[0]
     assert np.array_equal(host(sums)[1], S1)
     assert np.abs(S1).max() == 32 * 8 * 127
-    exact = host(ops.gemm_q8(wq, dev(bs), dev(bq)))
+    exact = host(ops.gemm_q8(cuda_core_weight(orc.DT_Q4_0, raw, m, k), dev(bs), dev(bq)))
     assert np.abs(host(out) - exact).max() <= 1e-5 * np.abs(exact).max()
 
 
-def test_gemm_tc_exact_extreme_lane_partials(ops, orc):
+def test_gemm_tc_exact_extreme_lane_partials(ops, orc, cuda_core_weight):
     """The bit-exact kernel on the largest lane partials (8 * 8 * 127 = 8128 per NEON lane group and block) and on
     low-bit patterns next to them: hand-built integer operands that survive both quantisers unchanged."""
     from wick_b200 import gguf_synth as gs
@@ -164,7 +164,7 @@ def test_gemm_tc_exact_extreme_lane_partials(ops, orc):
     S = orc.block_sums(orc.DT_Q4_0, raw, bq[0], m, k)[0]
     assert np.abs(S).max() == 32 * 8 * 127
     out = host(ops.gemm_q8_tc_exact(w, dev(bs), dev(bq)))
-    exact = host(ops.gemm_q8(w, dev(bs), dev(bq)))
+    exact = host(ops.gemm_q8(cuda_core_weight(orc.DT_Q4_0, raw, m, k), dev(bs), dev(bq)))
     assert np.array_equal(out.view(np.uint32), exact.view(np.uint32)), \
         f"{int((out.view(np.uint32) != exact.view(np.uint32)).sum())} outputs differ"
     for j in range(0, n, 7):
@@ -172,7 +172,7 @@ def test_gemm_tc_exact_extreme_lane_partials(ops, orc):
         assert np.array_equal(out[j].view(np.uint32), ref.view(np.uint32))
 
 
-def test_gemm_tc_properties_full_size(ops, orc):
+def test_gemm_tc_properties_full_size(ops, orc, cuda_core_weight):
     """Size-independent properties at n = 4096: power-of-two activation scales commute with the product
     bit for bit, tokens are independent of their position in the batch, and repeated runs are identical."""
     m, k, n = 2048, 2048, 4096
@@ -186,7 +186,7 @@ def test_gemm_tc_properties_full_size(ops, orc):
     assert torch.equal(ops.gemm_q8_tc(w, bs * 4.0, bq), out * 4.0)
     perm = torch.randperm(n, device="cuda")
     assert torch.equal(ops.gemm_q8_tc(w, bs[perm].contiguous(), bq[perm].contiguous()), out[perm])
-    exact = ops.gemm_q8(w, bs, bq)
+    exact = ops.gemm_q8(cuda_core_weight(orc.DT_Q4_0, raw, m, k), bs, bq)
     assert float((out - exact).abs().max()) <= 1e-5 * float(exact.abs().max())
     for j in (0, 2047, 4095):
         ref = orc.gemv(orc.DT_Q4_0, raw, host(bs[j]), host(bq[j]), m, k)

@@ -136,14 +136,17 @@ def test_gemm_q8_0_known_answer(ops, orc):
 
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("m,k,n", [(33, 96, 1), (40, 2048, 8), (65, 1056, 33), (256, 2080, 130), (100, 6912, 17)])
-def test_gemm_bit_exact_ragged(ops, orc, dtype, m, k, n):
+def test_gemm_bit_exact_ragged(ops, orc, cuda_core_weight, dtype, m, k, n):
     rng = np.random.default_rng(m + k + n)
     raw = rand_weights(rng, dtype, m, k)
     x = rng.standard_normal((n, k), dtype=F32)
     bs, bq = orc.quantize_q8_0(x)
     w = ops.QuantWeight(orc.QTYPE_ID[dtype], raw, m, k)
     out = host(ops.gemm_q8(w, dev(bs), dev(bq)))
-    assert_bit_equal(out.T, orc.gemm(orc.QTYPE_ID[dtype], raw, bs, bq, m, n, k), f"gemm {dtype} {m}x{k}x{n}")
+    want = orc.gemm(orc.QTYPE_ID[dtype], raw, bs, bq, m, n, k)
+    assert_bit_equal(out.T, want, f"gemm {dtype} {m}x{k}x{n}")
+    out = host(ops.gemm_q8(cuda_core_weight(orc.QTYPE_ID[dtype], raw, m, k), dev(bs), dev(bq)))
+    assert_bit_equal(out.T, want, f"gemm on the CUDA cores {dtype} {m}x{k}x{n}")
 
 
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
