@@ -757,14 +757,18 @@ cudaError_t encode_rows_map(const void* base, int rows, int k, int box_rows, CUt
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t device_sm_count(int* sms) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+}
+
 template <int BN, bool EXACT>
 cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_x, const float* x_scales, int n, int k,
                       int32_t* sums, uint32_t* err) {
-    // per device, like every attribute of a kernel: the first device of a process must not stand for the others
     const size_t smem = sizeof(TcSmem<BN>) + 1024;
-    int dev = 0, sm_count = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    int sm_count = 0;
+    cudaError_t e = device_sm_count(&sm_count);
     if (e != cudaSuccess) return e;
     static RaisedPerDevice limit, limit_sums;
     e = raise_dynamic_smem(limit, (const void*)k_gemm_tc<BN, false, EXACT>, smem);
@@ -844,14 +848,15 @@ cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, floa
     // 16-token or 8-token tiles: whichever needs less time in waves of one tile per SM.  A stage of the small tile takes 810
     // cycles against 1430 (0.57; 64 rows x 2048 x 6912 and 512 x 6144 x 2048), so it wins where it fills a last wave that
     // the large one would leave mostly empty: one wave instead of half of one, 3 instead of 2 (64 rows x 6144), and so on.
-    int row_tiles = 0;
+    int row_tiles = 0, sms = 0;
     for (int i = 0; i < count; i++) row_tiles += w[i]->m_pad / TC_BM;
-    constexpr int SMS = 148;
-    const int wide_waves = (row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) + SMS - 1) / SMS;
-    const int narrow_waves = (row_tiles * ((n + TC_EXACT_TOKENS / 2 - 1) / (TC_EXACT_TOKENS / 2)) + SMS - 1) / SMS;
+    cudaError_t e = device_sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    const int wide_waves = (row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) + sms - 1) / sms;
+    const int narrow_waves = (row_tiles * ((n + TC_EXACT_TOKENS / 2 - 1) / (TC_EXACT_TOKENS / 2)) + sms - 1) / sms;
     const bool narrow = narrow_waves * 62 < wide_waves * 100;  // (close calls go to the large tile: fewer weight reads)
     const int tok = narrow ? TC_EXACT_TOKENS / 2 : TC_EXACT_TOKENS;
-    cudaError_t e = fill_job(job, w, out, count, (n + tok - 1) / tok);
+    e = fill_job(job, w, out, count, (n + tok - 1) / tok);
     if (e != cudaSuccess) return e;
     job.xq = xq;
     return narrow ? launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, CUtensorMap{}, x_scales, n, w[0]->k, nullptr, err)
