@@ -13,16 +13,16 @@
 //
 // One MMA instruction covers exactly one quantisation block (K = 32 int8), writes a fresh 128 x BN
 // int32 tile into one of 512/BN tensor-memory buffers and never accumulates across blocks, because
-// each block has its own scale pair.  The epilogue warps drain a buffer (tcgen05.ld), hand it back,
-// and apply the scales on the CUDA cores: 3 instructions per (output, block), which is what bounds the
-// kernel (the tensor pipe needs about 1/6 of that time).
+// each block has its own scale pair.  The epilogue warps drain a stage's four buffers (tcgen05.ld), hand them back,
+// and apply the scales on the CUDA cores, which is what bounds the kernel: per (output, block) a conversion and half of
+// two packed instructions here, half of ten packed ones in the EXACT form (see the epilogue).
 //
-// Roles in a CTA (one CTA per SM, persistent over output tiles; 12 warps for EXACT, else 20):
+// Roles in a CTA (one CTA per SM, persistent over output tiles; 12 warps):
 //   warp 0  lane 0: TMA producer, one K=128 stage (4 blocks) of W rows (and, not for EXACT, activation rows) per step
 //   warp 1        : issues tcgen05.mma / tcgen05.commit from one elected lane and owns the TMEM allocation
 //   warp 2        : copies the stage's weight scales and (transposed) activation scales into smem (cp.async)
 //   warp 3        : EXACT: spreads the activation words over the lane-group rows of the operand (cp.async)
-//   warps 4..     : epilogue; warp w reads TMEM lanes 32*(w%4).. and its group's share of the columns
+//   warps 4..11   : epilogue; warp w reads TMEM lanes 32*(w%4).. and its group's half of the columns
 // Every wait is bounded: on expiry the kernel records an error code, all roles leave their loops and
 // the CTA frees its tensor memory and exits.
 #include <cuda.h>
@@ -44,6 +44,10 @@ constexpr int TC_KB_PER_STAGE = TC_KSTAGE / QK;  // 4 quantisation blocks per st
 // the MMA issuer needs it; with four stages that left about one microsecond, less than a loaded L2 round trip.
 template <int BN>
 __host__ __device__ constexpr int tc_stages() { return BN <= 32 ? 9 : 8; }
+// Hand-over units of tensor memory (512 columns), a stage's blocks each.  32-column tiles fill it with four: with two, a stage could
+// not take less than half the way round (release, MMA issue, MMAs, wait, loads), ~860 cycles for the work of ~400.
+template <int BN>
+__host__ __device__ constexpr int tc_units() { return 512 / (BN * TC_KB_PER_STAGE); }
 constexpr int TC_COL_GROUPS = 2;    // epilogue warps per TMEM lane quarter; each takes half of a tile's columns
 constexpr int TC_EPI_WARPS = 4 * TC_COL_GROUPS;
 constexpr int TC_THREADS = 32 * (4 + TC_EPI_WARPS);
@@ -70,8 +74,8 @@ struct TcSmem {
     uint32_t bias[TC_BIAS_BYTES / 4];           // exact GEMM only
     unsigned long long full[tc_stages<BN>()];   // TMA bytes landed + scales written
     unsigned long long empty[tc_stages<BN>()];  // MMAs of the stage retired + epilogue done with its scales
-    unsigned long long tmem_full[512 / BN];   // block sums of one k-block are in the buffer
-    unsigned long long tmem_empty[512 / BN];  // all epilogue warps have read the buffer
+    unsigned long long tmem_full[tc_units<BN>()];   // block sums of a stage are in the unit's part of tensor memory
+    unsigned long long tmem_empty[tc_units<BN>()];  // all epilogue warps have read them
     uint32_t tmem_base;
     volatile uint32_t abort;
 };
@@ -217,30 +221,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int32_t* r) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int32_t* r) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-        : "r"(taddr)
-        : "memory");
-}
 template <int COLS>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, int32_t* r) {
-    static_assert(COLS == 8 || COLS == 16 || COLS == 32, "one tcgen05.ld per k-block");
-    if constexpr (COLS == 8) tmem_ld8(taddr, r);
-    else if constexpr (COLS == 16) tmem_ld16(taddr, r);
+    static_assert(COLS == 16 || COLS == 32, "one tcgen05.ld per k-block");
+    if constexpr (COLS == 16) tmem_ld16(taddr, r);
     else tmem_ld32(taddr, r);
 }
 // Shared-memory loads by 32-bit address (a pointer derived from the aligned raw buffer is a generic one to the compiler)
 __device__ __forceinline__ float lds_f32(uint32_t a) {
     float v;
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ f32x2 lds_64(uint32_t a) {
-    f32x2 v;
-    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
     return v;
 }
 __device__ __forceinline__ void lds_2x64(uint32_t a, f32x2& v0, f32x2& v1) {
@@ -276,11 +266,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     pdl_trigger();
     extern __shared__ uint8_t tc_smem_raw[];
     TcSmem<BN>* sm = reinterpret_cast<TcSmem<BN>*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr int NBUF = 512 / BN;
     constexpr int UNIT = TC_KB_PER_STAGE;  // blocks per hand-over of tensor memory: a stage
-    // Hand-over units in flight.  32-column tiles fill tensor memory with four: with two, a stage could not take less than
-    // half the way round (release, MMA issue, MMAs, wait, loads), ~860 cycles for the work of ~400.
-    constexpr int NU = NBUF / UNIT;
+    constexpr int NU = tc_units<BN>();     // units in flight
     static_assert(NU >= 2 && (NU & (NU - 1)) == 0, "hand-over units that tile tensor memory");
     constexpr int TC_STAGES = tc_stages<BN>();
     constexpr int COLS = BN / TC_COL_GROUPS;  // columns per epilogue thread
@@ -288,7 +275,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     // spreads the words), so a tile covers BN/4 tokens and the MMA yields the four lane partials.  Column order inside a
     // pair of tokens is (lane group, token of the pair): the epilogue's packed arithmetic works on two tokens at a time.
     constexpr int TOK = EXACT ? BN / 4 : BN;  // tokens per tile
-    static_assert(!EXACT || ((COLS == 32 || COLS == 16 || COLS == 8) && !SUMS), "exact epilogue: 8, 4 or 2 tokens x 4 lane groups per thread");
+    static_assert(!EXACT || ((COLS == 32 || COLS == 16) && !SUMS), "exact epilogue: 8 or 4 tokens x 4 lane groups per thread");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = k / QK;
     const int k_stages = k / TC_KSTAGE;
@@ -301,7 +288,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             mbar_init(smem_u32(&sm->full[s]), 1 + 32 + (EXACT ? 1 : 0));
             mbar_init(smem_u32(&sm->empty[s]), 1);  // the MMA issuer alone, NU stages later (see there)
         }
-        for (int b = 0; b < NBUF; b++) {
+        for (int b = 0; b < NU; b++) {
             mbar_init(smem_u32(&sm->tmem_full[b]), 1);
             mbar_init(smem_u32(&sm->tmem_empty[b]), TC_EPI_WARPS);
         }
@@ -358,10 +345,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         // to issue, every descriptor going through general registers first, and this warp set the pace of the kernel.)
         const uint32_t leader = elect_one();
         const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-        // EXACT: every block's tile starts from 2^17 (a constant x constant product of the same shape), so that the
+        // EXACT: every block's tile starts from 2^17 (d_bias: a constant x constant product of the same shape), so that the
         // int32 results are positive: see the epilogue
-        const unsigned long long d_bias = EXACT ? umma_desc_plain32(smem_u32(sm->bias)) : 0ull;
-        (void)d_bias;
         // Asking a barrier costs 66 cycles even when it completed long ago: a stage's two questions go out together, and
         // only a "not yet" is followed by a wait.
         static_assert(UNIT == TC_KB_PER_STAGE, "one hand-over per stage");
@@ -381,6 +366,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                 // that wait also says that the epilogue is done with the scales of the stage NU before this one
                 if (g >= NU) mbar_arrive(smem_u32(&sm->empty[(g - NU) % TC_STAGES]));
                 if constexpr (EXACT) {
+                    const unsigned long long d_bias = umma_desc_plain32(smem_u32(sm->bias));
                     umma_i8_same_a<0>(d, d_bias, d_bias, idesc);
                     umma_i8_same_a<1>(d + BN, d_bias, d_bias, idesc);
                     umma_i8_same_a<1>(d + 2 * BN, d_bias, d_bias, idesc);
@@ -615,12 +601,8 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     auto scales = [&](const int kk) {
                         Scales c;
                         c.w = lds_f32(st_sw + kk * (TC_BM * 4));
-                        if constexpr (TP >= 2) {
 #pragma unroll
-                            for (int i = 0; i < TP; i += 2) lds_2x64(st_sx + kk * (BN * 4) + i * 8, c.x[i], c.x[i + 1]);
-                        } else {
-                            c.x[0] = lds_64(st_sx + kk * (BN * 4));
-                        }
+                        for (int i = 0; i < TP; i += 2) lds_2x64(st_sx + kk * (BN * 4) + i * 8, c.x[i], c.x[i + 1]);
                         return c;
                     };
                     auto chains = [&](const int32_t (&S)[COLS], const int p, const Scales& sc) {
