@@ -106,8 +106,8 @@ def test_operator_gemm_with_scales_that_are_not_f16(ops, orc, m, k, n):
     bs = (10.0 ** rng.uniform(-4, 0, size=(n, k // 32))).astype(F32)
     bs[2] = 10.0 ** rng.uniform(-44, -8, size=k // 32)
     bs[4, 1], bs[5, 2], bs[6, 3], bs[n - 1, 0] = 1e-12, 3e-39, 1e13, 1e30
-    bs[7], bs[8, 1:] = 2.0 ** -25, np.nextafter(F32(2.0 ** -25), F32(0))   # the last inside and the first outside
-    bs[9], bs[10, 0] = np.nextafter(F32(2.0 ** 40), F32(0)), 2.0 ** 40
+    bs[7], bs[8, 1:] = 2.0 ** -49, np.nextafter(F32(2.0 ** -49), F32(0))   # the last inside and the first outside
+    bs[9], bs[10, 0] = np.nextafter(F32(2.0 ** 16), F32(0)), 2.0 ** 16
     bq = rng.integers(-127, 128, size=(n, k), dtype=np.int8)
     w = ops.QuantWeight(ops.DT_Q4_0, raw, m, k)
     want = np.stack([orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], m, k) for j in range(n)])

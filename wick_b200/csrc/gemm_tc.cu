@@ -27,6 +27,7 @@
 // the CTA frees its tensor memory and exits.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -53,8 +54,8 @@ constexpr int TC_EPI_WARPS = 4 * TC_COL_GROUPS;
 constexpr int TC_THREADS = 32 * (4 + TC_EPI_WARPS);
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
 
-// Weight scales are stored times 2^72 (exact): what the exact epilogue needs, see there.
-constexpr float TC_SCALE_UP = 0x1p72f, TC_SCALE_DOWN = 0x1p-72f, TC_EXACT_DOWN = 0x1p77f;
+// Weight scales are stored times 2^96 (exact): what the exact epilogue needs, see there.
+constexpr float TC_SCALE_UP = 0x1p96f, TC_SCALE_DOWN = 0x1p-96f, TC_EXACT_DOWN = 0x1p53f;
 
 template <int BN>
 struct alignas(1024) TcStage {
@@ -78,6 +79,7 @@ struct TcSmem {
     unsigned long long tmem_empty[tc_units<BN>()];  // all epilogue warps have read them
     uint32_t tmem_base;
     volatile uint32_t abort;
+    volatile uint32_t odd_scale;              // ANY_SCALE: there is something to repair
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -257,7 +259,60 @@ __device__ __forceinline__ TcTile tc_decode_tile(const TcJob& job, int t, int ti
     return r;
 }
 
-template <int BN, bool SUMS, bool EXACT>
+// Activation scales with which the exact epilogue's chains are not the reference's: d = d_w * d_x must keep p * d * 2^-53 a normal
+// f32 and d * 2^96 finite for every finite f16 d_w (magnitudes [2^-24, 2^16)).  The library's quantiser rounds to f16 and stays
+// inside, an overflow to infinity apart; a caller of the operators may bring any f32.
+__device__ __forceinline__ bool tc_odd_scale(float x) {
+    constexpr uint32_t LOW = 0x27000000u, END = 0x47800000u;  // 2^-49, 2^16
+    const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+    return u != 0u && u - LOW >= END - LOW;
+}
+// Whether xs[0..count) holds one, as far as this thread looks: elements `first`, first + step, ...
+__device__ __forceinline__ bool tc_any_odd_scale(const float* xs, int first, int step, int count) {
+    bool odd = false;
+#pragma unroll 4
+    for (int i = first; i < count; i += step) {
+        float x;
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(xs + i));  // (not to be moved above the dependency wait)
+        odd |= tc_odd_scale(x);
+    }
+    return odd;
+}
+
+// One output in the reference's plain form, for tokens with such scales (not expected: no attempt at speed).
+__device__ __noinline__ float tc_exact_plain(const TcJob& job, int mat, int row, int tok, const float* x_scales, int k) {
+    const int nb = k / QK, m_pad = job.m_pad[mat];
+    const int *w = reinterpret_cast<const int*>(job.wq[mat] + (size_t)row * k), *x = reinterpret_cast<const int*>(job.xq + (size_t)tok * k);
+    const float *ws = job.scales_t[mat] + row, *xs = x_scales + (size_t)tok * nb;
+    float acc[2][4] = {};
+#pragma unroll 1
+    for (int b = 0; b < nb; b++, w += 8, x += 8, ws += m_pad) {
+        const float d = __fmul_rn(*ws * TC_SCALE_DOWN, xs[b]);
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            const float t = __fmul_rn((float)dp4a_ss(w[4 + l], x[4 + l], dp4a_ss(w[l], x[l], 0)), d);
+            if (b & 1) acc[1][l] = __fadd_rn(acc[1][l], t);
+            else acc[0][l] = __fadd_rn(acc[0][l], t);
+        }
+    }
+    const float e = __fadd_rn(__fadd_rn(acc[0][0], acc[0][1]), __fadd_rn(acc[0][2], acc[0][3]));
+    const float o = __fadd_rn(__fadd_rn(acc[1][0], acc[1][1]), __fadd_rn(acc[1][2], acc[1][3]));
+    return __fadd_rn(e, o);
+}
+
+// A tile's tokens with odd scales once more.
+__device__ __noinline__ void tc_repair_tile(const TcJob& job, const TcTile& tl, const float* x_scales, int n, int k, int tokens) {
+    const int nb = k / QK;
+    for (int tok = tl.n0; tok < min(n, tl.n0 + tokens); tok++) {
+        if (!__syncthreads_or(tc_any_odd_scale(x_scales + (size_t)tok * nb, threadIdx.x, blockDim.x, nb))) continue;
+        for (int row = tl.m0 + threadIdx.x; row < min(job.m[tl.mat], tl.m0 + TC_BM); row += blockDim.x)
+            job.out[tl.mat][(size_t)tok * job.m[tl.mat] + row] = tc_exact_plain(job, tl.mat, row, tok, x_scales, k);
+    }
+}
+
+// ANY_SCALE: the CTA looks at its tokens' scales while its first stage is on its way, and repairs its tiles if it must.  For the
+// small tiles only (a CTA has few of them); behind a GEMM of large ones k_tc_odd_scales does that.
+template <int BN, bool SUMS, bool EXACT, bool ANY_SCALE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap map_x,
           const float* __restrict__ x_scales,  // [n][k/32]
@@ -293,6 +348,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             mbar_init(smem_u32(&sm->tmem_empty[b]), TC_EPI_WARPS);
         }
         sm->abort = 0;
+        sm->odd_scale = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -554,14 +610,13 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             // multiply-adds + 2 packed additions + 1/2 + 1/2 for the scales, two tokens per instruction:
             //  - tensor memory holds v = p + 2^17 > 0 (the bias instruction).  Read as an f32, a positive integer below 2^23
             //    is the denormal v * 2^-149, which the FMA pipe takes at full rate: no conversion.
-            //  - d = f16(d_w) * d_x rounds the same when the weight scale is stored times 2^72 (D = d * 2^72), and 2^17 * D is
-            //    exact.  Hence fma(v * 2^-149, D, -2^-132 * D) rounds (v - 2^17) * d * 2^-77 once: it IS
-            //    RN(float(p) * d) * 2^-77, the reference's rounded product, and no contraction with the addition can occur.
-            //  - the chains run scaled by 2^-77.  Scales are f16 values, so every term is a multiple of 2^-48: nothing falls
+            //  - d = f16(d_w) * d_x rounds the same when the weight scale is stored times 2^96 (D = d * 2^96), and 2^17 * D is
+            //    exact.  Hence fma(v * 2^-149, D, -2^-132 * D) rounds (v - 2^17) * d * 2^-53 once: it IS
+            //    RN(float(p) * d) * 2^-53, the reference's rounded product, and no contraction with the addition can occur.
+            //  - the chains run scaled by 2^-53.  Scales are f16 values, so every term is a multiple of 2^-48: nothing falls
             //    into the denormal range (2^-125) and every rounding is the unscaled one; the final sum is multiplied back.
-            //  - scales outside launch_gemm_tc_exact's range are kept away from here: an infinite one would make every term
-            //    Inf - Inf.  (Looked for in this kernel - NaN outputs in the epilogue, scales in the loading warps - they cost
-            //    1 to 7 % of every product.)
+            //    Other scales: tc_odd_scale.  (Looked for here - NaN outputs in the epilogue, scales in the loading warps -
+            //    they cost the large tiles 1 to 7 %, mostly by what the compiler then made of the loop.)
             // 6144 x 2048 at 512 tokens: 157 -> 117 us (110 TFLOP/s); FMA pipe two thirds busy, the rest is the hand-over: both
             // warps of a scheduler wait at the same time.  Tried: columns split between the groups with barriers and MMAs of
             // their own (123), the groups kept half a stage apart (144), sixteen warps of 4 tokens (131), the next stage's
@@ -569,6 +624,11 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             constexpr int TP = COLS / 8;  // token pairs per thread
             const f32x2 unbias = pack2(-__uint_as_float(1u << 17), -__uint_as_float(1u << 17));  // -2^-132
             const uint32_t sw0 = smem_u32(&sm->stage[0].sw[0][row_in_tile]), sx0 = smem_u32(&sm->stage[0].sx[0][cg * 2 * TP]);
+            if constexpr (ANY_SCALE)
+                for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+                    const int n0 = tc_decode_tile(job, t, tiles_n, TOK).n0;
+                    if (tc_any_odd_scale(x_scales + (size_t)n0 * nb, threadIdx.x - 128, 32 * TC_EPI_WARPS, min(TOK, n - n0) * nb)) sm->odd_scale = 1;
+                }
             bool ready = false;  // the answer of a question asked during the stage before
             f32x2 acc2[TP][2][4];         // [pair][block parity][lane group], halves = the pair's tokens
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -666,6 +726,23 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
+    if constexpr (ANY_SCALE) {
+        if (sm->odd_scale && !sm->abort)
+            for (int t = blockIdx.x; t < tiles; t += gridDim.x) tc_repair_tile(job, tc_decode_tile(job, t, tiles_n, TOK), x_scales, n, k, TOK);
+    }
+}
+
+// Behind an exact GEMM of large tiles: one warp per CTA, four CTAs to an SM, which fit beside the GEMM's and so are there when it
+// ends.  Bound: latency, one launch and one trip to L2 (6144 x 2048 at 512 columns: 113.5 -> 115.2 us; with CTAs of eight warps
+// 116.5, which behind the small tiles were 8.7 -> 10.8).
+__global__ void __launch_bounds__(32) k_tc_odd_scales(const __grid_constant__ TcJob job, const float* x_scales, int n, int k) {
+    pdl_enter(x_scales);
+    const int nb = k / QK;
+    for (int tok = blockIdx.x; tok < n; tok += gridDim.x) {
+        if (!__any_sync(0xffffffffu, tc_any_odd_scale(x_scales + (size_t)tok * nb, threadIdx.x, 32, nb))) continue;
+        for (int mat = 0; mat < job.count; mat++)
+            for (int row = threadIdx.x; row < job.m[mat]; row += 32) job.out[mat][(size_t)tok * job.m[mat] + row] = tc_exact_plain(job, mat, row, tok, x_scales, k);
+    }
 }
 
 }  // namespace
@@ -745,7 +822,7 @@ cudaError_t device_sm_count(int* sms) {
     return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
-template <int BN, bool EXACT>
+template <int BN, bool EXACT, bool ANY_SCALE = false>
 cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_x, const float* x_scales, int n, int k,
                       int32_t* sums, uint32_t* err) {
     const size_t smem = sizeof(TcSmem<BN>) + 1024;
@@ -753,19 +830,19 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     cudaError_t e = device_sm_count(&sm_count);
     if (e != cudaSuccess) return e;
     static RaisedPerDevice limit, limit_sums;
-    e = raise_dynamic_smem(limit, (const void*)k_gemm_tc<BN, false, EXACT>, smem);
+    e = raise_dynamic_smem(limit, (const void*)k_gemm_tc<BN, false, EXACT, ANY_SCALE>, smem);
     if constexpr (!EXACT)
-        if (e == cudaSuccess) e = raise_dynamic_smem(limit_sums, (const void*)k_gemm_tc<BN, true, false>, smem);
+        if (e == cudaSuccess) e = raise_dynamic_smem(limit_sums, (const void*)k_gemm_tc<BN, true, false, false>, smem);
     if (e != cudaSuccess) return e;
     const int tiles = job.tile_start[job.count];
     const int grid = tiles < sm_count ? tiles : sm_count;
     g_kernel_launches++;
     if constexpr (!EXACT) {
         if (sums) {
-            return launch_pdl(st, k_gemm_tc<BN, true, false>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, sums, n, k, err);
+            return launch_pdl(st, k_gemm_tc<BN, true, false, false>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, sums, n, k, err);
         }
     }
-    return launch_pdl(st, k_gemm_tc<BN, false, EXACT>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, nullptr, n, k, err);
+    return launch_pdl(st, k_gemm_tc<BN, false, EXACT, ANY_SCALE>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, nullptr, n, k, err);
 }
 
 cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, int count, int tiles_n) {
@@ -777,6 +854,7 @@ cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, in
         if (i >= count) continue;
         if (w[i]->k != w[0]->k) return cudaErrorInvalidValue;
         job.map_w[i] = w[i]->map;
+        job.wq[i] = w[i]->q;
         job.scales_t[i] = w[i]->scales_t;
         job.out[i] = out[i];
         job.m[i] = w[i]->m;
@@ -823,7 +901,7 @@ cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* con
 }
 
 cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,
-                                 const float* x_scales, int n, uint32_t* err) {
+                                 const float* x_scales, int n, bool any_scale, uint32_t* err) {
     if (n <= 0 || count <= 0) return cudaSuccess;
     if (count > 3) return cudaErrorInvalidValue;
     TcJob job;
@@ -841,8 +919,13 @@ cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, floa
     e = fill_job(job, w, out, count, (n + tok - 1) / tok);
     if (e != cudaSuccess) return e;
     job.xq = xq;
-    return narrow ? launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, CUtensorMap{}, x_scales, n, w[0]->k, nullptr, err)
-                  : launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, CUtensorMap{}, x_scales, n, w[0]->k, nullptr, err);
+    const CUtensorMap none{};
+    if (narrow && any_scale) return launch_tc<2 * TC_EXACT_TOKENS, true, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
+    if (narrow) return launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
+    e = launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
+    if (e != cudaSuccess || !any_scale) return e;
+    g_kernel_launches++;
+    return launch_pdl(st, k_tc_odd_scales, dim3(std::min(n, 4 * sms)), dim3(32), 0, job, x_scales, n, w[0]->k);
 }
 
 }  // namespace wick

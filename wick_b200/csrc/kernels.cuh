@@ -132,8 +132,6 @@ struct GemvJob {
 void launch_gemv(cudaStream_t st, const GemvJob& job, const float* xs, const int8_t* xq);
 // Integer GEMM over n quantised tokens, out[j*m + i] (simd.rs:696-1019).
 void launch_gemm(cudaStream_t st, const DevWeight& w, const float* bs, const int8_t* bq, int n, float* out);
-// Behind launch_gemm_tc_exact where the activation scales are a caller's: recomputes the tokens whose scales it cannot take.
-void launch_gemm_odd_scales(cudaStream_t st, const DevWeight& w, const float* bs, const int8_t* bq, int n, float* out);
 void launch_block_sums(cudaStream_t st, const DevWeight& w, const int8_t* xq, int32_t* S);
 
 // Multi-sequence decode step (kernels_batch.cu): row j of n is the next token of its own sequence, with its own

@@ -225,45 +225,4 @@ void launch_gemm(cudaStream_t st, const DevWeight& w, const float* bs, const int
     else g_kernel_launches++, launch_pdl(st, k_gemm<DT_Q8_0>, dim3(grid), dim3(256), 0, w, bs, bq, n, out);
 }
 
-// ── behind the exact tensor-core GEMM: tokens whose scales it cannot take ───
-// It needs activation scales that are 0 or in [2^-25, 2^40) by magnitude.  The library's quantiser gives f16 values (an overflow to
-// infinity apart), but a caller of the operators may bring any f32.  A warp looks at one token's scales; the CTA computes the
-// outputs of the tokens that have others (not expected: no attempt at speed) as k_gemv does.  Bound: one launch and one trip to
-// L2, about 2 us where no token does.
-constexpr int ODD_TOKENS = 8;
-template <int DT>
-__global__ void __launch_bounds__(ODD_TOKENS * 32) k_gemm_odd_scales(DevWeight w, const float* __restrict__ bs, const int8_t* __restrict__ bq, int n,
-                                                                      float* __restrict__ out) {
-    pdl_enter(bs, bq, out);
-    __shared__ uint32_t odd[ODD_TOKENS];
-    constexpr uint32_t LOW = 0x33000000u, END = 0x53800000u;  // 2^-25, 2^40
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = w.k, nb = k / QK;
-    const int j0 = blockIdx.x * ODD_TOKENS;
-    bool mine = false;
-    for (int b = lane; b < nb && j0 + warp < n; b += 32) {
-        const uint32_t u = __float_as_uint(bs[(size_t)(j0 + warp) * nb + b]) & 0x7fffffffu;
-        mine |= u != 0u && u - LOW >= END - LOW;
-    }
-    mine = __any_sync(0xffffffffu, mine);
-    if (lane == 0) odd[warp] = mine;
-    __syncthreads();
-    for (int t = 0; t < ODD_TOKENS; t++) {
-        if (!odd[t]) continue;
-        const size_t j = j0 + t;
-        for (int g = warp; g < w.groups(); g += ODD_TOKENS) {
-            const float acc = reduce_row8(gemv_chain<DT>(w, g, lane, reinterpret_cast<const int*>(bq + j * k), bs + j * nb));
-            const int row = g * 4 + ((lane >> 2) & 3);
-            if ((lane & 19) == 0 && row < w.m) out[j * w.m + row] = acc;
-        }
-    }
-}
-
-void launch_gemm_odd_scales(cudaStream_t st, const DevWeight& w, const float* bs, const int8_t* bq, int n, float* out) {
-    if (!n || !w.m) return;
-    const dim3 grid((n + ODD_TOKENS - 1) / ODD_TOKENS), block(ODD_TOKENS * 32);
-    g_kernel_launches++;
-    if (w.dtype == DT_Q4_0) launch_pdl(st, k_gemm_odd_scales<DT_Q4_0>, grid, block, 0, w, bs, bq, n, out);
-    else launch_pdl(st, k_gemm_odd_scales<DT_Q8_0>, grid, block, 0, w, bs, bq, n, out);
-}
-
 }  // namespace wick

@@ -729,7 +729,7 @@ void run_gemms(wick_cuda_model* m, int n, std::initializer_list<GemmTarget> list
         const bool is_hs = tw[0]->k == hs;
         cudaError_t e;
         if (tc_exact) {
-            e = launch_gemm_tc_exact(st, tw, outs, c, m->q8q, m->q8s, n, m->tc_err);
+            e = launch_gemm_tc_exact(st, tw, outs, c, m->q8q, m->q8s, n, /*any_scale=*/false, m->tc_err);
         } else {
             e = launch_gemm_tc(st, tw, outs, c, is_hs ? m->map_x_hs : m->map_x_is, m->q8s, n, nullptr, m->tc_err);
         }
@@ -2113,8 +2113,7 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
             if (w->tc_exact) {
                 const TcWeight* tw[1] = {&w->tc};
                 float* outs[1] = {out_dev};
-                CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
-                launch_gemm_odd_scales(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
+                CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, /*any_scale=*/true, w->tc_err));
                 OP_END();
             }
         }
@@ -2150,8 +2149,7 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     const TcWeight* tw[1] = {&w->tc};
     float* outs[1] = {out_dev};
     if (w->tc_exact) {
-        CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
-        launch_gemm_odd_scales(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
+        CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, /*any_scale=*/true, w->tc_err));
     } else {
         launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
     }
