@@ -32,7 +32,6 @@ constexpr int NCT = NC * 32;
 constexpr int TEAM_WARPS = MEGA_TEAM_WARPS;  // consumer warps work on ring slots in teams
 constexpr int NTEAMS = MEGA_TEAMS;
 constexpr int TEAM_THREADS = TEAM_WARPS * 32;
-constexpr int SPLIT_PAIR_STEPS = 48;  // two groups in a slot are split over the team's warps above this many steps
 constexpr unsigned SPIN_LIMIT = 1u << 22;  // x ~0.25-2 us per iteration
 constexpr unsigned WAIT_NS = 2000;         // hardware suspend limit of one mbarrier test
 
@@ -1210,9 +1209,11 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                         if (c.stamp && nst < 4) c.stamp[nst * 4 + 1] = globaltimer_ns();
                         uint8_t* base = S.ring + (size_t)slot * P.slot_bytes;
                         const int n = nb >> 1;
-                        // One group (or two long ones) per team: the steps of each are shared out to the team's warps, the
-                        // owner takes the first part and adds the others' terms after the sync
-                        const bool split = ng == 1 || (ng == 2 && n > SPLIT_PAIR_STEPS);
+                        // One group for a team of three: its steps are shared out to the team's warps, the owner takes the first part
+                        // and adds the others' terms after the sync.  Two groups are left to two warps, whatever their length
+                        // (split as well: 431.6 against 426.7 us per token with rows of 3584 in Q8_0; 423.3 against 418.3 for the
+                        // 1.6B model's Q4_0).  The loop below is over that one group; without it 1.6B Q4_0 takes 420.
+                        const bool split = ng == 1;
                         const int part = ((n + TEAM_WARPS - 1) / TEAM_WARPS + 3) & ~3;  // whole batches
                         // residual-add epilogue: the old value of the row is fetched now, so that its latency runs
                         // under the chain step instead of after it (a warp owns at most two groups of a slot)
@@ -1224,7 +1225,7 @@ __device__ void consumer(const MegaParams& P, const Smem& S, int cta, int ncta) 
                                 if (gi < ng && row < wm) resid[q] = __ldcg(y + row);
                             }
                         }
-                        float first = 0.0f;  // split: the owner's part of its group
+                        float first = 0.0f;  // split: the owner's part of the group
                         if (split) {
                             for (int gi = 0; gi < ng; gi++) {
                                 uint32_t* q = reinterpret_cast<uint32_t*>(base + (size_t)gi * qgb) + w_at;
