@@ -280,12 +280,12 @@ def test_bounded_waits_report_timeout(wick, model_dir):
 
 
 def test_split_scores_long_context_decode(wick, orc, model_dir, monkeypatch):
-    """From 768 cached tokens on, decode computes the cached keys' scores in a phase of its own (keys split over
+    """From 1152 cached tokens on (models of few heads), decode computes the cached keys' scores in a phase of its own (keys split over
     all CTAs).  Same bits as the in-phase loop (switched back on by WICK_CUDA_NO_SPLIT_SCORES) and as the oracle,
     across the switch-over point and for the device-resident loop."""
     from wick_b200 import gguf_synth as gs
     path = _model_path(model_dir, "tiny-wide", "q4_0")
-    toks = gs.random_prompt(760, gs.SPECS["tiny-wide"].vocab, seed=12)
+    toks = gs.random_prompt(1144, gs.SPECS["tiny-wide"].vocab, seed=12)
     a = wick.CudaLfm2Model(path, 2048)
     sa = wick.InferenceState()
     la = a.forward_prefill(toks, 0, sa)
@@ -293,7 +293,7 @@ def test_split_scores_long_context_decode(wick, orc, model_dir, monkeypatch):
     lo = om.forward_prefill(toks, 0)
     assert_logits_equal(la, lo, "prefill")
     tok = orc.argmax(lo)
-    for i in range(20):                      # positions 760..779: the list switches at 768
+    for i in range(20):                      # positions 1144..1163: the list switches at 1152
         x, y = a.forward([tok], sa.seq_len, sa), om.forward(tok)
         assert_logits_equal(x, y, f"step {i}")
         tok = orc.argmax(y)
@@ -302,7 +302,7 @@ def test_split_scores_long_context_decode(wick, orc, model_dir, monkeypatch):
     monkeypatch.setenv("WICK_CUDA_NO_SPLIT_SCORES", "1")
     b = wick.CudaLfm2Model(path, 2048)
     sb = wick.InferenceState()
-    more = gs.random_prompt(900, gs.SPECS["tiny-wide"].vocab, seed=13)
+    more = gs.random_prompt(1300, gs.SPECS["tiny-wide"].vocab, seed=13)
     lb = b.forward_prefill(more, 0, sb)
     monkeypatch.delenv("WICK_CUDA_NO_SPLIT_SCORES")
     la2 = a.forward_prefill(more, 0, sa)

@@ -795,7 +795,7 @@ __device__ void phase_attention(Ctx& c, const MegaPhase& ph, int pos) {
     float* sc = c.S.xf;
     float *qs = c.S.head, *ks = c.S.head + 256;
     const int seq = pos + 1;
-    const int sl = LONG && 2 * n_heads * (hd / 16) <= c.ncta ? 8 : 16;  // output dims per item
+    const int sl = LONG && mega_narrow_slices(P, c.ncta) ? 8 : 16;  // output dims per item
     const int nq = hd / sl, items = n_heads * nq;
     const int nf = xf_floats(P);
     const int sc_pad = (seq + 3) & ~3;

@@ -102,6 +102,9 @@ struct MegaParams {
 // Longest hidden row a flag_in phase handles (15 consumer warps x 5 blocks x 32 elements).
 constexpr int MEGA_FLAGGED_MAX_K = 2400;
 
+// Long contexts: whether slices of 8 output dims leave no more items than CTAs (slices of 16 would leave half of them idle).
+__host__ __device__ inline bool mega_narrow_slices(const MegaParams& P, int ctas) { return 2 * P.n_heads * (P.head_dim / 16) <= ctas; }
+
 size_t mega_smem_bytes(const MegaParams& P);
 // Launches the persistent kernel (cooperative: one CTA per SM, all co-resident).
 cudaError_t launch_decode_mega(cudaStream_t st, const MegaParams& P, int n_ctas);

@@ -120,6 +120,7 @@ struct wick_cuda_model {
     int n_phases_long = 0;
     float* scores_g = nullptr;
     bool last_launch_long = false, long_ok = false;
+    uint32_t long_from = 0;  // cached keys from which decode takes that list
     MegaLayer* d_mlayers = nullptr;
     unsigned long long* d_sync = nullptr;  // [0] barrier counter, [1..2] argmax accumulators
     unsigned long long* hidden_flagged = nullptr;  // [hs] flagged copy of the hidden row (persistent decode kernel)
@@ -487,6 +488,12 @@ int32_t build_mega(wick_cuda_model* m) {
         PL.n_phases = m->n_phases_long;
         PL.phases = m->d_phases_long;
         m->long_ok = mega_max_ctas(PL) >= m->mega_ctas;
+        // One more grid barrier per attention layer and a scores phase, against a scores loop that grows with the keys and with the
+        // items per CTA.  us per token without / with them: 350M Q4_0 (8-wide slices, half the V bytes per item) at 1088 keys
+        // 441 / 443, at 1152 448 / 446; Q8_0 at 1152 445 / 450, at 1216 453 / 453; 1.6B Q4_0 (128 items of 16) at 1472 547 / 550, at
+        // 1536 552 / 551; Q8_0 at 1600 630 / 633, at 1664 639 / 637; 56 heads (224 items) Q4_0 at 896 367 / 370, at 1024 376 / 375.
+        const uint32_t items = (uint32_t)(P.n_heads * (P.head_dim / 16)), ctas = (uint32_t)std::max(m->mega_ctas, 1);
+        m->long_from = mega_narrow_slices(P, m->mega_ctas) ? 1152 : 1536 * ctas / std::max(items, ctas);
     }
     m->mega_ok = m->mega_ctas > 0;
     return WICK_CUDA_OK;
@@ -495,16 +502,12 @@ int32_t build_mega(wick_cuda_model* m) {
 // Runs n decode steps with the persistent kernel; ctl holds token / pos / step on entry.
 void logits_matvec(wick_cuda_model* m);
 
-// Contexts from this length on decode with the split-scores phase list (one extra grid barrier per attention layer,
-// ~2.5 us, against a scores loop that grows by ~12 ns per cached key and CTA).
-static const uint32_t MEGA_LONG_CTX = 768;
-
 // `embedding`: device row [hidden] that takes the place of the token's embedding (one step only).
 int32_t run_mega(wick_cuda_model* m, int n_tokens, bool greedy, const float* embedding = nullptr) {
     MegaParams P = m->mega;
     P.greedy = greedy ? 1 : 0;
     P.embedding = embedding;
-    m->last_launch_long = m->long_ok && m->seq_len >= MEGA_LONG_CTX && getenv("WICK_CUDA_NO_SPLIT_SCORES") == nullptr;
+    m->last_launch_long = m->long_ok && m->seq_len >= m->long_from && getenv("WICK_CUDA_NO_SPLIT_SCORES") == nullptr;
     if (m->last_launch_long) {
         P.phases = m->d_phases_long;
         P.n_phases = m->n_phases_long;
