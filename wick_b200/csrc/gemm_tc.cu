@@ -310,8 +310,8 @@ __device__ __noinline__ void tc_repair_tile(const TcJob& job, const TcTile& tl, 
     }
 }
 
-// ANY_SCALE: the CTA looks at its tokens' scales while its first stage is on its way, and repairs its tiles if it must.  For the
-// small tiles only (a CTA has few of them); behind a GEMM of large ones k_tc_odd_scales does that.
+// ANY_SCALE: the CTA looks at its tokens' scales while its first stage is on its way, and repairs its tiles if it must.  For launches
+// of few tiles per CTA; behind the others k_tc_odd_scales does that (launch_gemm_tc_exact).
 template <int BN, bool SUMS, bool EXACT, bool ANY_SCALE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap map_x,
@@ -732,7 +732,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     }
 }
 
-// Behind an exact GEMM of large tiles: one warp per CTA, four CTAs to an SM, which fit beside the GEMM's and so are there when it
+// Behind an exact GEMM of many tiles: one warp per CTA, four CTAs to an SM, which fit beside the GEMM's and so are there when it
 // ends.  Bound: latency, one launch and one trip to L2 (6144 x 2048 at 512 columns: 113.5 -> 115.2 us; with CTAs of eight warps
 // 116.5, which behind the small tiles were 8.7 -> 10.8).
 __global__ void __launch_bounds__(32) k_tc_odd_scales(const __grid_constant__ TcJob job, const float* x_scales, int n, int k) {
@@ -920,9 +920,15 @@ cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, floa
     if (e != cudaSuccess) return e;
     job.xq = xq;
     const CUtensorMap none{};
-    if (narrow && any_scale) return launch_tc<2 * TC_EXACT_TOKENS, true, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
-    if (narrow) return launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
-    e = launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
+    // Who looks at a caller's scales: the kernel itself costs the large tiles 0.3 to 0.9 us a wave (its loop is compiled worse with
+    // the second pass behind it), a kernel behind it 1.5 to 5 us: 3072 x 1024 at 81 columns, one wave, 11.1 / 16.0; 6144 x 2048 at
+    // 96, two, 25.0 / 25.7; at 256, six, 67.3 / 65.2 us.  The small tiles, 16.8 us with or without, always do it themselves.
+    const bool looks = any_scale && (narrow || wide_waves <= 2);
+    if (narrow) e = looks ? launch_tc<2 * TC_EXACT_TOKENS, true, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err)
+                          : launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
+    else e = looks ? launch_tc<4 * TC_EXACT_TOKENS, true, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err)
+                   : launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
+    any_scale = any_scale && !looks;
     if (e != cudaSuccess || !any_scale) return e;
     g_kernel_launches++;
     return launch_pdl(st, k_tc_odd_scales, dim3(std::min(n, 4 * sms)), dim3(32), 0, job, x_scales, n, w[0]->k);
