@@ -14,7 +14,8 @@
 //     quantised input from shared memory without bank conflicts (grouped layout, DevWeight);
 //   * the small operators between mat-vecs (RMSNorm + Q8_0 quantise, short-conv gating,
 //     SwiGLU, attention-output quantise) are recomputed by every CTA as the prologue of the
-//     phase that consumes them, so a phase boundary is exactly one grid-wide barrier;
+//     phase that consumes them, so a phase boundary is one grid-wide barrier, or none where the hidden row is handed
+//     over element by element in flagged words (33 of the 71 phases);
 //   * residual adds and the argmax are epilogues of the mat-vec that produces their input.
 // Arithmetic and its order are those of the per-kernel path (and of the CPU reference).
 //

@@ -701,7 +701,7 @@ void prof_collect(wick_cuda_model* m) {  // after the stream has been synchronis
     m->prof_used = 0;
 }
 
-// The int8 weight copies of the tensor-core GEMMs (1.7 bytes per parameter) are made by the first chunk of more than
+// The int8 weight copies of the tensor-core GEMMs (1.125 bytes per parameter) are made by the first chunk of more than
 // TC_BUILD_ABOVE tokens, so that decoding and the shortest prompts leave a model at its packed size.  Once they are there
 // the bit-exact GEMM uses them from two tokens on: its 8-token tile costs the same for 2 tokens as for 8, and the CUDA-core
 // kernel needs several times as long at any of these counts (350M, 9-token prompt: 3.7 -> 1.2 ms).  The fused-chain GEMM
@@ -805,8 +805,7 @@ void enqueue_prefill_chunk(wick_cuda_model* m, int n, int start_pos, bool flash,
 }
 
 // Tensor-core prefill GEMM: decided at load (tc_ok = the shapes allow it), built on first use (ensure_tc): the int8
-// copies of the layer matrices, the activation tensor maps and the masked-activation buffer cost about 1.7 bytes per
-// parameter, which a decode-only user never needs.
+// copies of the layer matrices cost 1.125 bytes per parameter, which a decode-only user never needs.
 int32_t build_tc(wick_cuda_model* m) {
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size;
     const char* mode = getenv("WICK_CUDA_PREFILL");
