@@ -618,9 +618,9 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             //    Other scales: tc_odd_scale.  (Looked for here - NaN outputs in the epilogue, scales in the loading warps -
             //    they cost the large tiles 1 to 7 %, mostly by what the compiler then made of the loop.)
             // 6144 x 2048 at 512 tokens: 157 -> 113.5 us (113 TFLOP/s).  Of the FMA pipe's time 48 % is this arithmetic, 6 % integer
-            // multiply-adds, 46 % idle at the hand-over: both warps of a scheduler wait at the same time.  Tried: columns split between the groups with barriers and MMAs of
-            // their own (123), the groups kept half a stage apart (144), sixteen warps of 4 tokens (131), the next stage's
-            // first block loaded before the last chains (145 to 179).
+            // multiply-adds, 46 % idle at the hand-over: both warps of a scheduler wait at the same time.  Tried: columns split
+            // between the groups with barriers and MMAs of their own (123), the groups kept half a stage apart (144), sixteen
+            // warps of 4 tokens (131), the next stage's first block loaded before the last chains (145 to 179).
             constexpr int TP = COLS / 8;  // token pairs per thread
             const f32x2 unbias = pack2(-__uint_as_float(1u << 17), -__uint_as_float(1u << 17));  // -2^-132
             const uint32_t sw0 = smem_u32(&sm->stage[0].sw[0][row_in_tile]), sx0 = smem_u32(&sm->stage[0].sx[0][cg * 2 * TP]);
