@@ -137,11 +137,9 @@ int32_t wick_cuda_shift_kv(wick_cuda_model* m, uint32_t n_keep, uint32_t shift);
  * runs; a single token or frame is a decode step, with the same bits).  Decode is not affected.
  * EXACT (default): the arithmetic of gemm_q*_q8_0_neon (simd.rs:696-1019) bit for bit, so logits and
  *   greedy tokens equal wick's CPU path.  When hidden and feed-forward sizes are multiples of 128 it
- *   runs on the tensor cores: tcgen05 int8 MMAs against lane-group-masked activations produce the
- *   four int32 lane partials of every block, and the epilogue keeps the reference's eight unfused f32
- *   chains per output; otherwise, and for weights with an infinite scale, on the CUDA-core kernel.  One limit: a
- *   block of activations above 65504 x 127 (8.3 million) has an infinite scale; its token's outputs are then NaN
- *   on the tensor cores, where the CPU path gives infinities and NaN (the operators below do as the CPU path does).
+ *   runs on the tensor cores: one MMA per lane group of a block gives its four integer lane partials, and
+ *   the reference's eight unfused f32 chains per output follow in the same registers; otherwise on the
+ *   CUDA-core kernel.
  * EXACT_CUDA_CORES (env WICK_CUDA_PREFILL=exact-cuda-cores): always the CUDA-core kernel (same bits).
  * TENSOR (env WICK_CUDA_PREFILL=tensor; needs the multiples of 128): the kernel described at
  *   wick_cuda_gemm_q8_tc.  Each product agrees with EXACT to f32 rounding, but the first last-bit
@@ -225,9 +223,9 @@ int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const 
 /* gemm_q4_0_q8_0_neon / gemm_q8_0_q8_0_neon (simd.rs:696-925, :937-1019) over n pre-quantised
  * columns; the result is token-major out[j*m + i] (the reference writes out[i*n + j]).  bq must be 4-byte aligned; bs may hold
  * any f32.  With more than 8 columns and k % 128 == 0 it runs on the tensor cores, with the same bits: the weight's first such
- * call makes an int8 copy of it (1.125 bytes per parameter, kept until the weight is destroyed) and waits for that; repeated
- * products are then 3.7 times as fast as on the CUDA cores, the first one 1.8 times.  Without memory for the copy, while `stream`
- * is captured before the copy exists, and for weights with an infinite scale it runs on the CUDA cores.  A weight created
+ * call makes a copy of it in operand order (1.125 bytes per parameter, kept until the weight is destroyed) and waits for that;
+ * repeated products are then 4 times as fast as on the CUDA cores, the first one 1.9 times.  Without memory for the copy, while
+ * `stream` is captured before the copy exists, and for columns that are not 16-byte aligned it runs on the CUDA cores.  A weight created
  * with WICK_CUDA_PREFILL=exact-cuda-cores in the environment always does, and never makes the copy. */
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev,
                           uint32_t n, float* out_dev, void* stream);
@@ -251,7 +249,7 @@ int32_t wick_cuda_gemm_q8_tc(wick_cuda_weight* w, const float* bs_dev, const int
                              float* out_dev, int32_t* block_sums_dev, void* stream);
 /* The bit-exact product on the tensor cores (the default GEMM of forward_prefill): same result as
  * wick_cuda_gemm_q8, bit for bit.  Needs k % 128 == 0.  Synchronises `stream` (operator entry point for
- * tests) and, like wick_cuda_gemm_q8_tc, makes the weight's int8 copy on its first call. */
+ * tests) and makes the weight's copy on its first call, like wick_cuda_gemm_q8 (wick_cuda_gemm_q8_tc has an int8 copy of its own). */
 int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n,
                                    float* out_dev, void* stream);
 /* int32 block dot sums S[i][b] = sum over the 32 elements of block b of row i (the vdotq_s32

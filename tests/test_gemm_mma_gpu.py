@@ -1,0 +1,55 @@
+"""The bit-exact GEMM on the tensor cores at the edges of its tiles, stages and rounds, against the CUDA-core kernel (itself
+compared with the oracle) for every output and the oracle for sampled ones."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+F32 = np.float32
+
+
+@pytest.fixture(scope="module")
+def ops(cuda_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import ops
+    return ops
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+# Row tiles of 16 in groups of 1, 2, 4 and 6, token tiles of 8, 16 and 32; stages of 256 elements, the last one half there (k = 128,
+# 384); more tiles than SMs, with fewer stages to a tile than producer groups.
+@pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("m,k,n", [(1, 128, 1), (16, 256, 8), (17, 384, 9), (95, 640, 16), (97, 1024, 33), (2400, 128, 7), (4808, 128, 65),
+                                   (1000, 384, 24), (9600, 256, 31), (96 * 160, 128, 40), (2048, 1152, 200), (520, 2304, 97)])
+def test_exact_gemm_at_its_edges(ops, orc, cuda_core_weight, dtype, m, k, n):
+    rng = np.random.default_rng(m + k + n)
+    raw = rng.integers(0, 256, size=(m, k // 32, 18 if dtype == "q4_0" else 34), dtype=np.uint8)  # every int8, -128 too
+    raw[:, :, :2] = rng.uniform(-0.02, 0.02, size=(m, k // 32)).astype(np.float16).view(np.uint8).reshape(m, k // 32, 2)
+    bq = rng.integers(-128, 128, size=(n, k), dtype=np.int8)
+    bs = rng.uniform(0.0, 0.1, size=(n, k // 32)).astype(np.float16).astype(F32)
+    dt = ops.QTYPE_ID[dtype]
+    got = ops.gemm_q8_tc_exact(ops.QuantWeight(dt, raw.reshape(-1), m, k), dev(bs), dev(bq))
+    assert torch.equal(got.view(torch.int32), ops.gemm_q8(cuda_core_weight(dt, raw.reshape(-1), m, k), dev(bs), dev(bq)).view(torch.int32))
+    for j in {0, n - 1}:
+        want = orc.gemv(dt, raw.reshape(m, -1), bs[j], bq[j], m, k)
+        assert np.array_equal(got[j].cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+def test_columns_that_are_not_16_byte_aligned(ops, orc):
+    """The tensor cores' kernel reads 16 bytes at a time; a caller's 4-byte aligned columns are served as before."""
+    from wick_b200 import gguf_synth as gs
+    rng = np.random.default_rng(0)
+    m, k, n = 130, 256, 20
+    raw = gs.quantize_q4_0((rng.standard_normal((m, k)) * 0.02).astype(F32))
+    bs, bq = orc.quantize_q8_0(rng.standard_normal((n, k), dtype=F32))
+    w = ops.QuantWeight(ops.DT_Q4_0, raw, m, k)
+    room = torch.zeros(n * k + 4, dtype=torch.int8, device="cuda")
+    room[4:] = dev(bq).flatten()
+    for f in (ops.gemm_q8, ops.gemm_q8_tc_exact):
+        got = f(w, dev(bs), room[4:].view(n, k)).cpu().numpy()
+        for j in range(n):
+            assert np.array_equal(got[j].view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], m, k).view(np.uint32))

@@ -8,20 +8,19 @@
 // S_b is the same integer the NEON kernels produce per block (simd.rs:696-1019, the four lane
 // partials added up); what differs from them is the f32 accumulation: one fused chain per output in
 // block order instead of 2 x 4 unfused lane chains, so outputs agree to f32 rounding (~1e-6 relative),
-// not bit for bit.  The EXACT instantiation (the default of forward_prefill) keeps the four lane partials apart as columns
-// and their eight chains in the epilogue, bit for bit; this one is the throughput option.
+// not bit for bit.  The throughput option; the bit-exact GEMM is gemm_mma.cu.
 //
 // One MMA instruction covers exactly one quantisation block (K = 32 int8), writes a fresh 128 x BN
 // int32 tile into one of 512/BN tensor-memory buffers and never accumulates across blocks, because
 // each block has its own scale pair.  The epilogue warps drain a stage's four buffers (tcgen05.ld), hand them back,
 // and apply the scales on the CUDA cores, which is what bounds the kernel: per (output, block) a conversion and half of
-// two packed instructions here, half of ten packed ones in the EXACT form (see the epilogue).
+// two packed instructions.
 //
 // Roles in a CTA (one CTA per SM, persistent over output tiles; 12 warps):
-//   warp 0  lane 0: TMA producer, one K=128 stage (4 blocks) of W rows (and, not for EXACT, activation rows) per step
+//   warp 0  lane 0: TMA producer, one K=128 stage (4 blocks) of W rows and activation rows per step
 //   warp 1        : issues tcgen05.mma / tcgen05.commit from one elected lane and owns the TMEM allocation
 //   warp 2        : copies the stage's weight scales and (transposed) activation scales into smem (cp.async)
-//   warp 3        : EXACT: spreads the activation words over the lane-group rows of the operand (cp.async)
+//   warp 3        : idle (a warp reads the TMEM lanes of quarter w % 4, so the epilogue starts at a multiple of 4)
 //   warps 4..11   : epilogue; warp w reads TMEM lanes 32*(w%4).. and its group's half of the columns
 // Every wait is bounded: on expiry the kernel records an error code, all roles leave their loops and
 // the CTA frees its tensor memory and exits.
@@ -40,22 +39,18 @@ namespace {
 constexpr int TC_BM = 128;          // weight rows per tile == TMEM lanes
 constexpr int TC_KSTAGE = 128;      // int8 elements (bytes) per row per stage == one 128B swizzle atom
 constexpr int TC_KB_PER_STAGE = TC_KSTAGE / QK;  // 4 quantisation blocks per stage
-// Shared-memory stages: as many as fit (27.6 KB each for 64-column tiles, 23.5 KB for 32).  A stage is
+// Shared-memory stages: as many as fit (27.6 KB each for 64-column tiles).  A stage is
 // only refilled after the epilogue has finished with its scales, and the refill has to be back from L2 before
 // the MMA issuer needs it; with four stages that left about one microsecond, less than a loaded L2 round trip.
 template <int BN>
-__host__ __device__ constexpr int tc_stages() { return BN <= 32 ? 9 : 8; }
-// Hand-over units of tensor memory (512 columns), a stage's blocks each.  32-column tiles fill it with four: with two, a stage could
-// not take less than half the way round (release, MMA issue, MMAs, wait, loads), ~860 cycles for the work of ~400.
+__host__ __device__ constexpr int tc_stages() { return 8; }
+// Hand-over units of tensor memory (512 columns), a stage's blocks each.
 template <int BN>
 __host__ __device__ constexpr int tc_units() { return 512 / (BN * TC_KB_PER_STAGE); }
 constexpr int TC_COL_GROUPS = 2;    // epilogue warps per TMEM lane quarter; each takes half of a tile's columns
 constexpr int TC_EPI_WARPS = 4 * TC_COL_GROUPS;
 constexpr int TC_THREADS = 32 * (4 + TC_EPI_WARPS);
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
-
-// Weight scales are stored times 2^96 (exact): what the exact epilogue needs, see there.
-constexpr float TC_SCALE_UP = 0x1p96f, TC_SCALE_DOWN = 0x1p-96f, TC_EXACT_DOWN = 0x1p53f;
 
 template <int BN>
 struct alignas(1024) TcStage {
@@ -65,21 +60,15 @@ struct alignas(1024) TcStage {
     float sx[TC_KB_PER_STAGE][BN];            // activation scales, transposed to [block][token]
 };
 
-// Bytes of the constant operand of the exact GEMM's bias instruction: 128 rows x 32 bytes, all equal (64 x 64 x 32 = 2^17).
-constexpr int TC_BIAS_BYTES = TC_BM * QK;
-constexpr uint32_t TC_BIAS_WORD = 0x40404040u;
-
 template <int BN>
 struct TcSmem {
     TcStage<BN> stage[tc_stages<BN>()];
-    uint32_t bias[TC_BIAS_BYTES / 4];           // exact GEMM only
     unsigned long long full[tc_stages<BN>()];   // TMA bytes landed + scales written
     unsigned long long empty[tc_stages<BN>()];  // MMAs of the stage retired + epilogue done with its scales
     unsigned long long tmem_full[tc_units<BN>()];   // block sums of a stage are in the unit's part of tensor memory
     unsigned long long tmem_empty[tc_units<BN>()];  // all epilogue warps have read them
     uint32_t tmem_base;
     volatile uint32_t abort;
-    volatile uint32_t odd_scale;              // ANY_SCALE: there is something to repair
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -157,39 +146,13 @@ __device__ __forceinline__ unsigned long long umma_desc_sw128(uint32_t smem_addr
     return d;
 }
 
-// K-major operand tile of 32-byte rows without swizzle: 8 x 16-byte core matrices of 128 bytes, the two halves of a row one
-// core matrix apart, 8-row groups 256 bytes apart (only ever used on a tile whose bytes are all equal).
-__device__ __forceinline__ unsigned long long umma_desc_plain32(uint32_t smem_addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((smem_addr >> 4) & 0x3FFF);
-    d |= (unsigned long long)(128 >> 4) << 16;
-    d |= (unsigned long long)(256 >> 4) << 32;
-    d |= 1ull << 46;
-    return d;
-}
-
-template <bool ACC>
 __device__ __forceinline__ void umma_i8(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 p, 0, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "n"(ACC ? 1 : 0)
+        "l"(da), "l"(db), "r"(idesc)
         : "memory");
-}
-// The constant product: several in a row read the same A operand, which stays in the collector (N = 32: 20 cycles instead
-// of 40, the A operand being read at 64 bytes a cycle).  WHICH: 0 first, 1 between, 2 last.
-template <int WHICH>
-__device__ __forceinline__ void umma_i8_same_a(uint32_t tmem_d, unsigned long long da, unsigned long long db, uint32_t idesc) {
-#define WICK_UMMA_COLLECT(how)                                                                                      \
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"                                                   \
-                 "tcgen05.mma.cta_group::1.kind::i8.collector::a::" how " [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), \
-                 "l"(da), "l"(db), "r"(idesc)                                                                       \
-                 : "memory")
-    if constexpr (WHICH == 0) WICK_UMMA_COLLECT("fill");
-    else if constexpr (WHICH == 1) WICK_UMMA_COLLECT("use");
-    else WICK_UMMA_COLLECT("lastuse");
-#undef WICK_UMMA_COLLECT
 }
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t p;
@@ -213,21 +176,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int32_t* r) {
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, int32_t* r) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-template <int COLS>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, int32_t* r) {
-    static_assert(COLS == 16 || COLS == 32, "one tcgen05.ld per k-block");
-    if constexpr (COLS == 16) tmem_ld16(taddr, r);
-    else tmem_ld32(taddr, r);
 }
 // Shared-memory loads by 32-bit address (a pointer derived from the aligned raw buffer is a generic one to the compiler)
 __device__ __forceinline__ float lds_f32(uint32_t a) {
@@ -259,60 +207,7 @@ __device__ __forceinline__ TcTile tc_decode_tile(const TcJob& job, int t, int ti
     return r;
 }
 
-// Activation scales with which the exact epilogue's chains are not the reference's: d = d_w * d_x must keep p * d * 2^-53 a normal
-// f32 and d * 2^96 finite for every finite f16 d_w (magnitudes [2^-24, 2^16)).  The library's quantiser rounds to f16 and stays
-// inside, an overflow to infinity apart; a caller of the operators may bring any f32.
-__device__ __forceinline__ bool tc_odd_scale(float x) {
-    constexpr uint32_t LOW = 0x27000000u, END = 0x47800000u;  // 2^-49, 2^16
-    const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
-    return u != 0u && u - LOW >= END - LOW;
-}
-// Whether xs[0..count) holds one, as far as this thread looks: elements `first`, first + step, ...
-__device__ __forceinline__ bool tc_any_odd_scale(const float* xs, int first, int step, int count) {
-    bool odd = false;
-#pragma unroll 4
-    for (int i = first; i < count; i += step) {
-        float x;
-        asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(xs + i));  // (not to be moved above the dependency wait)
-        odd |= tc_odd_scale(x);
-    }
-    return odd;
-}
-
-// One output in the reference's plain form, for tokens with such scales (not expected: no attempt at speed).
-__device__ __noinline__ float tc_exact_plain(const TcJob& job, int mat, int row, int tok, const float* x_scales, int k) {
-    const int nb = k / QK, m_pad = job.m_pad[mat];
-    const int *w = reinterpret_cast<const int*>(job.wq[mat] + (size_t)row * k), *x = reinterpret_cast<const int*>(job.xq + (size_t)tok * k);
-    const float *ws = job.scales_t[mat] + row, *xs = x_scales + (size_t)tok * nb;
-    float acc[2][4] = {};
-#pragma unroll 1
-    for (int b = 0; b < nb; b++, w += 8, x += 8, ws += m_pad) {
-        const float d = __fmul_rn(*ws * TC_SCALE_DOWN, xs[b]);
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const float t = __fmul_rn((float)dp4a_ss(w[4 + l], x[4 + l], dp4a_ss(w[l], x[l], 0)), d);
-            if (b & 1) acc[1][l] = __fadd_rn(acc[1][l], t);
-            else acc[0][l] = __fadd_rn(acc[0][l], t);
-        }
-    }
-    const float e = __fadd_rn(__fadd_rn(acc[0][0], acc[0][1]), __fadd_rn(acc[0][2], acc[0][3]));
-    const float o = __fadd_rn(__fadd_rn(acc[1][0], acc[1][1]), __fadd_rn(acc[1][2], acc[1][3]));
-    return __fadd_rn(e, o);
-}
-
-// A tile's tokens with odd scales once more.
-__device__ __noinline__ void tc_repair_tile(const TcJob& job, const TcTile& tl, const float* x_scales, int n, int k, int tokens) {
-    const int nb = k / QK;
-    for (int tok = tl.n0; tok < min(n, tl.n0 + tokens); tok++) {
-        if (!__syncthreads_or(tc_any_odd_scale(x_scales + (size_t)tok * nb, threadIdx.x, blockDim.x, nb))) continue;
-        for (int row = tl.m0 + threadIdx.x; row < min(job.m[tl.mat], tl.m0 + TC_BM); row += blockDim.x)
-            job.out[tl.mat][(size_t)tok * job.m[tl.mat] + row] = tc_exact_plain(job, tl.mat, row, tok, x_scales, k);
-    }
-}
-
-// ANY_SCALE: the CTA looks at its tokens' scales while its first stage is on its way, and repairs its tiles if it must.  For launches
-// of few tiles per CTA; behind the others k_tc_odd_scales does that (launch_gemm_tc_exact).
-template <int BN, bool SUMS, bool EXACT, bool ANY_SCALE>
+template <int BN, bool SUMS>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap map_x,
           const float* __restrict__ x_scales,  // [n][k/32]
@@ -326,11 +221,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
     static_assert(NU >= 2 && (NU & (NU - 1)) == 0, "hand-over units that tile tensor memory");
     constexpr int TC_STAGES = tc_stages<BN>();
     constexpr int COLS = BN / TC_COL_GROUPS;  // columns per epilogue thread
-    // EXACT: a column is (token, NEON lane group); each activation row of the operand is masked to one lane group (warp 3
-    // spreads the words), so a tile covers BN/4 tokens and the MMA yields the four lane partials.  Column order inside a
-    // pair of tokens is (lane group, token of the pair): the epilogue's packed arithmetic works on two tokens at a time.
-    constexpr int TOK = EXACT ? BN / 4 : BN;  // tokens per tile
-    static_assert(!EXACT || ((COLS == 32 || COLS == 16) && !SUMS), "exact epilogue: 8 or 4 tokens x 4 lane groups per thread");
+    constexpr int TOK = BN;  // tokens per tile
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = k / QK;
     const int k_stages = k / TC_KSTAGE;
@@ -339,8 +230,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < TC_STAGES; s++) {
-            // producer (with tx bytes) + every lane of the scale warp + the exact GEMM's activation warp
-            mbar_init(smem_u32(&sm->full[s]), 1 + 32 + (EXACT ? 1 : 0));
+            mbar_init(smem_u32(&sm->full[s]), 1 + 32);  // producer (with tx bytes) + every lane of the scale warp
             mbar_init(smem_u32(&sm->empty[s]), 1);  // the MMA issuer alone, NU stages later (see there)
         }
         for (int b = 0; b < NU; b++) {
@@ -348,15 +238,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             mbar_init(smem_u32(&sm->tmem_empty[b]), TC_EPI_WARPS);
         }
         sm->abort = 0;
-        sm->odd_scale = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if constexpr (EXACT) {
-        // the words that the lane-group masks zero are written once: every refill of a stage stores to the same other words
-        for (int s = 0; s < TC_STAGES; s++)
-            for (int i = threadIdx.x; i < BN * TC_KSTAGE / 16; i += TC_THREADS) reinterpret_cast<uint4*>(sm->stage[s].b)[i] = make_uint4(0u, 0u, 0u, 0u);
-        for (int i = threadIdx.x; i < TC_BIAS_BYTES / 4; i += TC_THREADS) sm->bias[i] = TC_BIAS_WORD;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
@@ -364,11 +246,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // Nothing up to here touches what another kernel writes.  The small tiles, whose kernels are short, also fetch their first
-    // weights (constant data) before they wait, and the other roles wait on their own (9-token prompt 851 -> 827 us); in
-    // the larger ones the waits inside the roles cost more than that gains (4096 tokens: 93.2 against 92.9 ms).
-    constexpr bool WAIT_LATE = EXACT && BN <= 32;
-    if constexpr (!WAIT_LATE) pdl_wait();
+    pdl_wait();  // (nothing up to here touches what another kernel writes)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -388,21 +266,18 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     ok = mbar_wait<BN, 256>(sm, smem_u32(&sm->empty[s]), (u & 1) ^ 1, err, 1);
                     if (!ok) break;
                     const uint32_t bar = smem_u32(&sm->full[s]);
-                    mbar_arrive_expect_tx(bar, (EXACT ? TC_BM : TC_BM + BN) * TC_KSTAGE);
+                    mbar_arrive_expect_tx(bar, (TC_BM + BN) * TC_KSTAGE);
                     tma_load_2d(smem_u32(sm->stage[s].a), mw, bar, ks * TC_KSTAGE, tl.m0);
-                    if constexpr (!EXACT) tma_load_2d(smem_u32(sm->stage[s].b), &map_x, bar, ks * TC_KSTAGE, tl.n0);
+                    tma_load_2d(smem_u32(sm->stage[s].b), &map_x, bar, ks * TC_KSTAGE, tl.n0);
                 }
             }
         }
     } else if (warp == 1) {
         // ── MMA issuer ───────────────────────────────────────────────────────
         // The whole warp runs the loop and one elected lane issues: descriptors and barrier addresses then stay in uniform
-        // registers.  (With a single-lane loop the eight instructions of an exact stage took about 1000 of its 1800 cycles
-        // to issue, every descriptor going through general registers first, and this warp set the pace of the kernel.)
+        // registers.
         const uint32_t leader = elect_one();
         const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-        // EXACT: every block's tile starts from 2^17 (d_bias: a constant x constant product of the same shape), so that the
-        // int32 results are positive: see the epilogue
         // Asking a barrier costs 66 cycles even when it completed long ago: a stage's two questions go out together, and
         // only a "not yet" is followed by a wait.
         static_assert(UNIT == TC_KB_PER_STAGE, "one hand-over per stage");
@@ -421,23 +296,15 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
             if (leader) {
                 // that wait also says that the epilogue is done with the scales of the stage NU before this one
                 if (g >= NU) mbar_arrive(smem_u32(&sm->empty[(g - NU) % TC_STAGES]));
-                if constexpr (EXACT) {
-                    const unsigned long long d_bias = umma_desc_plain32(smem_u32(sm->bias));
-                    umma_i8_same_a<0>(d, d_bias, d_bias, idesc);
-                    umma_i8_same_a<1>(d + BN, d_bias, d_bias, idesc);
-                    umma_i8_same_a<1>(d + 2 * BN, d_bias, d_bias, idesc);
-                    umma_i8_same_a<2>(d + 3 * BN, d_bias, d_bias, idesc);
-                }
 #pragma unroll
                 for (int kk = 0; kk < UNIT; kk++)  // 32 bytes further along K inside the swizzle atom: +2 in the address field
-                    umma_i8<EXACT>(d + kk * BN, da + kk * 2, db + kk * 2, idesc);
+                    umma_i8(d + kk * BN, da + kk * 2, db + kk * 2, idesc);
                 umma_commit(smem_u32(&sm->tmem_full[unit]));
             }
             __syncwarp();
         }
     } else if (warp == 2) {
         // ── scale loader ─────────────────────────────────────────────────────
-        if constexpr (WAIT_LATE) pdl_wait();
         uint32_t g = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -474,64 +341,16 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&sm->full[s])) : "memory");
             }
         }
-    } else if (EXACT && warp == 3) {
-        // ── activation warp (exact GEMM) ─────────────────────────────────────
-        if constexpr (WAIT_LATE) pdl_wait();
-        // Word l of a token's 16-byte half block belongs to lane group l (simd.rs:381-383: vdotq_s32 lane l), so it goes to
-        // row (pair of tokens, l, token of the pair) of the 128B-swizzled operand and the row's other words stay zero.  Done
-        // here the operand costs a quarter of the L2 reads of an expanded copy in memory, and no pass that writes one.
-        // A warp's 32 words of a token are 128 contiguous bytes of global memory and 32 different banks.
-        constexpr int LAG = 3;  // copies of so many stages are in flight before the oldest one is handed on
-        uint32_t g = 0, done = 0;
-        bool ok = true;
-        const int chunk = lane >> 2, l = lane & 3;
-        const uint32_t dst0 = l * 4 + (2 * l) * 128 + ((chunk ^ (2 * l)) << 4), dst1 = l * 4 + (2 * l + 1) * 128 + ((chunk ^ (2 * l + 1)) << 4);
-        auto hand_on = [&]() {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sm->full[done % TC_STAGES]));
-            done++;
-        };
-        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-            const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
-            const int8_t* src[TOK];
-#pragma unroll
-            for (int j = 0; j < TOK; j++)  // rows past the last token repeat it; their outputs are not stored
-                src[j] = job.xq + (size_t)min(tl.n0 + j, n - 1) * k + lane * 4;
-            for (int ks = 0; ks < k_stages; ks++, g++) {
-                const int s = g % TC_STAGES;
-                ok = mbar_wait<BN, 256>(sm, smem_u32(&sm->empty[s]), ((g / TC_STAGES) & 1) ^ 1, err, 7);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                // row 8 * (j / 2) + 2 * l + (j & 1); its place among the eight rows of a swizzle atom is 2 * l + (j & 1)
-                const uint32_t b = smem_u32(sm->stage[s].b);
-                const uint32_t b0 = b + dst0, b1 = b + dst1;
-#pragma unroll
-                for (int j = 0; j < TOK; j++) {
-                    cp_async_4(((j & 1) ? b1 : b0) + (j >> 1) * 1024, src[j]);
-                    src[j] += TC_KSTAGE;
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                if (g >= LAG) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
-                    hand_on();
-                }
-            }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (ok)
-            while (done < g) hand_on();
     } else if (warp >= 4) {
         // ── epilogue ─────────────────────────────────────────────────────────
-        if constexpr (WAIT_LATE) pdl_wait();
         const int quarter = warp & 3, cg = (warp - 4) >> 2;
         const int row_in_tile = quarter * 32 + lane;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cg * COLS);
         uint32_t g = 0;
         bool ok = true;
-        if constexpr (!EXACT) {
+        {
             // One fused chain per output: per block a conversion per output and one packed product and one packed multiply-add
-            // per two.  Same hand-over as below (2048-token prompt of the 1.6B model: 23.4 -> 18.4 ms).
+            // per two (2048-token prompt of the 1.6B model: 23.4 -> 18.4 ms).
             static_assert(COLS == 32, "64 tokens per tile");
             f32x2 acc[COLS / 2];
             bool ready = false;
@@ -553,7 +372,7 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     const uint32_t t0 = lane_base + unit * (UNIT * BN);
                     int32_t SA[COLS], SB[COLS];
                     auto chain = [&](const int32_t (&S)[COLS], const int kk) {
-                        const float sw = lds_f32(st_sw + kk * (TC_BM * 4)) * TC_SCALE_DOWN;
+                        const float sw = lds_f32(st_sw + kk * (TC_BM * 4));
                         const f32x2 sw2 = pack2(sw, sw);
 #pragma unroll
                         for (int c = 0; c < COLS; c += 4) {
@@ -571,15 +390,15 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                             }
                         }
                     };
-                    tmem_ld<COLS>(t0, SA);
+                    tmem_ld32(t0, SA);
                     tmem_ld_wait();
-                    tmem_ld<COLS>(t0 + BN, SB);
+                    tmem_ld32(t0 + BN, SB);
                     chain(SA, 0);
                     tmem_ld_wait();
-                    tmem_ld<COLS>(t0 + 2 * BN, SA);
+                    tmem_ld32(t0 + 2 * BN, SA);
                     chain(SB, 1);
                     tmem_ld_wait();
-                    tmem_ld<COLS>(t0 + 3 * BN, SB);
+                    tmem_ld32(t0 + 3 * BN, SB);
                     const bool q = mbar_test(smem_u32(&sm->tmem_full[(g + 1) % NU]), ((g + 1) / NU) & 1);
                     chain(SA, 2);
                     tmem_ld_wait();
@@ -600,119 +419,6 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
                     }
                 }
             }
-        } else {
-            // The arithmetic of gemm_q*_q8_0_neon (simd.rs:696-1019) bit for bit: per output eight unfused
-            // chains acc[parity of the block][lane group] += float(lane partial) * (f16(d_w) * d_x), blocks
-            // in ascending order, combined at the end as ((a0+a1)+(a2+a3)) per parity, even + odd.
-            //
-            // Bound: instruction issue and the FMA pipe.  Per (output, block) there are four lane partials p and, in the
-            // plain form, 4 int->float conversions + 4 products + 4 additions + the scale product.  Here it is 2 packed fused
-            // multiply-adds + 2 packed additions + 1/2 + 1/2 for the scales, two tokens per instruction:
-            //  - tensor memory holds v = p + 2^17 > 0 (the bias instruction).  Read as an f32, a positive integer below 2^23
-            //    is the denormal v * 2^-149, which the FMA pipe takes at full rate: no conversion.
-            //  - d = f16(d_w) * d_x rounds the same when the weight scale is stored times 2^96 (D = d * 2^96), and 2^17 * D is
-            //    exact.  Hence fma(v * 2^-149, D, -2^-132 * D) rounds (v - 2^17) * d * 2^-53 once: it IS
-            //    RN(float(p) * d) * 2^-53, the reference's rounded product, and no contraction with the addition can occur.
-            //  - the chains run scaled by 2^-53.  Scales are f16 values, so every term is a multiple of 2^-48: nothing falls
-            //    into the denormal range (2^-125) and every rounding is the unscaled one; the final sum is multiplied back.
-            //    Other scales: tc_odd_scale.  (Looked for here - NaN outputs in the epilogue, scales in the loading warps -
-            //    they cost the large tiles 1 to 7 %, mostly by what the compiler then made of the loop.)
-            // 6144 x 2048 at 512 tokens: 157 -> 113.5 us (113 TFLOP/s).  Of the FMA pipe's time 48 % is this arithmetic, 6 % integer
-            // multiply-adds, 46 % idle at the hand-over: both warps of a scheduler wait at the same time.  Tried: columns split
-            // between the groups with barriers and MMAs of their own (123), the groups kept half a stage apart (144), sixteen
-            // warps of 4 tokens (131), the next stage's first block loaded before the last chains (145 to 179).
-            constexpr int TP = COLS / 8;  // token pairs per thread
-            const f32x2 unbias = pack2(-__uint_as_float(1u << 17), -__uint_as_float(1u << 17));  // -2^-132
-            const uint32_t sw0 = smem_u32(&sm->stage[0].sw[0][row_in_tile]), sx0 = smem_u32(&sm->stage[0].sx[0][cg * 2 * TP]);
-            if constexpr (ANY_SCALE)
-                for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-                    const int n0 = tc_decode_tile(job, t, tiles_n, TOK).n0;
-                    if (tc_any_odd_scale(x_scales + (size_t)n0 * nb, threadIdx.x - 128, 32 * TC_EPI_WARPS, min(TOK, n - n0) * nb)) sm->odd_scale = 1;
-                }
-            bool ready = false;  // the answer of a question asked during the stage before
-            f32x2 acc2[TP][2][4];         // [pair][block parity][lane group], halves = the pair's tokens
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                const TcTile tl = tc_decode_tile(job, t, tiles_n, TOK);
-                const int m = job.m[tl.mat];
-                const int row = tl.m0 + row_in_tile;
-#pragma unroll
-                for (int i = 0; i < TP; i++)
-#pragma unroll
-                    for (int l = 0; l < 4; l++) acc2[i][0][l] = acc2[i][1][l] = pack2(0.f, 0.f);
-                for (int ks = 0; ks < k_stages && ok; ks++, g++) {
-                    static_assert(UNIT == TC_KB_PER_STAGE, "the exact epilogue takes a whole stage per hand-over");
-                    const uint32_t unit = g % NU;  // the part of tensor memory with the stage's 4 blocks
-                    // One wait and one arrival per stage.  The wait covers the stage's scales too: the MMA issuer had seen
-                    // their barrier (full[s]) before it issued what this one reports.  The arrival stands for both the tensor
-                    // memory and the scales, all of which are in registers by then.
-                    // (every lane of a warp runs the same wait on the same barrier and gets the same answer)
-                    if (!ready) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(sm, smem_u32(&sm->tmem_full[unit]), (g / NU) & 1, err, 6));
-                        if (!ok) break;
-                    }
-                    tc_fence_after();
-                    const uint32_t st_off = (g % TC_STAGES) * (uint32_t)sizeof(TcStage<BN>), st_sw = sw0 + st_off, st_sx = sx0 + st_off;
-                    // the load of block kk + 1 is in flight while the chains of block kk run
-                    int32_t SA[COLS], SB[COLS];
-                    struct Scales {
-                        float w;
-                        f32x2 x[TP];
-                    };
-                    auto scales = [&](const int kk) {
-                        Scales c;
-                        c.w = lds_f32(st_sw + kk * (TC_BM * 4));
-#pragma unroll
-                        for (int i = 0; i < TP; i += 2) lds_2x64(st_sx + kk * (BN * 4) + i * 8, c.x[i], c.x[i + 1]);
-                        return c;
-                    };
-                    auto chains = [&](const int32_t (&S)[COLS], const int p, const Scales& sc) {
-                        const f32x2 sw2 = pack2(sc.w, sc.w);
-#pragma unroll
-                        for (int i = 0; i < TP; i++) {
-                            const f32x2 d = mul2(sw2, sc.x[i]);
-                            const f32x2 c = mul2(d, unbias);
-#pragma unroll
-                            for (int l = 0; l < 4; l++) {
-                                const f32x2 v = pack2(__int_as_float(S[i * 8 + 2 * l]), __int_as_float(S[i * 8 + 2 * l + 1]));
-                                acc2[i][p][l] = add2(acc2[i][p][l], fma2(v, d, c));
-                            }
-                        }
-                    };
-                    const uint32_t t0 = lane_base + unit * (TC_KB_PER_STAGE * BN);
-                    tmem_ld<COLS>(t0, SA);
-                    const Scales c0 = scales(0), c1 = scales(1);
-                    tmem_ld_wait();
-                    tmem_ld<COLS>(t0 + BN, SB);
-                    chains(SA, 0, c0);
-                    const Scales c2 = scales(2);
-                    tmem_ld_wait();
-                    tmem_ld<COLS>(t0 + 2 * BN, SA);
-                    chains(SB, 1, c1);
-                    const Scales c3 = scales(3);
-                    tmem_ld_wait();
-                    tmem_ld<COLS>(t0 + 3 * BN, SB);
-                    const bool q = mbar_test(smem_u32(&sm->tmem_full[(g + 1) % NU]), ((g + 1) / NU) & 1);
-                    chains(SA, 0, c2);
-                    tmem_ld_wait();
-                    tc_fence_before();
-                    ready = __all_sync(0xffffffffu, q);
-                    if (lane == 0) mbar_arrive(smem_u32(&sm->tmem_empty[unit]));
-                    chains(SB, 1, c3);
-                }
-                if (ok && row < m) {
-                    float* out = job.out[tl.mat];
-#pragma unroll
-                    for (int i = 0; i < TP; i++) {
-                        const int tok = tl.n0 + cg * 2 * TP + 2 * i;
-                        const f32x2 e = add2(add2(acc2[i][0][0], acc2[i][0][1]), add2(acc2[i][0][2], acc2[i][0][3]));
-                        const f32x2 o = add2(add2(acc2[i][1][0], acc2[i][1][1]), add2(acc2[i][1][2], acc2[i][1][3]));
-                        float r0, r1;
-                        unpack2(add2(e, o), r0, r1);
-                        if (tok < n) out[(size_t)tok * m + row] = r0 * TC_EXACT_DOWN;
-                        if (tok + 1 < n) out[(size_t)(tok + 1) * m + row] = r1 * TC_EXACT_DOWN;
-                    }
-                }
-            }
         }
     }
 
@@ -726,23 +432,6 @@ k_gemm_tc(const __grid_constant__ TcJob job, const __grid_constant__ CUtensorMap
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
-    if constexpr (ANY_SCALE) {
-        if (sm->odd_scale && !sm->abort)
-            for (int t = blockIdx.x; t < tiles; t += gridDim.x) tc_repair_tile(job, tc_decode_tile(job, t, tiles_n, TOK), x_scales, n, k, TOK);
-    }
-}
-
-// Behind an exact GEMM of many tiles: one warp per CTA, four CTAs to an SM, which fit beside the GEMM's and so are there when it
-// ends.  Bound: latency, one launch and one trip to L2 (6144 x 2048 at 512 columns: 113.5 -> 115.2 us; with CTAs of eight warps
-// 116.5, which behind the small tiles were 8.7 -> 10.8).
-__global__ void __launch_bounds__(32) k_tc_odd_scales(const __grid_constant__ TcJob job, const float* x_scales, int n, int k) {
-    pdl_enter(x_scales);
-    const int nb = k / QK;
-    for (int tok = blockIdx.x; tok < n; tok += gridDim.x) {
-        if (!__any_sync(0xffffffffu, tc_any_odd_scale(x_scales + (size_t)tok * nb, threadIdx.x, 32, nb))) continue;
-        for (int mat = 0; mat < job.count; mat++)
-            for (int row = threadIdx.x; row < job.m[mat]; row += 32) job.out[mat][(size_t)tok * job.m[mat] + row] = tc_exact_plain(job, mat, row, tok, x_scales, k);
-    }
 }
 
 }  // namespace
@@ -751,8 +440,7 @@ __global__ void __launch_bounds__(32) k_tc_odd_scales(const __grid_constant__ Tc
 namespace {
 
 // One thread per (row, block): widen the block's quants to int8 and store its scale.
-// *infinite = 1 if a scale is infinite.
-__global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restrict__ scales_t, int m_pad, uint32_t* __restrict__ infinite) {
+__global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restrict__ scales_t, int m_pad) {
     const int nb = w.k / QK;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)w.m * nb) return;
@@ -761,8 +449,7 @@ __global__ void k_tc_unpack(DevWeight w, int8_t* __restrict__ q, float* __restri
     const __half* dg = w.d + (size_t)g * nb * 4;
     const uint32_t* qg = reinterpret_cast<const uint32_t*>(w.q + (size_t)g * w.q_group_bytes());
     const float d = __half2float(dg[b * 4 + r]);
-    scales_t[(size_t)b * m_pad + row] = d * TC_SCALE_UP;
-    if (isinf(d)) *infinite = 1;
+    scales_t[(size_t)b * m_pad + row] = d;
     uint32_t o[8];
     if (w.dtype == DT_Q4_0) {
 #pragma unroll
@@ -822,7 +509,7 @@ cudaError_t device_sm_count(int* sms) {
     return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
-template <int BN, bool EXACT, bool ANY_SCALE = false>
+template <int BN>
 cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_x, const float* x_scales, int n, int k,
                       int32_t* sums, uint32_t* err) {
     const size_t smem = sizeof(TcSmem<BN>) + 1024;
@@ -830,19 +517,13 @@ cudaError_t launch_tc(cudaStream_t st, const TcJob& job, const CUtensorMap& map_
     cudaError_t e = device_sm_count(&sm_count);
     if (e != cudaSuccess) return e;
     static RaisedPerDevice limit, limit_sums;
-    e = raise_dynamic_smem(limit, (const void*)k_gemm_tc<BN, false, EXACT, ANY_SCALE>, smem);
-    if constexpr (!EXACT)
-        if (e == cudaSuccess) e = raise_dynamic_smem(limit_sums, (const void*)k_gemm_tc<BN, true, false, false>, smem);
+    e = sums ? raise_dynamic_smem(limit_sums, (const void*)k_gemm_tc<BN, true>, smem) : raise_dynamic_smem(limit, (const void*)k_gemm_tc<BN, false>, smem);
     if (e != cudaSuccess) return e;
     const int tiles = job.tile_start[job.count];
     const int grid = tiles < sm_count ? tiles : sm_count;
     g_kernel_launches++;
-    if constexpr (!EXACT) {
-        if (sums) {
-            return launch_pdl(st, k_gemm_tc<BN, true, false, false>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, sums, n, k, err);
-        }
-    }
-    return launch_pdl(st, k_gemm_tc<BN, false, EXACT, ANY_SCALE>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, nullptr, n, k, err);
+    if (sums) return launch_pdl(st, k_gemm_tc<BN, true>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, sums, n, k, err);
+    return launch_pdl(st, k_gemm_tc<BN, false>, dim3(grid), dim3(TC_THREADS), smem, job, map_x, x_scales, nullptr, n, k, err);
 }
 
 cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, int count, int tiles_n) {
@@ -854,7 +535,6 @@ cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, in
         if (i >= count) continue;
         if (w[i]->k != w[0]->k) return cudaErrorInvalidValue;
         job.map_w[i] = w[i]->map;
-        job.wq[i] = w[i]->q;
         job.scales_t[i] = w[i]->scales_t;
         job.out[i] = out[i];
         job.m[i] = w[i]->m;
@@ -870,7 +550,7 @@ cudaError_t fill_job(TcJob& job, const TcWeight* const* w, float* const* out, in
 
 bool tc_gemm_supported(int m, int k) { return m > 0 && k > 0 && k % TC_KSTAGE == 0; }
 
-cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out, uint32_t* infinite) {
+cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out) {
     out->m = w.m;
     out->k = w.k;
     out->m_pad = (w.m + TC_BM - 1) / TC_BM * TC_BM;
@@ -880,7 +560,7 @@ cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out, u
     if (e != cudaSuccess) return e;
     const size_t n_blocks = (size_t)w.m * (w.k / QK);
     g_kernel_launches++;
-    k_tc_unpack<<<(unsigned)((n_blocks + 255) / 256), 256, 0, st>>>(w, out->q, out->scales_t, out->m_pad, infinite);
+    k_tc_unpack<<<(unsigned)((n_blocks + 255) / 256), 256, 0, st>>>(w, out->q, out->scales_t, out->m_pad);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return encode_rows_map(out->q, out->m_pad, out->k, TC_BM, &out->map);
@@ -897,41 +577,7 @@ cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* con
     TcJob job;
     cudaError_t e = fill_job(job, w, out, count, (n + TC_TENSOR_TOKENS - 1) / TC_TENSOR_TOKENS);
     if (e != cudaSuccess) return e;
-    return launch_tc<TC_TENSOR_TOKENS, false>(st, job, map_x, x_scales, n, w[0]->k, sums, err);
-}
-
-cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,
-                                 const float* x_scales, int n, bool any_scale, uint32_t* err) {
-    if (n <= 0 || count <= 0) return cudaSuccess;
-    if (count > 3) return cudaErrorInvalidValue;
-    TcJob job;
-    // 16-token or 8-token tiles: whichever needs less time in waves of one tile per SM.  A stage of the small tile takes 810
-    // cycles against 1430 (0.57; 64 rows x 2048 x 6912 and 512 x 6144 x 2048), so it wins where it fills a last wave that
-    // the large one would leave mostly empty: one wave instead of half of one, 3 instead of 2 (64 rows x 6144), and so on.
-    int row_tiles = 0, sms = 0;
-    for (int i = 0; i < count; i++) row_tiles += w[i]->m_pad / TC_BM;
-    cudaError_t e = device_sm_count(&sms);
-    if (e != cudaSuccess) return e;
-    const int wide_waves = (row_tiles * ((n + TC_EXACT_TOKENS - 1) / TC_EXACT_TOKENS) + sms - 1) / sms;
-    const int narrow_waves = (row_tiles * ((n + TC_EXACT_TOKENS / 2 - 1) / (TC_EXACT_TOKENS / 2)) + sms - 1) / sms;
-    const bool narrow = narrow_waves * 62 < wide_waves * 100;  // (close calls go to the large tile: fewer weight reads)
-    const int tok = narrow ? TC_EXACT_TOKENS / 2 : TC_EXACT_TOKENS;
-    e = fill_job(job, w, out, count, (n + tok - 1) / tok);
-    if (e != cudaSuccess) return e;
-    job.xq = xq;
-    const CUtensorMap none{};
-    // Who looks at a caller's scales: the kernel itself costs the large tiles 0.3 to 0.9 us a wave (its loop is compiled worse with
-    // the second pass behind it), a kernel behind it 1.5 to 5 us: 3072 x 1024 at 81 columns, one wave, 11.1 / 16.0; 6144 x 2048 at
-    // 96, two, 25.0 / 25.7; at 256, six, 67.3 / 65.2 us.  The small tiles, 16.8 us with or without, always do it themselves.
-    const bool looks = any_scale && (narrow || wide_waves <= 2);
-    if (narrow) e = looks ? launch_tc<2 * TC_EXACT_TOKENS, true, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err)
-                          : launch_tc<2 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
-    else e = looks ? launch_tc<4 * TC_EXACT_TOKENS, true, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err)
-                   : launch_tc<4 * TC_EXACT_TOKENS, true>(st, job, none, x_scales, n, w[0]->k, nullptr, err);
-    any_scale = any_scale && !looks;
-    if (e != cudaSuccess || !any_scale) return e;
-    g_kernel_launches++;
-    return launch_pdl(st, k_tc_odd_scales, dim3(std::min(n, 4 * sms)), dim3(32), 0, job, x_scales, n, w[0]->k);
+    return launch_tc<TC_TENSOR_TOKENS>(st, job, map_x, x_scales, n, w[0]->k, sums, err);
 }
 
 }  // namespace wick

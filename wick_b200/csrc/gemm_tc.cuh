@@ -11,7 +11,7 @@ namespace wick {
 // layout, plus its scales as f32, block-major so that one k-block's 128 row scales are contiguous.
 struct TcWeight {
     int8_t* q = nullptr;      // [m_pad][k]
-    float* scales_t = nullptr;  // [k/32][m_pad], times 2^96
+    float* scales_t = nullptr;  // [k/32][m_pad]
     int m = 0, k = 0, m_pad = 0;
     CUtensorMap map;          // rows of this matrix, box 128 bytes x 128 rows, 128B swizzle
     size_t q_bytes() const { return (size_t)m_pad * k; }
@@ -22,10 +22,8 @@ struct TcWeight {
 // Q + K + V): their tiles are scheduled as one grid so that narrow matrices do not leave SMs idle.
 struct TcJob {
     CUtensorMap map_w[3];
-    const int8_t* wq[3];  // what map_w describes
     const float* scales_t[3];
     float* out[3];        // [n][m[i]] each
-    const int8_t* xq;     // exact GEMM: the quantised activations [n][k] (the other one reads them through a tensor map)
     int m[3], m_pad[3];
     int tile_start[4];    // first linear tile of each matrix; [count..3] = total
     int count;
@@ -36,9 +34,8 @@ bool tc_gemm_supported(int m, int k);
 
 // Fills `out` (q / scales_t must already point at q_bytes() / s_bytes() of device memory, zeroed by
 // this call) from the grouped layout of `w`, and encodes its tensor map.  Returns cudaSuccess or the
-// failing CUDA error; a tensor-map failure is reported as cudaErrorInvalidValue.  *infinite (device or mapped host memory)
-// becomes 1 if a scale is infinite: the exact GEMM does not take such a matrix.
-cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out, uint32_t* infinite);
+// failing CUDA error; a tensor-map failure is reported as cudaErrorInvalidValue.
+cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out);
 
 // Tensor map over quantised activations xq [rows_cap][k] int8 with a box of bn rows.
 cudaError_t tc_make_activation_map(const int8_t* xq, int rows_cap, int k, int bn, CUtensorMap* out);
@@ -50,14 +47,5 @@ cudaError_t tc_make_activation_map(const int8_t* xq, int rows_cap, int k, int bn
 constexpr int TC_TENSOR_TOKENS = 64;  // tokens per tile
 cudaError_t launch_gemm_tc(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const CUtensorMap& map_x,
                            const float* x_scales, int n, int32_t* sums, uint32_t* err);
-
-// The bit-exact variant (the arithmetic of gemm_q*_q8_0_neon, simd.rs:696-1019, in its order): every token's activations
-// become four rows of the operand, one per NEON lane group with the other groups' bytes zero, so that one MMA yields the
-// four lane partials of a block as four columns; the epilogue keeps the reference's eight unfused chains per output.
-// xq: int8 [n][k], 4-byte aligned.  Weight scales must be finite.  any_scale: the activation scales may be any f32 (a caller's);
-// otherwise they are f16 values (the library's quantiser), and outputs of a token with an infinite one are NaN.
-constexpr int TC_EXACT_TOKENS = 16;  // tokens per tile (64 MMA columns)
-cudaError_t launch_gemm_tc_exact(cudaStream_t st, const TcWeight* const* w, float* const* out, int count, const int8_t* xq,
-                                 const float* x_scales, int n, bool any_scale, uint32_t* err);
 
 }  // namespace wick

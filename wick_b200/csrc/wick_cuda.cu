@@ -18,6 +18,7 @@
 #include "../../include/wick_cuda.h"
 #include "gguf.hpp"
 #include "decode_mega.cuh"
+#include "gemm_mma.cuh"
 #include "gemm_tc.cuh"
 #include "kernels.cuh"
 #include "word_pool.hpp"
@@ -46,13 +47,18 @@ static int32_t fail(int32_t code, const std::string& msg) {
 
 namespace {
 
+// Copies of a matrix for the GEMMs of several rows; null until the first call that uses them.
+struct GemmCopies {
+    MmaWeight exact;  // the bit-exact GEMM's (gemm_mma.cu)
+    TcWeight fused;   // the fused-chain GEMM's (gemm_tc.cu)
+};
+
 struct Layer {
     bool is_attn = false;
     int n_kv = 0;
     float *attn_norm = nullptr, *ffn_norm = nullptr, *q_norm = nullptr, *k_norm = nullptr, *conv_w = nullptr;
     DevWeight in_proj, out_proj, q, k, v, o, gate, up, down;
-    // int8 copies for the tensor-core prefill GEMM (gemm_tc.cu); q == nullptr when unavailable
-    TcWeight tc_in_proj, tc_out_proj, tc_q, tc_k, tc_v, tc_o, tc_gate, tc_up, tc_down;
+    GemmCopies tc_in_proj, tc_out_proj, tc_q, tc_k, tc_v, tc_o, tc_gate, tc_up, tc_down;
     float *k_cache = nullptr, *v_cache = nullptr;  // [max_seq][kv_dim]
     float* conv_state = nullptr;                   // [d_conv][hidden]
 };
@@ -62,11 +68,11 @@ struct Layer {
 struct wick_cuda_weight {
     DevWeight w;
     int device = 0;
-    // int8 copy for the tensor-core GEMMs, made by the first call that uses them; the lock is for that call only
+    // copies for the tensor-core GEMMs, each made by the first call that uses it; the lock is for that call only
     mutable std::mutex tc_lock;
-    mutable TcWeight tc;
+    mutable MmaWeight exact;  // the bit-exact product's
+    mutable TcWeight tc;      // the fused-chain product's
     bool cuda_cores = false;             // products stay on the CUDA cores (WICK_CUDA_PREFILL=exact-cuda-cores at creation): no copy is made
-    mutable bool tc_exact = false;       // the copy can serve the exact product (no infinite scale)
     mutable uint32_t* tc_err = nullptr;  // host word (TcErrorWords) the kernels write on an expired wait: reading it needs no copy
 };
 
@@ -77,7 +83,7 @@ struct wick_cuda_model {
     int head_dim = 0;
     std::vector<Layer> layers;
     DevWeight embd;
-    TcWeight tc_embd;       // tensor-core copy of the vocabulary matrix, made for the multi-sequence step only
+    GemmCopies tc_embd;     // of the vocabulary matrix, made for the multi-sequence step only
     bool embd_q6k = false;  // token_embd is Q6_K: embd6 is used for the embedding rows and the logits, embd is empty
     DevQ6K embd6;
     float* output_norm = nullptr;
@@ -86,8 +92,7 @@ struct wick_cuda_model {
     // tensor-core prefill GEMMs: available when every matrix meets tc_gemm_supported(); prefill_mode
     // picks the bit-exact one (default), the fused-chain one, or the bit-exact CUDA-core kernel
     bool tc_ok = false;     // the model's shapes allow the tensor-core GEMM
-    bool tc_built = false;  // its int8 weight copies and buffers exist (made by the first call that needs them)
-    bool tc_infinite = false;  // a copied matrix has an infinite scale: the exact GEMM stays on the CUDA cores
+    bool exact_built = false, fused_built = false;  // the layers' copies exist (made by the first call that needs them)
     int prefill_mode = WICK_CUDA_PREFILL_EXACT;
     CUtensorMap map_x_hs, map_x_is;  // activations [max_chunk][hs | is] for the fused-chain GEMM
     float* normed_last = nullptr;  // output-normed hidden row of the last prefilled token
@@ -701,10 +706,11 @@ void prof_collect(wick_cuda_model* m) {  // after the stream has been synchronis
     m->prof_used = 0;
 }
 
-// The int8 weight copies of the tensor-core GEMMs (1.125 bytes per parameter) are made by the first chunk of more than
+// The weight copies of the tensor-core GEMMs (1.125 bytes per parameter; the exact and the fused-chain GEMM have one each, made
+// when a mode first needs it) are made by the first chunk of more than
 // TC_BUILD_ABOVE tokens, so that decoding and the shortest prompts leave a model at its packed size.  Once they are there
 // the bit-exact GEMM uses them from two tokens on: its 8-token tile costs the same for 2 tokens as for 8, and the CUDA-core
-// kernel needs several times as long at any of these counts (350M, 9-token prompt: 3.7 -> 1.2 ms).  The fused-chain GEMM
+// kernel needs several times as long at any of these counts (350M, 9-token prompt: 3.7 -> 0.70 ms).  The fused-chain GEMM
 // keeps its lower limit, because below it the other kernels' results are the ones a caller has always had.
 // From TC_REQUIRED_FROM rows on a call without memory for the copies is an error; below, the CUDA cores serve it.
 constexpr int TC_BUILD_ABOVE = 8, TC_FUSED_MIN_TOKENS = 16, TC_REQUIRED_FROM = 16;
@@ -713,33 +719,31 @@ constexpr int TC_BUILD_ABOVE = 8, TC_FUSED_MIN_TOKENS = 16, TC_REQUIRED_FROM = 1
 // launch on the tensor cores when the chunk is wide enough to fill an MMA tile, else the exact CUDA-core kernel.
 struct GemmTarget {
     const DevWeight* w;
-    const TcWeight* t;
+    const GemmCopies* t;
     float* out;
 };
 void run_gemms(wick_cuda_model* m, int n, std::initializer_list<GemmTarget> list) {
     cudaStream_t st = m->stream;
-    const int hs = m->cfg.hidden_size;
-    const bool tc_exact = m->tc_built && !m->tc_infinite && n >= 2 && m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
-    const bool tc = tc_exact || (m->tc_built && n >= TC_FUSED_MIN_TOKENS && m->prefill_mode == WICK_CUDA_PREFILL_TENSOR);
-    if (tc) {
-        const TcWeight* tw[3] = {};
-        float* outs[3] = {};
-        int c = 0;
-        for (const GemmTarget& g : list) {
-            tw[c] = g.t;
-            outs[c++] = g.out;
-        }
-        const bool is_hs = tw[0]->k == hs;
-        cudaError_t e;
-        if (tc_exact) {
-            e = launch_gemm_tc_exact(st, tw, outs, c, m->q8q, m->q8s, n, /*any_scale=*/false, m->tc_err);
-        } else {
-            e = launch_gemm_tc(st, tw, outs, c, is_hs ? m->map_x_hs : m->map_x_is, m->q8s, n, nullptr, m->tc_err);
-        }
-        (void)e;  // surfaced by the cudaGetLastError() check after the chunk
-    } else {
-        for (const GemmTarget& g : list) launch_gemm(st, *g.w, m->q8s, m->q8q, n, g.out);
+    bool exact = m->exact_built && n >= 2 && m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
+    bool fused = m->fused_built && n >= TC_FUSED_MIN_TOKENS && m->prefill_mode == WICK_CUDA_PREFILL_TENSOR;
+    const MmaWeight* ew[3] = {};
+    const TcWeight* fw[3] = {};
+    float* outs[3] = {};
+    int c = 0;
+    for (const GemmTarget& g : list) {
+        ew[c] = &g.t->exact;
+        fw[c] = &g.t->fused;
+        outs[c++] = g.out;
+        exact = exact && g.t->exact.p;
+        fused = fused && g.t->fused.q;
     }
+    // (errors surface in the cudaGetLastError() check after the chunk)
+    if (exact)
+        (void)launch_gemm_mma(st, ew, outs, c, m->q8q, m->q8s, n, m->tc_err);
+    else if (fused)
+        (void)launch_gemm_tc(st, fw, outs, c, fw[0]->k == (int)m->cfg.hidden_size ? m->map_x_hs : m->map_x_is, m->q8s, n, nullptr, m->tc_err);
+    else
+        for (const GemmTarget& g : list) launch_gemm(st, *g.w, m->q8s, m->q8q, n, g.out);
 }
 
 // One internal prefill chunk of n <= max_chunk tokens already in m->tokens_dev
@@ -804,7 +808,7 @@ void enqueue_prefill_chunk(wick_cuda_model* m, int n, int start_pos, bool flash,
     }
 }
 
-// Tensor-core prefill GEMM: decided at load (tc_ok = the shapes allow it), built on first use (ensure_tc): the int8
+// Tensor-core prefill GEMM: decided at load (tc_ok = the shapes allow it), built on first use (ensure_tc): the
 // copies of the layer matrices cost 1.125 bytes per parameter, which a decode-only user never needs.
 int32_t build_tc(wick_cuda_model* m) {
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size;
@@ -819,27 +823,27 @@ int32_t build_tc(wick_cuda_model* m) {
     return WICK_CUDA_OK;
 }
 
-// After tc_weight_fill calls that report to the model's (otherwise idle) error word; synchronises.
-int32_t note_infinite_scales(wick_cuda_model* m) {
-    uint32_t found = 0;
-    CU_TRY(cudaMemcpyAsync(&found, m->tc_err, 4, cudaMemcpyDeviceToHost, m->stream));
-    CU_TRY(cudaMemsetAsync(m->tc_err, 0, 4, m->stream));
-    CU_TRY(cudaStreamSynchronize(m->stream));
-    m->tc_infinite = m->tc_infinite || found != 0;
+int32_t copy_for_exact(wick_cuda_model* m, const DevWeight& w, GemmCopies* t) {
+    t->exact.m = w.m;
+    t->exact.k = w.k;
+    t->exact.dtype = w.dtype;
+    W_TRY(dev_alloc(m, &t->exact.p, t->exact.bytes()));
+    CU_TRY(mma_weight_fill(m->stream, w, t->exact.p));
+    return WICK_CUDA_OK;
+}
+int32_t copy_for_fused(wick_cuda_model* m, const DevWeight& w, GemmCopies* t) {
+    t->fused.m_pad = (w.m + 127) / 128 * 128;
+    t->fused.m = w.m;
+    t->fused.k = w.k;
+    W_TRY(dev_alloc(m, &t->fused.q, t->fused.q_bytes()));
+    W_TRY(dev_alloc(m, &t->fused.scales_t, t->fused.s_bytes() / sizeof(float)));
+    CU_TRY(tc_weight_fill(m->stream, w, &t->fused));
     return WICK_CUDA_OK;
 }
 
-int32_t make_tc(wick_cuda_model* m) {
-    const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size;
-    auto fill = [&](const DevWeight& w, TcWeight* t) -> int32_t {
-        t->m_pad = (w.m + 127) / 128 * 128;
-        t->m = w.m;
-        t->k = w.k;
-        W_TRY(dev_alloc(m, &t->q, t->q_bytes()));
-        W_TRY(dev_alloc(m, &t->scales_t, t->s_bytes() / sizeof(float)));
-        CU_TRY(tc_weight_fill(m->stream, w, t, m->tc_err));
-        return WICK_CUDA_OK;
-    };
+// The layers' copies for the exact or the fused-chain GEMM.
+int32_t make_copies(wick_cuda_model* m, bool exact) {
+    auto fill = [&](const DevWeight& w, GemmCopies* t) { return exact ? copy_for_exact(m, w, t) : copy_for_fused(m, w, t); };
     for (Layer& L : m->layers) {
         if (L.is_attn) {
             W_TRY(fill(L.q, &L.tc_q));
@@ -854,20 +858,24 @@ int32_t make_tc(wick_cuda_model* m) {
         W_TRY(fill(L.up, &L.tc_up));
         W_TRY(fill(L.down, &L.tc_down));
     }
-    CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, hs, TC_TENSOR_TOKENS, &m->map_x_hs));
-    CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, is, TC_TENSOR_TOKENS, &m->map_x_is));
-    W_TRY(note_infinite_scales(m));
-    m->tc_built = true;
+    if (!exact) {
+        CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.hidden_size, TC_TENSOR_TOKENS, &m->map_x_hs));
+        CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.intermediate_size, TC_TENSOR_TOKENS, &m->map_x_is));
+    }
+    CU_TRY(cudaStreamSynchronize(m->stream));
+    (exact ? m->exact_built : m->fused_built) = true;
     return WICK_CUDA_OK;
 }
 
 // The copies for a call of `rows` rows.
 int32_t ensure_tc(wick_cuda_model* m, uint32_t rows) {
-    if (rows <= (uint32_t)TC_BUILD_ABOVE || !m->tc_ok || m->tc_built || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
+    const bool exact = m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
+    if (rows <= (uint32_t)TC_BUILD_ABOVE || !m->tc_ok || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
+    if (exact ? m->exact_built : m->fused_built) return WICK_CUDA_OK;
     RelaxedCapture relaxed;
     const size_t n = m->allocs.size();
     const uint64_t bytes = m->bytes;
-    const int32_t r = make_tc(m);
+    const int32_t r = make_copies(m, exact);
     if (r != WICK_CUDA_OK) undo_allocs(m, n, bytes);
     return r == WICK_CUDA_ERR_OOM && rows < (uint32_t)TC_REQUIRED_FROM ? WICK_CUDA_OK : r;
 }
@@ -1115,17 +1123,6 @@ int32_t with_slot(wick_cuda_model* m, uint32_t id, F&& fn) {
 
 constexpr uint32_t MAX_BATCH_ROWS = 1024;
 
-int32_t make_tc_embd(wick_cuda_model* m) {
-    TcWeight* t = &m->tc_embd;
-    t->m_pad = (m->embd.m + 127) / 128 * 128;
-    t->m = m->embd.m;
-    t->k = m->embd.k;
-    W_TRY(dev_alloc(m, &t->q, t->q_bytes()));
-    W_TRY(dev_alloc(m, &t->scales_t, t->s_bytes() / sizeof(float)));
-    CU_TRY(tc_weight_fill(m->stream, m->embd, t, m->tc_err));
-    return note_infinite_scales(m);
-}
-
 int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) {
     const size_t nl = m->layers.size();
     if ((int)rows > m->batch_cap) {
@@ -1139,15 +1136,19 @@ int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) 
         m->batch_cap = cap;
         m->rows_out_cap = 0;
     }
-    if (m->tc_built && !m->embd_q6k && !m->tc_embd.q && rows >= 2) {
-        // the vocabulary head of a batched step is a GEMM over all rows: worth a tensor-core copy of the matrix
+    const bool exact = m->prefill_mode == WICK_CUDA_PREFILL_EXACT && m->exact_built && !m->tc_embd.exact.p;
+    const bool fused = m->prefill_mode == WICK_CUDA_PREFILL_TENSOR && m->fused_built && !m->tc_embd.fused.q;
+    if ((exact || fused) && !m->embd_q6k && rows >= 2) {
+        // the vocabulary head of a batched step is a GEMM over all rows: worth a copy of the matrix
         RelaxedCapture relaxed;
         const size_t n_allocs = m->allocs.size();
         const uint64_t bytes = m->bytes;
-        const int32_t r = make_tc_embd(m);
+        const int32_t r = exact ? copy_for_exact(m, m->embd, &m->tc_embd) : copy_for_fused(m, m->embd, &m->tc_embd);
         if (r != WICK_CUDA_OK) {
             undo_allocs(m, n_allocs, bytes);
-            m->tc_embd = TcWeight();  // (its first plane may have been allocated, which is what the calls look at)
+            // (a first plane may have been allocated, which is what the calls look at)
+            if (exact) m->tc_embd.exact = MmaWeight();
+            else m->tc_embd.fused = TcWeight();
             if (r != WICK_CUDA_ERR_OOM || rows >= (uint32_t)TC_REQUIRED_FROM) return r;
         }
     }
@@ -1208,10 +1209,8 @@ int32_t enqueue_decode_rows(wick_cuda_model* m, int n, int seq_bound) {
     if (m->embd_q6k) {
         for (int j = 0; j < n; j++)
             launch_gemv_q6k(st, m->embd6, m->q8s + (size_t)j * (hs / QK), m->q8q + (size_t)j * hs, m->logits_rows + (size_t)j * m->cfg.vocab_size);
-    } else if (m->tc_embd.q) {
-        gemms({{&m->embd, &m->tc_embd, m->logits_rows}});
     } else {
-        launch_gemm(st, m->embd, m->q8s, m->q8q, n, m->logits_rows);
+        gemms({{&m->embd, &m->tc_embd, m->logits_rows}});
     }
     return WICK_CUDA_OK;
 }
@@ -1675,7 +1674,7 @@ int32_t wick_cuda_prefill_mode(const wick_cuda_model* m, int32_t* mode) {
 int32_t wick_cuda_prefill_uses_tensor_cores(const wick_cuda_model* m, int32_t* yes) {
     W_TRY(check_model(m));
     if (!yes) return fail(WICK_CUDA_ERR_BAD_ARG, "yes is NULL");
-    *yes = m->tc_ok && m->prefill_mode != WICK_CUDA_PREFILL_EXACT_CUDA_CORES && !(m->tc_infinite && m->prefill_mode == WICK_CUDA_PREFILL_EXACT);
+    *yes = m->tc_ok && m->prefill_mode != WICK_CUDA_PREFILL_EXACT_CUDA_CORES;
     return WICK_CUDA_OK;
 }
 
@@ -2002,6 +2001,7 @@ void wick_cuda_weight_destroy(wick_cuda_weight* w) {
     if (!w) return;
     cudaFree((void*)w->w.q);
     cudaFree((void*)w->w.d);
+    cudaFree(w->exact.p);
     cudaFree(w->tc.q);
     release_tc_error_word(w->tc_err);  // (cudaFree has waited for the weight's kernels)
     delete w;
@@ -2048,34 +2048,59 @@ static bool has_tc_weight(const wick_cuda_weight* w) {
     std::lock_guard<std::mutex> hold(w->tc_lock);
     return w->tc_err != nullptr;
 }
-
-// The int8 copy of an operator-API weight, made on first use (and finished before the call goes on: later calls may come
-// on other streams).
-static int32_t ensure_tc_weight(const wick_cuda_weight* w, cudaStream_t st) {
+static bool has_exact_copy(const wick_cuda_weight* w) {
     std::lock_guard<std::mutex> hold(w->tc_lock);
-    if (w->tc_err) return WICK_CUDA_OK;
+    return w->exact.p != nullptr;
+}
+
+// A copy of an operator-API weight, made on first use (and finished before the call goes on: later calls may come on other
+// streams).  `plane` is the copy's own pointer, null until it is complete; `fill(p)` fills it at p, `bytes` long.
+extern "C++" {
+template <class P, class F>
+int32_t ensure_copy(const wick_cuda_weight* w, cudaStream_t st, P*& plane, size_t bytes, F&& fill) {
+    std::lock_guard<std::mutex> hold(w->tc_lock);
+    if (plane) return WICK_CUDA_OK;
     RelaxedCapture relaxed;
+    P* p = nullptr;
+    uint32_t* err = w->tc_err ? w->tc_err : g_tc_error_words.take();
+    cudaError_t e = err ? cudaMalloc((void**)&p, bytes) : cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = fill(p);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // (not for the next launch to find)
+        cudaFree(p);
+        if (!w->tc_err) g_tc_error_words.give_back(err);
+        CU_TRY(e);
+    }
+    plane = p;
+    w->tc_err = err;
+    return WICK_CUDA_OK;
+}
+}
+static int32_t ensure_exact_copy(const wick_cuda_weight* w, cudaStream_t st) {
+    MmaWeight t;
+    t.m = w->w.m;
+    t.k = w->w.k;
+    return ensure_copy(w, st, w->exact.p, t.bytes(), [&](uint8_t* p) {
+        w->exact.m = w->w.m;  // (everything but p, which ensure_copy sets last)
+        w->exact.k = w->w.k;
+        w->exact.dtype = w->w.dtype;
+        return mma_weight_fill(st, w->w, p);
+    });
+}
+static int32_t ensure_fused_copy(const wick_cuda_weight* w, cudaStream_t st) {
     TcWeight t;
     t.m = w->w.m;
     t.k = w->w.k;
     t.m_pad = (w->w.m + 127) / 128 * 128;
-    uint32_t* err = g_tc_error_words.take();
-    cudaError_t e = err ? cudaMalloc((void**)&t.q, t.q_bytes() + t.s_bytes()) : cudaErrorMemoryAllocation;  // (q_bytes is a multiple of 128 * 128)
-    if (e == cudaSuccess) {
-        t.scales_t = reinterpret_cast<float*>(t.q + t.q_bytes());
-        e = tc_weight_fill(st, w->w, &t, err);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-        cudaGetLastError();  // (not for the next launch to find)
-        cudaFree(t.q);
-        g_tc_error_words.give_back(err);
-        CU_TRY(e);
-    }
-    w->tc_exact = __atomic_exchange_n(err, 0u, __ATOMIC_ACQ_REL) == 0;
-    w->tc = t;
-    w->tc_err = err;
-    return WICK_CUDA_OK;
+    return ensure_copy(w, st, w->tc.q, t.q_bytes() + t.s_bytes(), [&](int8_t* p) {  // (q_bytes is a multiple of 128 * 128)
+        t.q = p;
+        t.scales_t = reinterpret_cast<float*>(p + t.q_bytes());
+        const cudaError_t e = tc_weight_fill(st, w->w, &t);
+        t.q = nullptr;
+        w->tc = t;
+        return e;
+    });
 }
 
 // Reports and clears what a kernel of this weight left behind on an expired wait (one exchange: of two threads one gets it).
@@ -2101,23 +2126,21 @@ int32_t wick_cuda_debug_weight_error(const wick_cuda_weight* w, uint32_t code) {
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n, float* out_dev,
                           void* stream) {
     if (!w || !bs_dev || !bq_dev || !out_dev) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
-    if (n > (uint32_t)TC_BUILD_ABOVE && !w->cuda_cores && tc_gemm_supported(w->w.m, w->w.k)) {
-        // same bits on the tensor cores (6912 x 2048 at 2002 rows: 1.71 ms on the CUDA cores); asynchronous like the other
+    if (n > (uint32_t)TC_BUILD_ABOVE && !w->cuda_cores && mma_gemm_supported(w->w.m, w->w.k) && ((uintptr_t)bq_dev & 15) == 0) {
+        // same bits on the tensor cores (6912 x 2048 at 2002 rows: 1.71 ms on the CUDA cores, 0.43 there); asynchronous like the other
         // operators, so a wait that expired in an earlier call is reported by wick_cuda_weight_status or by the next call
         cudaStream_t st = (cudaStream_t)stream;
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CU_TRY(cudaStreamIsCapturing(st, &capturing));
         int32_t made = WICK_CUDA_ERR_OOM;  // (making the copy allocates and synchronises: not while the stream is captured)
-        if (capturing == cudaStreamCaptureStatusNone || has_tc_weight(w)) made = ensure_tc_weight(w, st);
+        if (capturing == cudaStreamCaptureStatusNone || has_exact_copy(w)) made = ensure_exact_copy(w, st);
         if (made != WICK_CUDA_OK && made != WICK_CUDA_ERR_OOM) return made;
         if (made == WICK_CUDA_OK) {
             W_TRY(take_tc_error(w));
-            if (w->tc_exact) {
-                const TcWeight* tw[1] = {&w->tc};
-                float* outs[1] = {out_dev};
-                CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, /*any_scale=*/true, w->tc_err));
-                OP_END();
-            }
+            const MmaWeight* tw[1] = {&w->exact};
+            float* outs[1] = {out_dev};
+            CU_TRY(launch_gemm_mma(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
+            OP_END();
         }
     }
     // also where there is no memory for the copy: the product itself needs none
@@ -2131,7 +2154,7 @@ int32_t wick_cuda_gemm_q8_tc(wick_cuda_weight* w, const float* bs_dev, const int
     if (!tc_gemm_supported(w->w.m, w->w.k)) return fail(WICK_CUDA_ERR_BAD_ARG, "tensor-core GEMM needs k to be a multiple of 128");
     if (n == 0) return WICK_CUDA_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    W_TRY(ensure_tc_weight(w, st));
+    W_TRY(ensure_fused_copy(w, st));
     CUtensorMap map_x;
     CU_TRY(tc_make_activation_map(bq_dev, (int)n, w->w.k, TC_TENSOR_TOKENS, &map_x));
     const TcWeight* tw[1] = {&w->tc};
@@ -2147,14 +2170,11 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     if (!tc_gemm_supported(w->w.m, w->w.k)) return fail(WICK_CUDA_ERR_BAD_ARG, "tensor-core GEMM needs k to be a multiple of 128");
     if (n == 0) return WICK_CUDA_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    W_TRY(ensure_tc_weight(w, st));
-    const TcWeight* tw[1] = {&w->tc};
+    W_TRY(ensure_exact_copy(w, st));
+    const MmaWeight* tw[1] = {&w->exact};
     float* outs[1] = {out_dev};
-    if (w->tc_exact) {
-        CU_TRY(launch_gemm_tc_exact(st, tw, outs, 1, bq_dev, bs_dev, (int)n, /*any_scale=*/true, w->tc_err));
-    } else {
-        launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
-    }
+    if ((uintptr_t)bq_dev & 15) launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);  // (the tensor cores' kernel reads 16 bytes at a time)
+    else CU_TRY(launch_gemm_mma(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
     CU_TRY(cudaGetLastError());
     CU_TRY(cudaStreamSynchronize(st));
     return take_tc_error(w);
