@@ -31,35 +31,34 @@ namespace wick {
 namespace {
 
 constexpr int KB = MMA_STAGE_BLOCKS;  // blocks per pipeline stage (256 elements of K)
-constexpr int PRODUCERS = 4;
 constexpr uint32_t MMA_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
 
-// R x 16 rows, NT x 8 tokens; a warp takes 16 rows and the blocks of one parity, so 2R consumer warps.
-template <int R, int NT>
+// R x 16 rows, NT x 8 tokens; a warp takes 16 rows and the blocks of one parity, so 2R consumer warps.  READY: the activations are
+// there in operand order (MmaInput) and come by bulk copies like the weights, issued by one warp; otherwise (operators: int8 columns
+// of the caller) four warps convert them.
+template <int R, int NT, bool READY>
 struct MmaShape {
-    static constexpr int CONSUMERS = 2 * R;
+    static constexpr int CONSUMERS = 2 * R, PRODUCERS = READY ? 1 : 4;
     static constexpr int THREADS = 32 * (CONSUMERS + PRODUCERS);
     static constexpr int TOKENS = 8 * NT;
-    static constexpr int SX_STRIDE = TOKENS + 4;  // floats: the blocks of a stage start in different banks
     static constexpr int CTAS = R >= 4 ? 1 : 2;  // per SM
-    static constexpr int W_BYTES = KB * MMA_CHUNK;  // of a row tile in a stage
+    static constexpr int W_BYTES = KB * MMA_CHUNK, X_BYTES = KB * MMA_X_CHUNK;  // of a row tile / token tile in a stage
     // As many stages as fit (up to 12): with five of them the small tiles had too few bytes of weights in flight.
-    static constexpr int STAGE_BYTES = R * W_BYTES + KB * (NT * 512 + SX_STRIDE * 4);
+    static constexpr int STAGE_BYTES = R * W_BYTES + NT * X_BYTES;
     static constexpr int FIT = (220000 / CTAS - R * NT * 512) / STAGE_BYTES, STAGES = FIT < 12 ? FIT : 12;
-    static constexpr int XW = NT, GROUPS = PRODUCERS / XW;  // producer warps to a stage; stages in the works at a time
+    static constexpr int XW = READY ? 1 : NT, GROUPS = PRODUCERS / XW;  // producer warps to a stage; stages in the works at a time
 };
 
-template <int R, int NT>
+template <int R, int NT, bool READY>
 struct MmaSmem {
-    using S = MmaShape<R, NT>;
+    using S = MmaShape<R, NT, READY>;
     struct Stage {
         alignas(16) uint8_t a[R][KB][MMA_CHUNK];      // as in memory
-        alignas(16) uint32_t b[KB][NT][32][4];        // f16 pairs: lane (token g, c), lane group l: elements 2c, 2c + 1
-        alignas(16) float sx[KB][S::SX_STRIDE];       // activation scales [block][token]
+        alignas(16) uint8_t b[NT][KB][MMA_X_CHUNK];   // as in an MmaInput: lane (token g, c)'s f16 pairs of the lane groups, scales
     };
     Stage stage[S::STAGES];
     alignas(16) float odd[R][NT][32][4];              // sums of the odd blocks, handed to the warp of the even ones
-    unsigned long long full[S::STAGES];               // weights landed + activations written
+    unsigned long long full[S::STAGES];               // weights and activations are there
     unsigned long long empty[S::STAGES];              // all consumer warps have read the stage
     unsigned long long odd_full[R], odd_empty[R];
     volatile uint32_t abort;
@@ -131,15 +130,6 @@ __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint3
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-__device__ __forceinline__ uint32_t hsub_1152(uint32_t v) {  // 1024 + (q + 128) -> q, both halves, exact
-    uint32_t r;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0xE480E480u));
-    return r;
-}
-// Bytes (q + 128) 0, 1 / 2, 3 of a word as f16 pairs.
-__device__ __forceinline__ uint32_t f16_pair_lo(uint32_t w) { return hsub_1152(__byte_perm(w, 0x64646464u, 0x4140)); }
-__device__ __forceinline__ uint32_t f16_pair_hi(uint32_t w) { return hsub_1152(__byte_perm(w, 0x64646464u, 0x4342)); }
-
 // D = A (16 x 8) * B (8 x 8): the dot products of one lane group, exact in f32.
 __device__ __forceinline__ void mma_16x8x8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
     asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
@@ -160,14 +150,14 @@ __device__ __forceinline__ MmaTile mma_decode_tile(const MmaJob& job, int t, int
     return r;
 }
 
-template <int R, int NT, bool Q8>
-__global__ void __launch_bounds__(MmaShape<R, NT>::THREADS, MmaShape<R, NT>::CTAS)
+template <int R, int NT, bool Q8, bool READY>
+__global__ void __launch_bounds__(MmaShape<R, NT, READY>::THREADS, MmaShape<R, NT, READY>::CTAS)
 k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 minus_zero, uint32_t* err) {
-    using S = MmaShape<R, NT>;
-    using Stage = typename MmaSmem<R, NT>::Stage;
+    using S = MmaShape<R, NT, READY>;
+    using Stage = typename MmaSmem<R, NT, READY>::Stage;
     pdl_trigger();
     extern __shared__ __align__(16) uint8_t mma_smem_raw[];
-    MmaSmem<R, NT>* sm = reinterpret_cast<MmaSmem<R, NT>*>(mma_smem_raw);
+    MmaSmem<R, NT, READY>* sm = reinterpret_cast<MmaSmem<R, NT, READY>*>(mma_smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = job.k / QK, k_stages = (nb + KB - 1) / KB;
     const int tiles_n = (job.n + S::TOKENS - 1) / S::TOKENS;
@@ -177,7 +167,7 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; s++) {
-            mbar_init(smem_u32(&sm->full[s]), 1 + S::XW);  // the weights' (with their bytes) + every producer warp's
+            mbar_init(smem_u32(&sm->full[s]), READY ? 1 : 1 + S::XW);  // the bulk copies' (with their bytes) + every converting warp's
             mbar_init(smem_u32(&sm->empty[s]), S::CONSUMERS);
         }
         for (int r = 0; r < R; r++) {
@@ -190,7 +180,52 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
     }
     __syncthreads();
 
-    if (warp >= S::CONSUMERS) {
+    if (READY && warp >= S::CONSUMERS) {
+        // ── producer: lane i < R copies row tile i of a stage, lane R + i token tile i (past the end: the last one again) ──
+        int wt = blockIdx.x, wks = 0, xt = blockIdx.x, xks = 0;  // tile and stage of it that is copied next
+        const int x_tiles = (job.n + MMA_X_ROWS - 1) / MMA_X_ROWS, x_item = min(max(lane - R, 0), NT - 1);
+        const uint8_t *wsrc = nullptr, *xsrc = nullptr;
+        const uint8_t* x = job.x;
+        auto copy_weights = [&](uint32_t s) {
+            if (wks == 0) {
+                const MmaTile tl = mma_decode_tile<R, S::TOKENS>(job, wt, tiles_n);
+                const int row_tiles = (job.m[tl.mat] + MMA_ROWS - 1) / MMA_ROWS;
+                wsrc = job.w[tl.mat] + (size_t)min(tl.row_tile0 + min(lane, R - 1), row_tiles - 1) * k_stages * S::W_BYTES;
+                wt += gridDim.x;
+            }
+            const uint32_t bar = fbar0 + s * 8;
+            if (lane == 0) mbar_arrive_expect_tx(bar, S::STAGE_BYTES);
+            __syncwarp();
+            if (lane < R) bulk_load(smem_u32(sm->stage[0].a[lane]) + s * (uint32_t)sizeof(Stage), wsrc, S::W_BYTES, bar);
+            wsrc += S::W_BYTES;
+            if (++wks == k_stages) wks = 0;
+        };
+        auto copy_activations = [&](uint32_t s) {
+            if (xks == 0) {
+                const int n0 = mma_decode_tile<R, S::TOKENS>(job, xt, tiles_n).n0;
+                xsrc = x + (size_t)min(n0 / MMA_X_ROWS + x_item, x_tiles - 1) * k_stages * S::X_BYTES;
+                xt += gridDim.x;
+            }
+            if (lane >= R && lane < R + NT) bulk_load(smem_u32(sm->stage[0].b[x_item]) + s * (uint32_t)sizeof(Stage), xsrc, S::X_BYTES, fbar0 + s * 8);
+            xsrc += S::X_BYTES;
+            if (++xks == k_stages) xks = 0;
+        };
+        const uint32_t ahead = min(g_total, (uint32_t)S::STAGES);  // stages whose weights are asked for before the activations are there
+        for (uint32_t g = 0; g < ahead; g++) copy_weights(g);
+        pdl_wait();
+        asm volatile("" : "+l"(x) : : "memory");
+        for (uint32_t g = 0; g < ahead; g++) copy_activations(g);
+        uint32_t s = 0, par = 0;
+        for (uint32_t g = ahead; g < g_total; g++) {
+            if (!mbar_wait(ebar0 + s * 8, par, &sm->abort, err, 1)) break;
+            copy_weights(s);
+            copy_activations(s);
+            if (++s == S::STAGES) {
+                s = 0;
+                par ^= 1;
+            }
+        }
+    } else if (warp >= S::CONSUMERS) {
         // ── producers: weights by bulk copies, activations converted to f16 in operand order ──
         // A stage belongs to XW warps (as many as there are token tiles), the stages go round the groups.  A warp takes four cycles and
         // more from one instruction to the next: with all four on every stage, ~150 instructions each, small tiles took 0.4 us a
@@ -271,7 +306,7 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
         Fetched f[DEPTH];
 #pragma unroll
         for (int d = 0; d < DEPTH; d++) fetch(f[d]);
-        const uint32_t b_dst = smem_u32(sm->stage[0].b[blk]) + (tok1 * 4 + 2 * half) * 16;
+        const uint32_t b_dst = smem_u32(sm->stage[0].b[0][blk]) + (tok1 * 4 + 2 * half) * 16;
         // the piece that is written first holds the bytes 0, 1 of the words in even blocks, 2, 3 in odd ones
         const uint32_t sel0 = piece ? 0x4342 : 0x4140, sel1 = piece ? 0x4140 : 0x4342;
         uint32_t s = grp, par = 1;
@@ -291,16 +326,19 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
                     uint32_t u[4], v[4];
 #pragma unroll
                     for (int l = 0; l < 4; l++) {
-                        u[l] = hsub_1152(__byte_perm(w[l], 0x64646464u, sel0));
-                        v[l] = hsub_1152(__byte_perm(w[l], 0x64646464u, sel1));
+                        u[l] = mma_hsub_1152(__byte_perm(w[l], 0x64646464u, sel0));
+                        v[l] = mma_hsub_1152(__byte_perm(w[l], 0x64646464u, sel1));
                     }
                     const int pair = i * S::XW + xw;  // tokens 2 * pair, 2 * pair + 1
-                    const uint32_t dst = b_dst + st + (pair >> 2) * 512 + (pair & 3) * 128;
+                    const uint32_t dst = b_dst + st + (pair >> 2) * S::X_BYTES + (pair & 3) * 128;
                     sts128(dst + piece * 16, u[0], u[1], u[2], u[3]);
                     sts128(dst + (piece ^ 1) * 16, v[0], v[1], v[2], v[3]);
                 }
 #pragma unroll
-                for (int i = 0; i < SCALES; i++) sm->stage[s].sx[lane % KB][((i * S::XW + xw) * 32 + lane) / KB] = f[d].s[i];
+                for (int i = 0; i < SCALES; i++) {
+                    const int tok = ((i * S::XW + xw) * 32 + lane) / KB;
+                    reinterpret_cast<float*>(sm->stage[s].b[tok / MMA_X_ROWS][lane % KB] + 512)[tok % MMA_X_ROWS] = f[d].s[i];
+                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(fbar0 + s * 8);
                 fetch(f[d]);
@@ -322,14 +360,14 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
             f32x2 sx[NT];
         };
         const uint32_t a_off = smem_u32(sm->stage[0].a[rt][parity]) + lane * 16, s_off = smem_u32(sm->stage[0].a[rt][parity]) + 512 + gid * 8;
-        const uint32_t b_off = smem_u32(sm->stage[0].b[parity][0][lane]), x_off = smem_u32(&sm->stage[0].sx[parity][2 * c]);
+        const uint32_t b_off = smem_u32(sm->stage[0].b[0][parity]) + lane * 16, x_off = smem_u32(sm->stage[0].b[0][parity]) + 512 + c * 8;
         auto load = [&](Frag& f, uint32_t st, int j) {  // j: which of the stage's blocks of this parity
             f.a = lds128(a_off + st + j * (2 * MMA_CHUNK));
             f.sw = lds64(s_off + st + j * (2 * MMA_CHUNK));
 #pragma unroll
             for (int n = 0; n < NT; n++) {
-                f.b[n] = lds128(b_off + st + j * (2 * NT * 512) + n * 512);
-                f.sx[n] = lds64(x_off + st + j * (2 * S::SX_STRIDE * 4) + n * 32);
+                f.b[n] = lds128(b_off + st + j * (2 * MMA_X_CHUNK) + n * S::X_BYTES);
+                f.sx[n] = lds64(x_off + st + j * (2 * MMA_X_CHUNK) + n * S::X_BYTES);
             }
         };
         f32x2 acc[NT][2][4];  // [token tile][row gid / gid + 8][lane group], halves = tokens 2c, 2c + 1
@@ -507,20 +545,21 @@ cudaError_t device_sm_count(int* sms) {
     return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
-template <int R, int NT, bool Q8>
-cudaError_t launch_shape(cudaStream_t st, const MmaJob& job, int sms, uint32_t* err) {
-    const size_t smem = sizeof(MmaSmem<R, NT>);
+template <int R, int NT, bool Q8, bool READY>
+cudaError_t launch_kernel(cudaStream_t st, const MmaJob& job, int sms, uint32_t* err) {
+    using S = MmaShape<R, NT, READY>;
+    const size_t smem = sizeof(MmaSmem<R, NT, READY>);
     static RaisedPerDevice limit;
-    const cudaError_t e = raise_dynamic_smem(limit, (const void*)k_gemm_mma<R, NT, Q8>, smem);
+    const cudaError_t e = raise_dynamic_smem(limit, (const void*)k_gemm_mma<R, NT, Q8, READY>, smem);
     if (e != cudaSuccess) return e;
     g_kernel_launches++;
     const f32x2 minus_zero = 0x8000000080000000ull;
-    return launch_pdl(st, k_gemm_mma<R, NT, Q8>, dim3(std::min(job.tile_start[3], sms * MmaShape<R, NT>::CTAS)), dim3(MmaShape<R, NT>::THREADS), smem, job,
-                      minus_zero, err);
+    return launch_pdl(st, k_gemm_mma<R, NT, Q8, READY>, dim3(std::min(job.tile_start[3], sms * S::CTAS)), dim3(S::THREADS), smem, job, minus_zero, err);
 }
 template <int R, int NT>
 cudaError_t launch_shape(cudaStream_t st, const MmaJob& job, bool q8, int sms, uint32_t* err) {
-    return q8 ? launch_shape<R, NT, true>(st, job, sms, err) : launch_shape<R, NT, false>(st, job, sms, err);
+    if (job.x) return q8 ? launch_kernel<R, NT, true, true>(st, job, sms, err) : launch_kernel<R, NT, false, true>(st, job, sms, err);
+    return q8 ? launch_kernel<R, NT, true, false>(st, job, sms, err) : launch_kernel<R, NT, false, false>(st, job, sms, err);
 }
 
 }  // namespace
@@ -537,15 +576,15 @@ cudaError_t mma_weight_fill(cudaStream_t st, const DevWeight& w, uint8_t* p) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const int8_t* xq, const float* xs,
-                            int n, uint32_t* err) {
+cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const uint8_t* x, const int8_t* xq,
+                            const float* xs, int n, uint32_t* err) {
     if (n <= 0 || count <= 0) return cudaSuccess;
     if (count > 3) return cudaErrorInvalidValue;
     for (int i = 1; i < count; i++) {
         if (w[i]->k != w[0]->k) return cudaErrorInvalidValue;
         if (w[i]->dtype != w[0]->dtype) {  // mixed types: a launch each
             for (int j = 0; j < count; j++) {
-                const cudaError_t e = launch_gemm_mma(st, w + j, out + j, 1, xq, xs, n, err);
+                const cudaError_t e = launch_gemm_mma(st, w + j, out + j, 1, x, xq, xs, n, err);
                 if (e != cudaSuccess) return e;
             }
             return cudaSuccess;
@@ -556,6 +595,7 @@ cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* c
     if (e != cudaSuccess) return e;
     MmaJob job;
     memset(&job, 0, sizeof(job));
+    job.x = x;
     job.xq = xq;
     job.xs = xs;
     job.n = n;

@@ -25,6 +25,7 @@ struct MmaJob {
     float* out[3];      // [n][m[i]] each
     int m[3];
     int tile_start[4];  // first linear tile of each matrix; [count..3] = total
+    const uint8_t* x;   // the activations in operand order (MmaInput::p, MmaWeight::stages() stages of blocks), or null and
     const int8_t* xq;   // quantised activations [n][k]
     const float* xs;    // [n][k / 32]
     int n, k;
@@ -39,7 +40,7 @@ cudaError_t mma_weight_fill(cudaStream_t st, const DevWeight& w, uint8_t* p);
 // out[i][j][r] for matrix i < count (<= 3, equal k), token j < n, row r < m_i (token-major, like launch_gemm), with the arithmetic of
 // gemm_q*_q8_0_neon (simd.rs:696-1019) in its order, for any f32 scales.  xq: 16-byte aligned.  err: word (device or mapped host
 // memory) that receives a non-zero code if a bounded wait expired.
-cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const int8_t* xq, const float* xs,
+cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const uint8_t* x, const int8_t* xq, const float* xs,
                             int n, uint32_t* err);
 
 }  // namespace wick

@@ -57,6 +57,46 @@ struct DecodeCtl {
     unsigned long long argmax;  // packed (key, index) accumulator of the argmax kernels
 };
 
+// Quantised rows in the order in which the bit-exact GEMM (gemm_mma.cu) takes them as operands: tiles of 8 rows, in a tile block
+// after block MMA_X_CHUNK bytes each: for every row g and c = 0 .. 3 the elements 2c, 2c + 1 of the four NEON lane groups as f16 pairs
+// (16 bytes at (4g + c) * 16), then the eight scales.  A tile has `blocks` blocks; those behind the row's last one stay zero.
+// The quantisers below write this form instead of q8s / q8q where they are given one (p not null).
+constexpr int MMA_X_ROWS = 8, MMA_X_CHUNK = 512 + MMA_X_ROWS * 4;
+struct MmaInput {
+    uint8_t* p = nullptr;
+    int blocks = 0;
+};
+__device__ __forceinline__ uint32_t mma_hsub_1152(uint32_t v) {  // 1024 + (q + 128) -> q, both halves, exact
+    uint32_t r;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0xE480E480u));
+    return r;
+}
+// Bytes (q + 128) 0, 1 / 2, 3 of a word as f16 pairs.
+__device__ __forceinline__ uint32_t f16_pair_lo(uint32_t w) { return mma_hsub_1152(__byte_perm(w, 0x64646464u, 0x4140)); }
+__device__ __forceinline__ uint32_t f16_pair_hi(uint32_t w) { return mma_hsub_1152(__byte_perm(w, 0x64646464u, 0x4342)); }
+__device__ __forceinline__ uint8_t* mma_x_chunk(const MmaInput& x, int row, int b) {
+    return x.p + ((size_t)(row / MMA_X_ROWS) * x.blocks + b) * MMA_X_CHUNK;
+}
+// Elements 4 e .. 4 e + 3 of a row's block (quantize_lane4's result); lane group e % 4, c = 2 (e / 4) and the next one.
+__device__ __forceinline__ void mma_x_store4(const MmaInput& x, int row, int b, int e, uint32_t q, float scale) {
+    uint8_t* chunk = mma_x_chunk(x, row, b);
+    const int g = row % MMA_X_ROWS;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(chunk + (g * 4 + (e >> 2) * 2) * 16) + (e & 3);
+    q ^= 0x80808080u;
+    dst[0] = f16_pair_lo(q);
+    dst[4] = f16_pair_hi(q);
+    if (e == 0) reinterpret_cast<float*>(chunk + 512)[g] = scale;
+}
+// The same from a warp that has one element of the block per lane.
+__device__ __forceinline__ void mma_x_store_lane(const MmaInput& x, int row, int b, int lane, int8_t q, float scale) {
+    uint8_t* chunk = mma_x_chunk(x, row, b);
+    const int g = row % MMA_X_ROWS;
+    const uint32_t v = (uint32_t)(uint8_t)q ^ 0x80u, next = __shfl_down_sync(0xffffffffu, v, 1);
+    if ((lane & 1) == 0)
+        reinterpret_cast<uint32_t*>(chunk + (g * 4 + (lane >> 4) * 2 + ((lane >> 1) & 1)) * 16)[(lane >> 2) & 3] = f16_pair_lo(v | next << 8);
+    if (lane == 0) reinterpret_cast<float*>(chunk + 512)[g] = scale;
+}
+
 // Re-layout of GGUF block rows into the quant / scale planes of DevWeight.
 void launch_repack(cudaStream_t st, const DevWeight& w, const uint8_t* raw, uint8_t* q, __half* d);
 
@@ -67,22 +107,22 @@ void launch_embed(cudaStream_t st, const DevWeight& w, const uint32_t* tokens, c
 // Optional residual add (hidden += add), RMSNorm (cpu.rs:577-594) and Q8_0 quantisation
 // (simd.rs:255-323) of n rows.  normed_out (f32) is optional.
 void launch_add_rmsnorm_quant(cudaStream_t st, float* hidden, const float* add, const float* weight, float eps,
-                              int n, int dim, float* q8s, int8_t* q8q, float* normed_out);
+                              int n, int dim, float* q8s, int8_t* q8q, float* normed_out, const MmaInput& x = MmaInput());
 // In-place RMSNorm of n rows (operator entry point).
 void launch_rmsnorm(cudaStream_t st, float* x, const float* weight, int n, int dim, float eps);
 // Q8_0 quantisation of n rows.
-void launch_quant_rows(cudaStream_t st, const float* x, int n, int k, float* q8s, int8_t* q8q);
+void launch_quant_rows(cudaStream_t st, const float* x, int n, int k, float* q8s, int8_t* q8q, const MmaInput& mx = MmaInput());
 // gate = silu(gate) * up (cpu.rs:668-673) over n rows of dim, then quantise -> q8; `act_out`
 // optional f32 copy.
 void launch_silu_mul_quant(cudaStream_t st, const float* gate, const float* up, int n, int dim, float* q8s,
-                           int8_t* q8q, float* act_out);
+                           int8_t* q8q, float* act_out, const MmaInput& x = MmaInput());
 void launch_silu_mul(cudaStream_t st, float* gate, const float* up, size_t count);
 void launch_expf(cudaStream_t st, const float* x, float* y, size_t count);
 
 // Gated short conv (lfm2.rs:688-725, :1316-1354) over n tokens, state [d_conv][hs] updated;
 // writes f32 out [n][hs] (optional) and its Q8_0 quantisation (optional).
 void launch_shortconv(cudaStream_t st, const float* proj, const float* conv_w, float* state, int n, int hs,
-                      int ksize, float* out, float* q8s, int8_t* q8q);
+                      int ksize, float* out, float* q8s, int8_t* q8q, const MmaInput& x = MmaInput());
 
 // Per-head QK RMSNorm + RoPE + KV append (lfm2.rs:783-855, :1544-1623).  q [n][hs] in place;
 // k, v [n][kv_dim] read; rows start_pos+j of the caches written.  start_pos < 0: read from ctl.
@@ -137,7 +177,7 @@ void launch_block_sums(cudaStream_t st, const DevWeight& w, const int8_t* xq, in
 // Multi-sequence decode step (kernels_batch.cu): row j of n is the next token of its own sequence, with its own
 // position and state.  `states`, `k_caches`, `v_caches` are device arrays of n per-row pointers.
 void launch_shortconv_rows(cudaStream_t st, const float* proj, const float* conv_w, float* const* states, int n, int hs, int ks,
-                           float* q8s, int8_t* q8q);
+                           float* q8s, int8_t* q8q, const MmaInput& x = MmaInput());
 void launch_qknorm_rope_kv_rows(cudaStream_t st, float* q, const float* k, const float* v, const float* q_norm, const float* k_norm,
                                 float eps, const float* rope_cos, const float* rope_sin, float* const* k_caches, float* const* v_caches,
                                 const uint32_t* positions, int n, int n_heads, int n_kv_heads, int head_dim);

@@ -71,8 +71,8 @@ void launch_embed(cudaStream_t st, const DevWeight& w, const uint32_t* tokens, c
 __global__ void __launch_bounds__(256) k_add_rmsnorm_quant(float* __restrict__ hidden, const float* __restrict__ add,
                                                           const float* __restrict__ weight, float eps, int dim,
                                                           float* __restrict__ q8s, int8_t* __restrict__ q8q,
-                                                          float* __restrict__ normed_out) {
-    pdl_enter(hidden, add, weight, q8s, q8q, normed_out);
+                                                          float* __restrict__ normed_out, MmaInput mx) {
+    pdl_enter(hidden, add, weight, q8s, q8q, normed_out, mx.p);
     extern __shared__ float xs[];
     __shared__ double red[32];
     const int row = blockIdx.x;
@@ -108,7 +108,9 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_quant(float* __restrict__ h
         if (q8q) {
             float sc;
             const uint32_t q = quantize_lane4(v, &sc);
-            if (in) {
+            if (in && mx.p) {
+                mma_x_store4(mx, row, b, lane & 7, q, sc);
+            } else if (in) {
                 *reinterpret_cast<uint32_t*>(q8q + (size_t)row * dim + i) = q;
                 if ((lane & 7) == 0) q8s[(size_t)row * nb + b] = sc;
             }
@@ -117,9 +119,9 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_quant(float* __restrict__ h
 }
 
 void launch_add_rmsnorm_quant(cudaStream_t st, float* hidden, const float* add, const float* weight, float eps, int n,
-                              int dim, float* q8s, int8_t* q8q, float* normed_out) {
+                              int dim, float* q8s, int8_t* q8q, float* normed_out, const MmaInput& x) {
     g_kernel_launches++;
-    launch_pdl(st, k_add_rmsnorm_quant, dim3(n), dim3(256), dim * sizeof(float), hidden, add, weight, eps, dim, q8s, q8q, normed_out);
+    launch_pdl(st, k_add_rmsnorm_quant, dim3(n), dim3(256), dim * sizeof(float), hidden, add, weight, eps, dim, q8s, q8q, normed_out, x);
 }
 
 __global__ void __launch_bounds__(256) k_rmsnorm_generic(float* __restrict__ x, const float* __restrict__ weight, int dim,
@@ -138,8 +140,8 @@ void launch_rmsnorm(cudaStream_t st, float* x, const float* weight, int n, int d
 
 // ── plain Q8_0 quantisation of rows ────────────────────────────────────────
 __global__ void k_quant_rows(const float* __restrict__ x, size_t total_blocks, float* __restrict__ q8s,
-                             int8_t* __restrict__ q8q) {
-    pdl_enter(x, q8s, q8q);
+                             int8_t* __restrict__ q8q, MmaInput mx, unsigned blocks_per_row) {
+    pdl_enter(x, q8s, q8q, mx.p);
     // 8 lanes per block, 4 consecutive elements per lane; lanes past the end still take part in the shuffles
     const size_t gt = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t b = gt >> 3;
@@ -148,24 +150,28 @@ __global__ void k_quant_rows(const float* __restrict__ x, size_t total_blocks, f
     const float4 v = in ? *reinterpret_cast<const float4*>(x + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     float sc;
     const uint32_t q = quantize_lane4(v, &sc);
-    if (in) {
+    if (in && mx.p) {
+        const unsigned row = (unsigned)b / blocks_per_row;
+        mma_x_store4(mx, row, (unsigned)b - row * blocks_per_row, threadIdx.x & 7, q, sc);
+    } else if (in) {
         *reinterpret_cast<uint32_t*>(q8q + i) = q;
         if ((threadIdx.x & 7) == 0) q8s[b] = sc;
     }
 }
 
-void launch_quant_rows(cudaStream_t st, const float* x, int n, int k, float* q8s, int8_t* q8q) {
+void launch_quant_rows(cudaStream_t st, const float* x, int n, int k, float* q8s, int8_t* q8q, const MmaInput& mx) {
     size_t total = (size_t)n * (k / QK);
     if (!total) return;
     unsigned grid = (unsigned)((total * 8 + 255) / 256);
     g_kernel_launches++;
-    launch_pdl(st, k_quant_rows, dim3(grid), dim3(256), 0, x, total, q8s, q8q);
+    launch_pdl(st, k_quant_rows, dim3(grid), dim3(256), 0, x, total, q8s, q8q, mx, (unsigned)(k / QK));
 }
 
 // ── SwiGLU + quantise ──────────────────────────────────────────────────────
 __global__ void k_silu_mul_quant(const float* __restrict__ gate, const float* __restrict__ up, size_t total_blocks,
-                                 float* __restrict__ q8s, int8_t* __restrict__ q8q, float* __restrict__ act_out) {
-    pdl_enter(gate, up, q8s, q8q, act_out);
+                                 float* __restrict__ q8s, int8_t* __restrict__ q8q, float* __restrict__ act_out, MmaInput mx,
+                                 unsigned blocks_per_row) {
+    pdl_enter(gate, up, q8s, q8q, act_out, mx.p);
     const size_t gt = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t b = gt >> 3;
     const bool in = b < total_blocks;
@@ -178,19 +184,22 @@ __global__ void k_silu_mul_quant(const float* __restrict__ gate, const float* __
     }
     float sc;
     const uint32_t q = quantize_lane4(a, &sc);
-    if (in) {
+    if (in && mx.p) {
+        const unsigned row = (unsigned)b / blocks_per_row;
+        mma_x_store4(mx, row, (unsigned)b - row * blocks_per_row, threadIdx.x & 7, q, sc);
+    } else if (in) {
         *reinterpret_cast<uint32_t*>(q8q + i) = q;
         if ((threadIdx.x & 7) == 0) q8s[b] = sc;
     }
 }
 
 void launch_silu_mul_quant(cudaStream_t st, const float* gate, const float* up, int n, int dim, float* q8s, int8_t* q8q,
-                           float* act_out) {
+                           float* act_out, const MmaInput& x) {
     size_t total = (size_t)n * (dim / QK);
     if (!total) return;
     unsigned grid = (unsigned)((total * 8 + 255) / 256);
     g_kernel_launches++;
-    launch_pdl(st, k_silu_mul_quant, dim3(grid), dim3(256), 0, gate, up, total, q8s, q8q, act_out);
+    launch_pdl(st, k_silu_mul_quant, dim3(grid), dim3(256), 0, gate, up, total, q8s, q8q, act_out, x, (unsigned)(dim / QK));
 }
 
 __global__ void k_silu_mul(float* __restrict__ gate, const float* __restrict__ up, size_t count) {
@@ -221,8 +230,8 @@ void launch_expf(cudaStream_t st, const float* x, float* y, size_t count) {
 // A warp owns 32 consecutive channels of one token = one Q8_0 block of the out_proj input.
 __global__ void k_shortconv(const float* __restrict__ proj, const float* __restrict__ conv_w,
                             const float* __restrict__ state, int n, int hs, int ks, float* __restrict__ out,
-                            float* __restrict__ q8s, int8_t* __restrict__ q8q) {
-    pdl_enter(proj, conv_w, state, out, q8s, q8q);
+                            float* __restrict__ q8s, int8_t* __restrict__ q8q, MmaInput mx) {
+    pdl_enter(proj, conv_w, state, out, q8s, q8q, mx.p);
     const int dc = ks - 1;
     size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
@@ -249,8 +258,12 @@ __global__ void k_shortconv(const float* __restrict__ proj, const float* __restr
     if (q8q) {
         float sc;
         int8_t q = quantize_lane(o, &sc);
-        q8q[(size_t)j * hs + ch] = q;
-        if (lane == 0) q8s[gw] = sc;
+        if (mx.p) {
+            mma_x_store_lane(mx, j, ch / QK, lane, q, sc);
+        } else {
+            q8q[(size_t)j * hs + ch] = q;
+            if (lane == 0) q8s[gw] = sc;
+        }
     }
 }
 
@@ -276,11 +289,11 @@ __global__ void k_shortconv_state(const float* __restrict__ proj, float* __restr
 }
 
 void launch_shortconv(cudaStream_t st, const float* proj, const float* conv_w, float* state, int n, int hs, int ks,
-                      float* out, float* q8s, int8_t* q8q) {
+                      float* out, float* q8s, int8_t* q8q, const MmaInput& x) {
     size_t warps = (size_t)n * (hs / QK);
     if (!warps) return;
     g_kernel_launches++;
-    launch_pdl(st, k_shortconv, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, state, n, hs, ks, out, q8s, q8q);
+    launch_pdl(st, k_shortconv, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, state, n, hs, ks, out, q8s, q8q, x);
     if (ks > 1) g_kernel_launches++, launch_pdl(st, k_shortconv_state, dim3((hs + 255) / 256), dim3(256), 0, proj, state, n, hs, ks);
 }
 

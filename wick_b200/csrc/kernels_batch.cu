@@ -13,8 +13,8 @@ namespace wick {
 // A warp owns 32 consecutive channels of one row = one Q8_0 block of the out_proj input.  The row's rolling
 // buffer [d_conv][hs] is read, used and advanced by the thread that owns the channel.
 __global__ void k_shortconv_rows(const float* __restrict__ proj, const float* __restrict__ conv_w, float* const* __restrict__ states,
-                                 int n, int hs, int ks, float* __restrict__ q8s, int8_t* __restrict__ q8q) {
-    pdl_enter(proj, conv_w, states, q8s, q8q);
+                                 int n, int hs, int ks, float* __restrict__ q8s, int8_t* __restrict__ q8q, MmaInput mx) {
+    pdl_enter(proj, conv_w, states, q8s, q8q, mx.p);
     const int dc = ks - 1;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -39,16 +39,20 @@ __global__ void k_shortconv_rows(const float* __restrict__ proj, const float* __
     if (dc > 0) state[(size_t)(dc - 1) * hs + ch] = bx;
     float sc;
     const int8_t q = quantize_lane(o, &sc);
-    q8q[(size_t)j * hs + ch] = q;
-    if (lane == 0) q8s[gw] = sc;
+    if (mx.p) {
+        mma_x_store_lane(mx, j, ch / QK, lane, q, sc);
+    } else {
+        q8q[(size_t)j * hs + ch] = q;
+        if (lane == 0) q8s[gw] = sc;
+    }
 }
 
 void launch_shortconv_rows(cudaStream_t st, const float* proj, const float* conv_w, float* const* states, int n, int hs, int ks,
-                           float* q8s, int8_t* q8q) {
+                           float* q8s, int8_t* q8q, const MmaInput& x) {
     const size_t warps = (size_t)n * (hs / QK);
     if (!warps) return;
     g_kernel_launches++;
-    launch_pdl(st, k_shortconv_rows, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, states, n, hs, ks, q8s, q8q);
+    launch_pdl(st, k_shortconv_rows, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, states, n, hs, ks, q8s, q8q, x);
 }
 
 // ── per-head QK RMSNorm + RoPE + KV append, per-row position and caches (lfm2.rs:783-855) ──

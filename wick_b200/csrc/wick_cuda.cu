@@ -92,6 +92,7 @@ struct wick_cuda_model {
     // tensor-core prefill GEMMs: available when every matrix meets tc_gemm_supported(); prefill_mode
     // picks the bit-exact one (default), the fused-chain one, or the bit-exact CUDA-core kernel
     bool tc_ok = false;     // the model's shapes allow the tensor-core GEMM
+    MmaInput x_hs, x_is;    // inputs of the exact GEMM in its operand order, max_chunk rows of hidden / feed-forward size
     bool exact_built = false, fused_built = false;  // the layers' copies exist (made by the first call that needs them)
     int prefill_mode = WICK_CUDA_PREFILL_EXACT;
     CUtensorMap map_x_hs, map_x_is;  // activations [max_chunk][hs | is] for the fused-chain GEMM
@@ -722,9 +723,13 @@ struct GemmTarget {
     const GemmCopies* t;
     float* out;
 };
-void run_gemms(wick_cuda_model* m, int n, std::initializer_list<GemmTarget> list) {
+// Where the inputs of n rows of k elements go if the exact GEMM multiplies them, else null.
+MmaInput mma_input(const wick_cuda_model* m, int n, int k) {
+    if (!m->exact_built || n < 2 || m->prefill_mode != WICK_CUDA_PREFILL_EXACT) return MmaInput();
+    return k == (int)m->cfg.hidden_size ? m->x_hs : m->x_is;
+}
+void run_gemms(wick_cuda_model* m, int n, const MmaInput& x, std::initializer_list<GemmTarget> list) {
     cudaStream_t st = m->stream;
-    bool exact = m->exact_built && n >= 2 && m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
     bool fused = m->fused_built && n >= TC_FUSED_MIN_TOKENS && m->prefill_mode == WICK_CUDA_PREFILL_TENSOR;
     const MmaWeight* ew[3] = {};
     const TcWeight* fw[3] = {};
@@ -734,12 +739,11 @@ void run_gemms(wick_cuda_model* m, int n, std::initializer_list<GemmTarget> list
         ew[c] = &g.t->exact;
         fw[c] = &g.t->fused;
         outs[c++] = g.out;
-        exact = exact && g.t->exact.p;
         fused = fused && g.t->fused.q;
     }
     // (errors surface in the cudaGetLastError() check after the chunk)
-    if (exact)
-        (void)launch_gemm_mma(st, ew, outs, c, m->q8q, m->q8s, n, m->tc_err);
+    if (x.p)
+        (void)launch_gemm_mma(st, ew, outs, c, x.p, nullptr, nullptr, n, m->tc_err);
     else if (fused)
         (void)launch_gemm_tc(st, fw, outs, c, fw[0]->k == (int)m->cfg.hidden_size ? m->map_x_hs : m->map_x_is, m->q8s, n, nullptr, m->tc_err);
     else
@@ -756,24 +760,25 @@ void enqueue_prefill_chunk(wick_cuda_model* m, int n, int start_pos, bool flash,
     cudaStream_t st = m->stream;
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size, hd = m->head_dim;
     const float eps = m->cfg.rms_norm_eps;
-    auto gemms = [&](std::initializer_list<GemmTarget> list) { run_gemms(m, n, list); };
+    const MmaInput xh = mma_input(m, n, hs), xi = mma_input(m, n, is);
+    auto gemms = [&](const MmaInput& x, std::initializer_list<GemmTarget> list) { run_gemms(m, n, x, list); };
     prof_begin(m);
     if (embed) embed_rows(m, m->tokens_dev, nullptr, n);
     prof_mark(m, PC_EMBED);
     const float* pending = nullptr;
     for (size_t li = 0; li < m->layers.size(); li++) {
         Layer& L = m->layers[li];
-        launch_add_rmsnorm_quant(st, m->hidden, pending, L.attn_norm, eps, n, hs, m->q8s, m->q8q, nullptr);
+        launch_add_rmsnorm_quant(st, m->hidden, pending, L.attn_norm, eps, n, hs, m->q8s, m->q8q, nullptr, xh);
         prof_mark(m, PC_NORM_QUANT);
         if (!L.is_attn) {
-            gemms({{&L.in_proj, &L.tc_in_proj, m->proj}});
+            gemms(xh, {{&L.in_proj, &L.tc_in_proj, m->proj}});
             prof_mark(m, PC_GEMM);
-            launch_shortconv(st, m->proj, L.conv_w, L.conv_state, n, hs, m->cfg.conv_kernel_size, nullptr, m->q8s, m->q8q);
+            launch_shortconv(st, m->proj, L.conv_w, L.conv_state, n, hs, m->cfg.conv_kernel_size, nullptr, m->q8s, m->q8q, xh);
             prof_mark(m, PC_SHORTCONV);
-            gemms({{&L.out_proj, &L.tc_out_proj, m->block_out}});
+            gemms(xh, {{&L.out_proj, &L.tc_out_proj, m->block_out}});
             prof_mark(m, PC_GEMM);
         } else {
-            gemms({{&L.q, &L.tc_q, m->qbuf}, {&L.k, &L.tc_k, m->kbuf}, {&L.v, &L.tc_v, m->vbuf}});
+            gemms(xh, {{&L.q, &L.tc_q, m->qbuf}, {&L.k, &L.tc_k, m->kbuf}, {&L.v, &L.tc_v, m->vbuf}});
             prof_mark(m, PC_GEMM);
             launch_qknorm_rope_kv(st, m->qbuf, m->kbuf, m->vbuf, L.q_norm, L.k_norm, eps, m->rope_cos, m->rope_sin, L.k_cache,
                                   L.v_cache, n, start_pos, nullptr, m->cfg.n_heads, L.n_kv, hd);
@@ -784,18 +789,18 @@ void enqueue_prefill_chunk(wick_cuda_model* m, int n, int start_pos, bool flash,
                 launch_attention_naive(st, m->qbuf, L.k_cache, L.v_cache, m->attn_out, n, start_pos, nullptr, m->cfg.n_heads,
                                        L.n_kv, hd, m->cfg.max_seq_len);
             prof_mark(m, PC_ATTENTION);
-            launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q);
+            launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q, xh);
             prof_mark(m, PC_ACT_QUANT);
-            gemms({{&L.o, &L.tc_o, m->block_out}});
+            gemms(xh, {{&L.o, &L.tc_o, m->block_out}});
             prof_mark(m, PC_GEMM);
         }
-        launch_add_rmsnorm_quant(st, m->hidden, m->block_out, L.ffn_norm, eps, n, hs, m->q8s, m->q8q, nullptr);
+        launch_add_rmsnorm_quant(st, m->hidden, m->block_out, L.ffn_norm, eps, n, hs, m->q8s, m->q8q, nullptr, xh);
         prof_mark(m, PC_NORM_QUANT);
-        gemms({{&L.gate, &L.tc_gate, m->gate}, {&L.up, &L.tc_up, m->up}});
+        gemms(xh, {{&L.gate, &L.tc_gate, m->gate}, {&L.up, &L.tc_up, m->up}});
         prof_mark(m, PC_GEMM);
-        launch_silu_mul_quant(st, m->gate, m->up, n, is, m->q8s, m->q8q, nullptr);
+        launch_silu_mul_quant(st, m->gate, m->up, n, is, m->q8s, m->q8q, nullptr, xi);
         prof_mark(m, PC_ACT_QUANT);
-        gemms({{&L.down, &L.tc_down, m->ffn_out}});
+        gemms(xi, {{&L.down, &L.tc_down, m->ffn_out}});
         prof_mark(m, PC_GEMM);
         pending = m->ffn_out;
     }
@@ -858,7 +863,17 @@ int32_t make_copies(wick_cuda_model* m, bool exact) {
         W_TRY(fill(L.up, &L.tc_up));
         W_TRY(fill(L.down, &L.tc_down));
     }
-    if (!exact) {
+    if (exact) {
+        auto input = [&](int k, MmaInput* x) -> int32_t {
+            x->blocks = (k / QK + MMA_STAGE_BLOCKS - 1) / MMA_STAGE_BLOCKS * MMA_STAGE_BLOCKS;
+            const size_t bytes = (size_t)(m->max_chunk + MMA_X_ROWS - 1) / MMA_X_ROWS * x->blocks * MMA_X_CHUNK;
+            W_TRY(dev_alloc(m, &x->p, bytes));
+            CU_TRY(cudaMemsetAsync(x->p, 0, bytes, m->stream));  // (blocks behind the last one are read, never written)
+            return WICK_CUDA_OK;
+        };
+        W_TRY(input(m->cfg.hidden_size, &m->x_hs));
+        W_TRY(input(m->cfg.intermediate_size, &m->x_is));
+    } else {
         CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.hidden_size, TC_TENSOR_TOKENS, &m->map_x_hs));
         CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.intermediate_size, TC_TENSOR_TOKENS, &m->map_x_is));
     }
@@ -1175,20 +1190,22 @@ int32_t enqueue_decode_rows(wick_cuda_model* m, int n, int seq_bound) {
     cudaStream_t st = m->stream;
     const int hs = m->cfg.hidden_size, is = m->cfg.intermediate_size, hd = m->head_dim, cap = m->batch_cap;
     const float eps = m->cfg.rms_norm_eps;
-    auto gemms = [&](std::initializer_list<GemmTarget> list) { run_gemms(m, n, list); };
+    const MmaInput xh = mma_input(m, n, hs), xi = mma_input(m, n, is);
+    const MmaInput x_head = m->tc_embd.exact.p ? xh : MmaInput();
+    auto gemms = [&](const MmaInput& x, std::initializer_list<GemmTarget> list) { run_gemms(m, n, x, list); };
     embed_rows(m, m->rows_tok, nullptr, n);
     const float* pending = nullptr;
     for (size_t li = 0; li < m->layers.size(); li++) {
         Layer& L = m->layers[li];
         float** p0 = m->rows_ptrs + (li * 2) * cap;
         float** p1 = m->rows_ptrs + (li * 2 + 1) * cap;
-        launch_add_rmsnorm_quant(st, m->hidden, pending, L.attn_norm, eps, n, hs, m->q8s, m->q8q, nullptr);
+        launch_add_rmsnorm_quant(st, m->hidden, pending, L.attn_norm, eps, n, hs, m->q8s, m->q8q, nullptr, xh);
         if (!L.is_attn) {
-            gemms({{&L.in_proj, &L.tc_in_proj, m->proj}});
-            launch_shortconv_rows(st, m->proj, L.conv_w, p0, n, hs, m->cfg.conv_kernel_size, m->q8s, m->q8q);
-            gemms({{&L.out_proj, &L.tc_out_proj, m->block_out}});
+            gemms(xh, {{&L.in_proj, &L.tc_in_proj, m->proj}});
+            launch_shortconv_rows(st, m->proj, L.conv_w, p0, n, hs, m->cfg.conv_kernel_size, m->q8s, m->q8q, xh);
+            gemms(xh, {{&L.out_proj, &L.tc_out_proj, m->block_out}});
         } else {
-            gemms({{&L.q, &L.tc_q, m->qbuf}, {&L.k, &L.tc_k, m->kbuf}, {&L.v, &L.tc_v, m->vbuf}});
+            gemms(xh, {{&L.q, &L.tc_q, m->qbuf}, {&L.k, &L.tc_k, m->kbuf}, {&L.v, &L.tc_v, m->vbuf}});
             launch_qknorm_rope_kv_rows(st, m->qbuf, m->kbuf, m->vbuf, L.q_norm, L.k_norm, eps, m->rope_cos, m->rope_sin, p0, p1, m->rows_pos, n,
                                        m->cfg.n_heads, L.n_kv, hd);
             if (m->attn_splitk)
@@ -1196,21 +1213,21 @@ int32_t enqueue_decode_rows(wick_cuda_model* m, int n, int seq_bound) {
                                         hd, m->cfg.max_seq_len);
             else
                 CU_TRY(launch_attention_rows(st, m->qbuf, p0, p1, m->rows_pos, m->attn_out, n, m->cfg.n_heads, L.n_kv, hd, seq_bound));
-            launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q);
-            gemms({{&L.o, &L.tc_o, m->block_out}});
+            launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q, xh);
+            gemms(xh, {{&L.o, &L.tc_o, m->block_out}});
         }
-        launch_add_rmsnorm_quant(st, m->hidden, m->block_out, L.ffn_norm, eps, n, hs, m->q8s, m->q8q, nullptr);
-        gemms({{&L.gate, &L.tc_gate, m->gate}, {&L.up, &L.tc_up, m->up}});
-        launch_silu_mul_quant(st, m->gate, m->up, n, is, m->q8s, m->q8q, nullptr);
-        gemms({{&L.down, &L.tc_down, m->ffn_out}});
+        launch_add_rmsnorm_quant(st, m->hidden, m->block_out, L.ffn_norm, eps, n, hs, m->q8s, m->q8q, nullptr, xh);
+        gemms(xh, {{&L.gate, &L.tc_gate, m->gate}, {&L.up, &L.tc_up, m->up}});
+        launch_silu_mul_quant(st, m->gate, m->up, n, is, m->q8s, m->q8q, nullptr, xi);
+        gemms(xi, {{&L.down, &L.tc_down, m->ffn_out}});
         pending = m->ffn_out;
     }
-    launch_add_rmsnorm_quant(st, m->hidden, pending, m->output_norm, eps, n, hs, m->q8s, m->q8q, nullptr);
+    launch_add_rmsnorm_quant(st, m->hidden, pending, m->output_norm, eps, n, hs, m->q8s, m->q8q, nullptr, x_head);
     if (m->embd_q6k) {
         for (int j = 0; j < n; j++)
             launch_gemv_q6k(st, m->embd6, m->q8s + (size_t)j * (hs / QK), m->q8q + (size_t)j * hs, m->logits_rows + (size_t)j * m->cfg.vocab_size);
     } else {
-        gemms({{&m->embd, &m->tc_embd, m->logits_rows}});
+        gemms(x_head, {{&m->embd, &m->tc_embd, m->logits_rows}});
     }
     return WICK_CUDA_OK;
 }
@@ -2139,7 +2156,7 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
             W_TRY(take_tc_error(w));
             const MmaWeight* tw[1] = {&w->exact};
             float* outs[1] = {out_dev};
-            CU_TRY(launch_gemm_mma(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
+            CU_TRY(launch_gemm_mma(st, tw, outs, 1, nullptr, bq_dev, bs_dev, (int)n, w->tc_err));
             OP_END();
         }
     }
@@ -2174,7 +2191,7 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     const MmaWeight* tw[1] = {&w->exact};
     float* outs[1] = {out_dev};
     if ((uintptr_t)bq_dev & 15) launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);  // (the tensor cores' kernel reads 16 bytes at a time)
-    else CU_TRY(launch_gemm_mma(st, tw, outs, 1, bq_dev, bs_dev, (int)n, w->tc_err));
+    else CU_TRY(launch_gemm_mma(st, tw, outs, 1, nullptr, bq_dev, bs_dev, (int)n, w->tc_err));
     CU_TRY(cudaGetLastError());
     CU_TRY(cudaStreamSynchronize(st));
     return take_tc_error(w);
