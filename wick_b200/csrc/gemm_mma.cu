@@ -33,34 +33,34 @@ namespace {
 constexpr int KB = MMA_STAGE_BLOCKS;  // blocks per pipeline stage (256 elements of K)
 constexpr uint32_t MMA_SPIN_LIMIT = 1u << 18;  // try_wait itself suspends for a while, so this is of the order of a second
 
-// R x 16 rows, NT x 8 tokens; a warp takes 16 rows and the blocks of one parity, so 2R consumer warps.  READY: the activations are
+// R x 16 rows, NT x 8 tokens; a warp takes 16 rows, the blocks of one parity and 4 / LS of the lane groups: 2 R LS consumer warps.  READY: the activations are
 // there in operand order (MmaInput) and come by bulk copies like the weights, issued by one warp; otherwise (operators: int8 columns
 // of the caller) four warps convert them.
-template <int R, int NT, bool READY>
+template <int R, int NT, bool READY, int LS>
 struct MmaShape {
-    static constexpr int CONSUMERS = 2 * R, PRODUCERS = READY ? 1 : 4;
+    static constexpr int CONSUMERS = 2 * R * LS, LG = 4 / LS, PRODUCERS = READY ? 1 : 4;
     static constexpr int THREADS = 32 * (CONSUMERS + PRODUCERS);
     static constexpr int TOKENS = 8 * NT;
     static constexpr int CTAS = R >= 4 ? 1 : 2;  // per SM
     static constexpr int W_BYTES = KB * MMA_CHUNK, X_BYTES = KB * MMA_X_CHUNK;  // of a row tile / token tile in a stage
     // As many stages as fit (up to 12): with five of them the small tiles had too few bytes of weights in flight.
     static constexpr int STAGE_BYTES = R * W_BYTES + NT * X_BYTES;
-    static constexpr int FIT = (220000 / CTAS - R * NT * 512) / STAGE_BYTES, STAGES = FIT < 12 ? FIT : 12;
+    static constexpr int FIT = (220000 / CTAS - R * (2 * LS - 1) * NT * 512) / STAGE_BYTES, STAGES = FIT < 12 ? FIT : 12;
     static constexpr int XW = READY ? 1 : NT, GROUPS = PRODUCERS / XW;  // producer warps to a stage; stages in the works at a time
 };
 
-template <int R, int NT, bool READY>
+template <int R, int NT, bool READY, int LS>
 struct MmaSmem {
-    using S = MmaShape<R, NT, READY>;
+    using S = MmaShape<R, NT, READY, LS>;
     struct Stage {
         alignas(16) uint8_t a[R][KB][MMA_CHUNK];      // as in memory
         alignas(16) uint8_t b[NT][KB][MMA_X_CHUNK];   // as in an MmaInput: lane (token g, c)'s f16 pairs of the lane groups, scales
     };
     Stage stage[S::STAGES];
-    alignas(16) float odd[R][NT][32][4];              // sums of the odd blocks, handed to the warp of the even ones
+    alignas(16) float part[R][2 * LS - 1][NT][32][4];  // sums of a row tile's other warps, handed to its first one
     unsigned long long full[S::STAGES];               // weights and activations are there
     unsigned long long empty[S::STAGES];              // all consumer warps have read the stage
-    unsigned long long odd_full[R], odd_empty[R];
+    unsigned long long part_full[R], part_empty[R];
     volatile uint32_t abort;
 };
 
@@ -116,10 +116,14 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  : "memory");
 }
 
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
+template <int N>
+__device__ __forceinline__ void lds_words(uint32_t (&v)[N], uint32_t a) {
+    if constexpr (N == 4)
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
+    else if constexpr (N == 2)
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(a));
+    else
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[0]) : "r"(a));
 }
 __device__ __forceinline__ f32x2 lds64(uint32_t a) {
     f32x2 v;
@@ -150,14 +154,14 @@ __device__ __forceinline__ MmaTile mma_decode_tile(const MmaJob& job, int t, int
     return r;
 }
 
-template <int R, int NT, bool Q8, bool READY>
-__global__ void __launch_bounds__(MmaShape<R, NT, READY>::THREADS, MmaShape<R, NT, READY>::CTAS)
+template <int R, int NT, bool Q8, bool READY, int LS>
+__global__ void __launch_bounds__(MmaShape<R, NT, READY, LS>::THREADS, MmaShape<R, NT, READY, LS>::CTAS)
 k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 minus_zero, uint32_t* err) {
-    using S = MmaShape<R, NT, READY>;
-    using Stage = typename MmaSmem<R, NT, READY>::Stage;
+    using S = MmaShape<R, NT, READY, LS>;
+    using Stage = typename MmaSmem<R, NT, READY, LS>::Stage;
     pdl_trigger();
     extern __shared__ __align__(16) uint8_t mma_smem_raw[];
-    MmaSmem<R, NT, READY>* sm = reinterpret_cast<MmaSmem<R, NT, READY>*>(mma_smem_raw);
+    MmaSmem<R, NT, READY, LS>* sm = reinterpret_cast<MmaSmem<R, NT, READY, LS>*>(mma_smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = job.k / QK, k_stages = (nb + KB - 1) / KB;
     const int tiles_n = (job.n + S::TOKENS - 1) / S::TOKENS;
@@ -171,8 +175,8 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
             mbar_init(smem_u32(&sm->empty[s]), S::CONSUMERS);
         }
         for (int r = 0; r < R; r++) {
-            mbar_init(smem_u32(&sm->odd_full[r]), 1);
-            mbar_init(smem_u32(&sm->odd_empty[r]), 1);
+            mbar_init(smem_u32(&sm->part_full[r]), 2 * LS - 1);
+            mbar_init(smem_u32(&sm->part_empty[r]), 1);
         }
         sm->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -351,64 +355,65 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
         }
     } else {
         // ── consumers ──
-        const int rt = warp >> 1, parity = warp & 1, gid = lane >> 2, c = lane & 3;
+        constexpr int LG = S::LG;
+        const int rt = warp / (2 * LS), role = warp % (2 * LS), parity = role & 1, part = role >> 1, gid = lane >> 2, c = lane & 3;
         pdl_wait();  // (the outputs may still be read by the predecessor)
         struct Frag {
-            uint4 a;
+            uint32_t a[LG];
             f32x2 sw;  // rows gid, gid + 8
-            uint4 b[NT];
+            uint32_t b[NT][LG];
             f32x2 sx[NT];
         };
-        const uint32_t a_off = smem_u32(sm->stage[0].a[rt][parity]) + lane * 16, s_off = smem_u32(sm->stage[0].a[rt][parity]) + 512 + gid * 8;
-        const uint32_t b_off = smem_u32(sm->stage[0].b[0][parity]) + lane * 16, x_off = smem_u32(sm->stage[0].b[0][parity]) + 512 + c * 8;
+        const uint32_t a_off = smem_u32(sm->stage[0].a[rt][parity]) + lane * 16 + part * (4 * LG), s_off = smem_u32(sm->stage[0].a[rt][parity]) + 512 + gid * 8;
+        const uint32_t b_off = smem_u32(sm->stage[0].b[0][parity]) + lane * 16 + part * (4 * LG), x_off = smem_u32(sm->stage[0].b[0][parity]) + 512 + c * 8;
         auto load = [&](Frag& f, uint32_t st, int j) {  // j: which of the stage's blocks of this parity
-            f.a = lds128(a_off + st + j * (2 * MMA_CHUNK));
+            lds_words(f.a, a_off + st + j * (2 * MMA_CHUNK));
             f.sw = lds64(s_off + st + j * (2 * MMA_CHUNK));
 #pragma unroll
             for (int n = 0; n < NT; n++) {
-                f.b[n] = lds128(b_off + st + j * (2 * MMA_X_CHUNK) + n * S::X_BYTES);
+                lds_words(f.b[n], b_off + st + j * (2 * MMA_X_CHUNK) + n * S::X_BYTES);
                 f.sx[n] = lds64(x_off + st + j * (2 * MMA_X_CHUNK) + n * S::X_BYTES);
             }
         };
-        f32x2 acc[NT][2][4];  // [token tile][row gid / gid + 8][lane group], halves = tokens 2c, 2c + 1
+        f32x2 acc[NT][2][LG];  // [token tile][row gid / gid + 8][lane group], halves = tokens 2c, 2c + 1
         auto chains = [&](const Frag& f) {
-            const uint32_t w[4] = {f.a.x, f.a.y, f.a.z, f.a.w};
-            uint32_t a0[4], a1[4];
+            uint32_t a0[LG], a1[LG];
 #pragma unroll
-            for (int l = 0; l < 4; l++) {
-                a0[l] = Q8 ? f16_pair_lo(w[l]) : __byte_perm(w[l], 0, 0x1404);  // (an e5m2 byte is the upper half of its f16)
-                a1[l] = Q8 ? f16_pair_hi(w[l]) : __byte_perm(w[l], 0, 0x3424);
+            for (int l = 0; l < LG; l++) {
+                a0[l] = Q8 ? f16_pair_lo(f.a[l]) : __byte_perm(f.a[l], 0, 0x1404);
+                a1[l] = Q8 ? f16_pair_hi(f.a[l]) : __byte_perm(f.a[l], 0, 0x3424);
             }
             float s0, s1;
             unpack2(f.sw, s0, s1);
             const f32x2 sw[2] = {pack2(s0, s0), pack2(s1, s1)};
 #pragma unroll
             for (int n = 0; n < NT; n++) {
-                const uint32_t b[4] = {f.b[n].x, f.b[n].y, f.b[n].z, f.b[n].w};
-                float p[4][4];
+                float p[LG][4];
 #pragma unroll
-                for (int l = 0; l < 4; l++) mma_16x8x8(p[l], a0[l], a1[l], b[l]);
+                for (int l = 0; l < LG; l++) mma_16x8x8(p[l], a0[l], a1[l], f.b[n][l]);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const f32x2 d = mul2(sw[h], f.sx[n]);
 #pragma unroll
-                    for (int l = 0; l < 4; l++)  // (+ -0: the product alone, which a packed mul + add would not stay)
+                    for (int l = 0; l < LG; l++)  // (+ -0: the product alone, which a packed mul + add would not stay)
                         acc[n][h][l] = add2(acc[n][h][l], fma2(pack2(p[l][2 * h], p[l][2 * h + 1]), d, minus_zero));
                 }
             }
         };
         uint32_t g = 0, tile_no = 0, s = 0, par = 0;
         bool ok = g_total == 0 || mbar_wait(fbar0, 0, &sm->abort, err, 2);
-        // A small tile's warp is alone with its latencies: the next block's operands are loaded under the chains of one, across
-        // stages too.  The large ones have three warps to a scheduler and no registers for that (R = 6: 107 against 98.7 us).
-        constexpr bool AHEAD = NT <= 2;
+        // A warp that is alone on its scheduler, or nearly, waits for its own loads: the next block's operands are loaded under the
+        // chains of one, across stages too.  From two token tiles on a block has work enough to hide them, and the registers
+        // are better left to the compiler (64 x 16 tiles: 2048 x 6912 at 64 tokens 19.0 against 17.6 us, at 512 121 against
+        // 108; R = 6, NT = 4: 103 against 96 us for 6144 x 2048).  Where converting warps share the schedulers, NT = 2 wants it too.
+        constexpr bool AHEAD = NT == 1 || (NT == 2 && !READY);
         Frag f0, f1;
         if (AHEAD) load(f0, 0, 0);
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, tile_no++) {
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
-                for (int l = 0; l < 4; l++) acc[n][0][l] = acc[n][1][l] = pack2(0.f, 0.f);
+                for (int l = 0; l < LG; l++) acc[n][0][l] = acc[n][1][l] = pack2(0.f, 0.f);
 #pragma unroll 1
             for (int ks = 0; ks < k_stages; ks++, g++) {
                 const uint32_t s1 = s + 1 == S::STAGES ? 0 : s + 1, npar = s1 ? par : par ^ 1;
@@ -449,30 +454,46 @@ k_gemm_mma(const __grid_constant__ MmaJob job, const __grid_constant__ f32x2 min
                 par = npar;
             }
             if (!ok) break;
-            f32x2 sum[NT][2];
+            f32x2 sum[NT][2];  // of this warp's lane groups
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
-                for (int h = 0; h < 2; h++) sum[n][h] = add2(add2(acc[n][h][0], acc[n][h][1]), add2(acc[n][h][2], acc[n][h][3]));
-            float* ex = &sm->odd[rt][0][lane][0];
-            if (parity) {
-                ok = mbar_wait(smem_u32(&sm->odd_empty[rt]), (tile_no & 1) ^ 1, &sm->abort, err, 3);
+                for (int h = 0; h < 2; h++) {
+                    sum[n][h] = acc[n][h][0];
+                    if constexpr (LG >= 2) sum[n][h] = add2(sum[n][h], acc[n][h][1]);
+                    if constexpr (LG == 4) sum[n][h] = add2(sum[n][h], add2(acc[n][h][2], acc[n][h][3]));
+                }
+            if (role) {
+                ok = mbar_wait(smem_u32(&sm->part_empty[rt]), (tile_no & 1) ^ 1, &sm->abort, err, 3);
                 if (!ok) break;
+                float* ex = &sm->part[rt][role - 1][0][lane][0];
 #pragma unroll
                 for (int n = 0; n < NT; n++) *reinterpret_cast<ulonglong2*>(ex + n * 128) = make_ulonglong2(sum[n][0], sum[n][1]);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm->odd_full[rt]));
+                if (lane == 0) mbar_arrive(smem_u32(&sm->part_full[rt]));
             } else {
-                ok = mbar_wait(smem_u32(&sm->odd_full[rt]), tile_no & 1, &sm->abort, err, 4);
+                ok = mbar_wait(smem_u32(&sm->part_full[rt]), tile_no & 1, &sm->abort, err, 4);
                 if (!ok) break;
+                auto other = [&](int n, int r) { return *reinterpret_cast<const ulonglong2*>(&sm->part[rt][r - 1][n][lane][0]); };
 #pragma unroll
-                for (int n = 0; n < NT; n++) {
-                    const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(ex + n * 128);
-                    sum[n][0] = add2(sum[n][0], o.x);
-                    sum[n][1] = add2(sum[n][1], o.y);
+                for (int n = 0; n < NT; n++) {  // ((a0 + a1) + (a2 + a3)) of a parity from its parts, then even + odd
+                    ulonglong2 v[2];
+#pragma unroll
+                    for (int par2 = 0; par2 < 2; par2++) {
+                        ulonglong2 q[LS];
+#pragma unroll
+                        for (int i = 0; i < LS; i++) q[i] = i == 0 && par2 == 0 ? make_ulonglong2(sum[n][0], sum[n][1]) : other(n, 2 * i + par2);
+#pragma unroll
+                        for (int w = LS; w > 1; w /= 2)
+#pragma unroll
+                            for (int i = 0; i < w / 2; i++) q[i] = make_ulonglong2(add2(q[2 * i].x, q[2 * i + 1].x), add2(q[2 * i].y, q[2 * i + 1].y));
+                        v[par2] = q[0];
+                    }
+                    sum[n][0] = add2(v[0].x, v[1].x);
+                    sum[n][1] = add2(v[0].y, v[1].y);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm->odd_empty[rt]));
+                if (lane == 0) mbar_arrive(smem_u32(&sm->part_empty[rt]));
                 const MmaTile tl = mma_decode_tile<R, S::TOKENS>(job, t, tiles_n);
                 const int m = job.m[tl.mat], row = (tl.row_tile0 + rt) * MMA_ROWS + gid;
                 float* out = job.out[tl.mat];
@@ -545,21 +566,20 @@ cudaError_t device_sm_count(int* sms) {
     return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
-template <int R, int NT, bool Q8, bool READY>
+template <int R, int NT, bool Q8, bool READY, int LS>
 cudaError_t launch_kernel(cudaStream_t st, const MmaJob& job, int sms, uint32_t* err) {
-    using S = MmaShape<R, NT, READY>;
-    const size_t smem = sizeof(MmaSmem<R, NT, READY>);
+    using S = MmaShape<R, NT, READY, LS>;
+    const size_t smem = sizeof(MmaSmem<R, NT, READY, LS>);
     static RaisedPerDevice limit;
-    const cudaError_t e = raise_dynamic_smem(limit, (const void*)k_gemm_mma<R, NT, Q8, READY>, smem);
+    const cudaError_t e = raise_dynamic_smem(limit, (const void*)k_gemm_mma<R, NT, Q8, READY, LS>, smem);
     if (e != cudaSuccess) return e;
     g_kernel_launches++;
     const f32x2 minus_zero = 0x8000000080000000ull;
-    return launch_pdl(st, k_gemm_mma<R, NT, Q8, READY>, dim3(std::min(job.tile_start[3], sms * S::CTAS)), dim3(S::THREADS), smem, job, minus_zero, err);
+    return launch_pdl(st, k_gemm_mma<R, NT, Q8, READY, LS>, dim3(std::min(job.tile_start[3], sms * S::CTAS)), dim3(S::THREADS), smem, job, minus_zero, err);
 }
-template <int R, int NT>
+template <int R, int NT, bool READY, int LS = 1>
 cudaError_t launch_shape(cudaStream_t st, const MmaJob& job, bool q8, int sms, uint32_t* err) {
-    if (job.x) return q8 ? launch_kernel<R, NT, true, true>(st, job, sms, err) : launch_kernel<R, NT, false, true>(st, job, sms, err);
-    return q8 ? launch_kernel<R, NT, true, false>(st, job, sms, err) : launch_kernel<R, NT, false, false>(st, job, sms, err);
+    return q8 ? launch_kernel<R, NT, true, READY, LS>(st, job, sms, err) : launch_kernel<R, NT, false, READY, LS>(st, job, sms, err);
 }
 
 }  // namespace
@@ -606,20 +626,28 @@ cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* c
         return t;
     };
     // The shape that needs least time: rounds of tiles times what a stage of one takes, in 1/100 us, measured with one CTA of it on an
-    // SM and with all that fit.  Wide tiles do more per stage (1.76 us for 96 x 32 outputs, 0.32 for 16 x 8), narrow ones end sooner where
-    // there are few: 2048 x 6912 at 64 tokens 47.8 us as 96 x 32, 34.2 as 64 x 32, 20.7 as 64 x 16 and 28.8 as 16 x 16; 6144 x 2048
-    // there 17.3, 22.5, 19.7, 26.9; at 6 tokens 5.9 as 64 x 8 and 8.1 as 16 x 8, but 2048 x 6912 12.8 and 11.0.
-    static constexpr struct {
+    // SM and with all that fit.  Wide tiles do a little more per stage (96 x 32 outputs in 1.56 us, 64 x 16 in 0.54, 16 x 8 in 0.28),
+    // narrow ones end sooner where there are few: 2048 x 6912 at 64 tokens 45.1 us as 96 x 32 and 17.6 as 64 x 16, at 96 tokens
+    // 32.3 as 64 x 16 (two rounds, the second with a third of the SMs) and 24.7 as 64 x 24, at 6 tokens 12.4 as 64 x 8 and 9.5 as
+    // 16 x 8, where two warps share a row tile's lane groups (11.3 with one).
+    struct Shape {
         int r, nt, ctas, one, all;
-    } SHAPES[] = {{6, 4, 1, 176, 176}, {4, 4, 1, 120, 120}, {4, 2, 1, 67, 67}, {4, 1, 1, 41, 41}, {2, 1, 2, 42, 46}, {1, 2, 2, 46, 51}, {1, 1, 2, 32, 40}};
+    };
+    static constexpr int N_SHAPES = 7;
+    static constexpr Shape READY_SHAPES[N_SHAPES] = {{6, 4, 1, 156, 156}, {6, 2, 1, 78, 78}, {4, 3, 1, 80, 80}, {4, 2, 1, 53, 54},
+                                                     {4, 1, 1, 38, 42},   {2, 1, 2, 36, 38}, {1, 1, 2, 27, 28}};
+    // (with the converting warps: two lane-group warps bring nothing, 1024 x 4608 at 9 tokens 8.4 against 8.1 us)
+    static constexpr Shape CONVERT_SHAPES[N_SHAPES] = {{6, 4, 1, 176, 176}, {4, 4, 1, 120, 120}, {4, 2, 1, 67, 67}, {4, 1, 1, 41, 41},
+                                                       {2, 1, 2, 42, 46},   {1, 2, 2, 46, 51},   {1, 1, 2, 32, 40}};
+    const Shape* shapes = x ? READY_SHAPES : CONVERT_SHAPES;
     int best = 0, best_cost = INT_MAX;
-    for (int i = 0; i < (int)(sizeof(SHAPES) / sizeof(SHAPES[0])); i++) {
-        const auto& s = SHAPES[i];
+    for (int i = 0; i < N_SHAPES; i++) {
+        const Shape& s = shapes[i];
         const int t = tiles(s.r * MMA_ROWS, s.nt * 8), slots = sms * s.ctas, rest = t % slots;
         const int cost = t / slots * s.all + (rest == 0 ? 0 : rest <= sms ? s.one : s.all);
         if (cost < best_cost) best = i, best_cost = cost;
     }
-    const int rows = SHAPES[best].r * MMA_ROWS, tokens = SHAPES[best].nt * 8;
+    const int rows = shapes[best].r * MMA_ROWS, tokens = shapes[best].nt * 8;
     int t = 0;
     for (int i = 0; i < 3; i++) {
         job.tile_start[i] = t;
@@ -631,14 +659,23 @@ cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* c
     }
     job.tile_start[3] = t;
     const bool q8 = w[0]->dtype == DT_Q8_0;
+    if (x) switch (best) {
+            case 0: return launch_shape<6, 4, true>(st, job, q8, sms, err);
+            case 1: return launch_shape<6, 2, true>(st, job, q8, sms, err);
+            case 2: return launch_shape<4, 3, true>(st, job, q8, sms, err);
+            case 3: return launch_shape<4, 2, true>(st, job, q8, sms, err);
+            case 4: return launch_shape<4, 1, true>(st, job, q8, sms, err);
+            case 5: return launch_shape<2, 1, true>(st, job, q8, sms, err);
+            default: return launch_shape<1, 1, true, 2>(st, job, q8, sms, err);
+        }
     switch (best) {
-        case 0: return launch_shape<6, 4>(st, job, q8, sms, err);
-        case 1: return launch_shape<4, 4>(st, job, q8, sms, err);
-        case 2: return launch_shape<4, 2>(st, job, q8, sms, err);
-        case 3: return launch_shape<4, 1>(st, job, q8, sms, err);
-        case 4: return launch_shape<2, 1>(st, job, q8, sms, err);
-        case 5: return launch_shape<1, 2>(st, job, q8, sms, err);
-        default: return launch_shape<1, 1>(st, job, q8, sms, err);
+        case 0: return launch_shape<6, 4, false>(st, job, q8, sms, err);
+        case 1: return launch_shape<4, 4, false>(st, job, q8, sms, err);
+        case 2: return launch_shape<4, 2, false>(st, job, q8, sms, err);
+        case 3: return launch_shape<4, 1, false>(st, job, q8, sms, err);
+        case 4: return launch_shape<2, 1, false>(st, job, q8, sms, err);
+        case 5: return launch_shape<1, 2, false>(st, job, q8, sms, err);
+        default: return launch_shape<1, 1, false>(st, job, q8, sms, err);
     }
 }
 
