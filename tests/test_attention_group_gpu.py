@@ -1,0 +1,43 @@
+"""Attention of a KV head's query heads together, with the quantised result handed to the exact GEMM in its operand order: against
+the oracle at the edges of the 64-key tiles, for every split of 1 to 8 heads over the threads, and with rows whose last pipeline
+stage is half empty (12 and 20 blocks)."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float32).view(np.uint32)
+
+
+@pytest.mark.parametrize("qtype", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("hidden,heads,n_kv,ffn", [(256, 4, 4, 512), (384, 6, 2, 640), (384, 6, 1, 640), (512, 8, 1, 1152)])
+def test_prompts_and_batched_steps_at_tile_edges(cuda_lib, orc, model_dir, monkeypatch, qtype, hidden, heads, n_kv, ffn):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import gguf_synth as gs
+    from wick_b200.model import CudaLfm2Model
+    name = f"group-{hidden}-{heads}-{n_kv}"
+    monkeypatch.setitem(gs.SPECS, name, dataclasses.replace(gs.SPECS["tiny"], name=name, hidden=hidden, n_heads=heads, n_kv_heads=n_kv, ffn=ffn))
+    path = gs.cached_model(name, qtype, 0, cache_dir=model_dir, norm_jitter=0.2, weight_std=0.05)
+    m = CudaLfm2Model(path, 512)
+    ids, nxt, oracles = [], [], []
+    for n in (200, 1, 2, 63, 64, 65, 127, 129):  # (the first one makes the copies of the weights)
+        o = orc.OracleModel(path, 512)
+        toks = gs.random_prompt(n, m.config().vocab_size, seed=n)
+        sid = m.seq_create()
+        want = o.forward_prefill(toks, 0)
+        assert np.array_equal(bits(m.seq_prefill(sid, toks, 0)), bits(want)), n
+        ids.append(sid)
+        nxt.append(orc.argmax(want))
+        oracles.append(o)
+    for rows in (len(ids), 3):
+        got = m.decode_batch_logits(nxt[:rows], ids[:rows])
+        for i in range(rows):
+            want = oracles[i].forward(int(nxt[i]))
+            assert np.array_equal(bits(got[i]), bits(want)), (rows, i)
+            nxt[i] = orc.argmax(want)

@@ -183,6 +183,12 @@ void launch_qknorm_rope_kv_rows(cudaStream_t st, float* q, const float* k, const
                                 const uint32_t* positions, int n, int n_heads, int n_kv_heads, int head_dim);
 cudaError_t launch_attention_rows(cudaStream_t st, const float* q, float* const* k_caches, float* const* v_caches, const uint32_t* positions,
                                   float* out, int n, int n_heads, int n_kv_heads, int head_dim, int max_seq);
+// The same attention for the query heads of a KV head together, its result quantised (into x where x.p is not null): n rows with caches of
+// their own (positions[j] = cached rows before row j's) or, k_single not null, n consecutive tokens of one sequence from start_pos.
+// max_seq: keys of the longest row.  *done is false, and nothing launched, for shapes it does not take.
+cudaError_t launch_attention_group(cudaStream_t st, const float* q, float* const* k_caches, float* const* v_caches, const float* k_single,
+                                   const float* v_single, const uint32_t* positions, int start_pos, int n, int n_heads, int n_kv_heads, int head_dim,
+                                   int max_seq, float* q8s, int8_t* q8q, const MmaInput& x, bool* done);
 // Opt-in split-K form of the single-query attention (keys of every (row, head) in runs of 256 + a merge pass; rounding
 // differs from the exact kernel).  Caches per row (k_caches / v_caches) or one pair for all rows (k_single / v_single);
 // positions[j] = cached rows before row j's token.  scratch: attention_splitk_scratch_floats() floats.

@@ -227,9 +227,12 @@ void launch_expf(cudaStream_t st, const float* x, float* y, size_t count) {
 // d_conv tokens, so every (token, channel) is independent given the incoming state:
 //   y = 0 + S_0*w_0 + ... + S_{dc-1}*w_{dc-1} + bx_j*w_dc     (products and adds rounded one by one)
 //   out = c * y
-// A warp owns 32 consecutive channels of one token = one Q8_0 block of the out_proj input.
+// A warp owns 32 consecutive channels of one token = one Q8_0 block of the out_proj input.  The first token's warp also does the others
+// that read the incoming state, and then replaces it: slot k <- bx[n - dc + k], or the old slot k + n while that is still inside
+// the old buffer (n < d_conv), ascending k, so the in-place shift never reads a slot it already overwrote.  (A kernel of its
+// own for the state was one of ten launches per prompt piece of 2 to 3 us each.)
 __global__ void k_shortconv(const float* __restrict__ proj, const float* __restrict__ conv_w,
-                            const float* __restrict__ state, int n, int hs, int ks, float* __restrict__ out,
+                            float* __restrict__ state, int n, int hs, int ks, float* __restrict__ out,
                             float* __restrict__ q8s, int8_t* __restrict__ q8q, MmaInput mx) {
     pdl_enter(proj, conv_w, state, out, q8s, q8q, mx.p);
     const int dc = ks - 1;
@@ -237,55 +240,40 @@ __global__ void k_shortconv(const float* __restrict__ proj, const float* __restr
     int lane = threadIdx.x & 31;
     int bpr = hs / QK;
     if (gw >= (size_t)n * bpr) return;
-    int j = (int)(gw / bpr), ch = (int)(gw % bpr) * QK + lane;
-    const float* pj = proj + (size_t)j * 3 * hs;
-    float sum = 0.0f;
-    for (int k = 0; k < dc; k++) {
-        int src = j - dc + k;
-        float s;
-        if (src >= 0) {
-            const float* ps = proj + (size_t)src * 3 * hs;
-            s = __fmul_rn(ps[ch], ps[2 * hs + ch]);
-        } else {
-            s = state[(size_t)(k + j) * hs + ch];
+    const int j0 = (int)(gw / bpr), ch = (int)(gw % bpr) * QK + lane;
+    if (j0 > 0 && j0 < dc) return;
+    const int j1 = j0 > 0 ? j0 + 1 : max(1, min(dc, n));
+    auto bx = [&](int j) {
+        const float* p = proj + (size_t)j * 3 * hs;
+        return __fmul_rn(p[ch], p[2 * hs + ch]);
+    };
+    for (int j = j0; j < j1; j++) {
+        float sum = 0.0f;
+        for (int k = 0; k < dc; k++) {
+            const int src = j - dc + k;
+            const float s = src >= 0 ? bx(src) : state[(size_t)(k + j) * hs + ch];
+            sum = __fadd_rn(sum, __fmul_rn(s, conv_w[ch * ks + k]));
         }
-        sum = __fadd_rn(sum, __fmul_rn(s, conv_w[ch * ks + k]));
-    }
-    float bx = __fmul_rn(pj[ch], pj[2 * hs + ch]);
-    sum = __fadd_rn(sum, __fmul_rn(bx, conv_w[ch * ks + dc]));
-    float o = __fmul_rn(pj[hs + ch], sum);
-    if (out) out[(size_t)j * hs + ch] = o;
-    if (q8q) {
-        float sc;
-        int8_t q = quantize_lane(o, &sc);
-        if (mx.p) {
-            mma_x_store_lane(mx, j, ch / QK, lane, q, sc);
-        } else {
-            q8q[(size_t)j * hs + ch] = q;
-            if (lane == 0) q8s[gw] = sc;
+        sum = __fadd_rn(sum, __fmul_rn(bx(j), conv_w[ch * ks + dc]));
+        float o = __fmul_rn(proj[(size_t)j * 3 * hs + hs + ch], sum);
+        if (out) out[(size_t)j * hs + ch] = o;
+        if (q8q) {
+            float sc;
+            int8_t q = quantize_lane(o, &sc);
+            if (mx.p) {
+                mma_x_store_lane(mx, j, ch / QK, lane, q, sc);
+            } else {
+                q8q[(size_t)j * hs + ch] = q;
+                if (lane == 0) q8s[(size_t)j * bpr + ch / QK] = sc;
+            }
         }
     }
-}
-
-// State after n tokens: slot k <- bx[n - dc + k], or the old slot k + n while that is still
-// inside the old buffer (n < d_conv).  One thread per channel, ascending k, so the in-place
-// shift never reads a slot it already overwrote.
-__global__ void k_shortconv_state(const float* __restrict__ proj, float* __restrict__ state, int n, int hs, int ks) {
-    pdl_enter(proj, state);
-    const int dc = ks - 1;
-    int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ch >= hs) return;
-    for (int k = 0; k < dc; k++) {
-        int src = n - dc + k;
-        float s;
-        if (src >= 0) {
-            const float* ps = proj + (size_t)src * 3 * hs;
-            s = __fmul_rn(ps[ch], ps[2 * hs + ch]);
-        } else {
-            s = state[(size_t)(k + n) * hs + ch];
+    if (j0 == 0)
+        for (int k = 0; k < dc; k++) {
+            const int src = n - dc + k;
+            const float s = src >= 0 ? bx(src) : state[(size_t)(k + n) * hs + ch];
+            state[(size_t)k * hs + ch] = s;
         }
-        state[(size_t)k * hs + ch] = s;
-    }
 }
 
 void launch_shortconv(cudaStream_t st, const float* proj, const float* conv_w, float* state, int n, int hs, int ks,
@@ -294,7 +282,6 @@ void launch_shortconv(cudaStream_t st, const float* proj, const float* conv_w, f
     if (!warps) return;
     g_kernel_launches++;
     launch_pdl(st, k_shortconv, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, proj, conv_w, state, n, hs, ks, out, q8s, q8q, x);
-    if (ks > 1) g_kernel_launches++, launch_pdl(st, k_shortconv_state, dim3((hs + 255) / 256), dim3(256), 0, proj, state, n, hs, ks);
 }
 
 // ── per-head QK RMSNorm + RoPE + KV append ─────────────────────────────────

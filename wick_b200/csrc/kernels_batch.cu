@@ -201,6 +201,170 @@ cudaError_t launch_attention_rows(cudaStream_t st, const float* q, float* const*
     return cudaSuccess;
 }
 
+// ── exact attention of the query heads of one KV head (prompts below the tiled kernel's length, batched steps) ──
+// attn_scores / softmax_inplace / attn_values like k_attention_naive and k_attention_rows, for heads of 64: a CTA takes one token and
+// the HEADS <= 8 query heads of one KV head, so that a cached row is fetched once for all of them, and K and V rows come 64 at a
+// time in one stream of asynchronous copies, two tiles in flight: the first V tiles land under the softmax.  Scores: two
+// threads per key, each with every other head, the key row in registers.  Weighted V: two threads per dim, likewise.  The results
+// leave quantised, a warp has the 32 dims of a block.
+// Bound by latency (two passes over a few tiles) and, with many rows, by the cached rows' bytes.  64 rows of ~150 keys on the
+// 1.6B-class model: 32.3 us with a CTA per query head and 3.3 for the quantiser, now 14.5 for both (the rows are 6 us at the copy
+// rate).  Three tiles of ring instead of four: four CTAs to an SM, so that 512 are one wave.
+constexpr int GROUP_THREADS = 128, GROUP_TILE = 64, GROUP_HD = 64, GROUP_STAGES = 3, GROUP_MAX_HEADS = 8;
+constexpr int GROUP_ROW = GROUP_HD + 4;  // floats: eight lanes that read 16 bytes of eight keys hit different banks
+
+static size_t attention_group_smem(int heads, int seq) {
+    return (size_t)(GROUP_STAGES * GROUP_TILE * GROUP_ROW + heads * GROUP_HD + heads * ((seq + 3) & ~3)) * sizeof(float);
+}
+
+template <int PER>  // heads of a thread: PER >= heads / 2
+__global__ void __launch_bounds__(GROUP_THREADS) k_attention_group(const float* __restrict__ q, float* const* __restrict__ k_caches,
+                                                                   float* const* __restrict__ v_caches, const float* __restrict__ k_single,
+                                                                   const float* __restrict__ v_single, const uint32_t* __restrict__ positions,
+                                                                   int start_pos, int heads, int sc_stride, float* __restrict__ q8s,
+                                                                   int8_t* __restrict__ q8q, MmaInput mx) {
+    pdl_enter(q, k_caches, v_caches, k_single, v_single, positions, q8s, q8q, mx.p);
+    extern __shared__ __align__(16) float sm[];
+    float* ring = sm;
+    float* qs = ring + GROUP_STAGES * GROUP_TILE * GROUP_ROW;  // [heads][64]
+    float* sc = qs + heads * GROUP_HD;                         // [heads][sc_stride]
+    const int kvh = blockIdx.x, j = blockIdx.y, n_kv = gridDim.x;
+    const int kv_dim = n_kv * GROUP_HD, hs = kv_dim * heads;
+    const int seq = (positions ? (int)positions[j] : start_pos + j) + 1, tiles = (seq + GROUP_TILE - 1) / GROUP_TILE;
+    const float* kc = (k_single ? k_single : k_caches[j]) + kvh * GROUP_HD;
+    const float* vc = (v_single ? v_single : v_caches[j]) + kvh * GROUP_HD;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto stage = [&](int i) {  // tile i of the K rows' and then the V rows' tiles
+        if (i < 2 * tiles) {
+            const int t0 = (i < tiles ? i : i - tiles) * GROUP_TILE, rows = min(GROUP_TILE, seq - t0);
+            const float* src = (i < tiles ? kc : vc) + (size_t)t0 * kv_dim;
+            float* dst = ring + (i % GROUP_STAGES) * GROUP_TILE * GROUP_ROW;
+            for (int p = tid; p < rows * (GROUP_HD / 4); p += GROUP_THREADS) {
+                const int r = p / (GROUP_HD / 4), c = p % (GROUP_HD / 4) * 4;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * GROUP_ROW + c)),
+                             "l"(src + (size_t)r * kv_dim + c)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < GROUP_STAGES - 1; i++) stage(i);
+    for (int i = tid; i < heads * GROUP_HD; i += GROUP_THREADS) qs[i] = q[(size_t)j * hs + kvh * heads * GROUP_HD + i];
+    const float scale = __fdiv_rn(1.0f, sqrtf((float)GROUP_HD));
+    const int col = tid & 63, first = tid >> 6;  // key of a tile / dim; heads first, first + 2, ...
+    for (int i = 0; i < tiles; i++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GROUP_STAGES - 2) : "memory");
+        __syncthreads();  // tile i is there, tile i - 1 done with
+        stage(i + GROUP_STAGES - 1);
+        const int t = i * GROUP_TILE + col;
+        if (t < seq) {
+            const float4* row = reinterpret_cast<const float4*>(ring + (i % GROUP_STAGES) * GROUP_TILE * GROUP_ROW + col * GROUP_ROW);
+            float4 kv[GROUP_HD / 4];
+#pragma unroll
+            for (int d = 0; d < GROUP_HD / 4; d++) kv[d] = row[d];
+#pragma unroll
+            for (int p = 0; p < PER; p++) {
+                const int h = first + 2 * p;
+                if (h >= heads) break;
+                const float4* qh = reinterpret_cast<const float4*>(qs + h * GROUP_HD);
+                float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // chains of qk_dot: dims c, c + 8, ...
+#pragma unroll
+                for (int d = 0; d < GROUP_HD / 4; d++) {
+                    const float4 qv = qh[d];
+                    float* a = s + (d & 1) * 4;
+                    a[0] = __fmaf_rn(qv.x, kv[d].x, a[0]);
+                    a[1] = __fmaf_rn(qv.y, kv[d].y, a[1]);
+                    a[2] = __fmaf_rn(qv.z, kv[d].z, a[2]);
+                    a[3] = __fmaf_rn(qv.w, kv[d].w, a[3]);
+                }
+                const float v0 = __fadd_rn(s[0], s[4]), v1 = __fadd_rn(s[1], s[5]), v2 = __fadd_rn(s[2], s[6]), v3 = __fadd_rn(s[3], s[7]);
+                sc[h * sc_stride + t] = __fmul_rn(__fadd_rn(__fadd_rn(v0, v1), __fadd_rn(v2, v3)), scale);
+            }
+        }
+    }
+    __syncthreads();
+    for (int h = warp; h < heads; h += GROUP_THREADS / 32) {
+        float* s = sc + h * sc_stride;
+        float mxv = __int_as_float(0xFF800000);
+        for (int t = lane; t < seq; t += 32) mxv = fmaxf(mxv, s[t]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mxv = fmaxf(mxv, __shfl_xor_sync(0xffffffffu, mxv, o));
+        double sum = 0.0;
+        for (int t = lane; t < seq; t += 32) {
+            const float e = ggml_expf(__fsub_rn(s[t], mxv));
+            s[t] = e;
+            sum += (double)e;
+        }
+        const float inv = (float)(1.0 / warp_sum_f64(sum));
+        for (int t = lane; t < seq; t += 32) s[t] = __fmul_rn(s[t], inv);
+    }
+    float acc[PER];
+#pragma unroll
+    for (int p = 0; p < PER; p++) acc[p] = 0.0f;
+    for (int i = tiles; i < 2 * tiles; i++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GROUP_STAGES - 2) : "memory");
+        __syncthreads();  // (the first time: the softmax is complete, too)
+        stage(i + GROUP_STAGES - 1);
+        const int t0 = (i - tiles) * GROUP_TILE, rows = min(GROUP_TILE, seq - t0);
+        const float* v = ring + (i % GROUP_STAGES) * GROUP_TILE * GROUP_ROW + col;
+        const float* s = sc + t0;
+        int r = 0;
+        for (; r + 8 <= rows; r += 8) {
+            float vv[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) vv[u] = v[(r + u) * GROUP_ROW];
+#pragma unroll
+            for (int p = 0; p < PER; p++) {
+                const int h = first + 2 * p;
+                if (h >= heads) break;
+                const float4 a = *reinterpret_cast<const float4*>(s + h * sc_stride + r), b = *reinterpret_cast<const float4*>(s + h * sc_stride + r + 4);
+                const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int u = 0; u < 8; u++) acc[p] = __fmaf_rn(w[u], vv[u], acc[p]);
+            }
+        }
+        for (; r < rows; r++)
+#pragma unroll
+            for (int p = 0; p < PER; p++)
+                if (first + 2 * p < heads) acc[p] = __fmaf_rn(s[(first + 2 * p) * sc_stride + r], v[r * GROUP_ROW], acc[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < PER; p++) {
+        const int h = first + 2 * p;  // (the same for all lanes of a warp)
+        if (h >= heads) break;
+        float scale8;
+        const int8_t q8 = quantize_lane(acc[p], &scale8);
+        const int e = (kvh * heads + h) * GROUP_HD + col, b = e / QK;
+        if (mx.p) {
+            mma_x_store_lane(mx, j, b, lane, q8, scale8);
+        } else {
+            q8q[(size_t)j * hs + e] = q8;
+            if (lane == 0) q8s[(size_t)j * (hs / QK) + b] = scale8;
+        }
+    }
+}
+
+cudaError_t launch_attention_group(cudaStream_t st, const float* q, float* const* k_caches, float* const* v_caches, const float* k_single,
+                                   const float* v_single, const uint32_t* positions, int start_pos, int n, int n_heads, int n_kv_heads, int head_dim,
+                                   int max_seq, float* q8s, int8_t* q8q, const MmaInput& x, bool* done) {
+    const int heads = n_heads / n_kv_heads;
+    const size_t smem = attention_group_smem(heads, max_seq);
+    *done = head_dim == GROUP_HD && heads <= GROUP_MAX_HEADS && smem <= 220 * 1024;
+    if (!*done || n <= 0) return cudaSuccess;
+    auto launch = [&](auto kernel, RaisedPerDevice& limit) {
+        const cudaError_t e = raise_dynamic_smem(limit, (const void*)kernel, smem);
+        if (e != cudaSuccess) return e;
+        g_kernel_launches++;
+        return launch_pdl(st, kernel, dim3(n_kv_heads, n), dim3(GROUP_THREADS), smem, q, k_caches, v_caches, k_single, v_single, positions, start_pos, heads,
+                          (max_seq + 3) & ~3, q8s, q8q, x);
+    };
+    static RaisedPerDevice limit1, limit2, limit4;
+    if (heads <= 2) return launch(k_attention_group<1>, limit1);
+    if (heads <= 4) return launch(k_attention_group<2>, limit2);
+    return launch(k_attention_group<4>, limit4);
+}
+
 // ── split-K single-query attention (opt-in) ────────────────────────────────
 // The exact kernel above keeps the reference's one serial chain per output dim over ALL keys, which at thousands of
 // cached keys is the whole cost of a decode step.  This pair splits the keys of every (row, head) into runs of

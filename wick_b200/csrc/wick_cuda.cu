@@ -783,13 +783,17 @@ void enqueue_prefill_chunk(wick_cuda_model* m, int n, int start_pos, bool flash,
             launch_qknorm_rope_kv(st, m->qbuf, m->kbuf, m->vbuf, L.q_norm, L.k_norm, eps, m->rope_cos, m->rope_sin, L.k_cache,
                                   L.v_cache, n, start_pos, nullptr, m->cfg.n_heads, L.n_kv, hd);
             prof_mark(m, PC_QK_ROPE_KV);
+            bool quantised = false;
+            if (!flash)
+                (void)launch_attention_group(st, m->qbuf, nullptr, nullptr, L.k_cache, L.v_cache, nullptr, start_pos, n, m->cfg.n_heads, L.n_kv, hd,
+                                             start_pos + n, m->q8s, m->q8q, xh, &quantised);
             if (flash)  // (shapes the tiled kernel does not take were refused when the model was created)
                 launch_attention_flash(st, m->qbuf, L.k_cache, L.v_cache, m->attn_out, n, start_pos, m->cfg.n_heads, L.n_kv, hd, m->tc_err);
-            else
+            else if (!quantised)
                 launch_attention_naive(st, m->qbuf, L.k_cache, L.v_cache, m->attn_out, n, start_pos, nullptr, m->cfg.n_heads,
                                        L.n_kv, hd, m->cfg.max_seq_len);
             prof_mark(m, PC_ATTENTION);
-            launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q, xh);
+            if (!quantised) launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q, xh);
             prof_mark(m, PC_ACT_QUANT);
             gemms(xh, {{&L.o, &L.tc_o, m->block_out}});
             prof_mark(m, PC_GEMM);
@@ -1208,12 +1212,16 @@ int32_t enqueue_decode_rows(wick_cuda_model* m, int n, int seq_bound) {
             gemms(xh, {{&L.q, &L.tc_q, m->qbuf}, {&L.k, &L.tc_k, m->kbuf}, {&L.v, &L.tc_v, m->vbuf}});
             launch_qknorm_rope_kv_rows(st, m->qbuf, m->kbuf, m->vbuf, L.q_norm, L.k_norm, eps, m->rope_cos, m->rope_sin, p0, p1, m->rows_pos, n,
                                        m->cfg.n_heads, L.n_kv, hd);
+            bool quantised = false;
+            if (!m->attn_splitk)
+                CU_TRY(launch_attention_group(st, m->qbuf, p0, p1, nullptr, nullptr, m->rows_pos, 0, n, m->cfg.n_heads, L.n_kv, hd, seq_bound, m->q8s, m->q8q,
+                                              xh, &quantised));
             if (m->attn_splitk)
                 launch_attention_splitk(st, m->qbuf, p0, p1, nullptr, nullptr, m->rows_pos, m->attn_out, m->splitk_scratch, n, m->cfg.n_heads, L.n_kv,
                                         hd, m->cfg.max_seq_len);
-            else
+            else if (!quantised)
                 CU_TRY(launch_attention_rows(st, m->qbuf, p0, p1, m->rows_pos, m->attn_out, n, m->cfg.n_heads, L.n_kv, hd, seq_bound));
-            launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q, xh);
+            if (!quantised) launch_quant_rows(st, m->attn_out, n, hs, m->q8s, m->q8q, xh);
             gemms(xh, {{&L.o, &L.tc_o, m->block_out}});
         }
         launch_add_rmsnorm_quant(st, m->hidden, m->block_out, L.ffn_norm, eps, n, hs, m->q8s, m->q8q, nullptr, xh);
