@@ -464,7 +464,7 @@ def main():
             extra["serving"] = serving_side_line(m, spec, args, gs, peak)
         except Exception as e:                              # e.g. not enough device memory for the sequence slots
             extra["serving"] = f"unavailable: {e}"
-        extra["prefill_paths"] = {"exact": "default: bit-exact GEMM on tcgen05 (lane partials in tensor memory, eight unfused chains) + exact-order attention",
+        extra["prefill_paths"] = {"exact": "default: bit-exact GEMM on mma.sync (lane groups as its K, eight unfused chains in the same registers) + exact-order attention",
                                   "tensor": "tcgen05 int8 GEMM (exact block sums, one fused f32 chain) + exact-order attention",
                                   "exact-cuda-cores": "bit-exact CUDA-core integer GEMM + exact-order attention"}
         line["extra"] = extra

@@ -11,14 +11,15 @@
 //
 // Bound: the registers' read ports, which the two pipes share.  An mma with a zero C takes 4.5 cycles of a scheduler, a packed
 // operation 2 to 2.4, and they add up: 54 cycles per (16 x 8, block) with every operand in shared memory, a ceiling of 170
-// TFLOP/s; the whole kernel reaches 127 (6144 x 2048 at 512 tokens 101 us, 6912 x 2048 at 2002 416), the rest being the waits
-// around each stage and the producers' share of the issue slots (5 %).
+// TFLOP/s; the whole kernel reaches 134 (6144 x 2048 at 512 tokens 96 us) with activations that arrive as operands and 127
+// (101 us, 6912 x 2048 at 2002 416) where it converts them: there four warps have 5 % of the issue slots, and in small
+// tiles a chain of their own.
 // tcgen05 was here before (int8, lane groups as zero-padded columns, sums handed over through tensor memory): 115 and 463 us
-// for those, 17 us for 1024 x 4608 at 9 tokens (now 9) and 23 for 2048 x 6912 at 16 (12): a hand-over per stage bound it, a round of
+// for those, 17 us for 1024 x 4608 at 9 tokens (now 7) and 23 for 2048 x 6912 at 16 (9.8): a hand-over per stage bound it, a round of
 // release, issue, MMAs and wait that small tiles cannot hide at all, and that no order of loads or number of units shortened
 // (next block loaded across stages 110, four smaller units 134).
-// Taken back here: the next operands loaded under the chains in the large tiles too (106 against 101 us; no registers for it), stages
-// of 128 elements (147), one warp fewer to the schedulers (R = 4: 109; it is the better one where R = 6 leaves a wave mostly empty).
+// Taken back here: stages of 128 elements (147 against 101 us); more warps to the schedulers (R = 7: 104, R = 8: 142 against
+// 96, for want of registers) and wider tiles with fewer (64 x 48: 114, 64 x 64: 161).
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <climits>
