@@ -41,3 +41,20 @@ def test_prompts_and_batched_steps_at_tile_edges(cuda_lib, orc, model_dir, monke
             want = oracles[i].forward(int(nxt[i]))
             assert np.array_equal(bits(got[i]), bits(want)), (rows, i)
             nxt[i] = orc.argmax(want)
+
+
+def test_rows_wider_than_a_thread_per_four_elements(cuda_lib, orc, model_dir, monkeypatch):
+    """Hidden rows above 4096 elements: the add + RMSNorm + quantise kernel has more than four of them per thread."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import gguf_synth as gs
+    from wick_b200.model import CudaLfm2Model
+    spec = dataclasses.replace(gs.SPECS["tiny"], name="wide-rows", hidden=4352, n_layers=2, attn_layers=(1,), n_heads=68, n_kv_heads=17, ffn=256, vocab=256)
+    monkeypatch.setitem(gs.SPECS, spec.name, spec)
+    path = gs.cached_model(spec.name, "q4_0", 0, cache_dir=model_dir, norm_jitter=0.2)
+    m, o = CudaLfm2Model(path, 64), orc.OracleModel(path, 64)
+    sid = m.seq_create()
+    toks = gs.random_prompt(17, spec.vocab, seed=3)
+    want = o.forward_prefill(toks, 0)
+    assert np.array_equal(bits(m.seq_prefill(sid, toks, 0)), bits(want))
+    assert np.array_equal(bits(m.decode_batch_logits([orc.argmax(want)], [sid])[0]), bits(o.forward(orc.argmax(want))))

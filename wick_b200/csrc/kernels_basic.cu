@@ -141,8 +141,10 @@ __global__ void __launch_bounds__(1024) k_add_rmsnorm_quant(float* __restrict__ 
 void launch_add_rmsnorm_quant(cudaStream_t st, float* hidden, const float* add, const float* weight, float eps, int n,
                               int dim, float* q8s, int8_t* q8q, float* normed_out, const MmaInput& x) {
     g_kernel_launches++;
-    const int quads = dim / 4, threads = std::min(1024, (quads + 31) / 32 * 32), per = (quads + threads - 1) / threads;
-    auto kernel = per == 1 ? k_add_rmsnorm_quant<1> : per == 2 ? k_add_rmsnorm_quant<2> : k_add_rmsnorm_quant<4>;  // (rows of up to 16384)
+    // (rows beyond 16384 elements: more threads than a CTA can have, which the launch refuses)
+    const int quads = dim / 4, least = (quads + 1023) / 1024, per = least <= 2 ? std::max(least, 1) : 4;
+    const int threads = ((quads + per - 1) / per + 31) / 32 * 32;
+    auto kernel = per == 1 ? k_add_rmsnorm_quant<1> : per == 2 ? k_add_rmsnorm_quant<2> : k_add_rmsnorm_quant<4>;
     launch_pdl(st, kernel, dim3(n), dim3(threads), 0, hidden, add, weight, eps, dim, q8s, q8q, normed_out, x);
 }
 
