@@ -257,7 +257,7 @@ def serving_side_line(m, spec, args, gs, hbm_peak):
         "prefill_tok_s_wall": SERVE_SEQUENCES * SERVE_PROMPT / prefill_s,
         "roofline": {"bound": "hbm", "achieved": bpt / (dev / steps) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                      "frac": bpt / (dev / steps) / 1e9 / hbm_peak,
-                     "note": "weight bytes once per batched step; at 64 rows the step is bound by the exact GEMM's epilogue, not by HBM"},
+                     "note": "weight bytes once per batched step; at 64 rows the step is bound by the exact GEMM, not by HBM"},
     }
 
 

@@ -13,7 +13,7 @@ extern thread_local unsigned long long g_kernel_launches;
 // Programmatic dependent launch.  Kernels launched with launch_pdl may start while their predecessor in the stream is still
 // running; pdl_enter() lets the successor do the same and then waits until the predecessor has finished and its writes are
 // visible, so it stands before the first access to memory that any other kernel writes or reads.  A prompt or a batched
-// step is a chain of ~150 kernels of 2 to 20 us: the launch and the ramp of one now lie under the tail of the one before.
+// step is a chain of ~135 kernels of 2 to 35 us: the launch and the ramp of one now lie under the tail of the one before.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // `p`: the kernel's pointers.  A load through a const __restrict__ parameter may be moved anywhere by the compiler, above the
