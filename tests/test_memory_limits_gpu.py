@@ -88,3 +88,44 @@ def test_few_rows_without_memory_for_the_copies(ops, orc, model_dir):
         cm.forward_prefill([tok], 0, s)
         alone.append(cm.forward([tok + 2], 1, s))
     assert np.array_equal(first.view(np.uint32), np.stack(alone).view(np.uint32))
+
+
+def test_both_gemms_of_a_model_share_the_memory_of_its_copies(ops, model_dir):
+    """Switching the mode of a live model needs no memory, whichever came first, and the new mode's GEMM runs at once."""
+    import wick_b200.model as wick
+    from wick_b200 import gguf_synth as gs
+    path = gs.cached_model("lfm2-350m", "q4_0", 0, cache_dir=model_dir)
+    toks = gs.random_prompt(40, gs.SPECS["lfm2-350m"].vocab)
+
+    def step(m, ids):
+        """Kernels of a step of two rows, and its logits."""
+        before = m.kernel_launches()
+        return m.decode_batch_logits([3, 4], ids), m.kernel_launches() - before
+
+    def fresh(mode):
+        m = wick.CudaLfm2Model(path, 256)
+        m.set_prefill_mode(mode)
+        logits = m.forward_prefill(toks, 0, wick.InferenceState())
+        ids = [m.seq_create() for _ in range(2)]
+        return m, logits, ids, step(m, ids)[0]
+    exact, exact_logits, exact_ids, exact_first = fresh("exact")
+    kernels = step(exact, exact_ids)[1]
+    tensor, tensor_logits, tensor_ids, tensor_first = fresh("tensor")
+    assert exact_ids == tensor_ids
+    assert np.array_equal(tensor_first.view(np.uint32), exact_first.view(np.uint32))  # (two rows are exact in either mode)
+    size = exact.gpu_memory_bytes()
+    assert tensor.gpu_memory_bytes() == size
+    tensor.set_prefill_mode("exact")
+    step(tensor, tensor_ids)
+    assert step(tensor, tensor_ids)[1] == kernels         # two rows are enough to go over to the exact GEMM
+    with Filled(48 << 20):
+        for m in (exact, tensor):
+            for mode, want in (("tensor", tensor_logits), ("exact", exact_logits), ("tensor", tensor_logits)):
+                m.set_prefill_mode(mode)
+                assert np.array_equal(m.forward_prefill(toks, 0, wick.InferenceState()).view(np.uint32), want.view(np.uint32)), mode
+            m.set_prefill_mode("exact")
+            for i in exact_ids:
+                m.seq_destroy(i)
+                assert m.seq_create() == i
+            assert np.array_equal(step(m, exact_ids)[0].view(np.uint32), exact_first.view(np.uint32))
+            assert step(m, exact_ids)[1] == kernels and m.gpu_memory_bytes() == size

@@ -554,10 +554,12 @@ cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out) {
     out->m = w.m;
     out->k = w.k;
     out->m_pad = (w.m + TC_BM - 1) / TC_BM * TC_BM;
-    cudaError_t e = cudaMemsetAsync(out->q, 0, out->q_bytes(), st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(out->scales_t, 0, out->s_bytes(), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (out->m_pad > out->m) {  // (the rows behind the last one; the kernel writes all others)
+        e = cudaMemsetAsync(out->q + (size_t)out->m * out->k, 0, out->q_bytes() - (size_t)out->m * out->k, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(out->scales_t, 0, out->s_bytes(), st);
+        if (e != cudaSuccess) return e;
+    }
     const size_t n_blocks = (size_t)w.m * (w.k / QK);
     g_kernel_launches++;
     k_tc_unpack<<<(unsigned)((n_blocks + 255) / 256), 256, 0, st>>>(w, out->q, out->scales_t, out->m_pad);

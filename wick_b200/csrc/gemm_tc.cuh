@@ -32,8 +32,8 @@ struct TcJob {
 // True when the shapes meet the kernel's requirements (k a multiple of 128).
 bool tc_gemm_supported(int m, int k);
 
-// Fills `out` (q / scales_t must already point at q_bytes() / s_bytes() of device memory, zeroed by
-// this call) from the grouped layout of `w`, and encodes its tensor map.  Returns cudaSuccess or the
+// Fills `out` (q / scales_t must already point at q_bytes() / s_bytes() of device memory; the rows behind
+// the last one become zeros) from the grouped layout of `w`, and encodes its tensor map.  Returns cudaSuccess or the
 // failing CUDA error; a tensor-map failure is reported as cudaErrorInvalidValue.
 cudaError_t tc_weight_fill(cudaStream_t st, const DevWeight& w, TcWeight* out);
 

@@ -47,18 +47,21 @@ static int32_t fail(int32_t code, const std::string& msg) {
 
 namespace {
 
-// Copies of a matrix for the GEMMs of several rows; null until the first call that uses them.
-struct GemmCopies {
-    MmaWeight exact;  // the bit-exact GEMM's (gemm_mma.cu)
-    TcWeight fused;   // the fused-chain GEMM's (gemm_tc.cu)
+// The copy of a matrix for the GEMMs of several rows, in the order of the one that used it last: at most one of exact.p and fused.q is
+// set, and points at `mem`.  A model has one copy for both modes; a call in the other mode has it filled anew.
+struct GemmCopy {
+    uint8_t* mem = nullptr;  // room for either order, null until the first call that uses it
+    MmaWeight exact;         // the bit-exact GEMM's (gemm_mma.cu)
+    TcWeight fused;          // the fused-chain GEMM's (gemm_tc.cu)
 };
+enum class CopyOrder { NONE, EXACT, FUSED };
 
 struct Layer {
     bool is_attn = false;
     int n_kv = 0;
     float *attn_norm = nullptr, *ffn_norm = nullptr, *q_norm = nullptr, *k_norm = nullptr, *conv_w = nullptr;
     DevWeight in_proj, out_proj, q, k, v, o, gate, up, down;
-    GemmCopies tc_in_proj, tc_out_proj, tc_q, tc_k, tc_v, tc_o, tc_gate, tc_up, tc_down;
+    GemmCopy tc_in_proj, tc_out_proj, tc_q, tc_k, tc_v, tc_o, tc_gate, tc_up, tc_down;
     float *k_cache = nullptr, *v_cache = nullptr;  // [max_seq][kv_dim]
     float* conv_state = nullptr;                   // [d_conv][hidden]
 };
@@ -83,7 +86,7 @@ struct wick_cuda_model {
     int head_dim = 0;
     std::vector<Layer> layers;
     DevWeight embd;
-    GemmCopies tc_embd;     // of the vocabulary matrix, made for the multi-sequence step only
+    GemmCopy tc_embd;       // of the vocabulary matrix, made for the multi-sequence step only
     bool embd_q6k = false;  // token_embd is Q6_K: embd6 is used for the embedding rows and the logits, embd is empty
     DevQ6K embd6;
     float* output_norm = nullptr;
@@ -93,7 +96,7 @@ struct wick_cuda_model {
     // picks the bit-exact one (default), the fused-chain one, or the bit-exact CUDA-core kernel
     bool tc_ok = false;     // the model's shapes allow the tensor-core GEMM
     MmaInput x_hs, x_is;    // inputs of the exact GEMM in its operand order, max_chunk rows of hidden / feed-forward size
-    bool exact_built = false, fused_built = false;  // the layers' copies exist (made by the first call that needs them)
+    CopyOrder copies = CopyOrder::NONE;  // the order of the layers' copies (made by the first call that needs them)
     int prefill_mode = WICK_CUDA_PREFILL_EXACT;
     CUtensorMap map_x_hs, map_x_is;  // activations [max_chunk][hs | is] for the fused-chain GEMM
     float* normed_last = nullptr;  // output-normed hidden row of the last prefilled token
@@ -707,12 +710,14 @@ void prof_collect(wick_cuda_model* m) {  // after the stream has been synchronis
     m->prof_used = 0;
 }
 
-// The weight copies of the tensor-core GEMMs (1.125 bytes per parameter; the exact and the fused-chain GEMM have one each, made
-// when a mode first needs it) are made by the first chunk of more than
+// The weight copies of the tensor-core GEMMs (1.125 bytes per parameter, in the order of the exact or of the fused-chain GEMM) are
+// made by the first chunk of more than
 // TC_BUILD_ABOVE tokens, so that decoding and the shortest prompts leave a model at its packed size.  Once they are there
 // the bit-exact GEMM uses them from two tokens on: its 8-token tile costs the same for 2 tokens as for 8, and the CUDA-core
 // kernel needs several times as long at any of these counts (350M, 9-token prompt: 3.7 -> 0.70 ms).  The fused-chain GEMM
-// keeps its lower limit, because below it the other kernels' results are the ones a caller has always had.
+// keeps its lower limit, because below it the other kernels' results are the ones a caller has always had.  A call that uses
+// them in the other order (the mode was switched) fills the same memory again (0.9 ms for
+// the 1.6B-class model, 0.5 for the 350M-class one) instead of holding 1.125 more bytes per parameter for good.
 // From TC_REQUIRED_FROM rows on a call without memory for the copies is an error; below, the CUDA cores serve it.
 constexpr int TC_BUILD_ABOVE = 8, TC_FUSED_MIN_TOKENS = 16, TC_REQUIRED_FROM = 16;
 
@@ -720,17 +725,17 @@ constexpr int TC_BUILD_ABOVE = 8, TC_FUSED_MIN_TOKENS = 16, TC_REQUIRED_FROM = 1
 // launch on the tensor cores when the chunk is wide enough to fill an MMA tile, else the exact CUDA-core kernel.
 struct GemmTarget {
     const DevWeight* w;
-    const GemmCopies* t;
+    const GemmCopy* t;
     float* out;
 };
 // Where the inputs of n rows of k elements go if the exact GEMM multiplies them, else null.
 MmaInput mma_input(const wick_cuda_model* m, int n, int k) {
-    if (!m->exact_built || n < 2 || m->prefill_mode != WICK_CUDA_PREFILL_EXACT) return MmaInput();
+    if (m->copies != CopyOrder::EXACT || n < 2 || m->prefill_mode != WICK_CUDA_PREFILL_EXACT) return MmaInput();
     return k == (int)m->cfg.hidden_size ? m->x_hs : m->x_is;
 }
 void run_gemms(wick_cuda_model* m, int n, const MmaInput& x, std::initializer_list<GemmTarget> list) {
     cudaStream_t st = m->stream;
-    bool fused = m->fused_built && n >= TC_FUSED_MIN_TOKENS && m->prefill_mode == WICK_CUDA_PREFILL_TENSOR;
+    bool fused = m->copies == CopyOrder::FUSED && n >= TC_FUSED_MIN_TOKENS && m->prefill_mode == WICK_CUDA_PREFILL_TENSOR;
     const MmaWeight* ew[3] = {};
     const TcWeight* fw[3] = {};
     float* outs[3] = {};
@@ -832,71 +837,91 @@ int32_t build_tc(wick_cuda_model* m) {
     return WICK_CUDA_OK;
 }
 
-int32_t copy_for_exact(wick_cuda_model* m, const DevWeight& w, GemmCopies* t) {
-    t->exact.m = w.m;
-    t->exact.k = w.k;
+// Memory for a matrix's copy in either order.
+int32_t alloc_copy(wick_cuda_model* m, const DevWeight& w, GemmCopy* t) {
+    t->exact.m = t->fused.m = w.m;
+    t->exact.k = t->fused.k = w.k;
     t->exact.dtype = w.dtype;
-    W_TRY(dev_alloc(m, &t->exact.p, t->exact.bytes()));
-    CU_TRY(mma_weight_fill(m->stream, w, t->exact.p));
-    return WICK_CUDA_OK;
-}
-int32_t copy_for_fused(wick_cuda_model* m, const DevWeight& w, GemmCopies* t) {
     t->fused.m_pad = (w.m + 127) / 128 * 128;
-    t->fused.m = w.m;
-    t->fused.k = w.k;
-    W_TRY(dev_alloc(m, &t->fused.q, t->fused.q_bytes()));
-    W_TRY(dev_alloc(m, &t->fused.scales_t, t->fused.s_bytes() / sizeof(float)));
-    CU_TRY(tc_weight_fill(m->stream, w, &t->fused));
+    return dev_alloc(m, &t->mem, std::max(t->exact.bytes(), t->fused.q_bytes() + t->fused.s_bytes()));
+}
+// Fills it in the order of the exact or of the fused-chain GEMM, behind what the stream still does with its former content.
+int32_t fill_copy(wick_cuda_model* m, const DevWeight& w, GemmCopy* t, bool exact) {
+    t->exact.p = nullptr;
+    t->fused.q = nullptr;
+    if (exact) {
+        CU_TRY(mma_weight_fill(m->stream, w, t->mem));
+        t->exact.p = t->mem;
+        return WICK_CUDA_OK;
+    }
+    TcWeight f = t->fused;
+    f.q = reinterpret_cast<int8_t*>(t->mem);
+    f.scales_t = reinterpret_cast<float*>(t->mem + f.q_bytes());  // (q_bytes is a multiple of 128 * 128)
+    CU_TRY(tc_weight_fill(m->stream, w, &f));
+    t->fused = f;
     return WICK_CUDA_OK;
 }
 
-// The layers' copies for the exact or the fused-chain GEMM.
-int32_t make_copies(wick_cuda_model* m, bool exact) {
-    auto fill = [&](const DevWeight& w, GemmCopies* t) { return exact ? copy_for_exact(m, w, t) : copy_for_fused(m, w, t); };
+template <class F>  // f(matrix, its copy) for every matrix of the layers
+int32_t for_each_copy(wick_cuda_model* m, F&& f) {
     for (Layer& L : m->layers) {
         if (L.is_attn) {
-            W_TRY(fill(L.q, &L.tc_q));
-            W_TRY(fill(L.k, &L.tc_k));
-            W_TRY(fill(L.v, &L.tc_v));
-            W_TRY(fill(L.o, &L.tc_o));
+            W_TRY(f(L.q, &L.tc_q));
+            W_TRY(f(L.k, &L.tc_k));
+            W_TRY(f(L.v, &L.tc_v));
+            W_TRY(f(L.o, &L.tc_o));
         } else {
-            W_TRY(fill(L.in_proj, &L.tc_in_proj));
-            W_TRY(fill(L.out_proj, &L.tc_out_proj));
+            W_TRY(f(L.in_proj, &L.tc_in_proj));
+            W_TRY(f(L.out_proj, &L.tc_out_proj));
         }
-        W_TRY(fill(L.gate, &L.tc_gate));
-        W_TRY(fill(L.up, &L.tc_up));
-        W_TRY(fill(L.down, &L.tc_down));
+        W_TRY(f(L.gate, &L.tc_gate));
+        W_TRY(f(L.up, &L.tc_up));
+        W_TRY(f(L.down, &L.tc_down));
     }
-    if (exact) {
-        auto input = [&](int k, MmaInput* x) -> int32_t {
-            x->blocks = (k / QK + MMA_STAGE_BLOCKS - 1) / MMA_STAGE_BLOCKS * MMA_STAGE_BLOCKS;
-            const size_t bytes = (size_t)(m->max_chunk + MMA_X_ROWS - 1) / MMA_X_ROWS * x->blocks * MMA_X_CHUNK;
-            W_TRY(dev_alloc(m, &x->p, bytes));
-            CU_TRY(cudaMemsetAsync(x->p, 0, bytes, m->stream));  // (blocks behind the last one are read, never written)
-            return WICK_CUDA_OK;
-        };
-        W_TRY(input(m->cfg.hidden_size, &m->x_hs));
-        W_TRY(input(m->cfg.intermediate_size, &m->x_is));
-    } else {
-        CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.hidden_size, TC_TENSOR_TOKENS, &m->map_x_hs));
-        CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.intermediate_size, TC_TENSOR_TOKENS, &m->map_x_is));
-    }
-    CU_TRY(cudaStreamSynchronize(m->stream));
-    (exact ? m->exact_built : m->fused_built) = true;
     return WICK_CUDA_OK;
 }
 
-// The copies for a call of `rows` rows.
+// Memory for the layers' copies and for the exact GEMM's inputs (all of it whatever the mode: a switch must not need more).
+int32_t alloc_copies(wick_cuda_model* m) {
+    W_TRY(for_each_copy(m, [&](const DevWeight& w, GemmCopy* t) { return alloc_copy(m, w, t); }));
+    auto input = [&](int k, MmaInput* x) -> int32_t {
+        x->blocks = (k / QK + MMA_STAGE_BLOCKS - 1) / MMA_STAGE_BLOCKS * MMA_STAGE_BLOCKS;
+        const size_t bytes = (size_t)(m->max_chunk + MMA_X_ROWS - 1) / MMA_X_ROWS * x->blocks * MMA_X_CHUNK;
+        W_TRY(dev_alloc(m, &x->p, bytes));
+        CU_TRY(cudaMemsetAsync(x->p, 0, bytes, m->stream));  // (blocks behind the last one are read, never written)
+        return WICK_CUDA_OK;
+    };
+    W_TRY(input(m->cfg.hidden_size, &m->x_hs));
+    W_TRY(input(m->cfg.intermediate_size, &m->x_is));
+    CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.hidden_size, TC_TENSOR_TOKENS, &m->map_x_hs));
+    CU_TRY(tc_make_activation_map(m->q8q, m->max_chunk, m->cfg.intermediate_size, TC_TENSOR_TOKENS, &m->map_x_is));
+    return WICK_CUDA_OK;
+}
+
+// The layers' copies for a call of `rows` rows, in the order its mode takes.
 int32_t ensure_tc(wick_cuda_model* m, uint32_t rows) {
+    if (!m->tc_ok || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
     const bool exact = m->prefill_mode == WICK_CUDA_PREFILL_EXACT;
-    if (rows <= (uint32_t)TC_BUILD_ABOVE || !m->tc_ok || m->prefill_mode == WICK_CUDA_PREFILL_EXACT_CUDA_CORES) return WICK_CUDA_OK;
-    if (exact ? m->exact_built : m->fused_built) return WICK_CUDA_OK;
+    const CopyOrder want = exact ? CopyOrder::EXACT : CopyOrder::FUSED;
+    const bool there = m->layers[0].tc_gate.mem != nullptr;
+    if (m->copies == want || rows < (uint32_t)(!there ? TC_BUILD_ABOVE + 1 : exact ? 2 : TC_FUSED_MIN_TOKENS)) return WICK_CUDA_OK;
     RelaxedCapture relaxed;
-    const size_t n = m->allocs.size();
-    const uint64_t bytes = m->bytes;
-    const int32_t r = make_copies(m, exact);
-    if (r != WICK_CUDA_OK) undo_allocs(m, n, bytes);
-    return r == WICK_CUDA_ERR_OOM && rows < (uint32_t)TC_REQUIRED_FROM ? WICK_CUDA_OK : r;
+    if (!there) {
+        const size_t n = m->allocs.size();
+        const uint64_t bytes = m->bytes;
+        const int32_t r = alloc_copies(m);
+        if (r != WICK_CUDA_OK) {
+            undo_allocs(m, n, bytes);
+            W_TRY(for_each_copy(m, [](const DevWeight&, GemmCopy* t) { return *t = GemmCopy(), WICK_CUDA_OK; }));
+            m->x_hs = m->x_is = MmaInput();
+            return r == WICK_CUDA_ERR_OOM && rows < (uint32_t)TC_REQUIRED_FROM ? WICK_CUDA_OK : r;
+        }
+    }
+    m->copies = CopyOrder::NONE;
+    W_TRY(for_each_copy(m, [&](const DevWeight& w, GemmCopy* t) { return fill_copy(m, w, t, exact); }));
+    CU_TRY(cudaStreamSynchronize(m->stream));  // (a GEMM asks for its first weights ahead of its predecessors' end)
+    m->copies = want;
+    return WICK_CUDA_OK;
 }
 
 // Floats of all conv buffers of one sequence, one after another in layer order.
@@ -1155,20 +1180,22 @@ int32_t ensure_batch_buffers(wick_cuda_model* m, uint32_t rows, uint32_t steps) 
         m->batch_cap = cap;
         m->rows_out_cap = 0;
     }
-    const bool exact = m->prefill_mode == WICK_CUDA_PREFILL_EXACT && m->exact_built && !m->tc_embd.exact.p;
-    const bool fused = m->prefill_mode == WICK_CUDA_PREFILL_TENSOR && m->fused_built && !m->tc_embd.fused.q;
+    // The vocabulary head of a batched step is a GEMM over all rows: worth a copy of the matrix (in the order that this call takes).
+    const bool exact = m->prefill_mode == WICK_CUDA_PREFILL_EXACT && m->copies == CopyOrder::EXACT && !m->tc_embd.exact.p;
+    const bool fused = m->prefill_mode == WICK_CUDA_PREFILL_TENSOR && m->copies == CopyOrder::FUSED && !m->tc_embd.fused.q &&
+                       (!m->tc_embd.mem || rows >= (uint32_t)TC_FUSED_MIN_TOKENS);
     if ((exact || fused) && !m->embd_q6k && rows >= 2) {
-        // the vocabulary head of a batched step is a GEMM over all rows: worth a copy of the matrix
         RelaxedCapture relaxed;
         const size_t n_allocs = m->allocs.size();
         const uint64_t bytes = m->bytes;
-        const int32_t r = exact ? copy_for_exact(m, m->embd, &m->tc_embd) : copy_for_fused(m, m->embd, &m->tc_embd);
+        const int32_t r = m->tc_embd.mem ? WICK_CUDA_OK : alloc_copy(m, m->embd, &m->tc_embd);
         if (r != WICK_CUDA_OK) {
             undo_allocs(m, n_allocs, bytes);
-            // (a first plane may have been allocated, which is what the calls look at)
-            if (exact) m->tc_embd.exact = MmaWeight();
-            else m->tc_embd.fused = TcWeight();
+            m->tc_embd = GemmCopy();
             if (r != WICK_CUDA_ERR_OOM || rows >= (uint32_t)TC_REQUIRED_FROM) return r;
+        } else {
+            W_TRY(fill_copy(m, m->embd, &m->tc_embd, exact));
+            CU_TRY(cudaStreamSynchronize(m->stream));
         }
     }
     const size_t out_need = (size_t)steps * rows;
