@@ -39,17 +39,19 @@ def test_exact_gemm_at_its_edges(ops, orc, cuda_core_weight, dtype, m, k, n):
         assert np.array_equal(got[j].cpu().numpy().view(np.uint32), want.view(np.uint32))
 
 
-def test_columns_that_are_not_16_byte_aligned(ops, orc):
-    """The tensor cores' kernel reads 16 bytes at a time; a caller's 4-byte aligned columns are served as before."""
-    from wick_b200 import gguf_synth as gs
-    rng = np.random.default_rng(0)
-    m, k, n = 130, 256, 20
+@pytest.mark.parametrize("m,k,n,off", [(130, 256, 20, 4), (97, 384, 33, 8), (16, 640, 9, 12), (9600, 384, 31, 4), (2400, 128, 40, 12), (2048, 1152, 200, 4)])
+def test_columns_that_are_not_16_byte_aligned(ops, orc, cuda_core_weight, m, k, n, off):
+    """A caller's 4-byte aligned columns run on the tensor cores, too."""
+    from wick_b200 import _lib, gguf_synth as gs
+    rng = np.random.default_rng(m + n)
     raw = gs.quantize_q4_0((rng.standard_normal((m, k)) * 0.02).astype(F32))
     bs, bq = orc.quantize_q8_0(rng.standard_normal((n, k), dtype=F32))
-    w = ops.QuantWeight(ops.DT_Q4_0, raw, m, k)
-    room = torch.zeros(n * k + 4, dtype=torch.int8, device="cuda")
-    room[4:] = dev(bq).flatten()
+    room = torch.zeros(n * k + off, dtype=torch.int8, device="cuda")
+    room[off:] = dev(bq).flatten()
+    want = ops.gemm_q8(cuda_core_weight(ops.DT_Q4_0, raw, m, k), dev(bs), dev(bq))
+    assert np.array_equal(want[n - 1].cpu().numpy().view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[n - 1], bq[n - 1], m, k).view(np.uint32))
     for f in (ops.gemm_q8, ops.gemm_q8_tc_exact):
-        got = f(w, dev(bs), room[4:].view(n, k)).cpu().numpy()
-        for j in range(n):
-            assert np.array_equal(got[j].view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], m, k).view(np.uint32))
+        w = ops.QuantWeight(ops.DT_Q4_0, raw, m, k)
+        got = f(w, dev(bs), room[off:].view(n, k))
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+        assert w._lib.wick_cuda_debug_weight_error(w._h, 0) == _lib.OK  # (BAD_ARG where no product has used the tensor cores)

@@ -38,7 +38,7 @@ bool mma_gemm_supported(int m, int k);
 cudaError_t mma_weight_fill(cudaStream_t st, const DevWeight& w, uint8_t* p);
 
 // out[i][j][r] for matrix i < count (<= 3, equal k), token j < n, row r < m_i (token-major, like launch_gemm), with the arithmetic of
-// gemm_q*_q8_0_neon (simd.rs:696-1019) in its order, for any f32 scales.  xq: 16-byte aligned.  err: word (device or mapped host
+// gemm_q*_q8_0_neon (simd.rs:696-1019) in its order, for any f32 scales.  xq: 4-byte aligned.  err: word (device or mapped host
 // memory) that receives a non-zero code if a bounded wait expired.
 cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const uint8_t* x, const int8_t* xq, const float* xs,
                             int n, uint32_t* err);

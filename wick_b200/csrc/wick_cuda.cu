@@ -2178,7 +2178,7 @@ int32_t wick_cuda_debug_weight_error(const wick_cuda_weight* w, uint32_t code) {
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n, float* out_dev,
                           void* stream) {
     if (!w || !bs_dev || !bq_dev || !out_dev) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
-    if (n > (uint32_t)TC_BUILD_ABOVE && !w->cuda_cores && mma_gemm_supported(w->w.m, w->w.k) && ((uintptr_t)bq_dev & 15) == 0) {
+    if (n > (uint32_t)TC_BUILD_ABOVE && !w->cuda_cores && mma_gemm_supported(w->w.m, w->w.k)) {
         // same bits on the tensor cores (6912 x 2048 at 2002 rows: 1.71 ms on the CUDA cores, 0.43 there); asynchronous like the other
         // operators, so a wait that expired in an earlier call is reported by wick_cuda_weight_status or by the next call
         cudaStream_t st = (cudaStream_t)stream;
@@ -2225,9 +2225,7 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     W_TRY(ensure_exact_copy(w, st));
     const MmaWeight* tw[1] = {&w->exact};
     float* outs[1] = {out_dev};
-    if ((uintptr_t)bq_dev & 15) launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);  // (the tensor cores' kernel reads 16 bytes at a time)
-    else CU_TRY(launch_gemm_mma(st, tw, outs, 1, nullptr, bq_dev, bs_dev, (int)n, w->tc_err));
-    CU_TRY(cudaGetLastError());
+    CU_TRY(launch_gemm_mma(st, tw, outs, 1, nullptr, bq_dev, bs_dev, (int)n, w->tc_err));
     CU_TRY(cudaStreamSynchronize(st));
     return take_tc_error(w);
 }
