@@ -227,7 +227,7 @@ int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const 
  * any f32.  With more than 8 columns and k % 128 == 0 it runs on the tensor cores, with the same bits: the weight's first such
  * call makes a copy of it in operand order (1.125 bytes per parameter, kept until the weight is destroyed) and waits for that;
  * repeated products are then 4 times as fast as on the CUDA cores, the first one 1.9 times.  Without memory for the copy, and
- * while `stream` is captured before the copy exists, it runs on the CUDA cores.  A weight created
+ * while `stream` is captured before the copy exists (nor that of wick_cuda_gemm_q8_tc), it runs on the CUDA cores.  A weight created
  * with WICK_CUDA_PREFILL=exact-cuda-cores in the environment always does, and never makes the copy. */
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev,
                           uint32_t n, float* out_dev, void* stream);
@@ -251,7 +251,8 @@ int32_t wick_cuda_gemm_q8_tc(wick_cuda_weight* w, const float* bs_dev, const int
                              float* out_dev, int32_t* block_sums_dev, void* stream);
 /* The bit-exact product on the tensor cores (the default GEMM of forward_prefill): same result as
  * wick_cuda_gemm_q8, bit for bit.  Needs k % 128 == 0.  Synchronises `stream` (operator entry point for
- * tests) and makes the weight's copy on its first call, like wick_cuda_gemm_q8 (wick_cuda_gemm_q8_tc has an int8 copy of its own). */
+ * tests) and makes the weight's copy on its first call, like wick_cuda_gemm_q8 (wick_cuda_gemm_q8_tc has an int8 copy of its own;
+ * without memory for this one a weight that has that one is served by the CUDA cores). */
 int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n,
                                    float* out_dev, void* stream);
 /* int32 block dot sums S[i][b] = sum over the 32 elements of block b of row i (the vdotq_s32

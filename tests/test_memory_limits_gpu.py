@@ -57,6 +57,21 @@ def test_operator_product_without_memory_for_the_copy(ops, orc):
     assert np.array_equal(out[n - 1].cpu().numpy().view(np.uint32), want.view(np.uint32))
 
 
+def test_operator_weight_with_one_copy_and_no_memory_for_the_other(ops, orc):
+    m, k, n = 65536, 1024, 20                            # copies of 75 MB
+    rng = np.random.default_rng(1)
+    raw = rng.integers(0, 256, size=(m, k // 32, 18), dtype=np.uint8)
+    raw[:, :, :2] = np.full((m, k // 32, 1), 0.01, np.float16).view(np.uint8).reshape(m, k // 32, 2)
+    w = ops.QuantWeight(ops.DT_Q4_0, raw.reshape(-1), m, k)
+    bs, bq = orc.quantize_q8_0(rng.standard_normal((n, k), dtype=F32))
+    dbs, dbq = dev(bs), dev(bq)
+    ops.gemm_q8_tc(w, dbs, dbq)
+    want = orc.gemv(orc.DT_Q4_0, raw.reshape(m, -1), bs[n - 1], bq[n - 1], m, k)
+    with Filled(48 << 20):
+        got = ops.gemm_q8_tc_exact(w, dbs, dbq)          # (its output: 5 MB)
+        assert np.array_equal(got[n - 1].cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
 def test_few_rows_without_memory_for_the_copies(ops, orc, model_dir):
     """9 to 15 rows: served by the CUDA cores, bit for bit the same; nothing stays allocated; more rows are refused as ever."""
     import wick_b200.model as wick

@@ -115,6 +115,25 @@ def test_captured_products(ops, orc):
             assert np.array_equal(out[j].cpu().numpy().view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], w.m, w.k).view(np.uint32))
 
 
+def test_captured_product_of_a_weight_with_the_other_copy(ops, orc):
+    """A weight that gemm_q8_tc has used runs on the tensor cores from a capture on, too: its copy for them is made beside the capture."""
+    w, raw, bs, bq = make(ops, orc, m=16384, k=1024, n=20)
+    xs, xq, out = dev(bs), dev(bq), torch.empty((20, w.m), device="cuda")
+    ops.gemm_q8_tc(w, xs, xq)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        ops.gemm_q8(w, xs, xq, out)
+    assert torch.cuda.mem_get_info()[0] < free - (16 << 20)                 # 18.9 MB
+    _, _, bs, bq = make(ops, orc, n=20, k=1024, seed=1)
+    xs.copy_(dev(bs)), xq.copy_(dev(bq))
+    g.replay()
+    w.check_products()
+    for j in (0, 19):
+        assert np.array_equal(out[j].cpu().numpy().view(np.uint32), orc.gemv(orc.DT_Q4_0, raw, bs[j], bq[j], w.m, w.k).view(np.uint32))
+
+
 def test_weight_that_stays_on_the_cuda_cores(ops, orc, monkeypatch):
     """The environment switch of the models, for operator weights: no copy, the same bits."""
     from wick_b200 import _lib

@@ -2104,6 +2104,10 @@ static bool has_exact_copy(const wick_cuda_weight* w) {
     std::lock_guard<std::mutex> hold(w->tc_lock);
     return w->exact.p != nullptr;
 }
+static bool has_fused_copy(const wick_cuda_weight* w) {
+    std::lock_guard<std::mutex> hold(w->tc_lock);
+    return w->tc.q != nullptr;
+}
 
 // A copy of an operator-API weight, made on first use (and finished before the call goes on: later calls may come on other
 // streams).  `plane` is the copy's own pointer, null until it is complete; `fill(p)` fills it at p, `bytes` long.
@@ -2139,6 +2143,15 @@ static int32_t ensure_exact_copy(const wick_cuda_weight* w, cudaStream_t st) {
         w->exact.dtype = w->w.dtype;
         return mma_weight_fill(st, w->w, p);
     });
+}
+// The same while the caller's stream is captured: filled on a stream of its own.
+static int32_t ensure_exact_copy_beside_capture(const wick_cuda_weight* w) {
+    RelaxedCapture relaxed;
+    cudaStream_t own = nullptr;
+    CU_TRY(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+    const int32_t made = ensure_exact_copy(w, own);
+    cudaStreamDestroy(own);
+    return made;
 }
 static int32_t ensure_fused_copy(const wick_cuda_weight* w, cudaStream_t st) {
     TcWeight t;
@@ -2184,8 +2197,11 @@ int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const 
         cudaStream_t st = (cudaStream_t)stream;
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CU_TRY(cudaStreamIsCapturing(st, &capturing));
-        int32_t made = WICK_CUDA_ERR_OOM;  // (making the copy allocates and synchronises: not while the stream is captured)
+        // (A weight that no product has brought to the tensor cores yet gets no memory in a capture; one that
+        // wick_cuda_gemm_q8_tc has made its own copy of was served by that copy when both had one, and goes on being served.)
+        int32_t made = WICK_CUDA_ERR_OOM;
         if (capturing == cudaStreamCaptureStatusNone || has_exact_copy(w)) made = ensure_exact_copy(w, st);
+        else if (has_fused_copy(w)) made = ensure_exact_copy_beside_capture(w);
         if (made != WICK_CUDA_OK && made != WICK_CUDA_ERR_OOM) return made;
         if (made == WICK_CUDA_OK) {
             W_TRY(take_tc_error(w));
@@ -2222,10 +2238,16 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     if (!tc_gemm_supported(w->w.m, w->w.k)) return fail(WICK_CUDA_ERR_BAD_ARG, "tensor-core GEMM needs k to be a multiple of 128");
     if (n == 0) return WICK_CUDA_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    W_TRY(ensure_exact_copy(w, st));
-    const MmaWeight* tw[1] = {&w->exact};
-    float* outs[1] = {out_dev};
-    CU_TRY(launch_gemm_mma(st, tw, outs, 1, nullptr, bq_dev, bs_dev, (int)n, w->tc_err));
+    const int32_t made = ensure_exact_copy(w, st);
+    if (made == WICK_CUDA_ERR_OOM && has_fused_copy(w)) {  // (a weight that has one of the copies is not refused for want of the other)
+        launch_gemm(st, w->w, bs_dev, bq_dev, (int)n, out_dev);
+        CU_TRY(cudaGetLastError());
+    } else {
+        W_TRY(made);
+        const MmaWeight* tw[1] = {&w->exact};
+        float* outs[1] = {out_dev};
+        CU_TRY(launch_gemm_mma(st, tw, outs, 1, nullptr, bq_dev, bs_dev, (int)n, w->tc_err));
+    }
     CU_TRY(cudaStreamSynchronize(st));
     return take_tc_error(w);
 }
