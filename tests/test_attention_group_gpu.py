@@ -43,6 +43,36 @@ def test_prompts_and_batched_steps_at_tile_edges(cuda_lib, orc, model_dir, monke
             nxt[i] = orc.argmax(want)
 
 
+@pytest.mark.parametrize("heads,n_kv,rows", [(8, 1, 33), (12, 2, 17)])
+def test_many_heads_to_a_kv_head_in_small_batches(cuda_lib, orc, model_dir, monkeypatch, heads, n_kv, rows):
+    """More than four heads and at most 32 (row, KV head) pairs: the kernels of one head to a CTA, with a quantiser of their own; one row more: this one."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import gguf_synth as gs
+    from wick_b200.model import CudaLfm2Model
+    spec = dataclasses.replace(gs.SPECS["tiny"], name=f"small-batch-{heads}-{n_kv}", hidden=64 * heads, n_heads=heads, n_kv_heads=n_kv)
+    monkeypatch.setitem(gs.SPECS, spec.name, spec)
+    path = gs.cached_model(spec.name, "q4_0", 0, cache_dir=model_dir, norm_jitter=0.2, weight_std=0.05)
+    m, ids, oracles, toks = CudaLfm2Model(path, 128), [], [], []
+    for i in range(rows):
+        ids.append(m.seq_create())
+        oracles.append(orc.OracleModel(path, 128))
+        prompt = gs.random_prompt(9 + 3 * i, spec.vocab, seed=i)
+        m.seq_prefill(ids[i], prompt, 0)
+        toks.append(orc.argmax(oracles[i].forward_prefill(prompt, 0)))
+    kernels = []
+    for step in range(2):  # (the first one of each size makes buffers)
+        for n in (rows - 1, rows):
+            before = m.kernel_launches()
+            got = m.decode_batch_logits(toks[:n], ids[:n])
+            kernels.append(m.kernel_launches() - before)
+            for i in range(n):
+                want = oracles[i].forward(int(toks[i]))
+                assert np.array_equal(bits(got[i]), bits(want)), (step, n, i)
+                toks[i] = orc.argmax(want)
+    assert kernels[2] == kernels[3] + len(spec.attn_layers)
+
+
 def test_rows_wider_than_a_thread_per_four_elements(cuda_lib, orc, model_dir, monkeypatch):
     """Hidden rows above 4096 elements: the add + RMSNorm + quantise kernel has more than four of them per thread."""
     if not torch.cuda.is_available():

@@ -185,7 +185,8 @@ cudaError_t launch_attention_rows(cudaStream_t st, const float* q, float* const*
                                   float* out, int n, int n_heads, int n_kv_heads, int head_dim, int max_seq);
 // The same attention for the query heads of a KV head together, its result quantised (into x where x.p is not null): n rows with caches of
 // their own (positions[j] = cached rows before row j's) or, k_single not null, n consecutive tokens of one sequence from start_pos.
-// max_seq: keys of the longest row.  *done is false, and nothing launched, for shapes it does not take.
+// max_seq: keys of the longest row.  *done is false, and nothing launched, for shapes it does not take or
+// at which the kernels of one head to a CTA are faster.
 cudaError_t launch_attention_group(cudaStream_t st, const float* q, float* const* k_caches, float* const* v_caches, const float* k_single,
                                    const float* v_single, const uint32_t* positions, int start_pos, int n, int n_heads, int n_kv_heads, int head_dim,
                                    int max_seq, float* q8s, int8_t* q8q, const MmaInput& x, bool* done);

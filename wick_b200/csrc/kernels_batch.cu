@@ -350,7 +350,13 @@ cudaError_t launch_attention_group(cudaStream_t st, const float* q, float* const
                                    int max_seq, float* q8s, int8_t* q8q, const MmaInput& x, bool* done) {
     const int heads = n_heads / n_kv_heads;
     const size_t smem = attention_group_smem(heads, max_seq);
-    *done = head_dim == GROUP_HD && heads <= GROUP_MAX_HEADS && smem <= 220 * 1024;
+    // More than four heads are three or four in a row for a thread, which a CTA per head does side by side where the GPU has room for
+    // them: with 32 CTAs or fewer this kernel takes 1.03 to 1.4 times as long as the others, at 150, 1000 and 4000 keys (8 heads, one
+    // KV head, 8 rows: 18 against 15 us, 61 against 48, 209 against 159), with 64 0.66 to 1.06 times.  Up to four heads it is the
+    // faster one at every size measured (2 to 255 rows or tokens, 150 to 8000 keys: 0.31 to 0.95 times; the 1.6B-class model's four
+    // heads, 2 rows of 4000 keys: 133 against 169 us, 64 rows: 516 against 976).
+    const bool wins = heads <= 4 || n * n_kv_heads > 32;
+    *done = head_dim == GROUP_HD && heads <= GROUP_MAX_HEADS && smem <= 220 * 1024 && wins;
     if (!*done || n <= 0) return cudaSuccess;
     auto launch = [&](auto kernel, RaisedPerDevice& limit) {
         const cudaError_t e = raise_dynamic_smem(limit, (const void*)kernel, smem);
