@@ -173,3 +173,30 @@ def test_decode_with_a_short_ring_and_one_row_prefills(cuda_lib, orc, model_dir,
     assert_bits(cm.forward_embedding([int(toks[2])], 44, st), om.forward_embedding(int(toks[2])), "hidden row")
     assert list(cm.generate_greedy(6, 4, st)) == list(om.generate_greedy(6, 4))
     assert_bits(cm.forward_prefill(toks[:1], 0, st), om.forward_prefill(toks[:1], 0), "one-token prompt")
+
+
+def test_attention_whose_scores_just_fit_the_default_shared_memory(cuda_lib, orc, model_dir):
+    """8100 keys of 64: 47.9 KB of dynamic shared memory and the kernel's static 384 bytes are more than the 48 KB that need no opt-in.  (A
+    process of its own: one larger call before would have raised the limit.)"""
+    import os, subprocess, sys
+    from wick_b200 import gguf_synth as gs
+    code = """
+import os, sys
+os.environ["WICK_CUDA_DECODE"] = "graph"
+import numpy as np, torch
+from oracle import oracle as orc
+from wick_b200 import ops
+import wick_b200.model as wick
+cm, om = wick.CudaLfm2Model(sys.argv[1], 8100), orc.OracleModel(sys.argv[1], 8100)
+st, toks = wick.InferenceState(), list(range(5, 35))
+first = orc.argmax(om.forward_prefill(toks, 0))
+assert orc.argmax(cm.forward_prefill(toks, 0, st)) == first
+assert list(cm.generate_greedy(first, 8, st)) == list(om.generate_greedy(first, 8))
+q, k, v = (torch.randn(n, 64, device="cuda") for n in (1, 8100, 8100))
+short = ops.attention_decode(q, k[:8000], v[:8000], 1, 1, 64, 8000)
+v[8000:], k[8000:] = 0, -100 * torch.sign(q)   # the last hundred keys count for nothing
+assert torch.equal(ops.attention_decode(q, k, v, 1, 1, 64, 8100), short)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code, gs.cached_model("tiny-longctx", "q4_0", 0, cache_dir=model_dir, norm_jitter=0.2, weight_std=0.05)],
+                   check=True, cwd=root, timeout=300)

@@ -39,6 +39,8 @@ inline cudaError_t launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, 
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Dynamic shared memory that a kernel may ask for without opting in: 48 KB, less the static arrays of the kernels that ask (under 1 KB).
+constexpr size_t SMEM_WITHOUT_OPT_IN = 47 * 1024;
 // Raises a kernel's opt-in shared memory on the current device; `state`: the kernel's own static object.
 inline cudaError_t raise_dynamic_smem(RaisedPerDevice& state, const void* kernel, size_t bytes) {
     int dev = 0;
@@ -138,7 +140,7 @@ void launch_rope(cudaStream_t st, float* q, float* k, const float* cos_row, cons
 void launch_attention_naive(cudaStream_t st, const float* q, const float* k_cache, const float* v_cache, float* out,
                             int n, int start_pos, const DecodeCtl* ctl, int n_heads, int n_kv_heads, int head_dim,
                             int max_seq);
-// Opt-in to more than 48 KB of dynamic shared memory for the kernel above; call before any
+// Opt-in to the dynamic shared memory that the kernel above needs, where that takes one; call before any
 // stream capture that contains it.
 void configure_naive_attention_smem(size_t bytes);
 // Dynamic shared memory the kernel needs for this head size and longest sequence.

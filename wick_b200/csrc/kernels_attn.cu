@@ -124,8 +124,7 @@ __global__ void __launch_bounds__(NAIVE_THREADS) k_attention_naive(const float* 
 // lower the limit under a model that still launches with its own, larger size).
 static cudaError_t raise_naive_attention_smem(size_t bytes) {
     static RaisedPerDevice limit;
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return raise_dynamic_smem(limit, (const void*)k_attention_naive, bytes);
+    return bytes <= SMEM_WITHOUT_OPT_IN ? cudaSuccess : raise_dynamic_smem(limit, (const void*)k_attention_naive, bytes);
 }
 
 void configure_naive_attention_smem(size_t bytes) { raise_naive_attention_smem(bytes); }
@@ -513,7 +512,7 @@ static cudaError_t launch_flash_hd(cudaStream_t st, const float* q, const float*
     }
     const size_t smem = 64 + (size_t)(4 * FLASH_TILE + n_cw * 8 * BQ) * (HD + 4) * sizeof(float);
     static RaisedPerDevice limit, carveout;
-    if (smem > 48 * 1024) {
+    if (smem > SMEM_WITHOUT_OPT_IN) {
         e = raise_dynamic_smem(limit, (const void*)k_attention_flash<HD, BQ>, smem);
         if (e != cudaSuccess) return e;
     }

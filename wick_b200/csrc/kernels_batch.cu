@@ -191,7 +191,7 @@ cudaError_t launch_attention_rows(cudaStream_t st, const float* q, float* const*
                                   float* out, int n, int n_heads, int n_kv_heads, int head_dim, int max_seq) {
     static RaisedPerDevice limit;
     const size_t smem = naive_attention_smem_bytes(head_dim, max_seq);
-    if (smem > 48 * 1024) {
+    if (smem > SMEM_WITHOUT_OPT_IN) {
         const cudaError_t e = raise_dynamic_smem(limit, (const void*)k_attention_rows, smem);
         if (e != cudaSuccess) return e;
     }

@@ -1097,9 +1097,7 @@ int32_t build_model(wick_cuda_model* m, const GgufImage& g, uint32_t context_siz
     memset(m->h_ctl, 0, sizeof(DecodeCtl));
     CU_TRY(cudaMemset(m->ctl, 0, sizeof(DecodeCtl)));
     W_TRY(reset_sequence(m));
-    if (naive_attn_smem(m) > 48 * 1024) {
-        configure_naive_attention_smem(naive_attn_smem(m));
-    }
+    configure_naive_attention_smem(naive_attn_smem(m));
     CU_TRY(cudaEventCreate(&m->ev0));
     CU_TRY(cudaEventCreate(&m->ev1));
     {
@@ -2358,9 +2356,6 @@ int32_t wick_cuda_attention_prefill(const float* q_dev, const float* k_cache_dev
     } else {
         size_t smem = naive_attention_smem_bytes((int)head_dim, (int)(start_pos + n));
         if (smem > 200 * 1024) return fail(WICK_CUDA_ERR_BAD_ARG, "sequence too long for the per-token attention kernel");
-        if (smem > 48 * 1024) {
-                configure_naive_attention_smem(smem);
-        }
         launch_attention_naive((cudaStream_t)stream, q_dev, k_cache_dev, v_cache_dev, out_dev, (int)n, (int)start_pos, nullptr,
                                (int)n_heads, (int)n_kv_heads, (int)head_dim, (int)(start_pos + n));
     }
