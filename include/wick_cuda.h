@@ -255,6 +255,19 @@ int32_t wick_cuda_gemm_q8_tc(wick_cuda_weight* w, const float* bs_dev, const int
  * without memory for this one a weight that has that one is served by the CUDA cores). */
 int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev, uint32_t n,
                                    float* out_dev, void* stream);
+/* Test hooks: kernels of forward_prefill and wick_cuda_decode_batch one by one, fed as inside a model.  They synchronise `stream`.
+ * gemm_rows: the bit-exact product of n f32 rows x [n][k] after the Q8_0 quantiser.  ready != 0: in the form that a model's own
+ *   quantisers write; 0: in that of wick_cuda_gemm_q8.  tile: NULL, or three values: the index of the tile shape to take (0 .. 6; -1
+ *   for the rule's choice), then the shape that ran, in rows and tokens.
+ * attention_group: attention of prompts below 256 tokens and of batched steps, arguments as wick_cuda_attention_prefill (head_dim 64),
+ *   quantised result; BAD_ARG for shapes that other kernels serve.
+ * add_rmsnorm_quant: hidden [n][dim] += add (NULL: none), RMSNorm with `weight`, quantised and, normed_dev not NULL, in f32. */
+int32_t wick_cuda_debug_gemm_rows(const wick_cuda_weight* w, const float* x_dev, uint32_t n, int32_t ready, int32_t* tile, float* out_dev,
+                                  void* stream);
+int32_t wick_cuda_debug_attention_group(const float* q_dev, const float* k_cache_dev, const float* v_cache_dev, float* xs_dev, int8_t* xq_dev,
+                                        uint32_t n, uint32_t start_pos, uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim, void* stream);
+int32_t wick_cuda_debug_add_rmsnorm_quant(float* hidden_dev, const float* add_dev, const float* weight_dev, uint32_t n, uint32_t dim, float eps,
+                                          float* normed_dev, float* xs_dev, int8_t* xq_dev, void* stream);
 /* int32 block dot sums S[i][b] = sum over the 32 elements of block b of row i (the vdotq_s32
  * lanes of simd.rs:381-383 added up) against one quantised column. */
 int32_t wick_cuda_block_sums(const wick_cuda_weight* w, const int8_t* xq_dev, int32_t* s_dev, void* stream);

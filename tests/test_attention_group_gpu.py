@@ -73,6 +73,54 @@ def test_many_heads_to_a_kv_head_in_small_batches(cuda_lib, orc, model_dir, monk
     assert kernels[2] == kernels[3] + len(spec.attn_layers)
 
 
+@pytest.mark.parametrize("heads,n_kv", [(1, 8), (2, 3), (3, 2), (4, 8), (5, 1), (6, 3), (7, 1), (8, 2)])
+@pytest.mark.parametrize("n,start", [(33, 0), (40, 31), (34, 64), (36, 1000), (33, 4003)])
+def test_kernel_against_the_per_head_one(cuda_lib, heads, n_kv, n, start):
+    """Every split of 1 to 8 heads over the threads, contexts of one tile to many, against attention_prefill (itself compared with the oracle) and
+    the quantiser; and the result's place among other rows: nothing is written behind the last one."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(heads * 10 + n)
+    nh, kv = heads * n_kv, n_kv * 64
+    q = torch.randn((n, nh * 64), generator=g, device="cuda")
+    k, v = (torch.randn((start + n, kv), generator=g, device="cuda") for _ in range(2))
+    want_s, want_q = ops.quantize_f32_to_q8_0(ops.attention_prefill(q, k, v, n, start, nh, n_kv, 64, False))
+    s, b = torch.full((n + 1, nh * 2), 7.0, device="cuda"), torch.full((n + 1, nh * 64), 7, dtype=torch.int8, device="cuda")
+    _lib.check(cuda_lib.wick_cuda_debug_attention_group(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), b.data_ptr(), n, start, nh, n_kv, 64,
+                                                        torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(s[:n].view(torch.int32), want_s.view(torch.int32)) and torch.equal(b[:n], want_q)
+    assert (s[n] == 7).all() and (b[n] == 7).all()
+
+
+@pytest.mark.parametrize("dim", [32, 1024, 4064, 4096, 4128, 8160, 8192, 8224, 12320, 16384, 16416])
+def test_add_rmsnorm_quant_by_row_length(cuda_lib, dim):
+    """One, two and four quads to a thread and the edges between them, against the operators one by one; longer rows are refused."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    n = 3
+    h, add = (torch.randn((n, dim), generator=g, device="cuda") * 3 for _ in range(2))
+    w = torch.rand(dim, generator=g, device="cuda") + 0.5
+    for a in (add, None):
+        hidden, normed = h.clone(), torch.empty_like(h)
+        s, b = torch.empty((n, dim // 32), device="cuda"), torch.empty((n, dim), dtype=torch.int8, device="cuda")
+        r = cuda_lib.wick_cuda_debug_add_rmsnorm_quant(hidden.data_ptr(), a.data_ptr() if a is not None else None, w.data_ptr(), n, dim, 1e-5,
+                                                       normed.data_ptr(), s.data_ptr(), b.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        if dim > 16384:
+            assert r == _lib.ERR_CUDA
+            continue
+        _lib.check(r)
+        total = h + a if a is not None else h
+        assert torch.equal(hidden, total)
+        want = ops.rmsnorm_(total.clone(), w, 1e-5)
+        # (the f64 sums are added in different fixed orders: at most the last bit of the factor, so of a value, may differ)
+        assert (normed.view(torch.int32) - want.view(torch.int32)).abs().max() <= 1
+        want_s, want_q = ops.quantize_f32_to_q8_0(normed)
+        assert torch.equal(s, want_s) and torch.equal(b, want_q)
+
+
 def test_rows_wider_than_a_thread_per_four_elements(cuda_lib, orc, model_dir, monkeypatch):
     """Hidden rows above 4096 elements: the add + RMSNorm + quantise kernel has more than four of them per thread."""
     if not torch.cuda.is_available():

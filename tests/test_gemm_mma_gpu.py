@@ -55,3 +55,50 @@ def test_columns_that_are_not_16_byte_aligned(ops, orc, cuda_core_weight, m, k, 
         got = f(w, dev(bs), room[off:].view(n, k))
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
         assert w._lib.wick_cuda_debug_weight_error(w._h, 0) == _lib.OK  # (BAD_ARG where no product has used the tensor cores)
+
+
+# Rows and tokens of the tile shapes: of the form with activations in operand order, which every prompt and batched step of a model
+# takes, and of that with int8 columns (gemm_q8).
+TILES = {True: [(96, 32), (96, 16), (64, 24), (64, 16), (64, 8), (32, 8), (16, 8)],
+         False: [(96, 32), (64, 32), (64, 16), (64, 8), (32, 8), (16, 16), (16, 8)]}
+
+
+def gemm_rows(w, x, ready, tile=-1):
+    """The product of f32 rows by a tile shape (-1: the rule's) and the shape that ran."""
+    import ctypes as C
+    from wick_b200 import _lib
+    out, t = torch.empty((x.shape[0], w.m), device="cuda"), (C.c_int32 * 3)(tile, 0, 0)
+    _lib.check(w._lib.wick_cuda_debug_gemm_rows(w._h, x.data_ptr(), x.shape[0], int(ready), t, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    return out, (t[1], t[2])
+
+
+@pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("ready", [True, False])
+@pytest.mark.parametrize("tile", range(7))
+def test_every_tile_shape(ops, orc, cuda_core_weight, dtype, ready, tile):
+    """A row and a token more than a tile, fewer than three of each, and more tiles than SMs; k = 128 * odd leaves half of the last stage empty."""
+    rows, tokens = TILES[ready][tile]
+    for m, k, n in ((rows + 1, 128, tokens + 1), (3 * rows - 5, 384, 2 * tokens - 1), (rows * 150 + 7, 640, 3 * tokens + 2), (1, 1152, 1)):
+        rng = np.random.default_rng(m + k + n)
+        raw = rng.integers(0, 256, size=(m, k // 32, 18 if dtype == "q4_0" else 34), dtype=np.uint8)  # every int8, -128 too
+        raw[:, :, :2] = rng.uniform(-0.02, 0.02, size=(m, k // 32)).astype(np.float16).view(np.uint8).reshape(m, k // 32, 2)
+        dt = ops.QTYPE_ID[dtype]
+        x = dev(rng.standard_normal((n, k), dtype=F32) * np.exp(rng.standard_normal((n, 1), dtype=F32)))
+        x[n // 2, :32] = 0
+        got, ran = gemm_rows(ops.QuantWeight(dt, raw.reshape(-1), m, k), x, ready, tile)
+        assert ran == (rows, tokens)
+        bs, bq = ops.quantize_f32_to_q8_0(x)
+        assert torch.equal(got.view(torch.int32), ops.gemm_q8(cuda_core_weight(dt, raw.reshape(-1), m, k), bs, bq).view(torch.int32)), (m, k, n)
+        want = orc.gemv(dt, raw.reshape(m, -1), bs[n - 1].cpu().numpy(), bq[n - 1].cpu().numpy(), m, k)
+        assert np.array_equal(got[n - 1].cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("ready,m,n,tile", [(True, 6144, 512, 0), (True, 2048, 96, 1), (True, 65536, 24, 2), (True, 2048, 64, 3), (True, 1024, 33, 4),
+                                            (True, 65536, 6, 5), (True, 2048, 6, 6), (False, 6912, 2002, 0), (False, 2048, 96, 1), (False, 2048, 64, 2),
+                                            (False, 1024, 33, 3), (False, 2048, 9, 6)])
+def test_tile_shapes_of_ordinary_sizes(ops, ready, m, n, tile):
+    """What the rule takes on 148 SMs."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the rule goes by the device's SMs")
+    w = ops.QuantWeight(ops.DT_Q4_0, np.zeros(m * 4 * 18, np.uint8), m, 128)
+    assert gemm_rows(w, torch.ones((n, 128), device="cuda"), ready)[1] == TILES[ready][tile]

@@ -96,6 +96,9 @@ SIGNATURES = {
     "wick_cuda_debug_weight_error": [_vp, _u32],
     "wick_cuda_gemm_q8_tc": [_vp, _vp, _vp, _u32, _vp, _vp, _vp],
     "wick_cuda_gemm_q8_tc_exact": [_vp, _vp, _vp, _u32, _vp, _vp],
+    "wick_cuda_debug_gemm_rows": [_vp, _vp, _u32, _i32, C.POINTER(_i32), _vp, _vp],
+    "wick_cuda_debug_attention_group": [_vp, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp],
+    "wick_cuda_debug_add_rmsnorm_quant": [_vp, _vp, _vp, _u32, _u32, _f, _vp, _vp, _vp, _vp],
     "wick_cuda_block_sums": [_vp, _vp, _vp, _vp],
     "wick_cuda_rmsnorm": [_vp, _vp, _u32, _u32, _f, _vp],
     "wick_cuda_silu_mul": [_vp, _vp, _u64, _vp],

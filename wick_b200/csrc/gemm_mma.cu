@@ -613,14 +613,14 @@ cudaError_t mma_weight_fill(cudaStream_t st, const DevWeight& w, uint8_t* p) {
 }
 
 cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const uint8_t* x, const int8_t* xq,
-                            const float* xs, int n, uint32_t* err) {
+                            const float* xs, int n, uint32_t* err, MmaTileShape* tile) {
     if (n <= 0 || count <= 0) return cudaSuccess;
     if (count > 3) return cudaErrorInvalidValue;
     for (int i = 1; i < count; i++) {
         if (w[i]->k != w[0]->k) return cudaErrorInvalidValue;
         if (w[i]->dtype != w[0]->dtype) {  // mixed types: a launch each
             for (int j = 0; j < count; j++) {
-                const cudaError_t e = launch_gemm_mma(st, w + j, out + j, 1, x, xq, xs, n, err);
+                const cudaError_t e = launch_gemm_mma(st, w + j, out + j, 1, x, xq, xs, n, err, tile);
                 if (e != cudaSuccess) return e;
             }
             return cudaSuccess;
@@ -649,21 +649,22 @@ cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* c
     struct Shape {
         int r, nt, ctas, one, all;
     };
-    static constexpr int N_SHAPES = 7;
-    static constexpr Shape READY_SHAPES[N_SHAPES] = {{6, 4, 1, 156, 156}, {6, 2, 1, 78, 78}, {4, 3, 1, 80, 80}, {4, 2, 1, 53, 54},
+    static constexpr Shape READY_SHAPES[MMA_SHAPES] = {{6, 4, 1, 156, 156}, {6, 2, 1, 78, 78}, {4, 3, 1, 80, 80}, {4, 2, 1, 53, 54},
                                                      {4, 1, 1, 38, 42},   {2, 1, 2, 36, 38}, {1, 1, 2, 27, 28}};
     // (with the converting warps: two lane-group warps bring nothing, 1024 x 4608 at 9 tokens 8.4 against 8.1 us)
-    static constexpr Shape CONVERT_SHAPES[N_SHAPES] = {{6, 4, 1, 176, 176}, {4, 4, 1, 120, 120}, {4, 2, 1, 67, 67}, {4, 1, 1, 41, 41},
+    static constexpr Shape CONVERT_SHAPES[MMA_SHAPES] = {{6, 4, 1, 176, 176}, {4, 4, 1, 120, 120}, {4, 2, 1, 67, 67}, {4, 1, 1, 41, 41},
                                                        {2, 1, 2, 42, 46},   {1, 2, 2, 46, 51},   {1, 1, 2, 32, 40}};
     const Shape* shapes = x ? READY_SHAPES : CONVERT_SHAPES;
     int best = 0, best_cost = INT_MAX;
-    for (int i = 0; i < N_SHAPES; i++) {
+    for (int i = 0; i < MMA_SHAPES; i++) {
         const Shape& s = shapes[i];
         const int t = tiles(s.r * MMA_ROWS, s.nt * 8), slots = sms * s.ctas, rest = t % slots;
         const int cost = t / slots * s.all + (rest == 0 ? 0 : rest <= sms ? s.one : s.all);
         if (cost < best_cost) best = i, best_cost = cost;
     }
+    if (tile && tile->index >= 0 && tile->index < MMA_SHAPES) best = tile->index;
     const int rows = shapes[best].r * MMA_ROWS, tokens = shapes[best].nt * 8;
+    if (tile) *tile = MmaTileShape{best, rows, tokens};
     int t = 0;
     for (int i = 0; i < 3; i++) {
         job.tile_start[i] = t;

@@ -39,8 +39,12 @@ cudaError_t mma_weight_fill(cudaStream_t st, const DevWeight& w, uint8_t* p);
 
 // out[i][j][r] for matrix i < count (<= 3, equal k), token j < n, row r < m_i (token-major, like launch_gemm), with the arithmetic of
 // gemm_q*_q8_0_neon (simd.rs:696-1019) in its order, for any f32 scales.  xq: 4-byte aligned.  err: word (device or mapped host
-// memory) that receives a non-zero code if a bounded wait expired.
+// memory) that receives a non-zero code if a bounded wait expired.  tile (tests): a shape to take, or -1 for the rule's; receives what ran.
+struct MmaTileShape {
+    int index = -1, rows = 0, tokens = 0;
+};
 cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* const* out, int count, const uint8_t* x, const int8_t* xq, const float* xs,
-                            int n, uint32_t* err);
+                            int n, uint32_t* err, MmaTileShape* tile = nullptr);
+constexpr int MMA_SHAPES = 7;
 
 }  // namespace wick

@@ -2250,6 +2250,68 @@ int32_t wick_cuda_gemm_q8_tc_exact(wick_cuda_weight* w, const float* bs_dev, con
     return take_tc_error(w);
 }
 
+int32_t wick_cuda_debug_gemm_rows(const wick_cuda_weight* w, const float* x_dev, uint32_t n, int32_t ready, int32_t* tile, float* out_dev, void* stream) {
+    if (!w || !x_dev || !out_dev || n == 0) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument or no rows");
+    if (!mma_gemm_supported(w->w.m, w->w.k)) return fail(WICK_CUDA_ERR_BAD_ARG, "tensor-core GEMM needs k to be a multiple of 128");
+    if (tile && tile[0] >= MMA_SHAPES) return fail(WICK_CUDA_ERR_BAD_ARG, "no such tile shape");
+    cudaStream_t st = (cudaStream_t)stream;
+    W_TRY(ensure_exact_copy(w, st));
+    const int k = w->w.k;
+    MmaInput x;
+    x.blocks = w->exact.stages() * MMA_STAGE_BLOCKS;
+    const size_t x_bytes = ((size_t)n + MMA_X_ROWS - 1) / MMA_X_ROWS * x.blocks * MMA_X_CHUNK, s_bytes = (size_t)n * (k / QK) * sizeof(float);
+    uint8_t* scratch = nullptr;
+    CU_TRY(cudaMallocAsync((void**)&scratch, ready ? x_bytes : s_bytes + (size_t)n * k, st));
+    float* q8s = reinterpret_cast<float*>(scratch);
+    int8_t* q8q = reinterpret_cast<int8_t*>(scratch + s_bytes);  // (s_bytes is a multiple of 16: k is one of 128)
+    cudaError_t e = cudaSuccess;
+    if (ready) {
+        x.p = scratch;
+        e = cudaMemsetAsync(scratch, 0, x_bytes, st);
+    }
+    if (e == cudaSuccess) {
+        launch_quant_rows(st, x_dev, (int)n, k, q8s, q8q, x);
+        e = cudaGetLastError();
+    }
+    MmaTileShape shape;
+    if (tile) shape.index = tile[0];
+    const MmaWeight* tw[1] = {&w->exact};
+    float* outs[1] = {out_dev};
+    if (e == cudaSuccess) e = launch_gemm_mma(st, tw, outs, 1, x.p, ready ? nullptr : q8q, ready ? nullptr : q8s, (int)n, w->tc_err, &shape);
+    if (tile) {
+        tile[0] = shape.index;
+        tile[1] = shape.rows;
+        tile[2] = shape.tokens;
+    }
+    cudaFreeAsync(scratch, st);
+    CU_TRY(e);
+    CU_TRY(cudaStreamSynchronize(st));
+    return take_tc_error(w);
+}
+
+int32_t wick_cuda_debug_attention_group(const float* q_dev, const float* k_cache_dev, const float* v_cache_dev, float* xs_dev, int8_t* xq_dev,
+                                        uint32_t n, uint32_t start_pos, uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim, void* stream) {
+    if (!q_dev || !k_cache_dev || !v_cache_dev || !xs_dev || !xq_dev) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
+    if (!n_kv_heads || n_heads % n_kv_heads || n == 0) return fail(WICK_CUDA_ERR_BAD_ARG, "bad attention shape");
+    cudaStream_t st = (cudaStream_t)stream;
+    bool done = false;
+    CU_TRY(launch_attention_group(st, q_dev, nullptr, nullptr, k_cache_dev, v_cache_dev, nullptr, (int)start_pos, (int)n, (int)n_heads, (int)n_kv_heads,
+                                  (int)head_dim, (int)(start_pos + n), xs_dev, xq_dev, MmaInput(), &done));
+    if (!done) return fail(WICK_CUDA_ERR_BAD_ARG, "a shape that the other attention kernels serve");
+    CU_TRY(cudaStreamSynchronize(st));
+    OP_END();
+}
+
+int32_t wick_cuda_debug_add_rmsnorm_quant(float* hidden_dev, const float* add_dev, const float* weight_dev, uint32_t n, uint32_t dim, float eps,
+                                          float* normed_dev, float* xs_dev, int8_t* xq_dev, void* stream) {
+    if (!hidden_dev || !weight_dev || !xs_dev || !xq_dev || n == 0) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument or no rows");
+    if (dim == 0 || dim % QK) return fail(WICK_CUDA_ERR_BAD_ARG, "dim must be a positive multiple of 32");
+    launch_add_rmsnorm_quant((cudaStream_t)stream, hidden_dev, add_dev, weight_dev, eps, (int)n, (int)dim, xs_dev, xq_dev, normed_dev);
+    CU_TRY(cudaGetLastError());
+    CU_TRY(cudaStreamSynchronize((cudaStream_t)stream));
+    OP_END();
+}
+
 int32_t wick_cuda_block_sums(const wick_cuda_weight* w, const int8_t* xq_dev, int32_t* s_dev, void* stream) {
     if (!w || !xq_dev || !s_dev) return fail(WICK_CUDA_ERR_BAD_ARG, "NULL argument");
     launch_block_sums((cudaStream_t)stream, w->w, xq_dev, s_dev);
