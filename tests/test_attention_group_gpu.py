@@ -136,3 +136,20 @@ def test_rows_wider_than_a_thread_per_four_elements(cuda_lib, orc, model_dir, mo
     want = o.forward_prefill(toks, 0)
     assert np.array_equal(bits(m.seq_prefill(sid, toks, 0)), bits(want))
     assert np.array_equal(bits(m.decode_batch_logits([orc.argmax(want)], [sid])[0]), bits(o.forward(orc.argmax(want))))
+
+
+@pytest.mark.parametrize("hidden", [16384, 16416, 1 << 20])
+def test_hidden_rows_that_no_kernel_holds_are_refused_at_load(cuda_lib, model_dir, hidden):
+    """A launch with such rows is refused, and the captured decode step was left without it: all logits 0, and no error.  (16384 itself is
+    a length that the kernel takes: this file is turned down for its head size.)"""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wick_b200 import _lib, gguf_synth as gs
+    from wick_b200.model import CudaLfm2Model
+    data = bytearray(open(gs.cached_model("tiny", "q4_0", 0, cache_dir=model_dir), "rb").read())
+    key = b"lfm2.embedding_length" + (gs.T_UINT32).to_bytes(4, "little")
+    at = data.index(key) + len(key)
+    data[at:at + 4] = hidden.to_bytes(4, "little")
+    with pytest.raises(_lib.WickCudaError) as e:
+        CudaLfm2Model.from_bytes(bytes(data), 64)
+    assert e.value.code == _lib.ERR_BAD_GGUF and ("16384" in str(e.value)) == (hidden > 16384)

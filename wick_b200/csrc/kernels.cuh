@@ -107,7 +107,8 @@ void launch_repack(cudaStream_t st, const DevWeight& w, const uint8_t* raw, uint
 void launch_embed(cudaStream_t st, const DevWeight& w, const uint32_t* tokens, const DecodeCtl* ctl, float* out, int n);
 
 // Optional residual add (hidden += add), RMSNorm (cpu.rs:577-594) and Q8_0 quantisation
-// (simd.rs:255-323) of n rows.  normed_out (f32) is optional.
+// (simd.rs:255-323) of n rows.  normed_out (f32) is optional.  The launch of longer rows than this is refused.
+constexpr int ADD_RMSNORM_MAX_DIM = 16384;
 void launch_add_rmsnorm_quant(cudaStream_t st, float* hidden, const float* add, const float* weight, float eps,
                               int n, int dim, float* q8s, int8_t* q8q, float* normed_out, const MmaInput& x = MmaInput());
 // In-place RMSNorm of n rows (operator entry point).

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(1024) k_add_rmsnorm_quant(float* __restrict__ 
 void launch_add_rmsnorm_quant(cudaStream_t st, float* hidden, const float* add, const float* weight, float eps, int n,
                               int dim, float* q8s, int8_t* q8q, float* normed_out, const MmaInput& x) {
     g_kernel_launches++;
-    // (rows beyond 16384 elements: more threads than a CTA can have, which the launch refuses)
+    // (rows beyond ADD_RMSNORM_MAX_DIM: more threads than a CTA can have, which the launch refuses)
     const int quads = dim / 4, least = (quads + 1023) / 1024, per = least <= 2 ? std::max(least, 1) : 4;
     const int threads = ((quads + per - 1) / per + 31) / 32 * 32;
     auto kernel = per == 1 ? k_add_rmsnorm_quant<1> : per == 2 ? k_add_rmsnorm_quant<2> : k_add_rmsnorm_quant<4>;

@@ -662,9 +662,15 @@ int32_t capture_graph(wick_cuda_model* m, bool greedy, cudaGraphExec_t* out, uin
     cudaGraph_t graph = nullptr;
     CU_TRY(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
     const unsigned long long before = g_kernel_launches;
+    const bool clean = cudaPeekAtLastError() == cudaSuccess;  // (an error that an earlier call left behind is not this one's)
     enqueue_decode(m, greedy);
     *nodes = g_kernel_launches - before;
+    const cudaError_t refused = clean ? cudaGetLastError() : cudaSuccess;  // (a refused launch leaves a graph without that kernel, not an invalid capture)
     cudaError_t e = cudaStreamEndCapture(m->stream, &graph);
+    if (e == cudaSuccess && refused != cudaSuccess) {
+        cudaGraphDestroy(graph);
+        e = refused;
+    }
     if (e != cudaSuccess) return fail(WICK_CUDA_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(out, graph, 0);
     cudaGraphDestroy(graph);
@@ -977,6 +983,8 @@ int32_t build_model(wick_cuda_model* m, const GgufImage& g, uint32_t context_siz
     m->head_dim = hs / c.n_heads;
     const int hd = m->head_dim;
     if (hs % QK || is % QK) return fail(WICK_CUDA_ERR_BAD_GGUF, "hidden and feed-forward sizes must be multiples of 32");
+    if (hs > ADD_RMSNORM_MAX_DIM)
+        return fail(WICK_CUDA_ERR_BAD_GGUF, "hidden size " + std::to_string(hs) + ": rows of more than " + std::to_string(ADD_RMSNORM_MAX_DIM) + " elements are not supported");
     if (hd % 8 || hd > 256) return fail(WICK_CUDA_ERR_BAD_GGUF, "head_dim must be a multiple of 8 and <= 256");
     if (c.conv_kernel_size < 1 || c.conv_kernel_size > 8) return fail(WICK_CUDA_ERR_BAD_GGUF, "unsupported shortconv.l_cache");
     if (naive_attn_smem(m) > 200 * 1024)
