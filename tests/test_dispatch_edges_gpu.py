@@ -29,7 +29,7 @@ def assert_bits(got, want, what):
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("scales", ["smallest", "largest", "mixed"])
 def test_exact_gemm_keeps_every_f16_scale(ops, orc, dtype, scales):
-    """The epilogue works on scaled-down chains: f16 scales from the smallest subnormal to the largest value must not show."""
+    """f16 scales from the smallest subnormal to the largest value, and zero, in weights and activations."""
     rng = np.random.default_rng(3)
     m, k, n = 130, 384, 19
     bb = 18 if dtype == "q4_0" else 34
@@ -45,7 +45,7 @@ def test_exact_gemm_keeps_every_f16_scale(ops, orc, dtype, scales):
 
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("where", ["weights", "activations", "both"])
-@pytest.mark.parametrize("m,k,n", [(130, 384, 19), (6144, 128, 90), (6144, 128, 130)])  # 8-token tiles; two waves of 16-token tiles; three
+@pytest.mark.parametrize("m,k,n", [(130, 384, 19), (6144, 128, 90), (6144, 128, 130)])  # tiles of 16 x 8; two rounds of 64 x 32; six of 64 x 16
 def test_exact_gemm_with_infinite_scales(ops, orc, dtype, where, m, k, n):
     """Scales beyond f16 (a block of activations above 8.3 million; an infinity or NaN in a file): the reference's infinities and
     NaNs, not NaN throughout.  Only the sign and payload of a NaN are free."""
@@ -97,7 +97,7 @@ def test_model_with_infinite_weight_scales(cuda_lib, orc, model_dir, tmp_path):
         assert_bits(np.where(np.isnan(got), F32(0), got), np.where(np.isnan(want), F32(0), want), f"step {step}")
 
 
-@pytest.mark.parametrize("m,k,n", [(130, 384, 19), (6144, 128, 90), (6144, 128, 130)])  # 8-token tiles; two waves of 16-token tiles; three
+@pytest.mark.parametrize("m,k,n", [(130, 384, 19), (6144, 128, 90), (6144, 128, 130)])  # tiles of 16 x 8; two rounds of 64 x 32; six of 64 x 16
 def test_operator_gemm_with_scales_that_are_not_f16(ops, orc, m, k, n):
     """A caller's own quantiser need not round its scales to f16: tiny, subnormal and huge ones, alone and beside ordinary ones."""
     from wick_b200 import gguf_synth as gs

@@ -20,8 +20,8 @@ def dev(a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
 
 
-# Row tiles of 16 in groups of 1, 2, 4 and 6, token tiles of 8, 16 and 32; stages of 256 elements, the last one half there (k = 128,
-# 384); more tiles than SMs, with fewer stages to a tile than producer groups.
+# On 148 SMs the rule takes tiles of 16 x 8, 64 x 8, 64 x 16 and 96 x 32 for these, one round and several; stages of 256 elements, the last
+# one half there (k = 128, 384).  Every shape, and more tiles than SMs with fewer stages to a tile than producer groups: test_every_tile_shape.
 @pytest.mark.parametrize("dtype", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("m,k,n", [(1, 128, 1), (16, 256, 8), (17, 384, 9), (95, 640, 16), (97, 1024, 33), (2400, 128, 7), (4808, 128, 65),
                                    (1000, 384, 24), (9600, 256, 31), (96 * 160, 128, 40), (2048, 1152, 200), (520, 2304, 97)])

@@ -1,4 +1,4 @@
-"""Calls that need no int8 weight copy still work where there is no memory for one: the copy is a matter of speed."""
+"""Calls that can do without a weight copy still work where there is no memory for one: the copy is a matter of speed."""
 import numpy as np
 import pytest
 

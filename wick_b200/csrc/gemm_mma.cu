@@ -9,11 +9,12 @@
 // other lane groups.  What is left is packed f32x2 arithmetic, two tokens per instruction: per 16 x 8 outputs and block 4 mma,
 // 8 products, 8 additions and 2 scale products.
 //
-// Bound: the registers' read ports, which the two pipes share.  An mma with a zero C takes 4.5 cycles of a scheduler, a packed
-// operation 2 to 2.4, and they add up: 54 cycles per (16 x 8, block) with every operand in shared memory, a ceiling of 170
-// TFLOP/s; the whole kernel reaches 134 (6144 x 2048 at 512 tokens 96 us) with activations that arrive as operands and 127
-// (101 us, 6912 x 2048 at 2002 416) where it converts them: there four warps have 5 % of the issue slots, and in small
-// tiles a chain of their own.
+// Bound: the MMAs and the packed arithmetic one after the other.  In loops of their own an mma with a zero C takes 4.5 cycles of a
+// scheduler, a packed operation 2 to 2.4, and both together the sum (they share something, the registers' read ports by
+// guess): 54 cycles per (16 x 8, block) with every operand in shared memory, a ceiling of 170 TFLOP/s.  The whole kernel
+// reaches 134 (6144 x 2048 at 512 tokens 96 us; by ncu FMA pipe 60 %, MMAs 27, issue 54, 3.2 warps per scheduler: the rest
+// is latency) with activations that arrive as operands and 127 (101 us; 6912 x 2048 at 2002 433) where it converts
+// them: there four warps have 5 % of the issue slots, and in small tiles a chain of their own.
 // tcgen05 was here before (int8, lane groups as zero-padded columns, sums handed over through tensor memory): 115 and 463 us
 // for those, 17 us for 1024 x 4608 at 9 tokens (now 7) and 23 for 2048 x 6912 at 16 (9.8): a hand-over per stage bound it, a round of
 // release, issue, MMAs and wait that small tiles cannot hide at all, and that no order of loads or number of units shortened
@@ -651,7 +652,8 @@ cudaError_t launch_gemm_mma(cudaStream_t st, const MmaWeight* const* w, float* c
     };
     static constexpr Shape READY_SHAPES[MMA_SHAPES] = {{6, 4, 1, 156, 156}, {6, 2, 1, 78, 78}, {4, 3, 1, 80, 80}, {4, 2, 1, 53, 54},
                                                      {4, 1, 1, 38, 42},   {2, 1, 2, 36, 38}, {1, 1, 2, 27, 28}};
-    // (with the converting warps: two lane-group warps bring nothing, 1024 x 4608 at 9 tokens 8.4 against 8.1 us)
+    // (with the converting warps: two lane-group warps bring nothing, 1024 x 4608 at 9 tokens 8.4 against 8.1 us.  32 x 8 and 16 x 16 are
+    // for narrow matrices with many columns: 96 x 6912 at 600 16.8 us as 32 x 8, without the two 22.6; 16 x 2048 at 2400 8.7 and 10.2)
     static constexpr Shape CONVERT_SHAPES[MMA_SHAPES] = {{6, 4, 1, 176, 176}, {4, 4, 1, 120, 120}, {4, 2, 1, 67, 67}, {4, 1, 1, 41, 41},
                                                        {2, 1, 2, 42, 46},   {1, 2, 2, 46, 51},   {1, 1, 2, 32, 40}};
     const Shape* shapes = x ? READY_SHAPES : CONVERT_SHAPES;
