@@ -226,7 +226,7 @@ int32_t wick_cuda_gemv_q8(const wick_cuda_weight* w, const float* xs_dev, const 
  * columns; the result is token-major out[j*m + i] (the reference writes out[i*n + j]).  bq must be 4-byte aligned; bs may hold
  * any f32.  With more than 8 columns and k % 128 == 0 it runs on the tensor cores, with the same bits: the weight's first such
  * call makes a copy of it in operand order (1.125 bytes per parameter, kept until the weight is destroyed) and waits for that;
- * repeated products are then 4 times as fast as on the CUDA cores, the first one 1.9 times.  Without memory for the copy, and
+ * repeated products are then 4 times as fast as on the CUDA cores, the first one 1.6 to 1.9 times.  Without memory for the copy, and
  * while `stream` is captured before the copy exists (nor that of wick_cuda_gemm_q8_tc), it runs on the CUDA cores.  A weight created
  * with WICK_CUDA_PREFILL=exact-cuda-cores in the environment always does, and never makes the copy. */
 int32_t wick_cuda_gemm_q8(const wick_cuda_weight* w, const float* bs_dev, const int8_t* bq_dev,
