@@ -13,8 +13,8 @@
 // One MMA instruction covers exactly one quantisation block (K = 32 int8), writes a fresh 128 x BN
 // int32 tile into one of 512/BN tensor-memory buffers and never accumulates across blocks, because
 // each block has its own scale pair.  The epilogue warps drain a stage's four buffers (tcgen05.ld), hand them back,
-// and apply the scales on the CUDA cores, which is what bounds the kernel: per (output, block) a conversion and half of
-// two packed instructions.
+// and apply the scales on the CUDA cores, where the kernel's time goes: per (output, block) a conversion and half of
+// two packed instructions.  No unit is full (6144 x 2048 at 512 tokens: issue slots 51 %, ALU 41, FMA 36, tensor 8).
 //
 // Roles in a CTA (one CTA per SM, persistent over output tiles; 12 warps):
 //   warp 0  lane 0: TMA producer, one K=128 stage (4 blocks) of W rows and activation rows per step
